@@ -250,12 +250,13 @@ static int sm_count()
  * the work queue until it runs dry. */
 /* Warps per CTA for an exact launch: the choice among 4, 2, 1 that keeps
  * the most warps resident per SM (shared memory per warp grows with the ROI
- * side). */
-static int pick_wpb_exact(int side_max, int opt_model, int *per_sm_out)
+ * side).  A batch of few ROIs, no more than the GPU has schedulers, takes one
+ * chain per CTA: the chains are then spread over all SMs. */
+static int pick_wpb_exact(int side_max, bool few, int opt_model, int *per_sm_out)
 {
     int best_w = 0, best_wpb = 4, best_per = 0;
     const int cand[3] = {4, 2, 1};
-    for (int i = 0; i < 3; ++i) {
+    for (int i = few ? 2 : 0; i < 3; ++i) {
         int per = blocks_per_sm_exact(side_max, cand[i], opt_model);
         if (per * cand[i] > best_w) {
             best_w = per * cand[i];
@@ -295,11 +296,15 @@ static bamf_status launch_batch(bamf_workspace *ws, const SamplerConsts &K, Samp
             Bc.side_max = std::min(class_side(c), B.side_max);
         }
         int per_sm = 0, wpb = 0, mc = 2;
-        if (exact) wpb = pick_wpb_exact(Bc.side_max, K.opt_model, &per_sm);
+        /* Few ROIs in exact arithmetic, no more than two per SM: a team of warps
+         * on each chain, one CTA per chain (two such CTAs fill an SM's
+         * schedulers twice; beyond, a warp per chain keeps more chains going). */
+        const bool team = exact && K.opt_model == 0 && B.n_rois <= 2 * sms;
+        if (exact) wpb = pick_wpb_exact(Bc.side_max, B.n_rois <= 4 * sms, K.opt_model, &per_sm);
         else per_sm = best_fast_shape(Bc.side_max, K.opt_model, &wpb, &mc);
         if (per_sm < 1) return BAMF_ERR_TOO_LARGE;
         const int tw = ws->tuned_wpb[exact ? 0 : 1][c], tm = exact ? 0 : ws->tuned_min_ctas[c];
-        if (tw > 0) {
+        if (tw > 0 && !team) {
             int pt = exact ? blocks_per_sm_exact(Bc.side_max, tw, K.opt_model)
                            : blocks_per_sm_fast(Bc.side_max, tw, tm, K.opt_model);
             if (pt > 0) {
@@ -316,8 +321,9 @@ static bamf_status launch_batch(bamf_workspace *ws, const SamplerConsts &K, Samp
             cs = ws->cls_stream[c];
             CU(cudaStreamWaitEvent(cs, ws->fork_ev, 0));
         }
-        cudaError_t e = exact ? launch_rjmcmc_exact(Kl, Bc, Bc.side_max, blocks, wpb, cs)
-                              : launch_rjmcmc_fast(Kl, Bc, Bc.side_max, blocks, wpb, mc, cs);
+        cudaError_t e = team    ? launch_rjmcmc_exact_team(Kl, Bc, Bc.side_max, blocks, cs)
+                        : exact ? launch_rjmcmc_exact(Kl, Bc, Bc.side_max, blocks, wpb, cs)
+                                : launch_rjmcmc_fast(Kl, Bc, Bc.side_max, blocks, wpb, mc, cs);
         if (e != cudaSuccess) return cuda_fail(e, "rjmcmc kernel launch");
         if (fork) {
             CU(cudaEventRecord(ws->join_ev[c], cs));

@@ -6,7 +6,7 @@
 #include <cuda_runtime.h>
 
 #include "bamf.h"
-#include "bamf_parity_math.h"
+#include "parity_quick.cuh"
 
 /* a failed CUDA runtime call: clear its error so that a later call on this
  * thread does not report it again */
@@ -85,15 +85,15 @@ extern "C" bamf_status bamf_probe_peaks(double *fp32_flops, double *mufu_ops)
     return err == cudaSuccess ? BAMF_OK : BAMF_ERR_CUDA;
 }
 
-/* The parity math of the exact sampler (include/bamf_parity_math.h) on the
- * device: out[i] = f(x[i]) for f = erf (0), log (1), exp (2); a host caller
- * compares with the same header compiled for the CPU. */
+/* The parity math of the exact sampler (parity_quick.cuh) on the device:
+ * out[i] = f(x[i]) for f = erf (0), log (1), exp (2); a host caller compares
+ * with include/bamf_parity_math.h compiled for the CPU. */
 __global__ void parity_math_kernel(const float *__restrict__ x, int n, int fn, float *__restrict__ out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float v = x[i];
-    out[i] = fn == 0 ? bamf_pm_erff(v) : (fn == 1 ? bamf_pm_logf(v) : bamf_pm_expf(v));
+    out[i] = fn == 0 ? bamf::pq::erf_q(v) : (fn == 1 ? bamf::pq::log_q(v) : bamf::pq::exp_q(v));
 }
 
 extern "C" bamf_status bamf_parity_math_device(int fn, const float *x, int n, float *out)

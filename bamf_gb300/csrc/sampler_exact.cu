@@ -15,6 +15,16 @@ cudaError_t launch_exact_gauss(const SamplerConsts &K, const SamplerBatch &B, si
     return launch_kernel(rjmcmc_kernel<true, false>, K, B, smem, blocks, threads, stream);
 }
 
+/* few chains: EXACT_TEAM warps on each, one chain per CTA */
+constexpr int EXACT_TEAM = 4;
+
+cudaError_t launch_rjmcmc_exact_team(const SamplerConsts &K, const SamplerBatch &B, int side_max, int blocks,
+                                     cudaStream_t stream)
+{
+    return launch_kernel(rjmcmc_kernel_team<EXACT_TEAM>, K, B, (size_t)warp_smem_floats(side_max, true) * sizeof(float),
+                         blocks, 32 * EXACT_TEAM, stream);
+}
+
 int occupancy_exact_gauss(size_t smem, int threads) { return resident_ctas(rjmcmc_kernel<true, false>, smem, threads); }
 
 cudaError_t launch_rjmcmc_exact(const SamplerConsts &K, const SamplerBatch &B, int side_max, int blocks,

@@ -34,6 +34,7 @@
 
 #include "bamf.h"
 #include "bamf_parity_math.h"
+#include "parity_quick.cuh"
 #include "bamf_philox.h"
 #include "sampler_common.h"
 
@@ -57,9 +58,9 @@ struct SMath;
 
 template <>
 struct SMath<true> {
-    static __device__ __forceinline__ float erf_(float x) { return bamf_pm_erff(x); }
-    static __device__ __forceinline__ float log_(float x) { return bamf_pm_logf(x); }
-    static __device__ __forceinline__ float exp_(float x) { return bamf_pm_expf(x); }
+    static __device__ __forceinline__ float erf_(float x) { return pq::erf_q(x); }
+    static __device__ __forceinline__ float log_(float x) { return pq::log_q(x); }
+    static __device__ __forceinline__ float exp_(float x) { return pq::exp_q(x); }
     static __device__ __forceinline__ float powf_(float x, float y) { return bamf_pm_powf(x, y); }
 };
 
@@ -72,7 +73,9 @@ struct SMath<false> {
 };
 
 /* Per-warp shared-memory carve-out, in floats.  Exact: data D, model M,
- * proposal model Mt, per-pixel work E, sCMOS, proposal stencils NX/NY.
+ * proposal model Mt, per-pixel work E, sCMOS (each rounded up to 16 bytes,
+ * for the vector loads of the serial sums), a pool of 2 x 32 stencil rows
+ * NX/NY shared by A and T, 128 buffered uniforms.
  * Fast: D, M, Mt and the compact stencil rows SXo/SYo (old, of A) and
  * SXn/SYn (new, of T); log2 M is recomputed in each likelihood pass (the
  * SFU has room; the smaller carve-out keeps 3 CTAs of 8 chains resident
@@ -83,10 +86,13 @@ struct SMath<false> {
  * (rare: a jump of a cluster of more than 4 emitters) and periodic rebuilds
  * stream the model one emitter at a time. */
 #define FAST_ROWS 4
+#define EXACT_ROWS (2 * BAMF_NMAX) /* stencil rows of the exact sampler's pool */
+#define EXACT_UBUF 128
+__host__ __device__ inline int exact_npix(int side_max) { return (side_max * side_max + 3) & ~3; }
 __host__ __device__ inline int warp_smem_floats(int side_max, bool exact)
 {
     int npix = side_max * side_max, nxs = BAMF_NMAX * side_max;
-    return exact ? 5 * npix + 4 * nxs + C_COUNT + BAMF_NMAX + 2 /* D M Mt E sCMOS, NX NY of A and of T */
+    return exact ? 5 * exact_npix(side_max) + 4 * nxs + EXACT_UBUF + C_COUNT + BAMF_NMAX + 2
                  : 3 * npix + 4 * FAST_ROWS * side_max + C_COUNT + BAMF_NMAX + 2; /* D M Mt SXo SYo SXn SYn */
 }
 
@@ -274,7 +280,19 @@ static __device__ __noinline__ float normpdf_f(float x, float u, float s)
     return 1.0f / (sq2pi * s) * SMath<EXACT>::exp_(-d * d / (2.0f * s * s));
 }
 
-template <bool EXACT, bool NUM>
+/* Exact mode, a chain run by a team of TEAM warps: what its first warp asks
+ * the others to do with their share of the pixels (TeamCmd::ASK_*), and the
+ * state they need for it. */
+struct TeamCmd {
+    enum { ASK_END, ASK_MODEL, ASK_SCORE };
+    int ask, X, Y, n;
+    float BG, ABG, BBG;
+    const float *D, *M, *NX, *NY, *scm;
+    float *E, *out, *sink;
+    int row[BAMF_NMAX];
+};
+
+template <bool EXACT, bool NUM, int TEAM = 1>
 struct ChainWarp {
     typedef SMath<EXACT> MT;
     const SamplerConsts *K;
@@ -283,12 +301,17 @@ struct ChainWarp {
     int roi;
     /* geometry */
     int X, Y, npix;
-    int px_dx, px_dy; /* pixel p -> p+32 moves x by px_dx and y by px_dy (then wraps) */
+    static constexpr int STEP = 32 * TEAM; /* pixels of a pass */
+    int px_dx, px_dy; /* pixel p -> p + STEP moves x by px_dx and y by px_dy (then wraps) */
+    TeamCmd *cmd;     /* TEAM > 1: shared memory */
     float sigma, Cst, MeanN;
     /* shared memory */
     float *D, *M, *Mt, *E, *NX, *NY;
-    float *NXt, *NYt; /* exact mode: stencil rows of T (NX, NY hold A's) */
-    int tsrc;         /* exact mode: the A slot T's emitter in this lane came from, -1 if changed */
+    /* exact mode: row r of the pool is NX[r X ..], NY[r Y ..]; arow / trow is
+     * the row of this lane's emitter of A / of T (an emitter T left unchanged
+     * keeps A's row; -1: changed or new, not evaluated yet) */
+    int arow, trow;
+    float *ubuf; /* exact mode: uniforms base * 4 .. base * 4 + 127 */
     float *SXo, *SYo, *SXn, *SYn; /* fast mode: compact stencil rows */
     const float *scm; /* sCMOS: shared memory (exact) or global/null (fast) */
     /* sampled PSF (OptModel 1): [P0 y][P1 x][P2 y-sub][P3 x-sub], y fastest;
@@ -309,8 +332,9 @@ struct ChainWarp {
     float tBG, tABG, tBBG;
     bool t_overflow;
     /* uniform stream */
-    uint32_t seed, chain, idx, base;
-    uint32_t r0, r1, r2, r3;
+    uint32_t seed, chain, base;
+    uint32_t idx;            /* exact mode: next uniform of ubuf, else of the stream */
+    uint32_t r0, r1, r2, r3; /* fast mode: this lane's block of the buffer */
     /* phase */
     int is_burnin;
     float P[8];
@@ -320,7 +344,7 @@ struct ChainWarp {
     /* incremental-model bookkeeping (fast mode) */
     uint32_t a_dirty, t_dirty;
     int llr_box; /* pixels the last likelihood pass changed: x0 | x1 << 8 | y0 << 16 | y1 << 24 */
-    float pdf_aBG; /* fast mode: offset-prior density of aBG */
+    float pdf_aBG; /* offset-prior density of aBG */
     /* move-synchronous mode: the jump sub-branch uniform comes from the CTA */
     bool use_shared_ub;
     float shared_ub;
@@ -328,11 +352,29 @@ struct ChainWarp {
     /* ---------------------------------------------------------- RNG */
     __device__ __forceinline__ void refill()
     {
+        if (EXACT) {
+            /* block numbers wrap where a 32-bit stream index wraps */
+            const uint4 b = philox_block((base + (uint32_t)lane) & 0x3fffffffu, seed, chain);
+            __syncwarp();
+            reinterpret_cast<float4 *>(ubuf)[lane] =
+                make_float4(bamf_u31_to_float(b.x >> 1), bamf_u31_to_float(b.y >> 1), bamf_u31_to_float(b.z >> 1),
+                            bamf_u31_to_float(b.w >> 1));
+            __syncwarp();
+            return;
+        }
         uint4 b = philox_block(base + (uint32_t)lane, seed, chain);
         r0 = b.x; r1 = b.y; r2 = b.z; r3 = b.w;
     }
     __device__ __forceinline__ float urand()
     {
+        if (EXACT) {
+            if (idx >= (uint32_t)EXACT_UBUF) {
+                base += EXACT_UBUF / 4;
+                idx = 0u;
+                refill();
+            }
+            return ubuf[idx++];
+        }
         uint32_t blk = idx >> 2;
         if (blk - base >= 32u) {
             base = blk;
@@ -352,7 +394,15 @@ struct ChainWarp {
     {
         if (EXACT) {
             float t = 0;
-            for (int k = 0; k < 12; ++k) t = t + urand();
+            if (idx + 12u <= (uint32_t)EXACT_UBUF) { /* all twelve buffered: loads in flight together */
+                const float *u = ubuf + idx;
+#pragma unroll
+                for (int k = 0; k < 12; ++k) t = t + u[k];
+                idx += 12u;
+            } else {
+#pragma unroll 1
+                for (int k = 0; k < 12; ++k) t = t + urand();
+            }
             return t - 6.0f;
         }
         if (((idx + 11u) >> 2) - base >= 32u) {
@@ -362,6 +412,27 @@ struct ChainWarp {
         float u = irwin_hall12(idx, base, r0, r1, r2, r3, lane);
         idx += 12u;
         return u;
+    }
+
+    /* Three consecutive randn().  Exact mode:
+     * lane k adds the k-th draw's twelve uniforms, in draw order. */
+    __device__ __forceinline__ void randn3(float &a, float &b, float &c)
+    {
+        if (EXACT && idx + 36u <= (uint32_t)EXACT_UBUF) {
+            const float *u = ubuf + idx + 12 * min(lane, 2);
+            float t = 0;
+#pragma unroll
+            for (int k = 0; k < 12; ++k) t = t + u[k];
+            t = t - 6.0f;
+            idx += 36u;
+            a = __shfl_sync(BAMF_FULL, t, 0);
+            b = __shfl_sync(BAMF_FULL, t, 1);
+            c = __shfl_sync(BAMF_FULL, t, 2);
+        } else {
+            a = randn();
+            b = randn();
+            c = randn();
+        }
     }
 
     /* ------------------------------------------------------ lane access */
@@ -378,7 +449,7 @@ struct ChainWarp {
             tI = I;
             tX = x;
             tY = y;
-            if (EXACT) tsrc = -1;
+            if (EXACT) trow = -1;
         }
         if (!EXACT) t_dirty |= 1u << k;
     }
@@ -393,7 +464,7 @@ struct ChainWarp {
             tX = x;
             tY = y;
             tS = s;
-            if (EXACT) tsrc = -1;
+            if (EXACT) trow = -1;
         }
         if (!EXACT) t_dirty |= 1u << tn;
         tn++;
@@ -405,10 +476,10 @@ struct ChainWarp {
         float vX = __shfl_down_sync(BAMF_FULL, tX, 1);
         float vY = __shfl_down_sync(BAMF_FULL, tY, 1);
         int vS = __shfl_down_sync(BAMF_FULL, tS, 1);
-        int vsrc = EXACT ? __shfl_down_sync(BAMF_FULL, tsrc, 1) : 0;
+        int vrow = EXACT ? __shfl_down_sync(BAMF_FULL, trow, 1) : 0;
         if (lane >= id) {
             tI = vI; tX = vX; tY = vY; tS = vS;
-            if (EXACT) tsrc = vsrc;
+            if (EXACT) trow = vrow;
         }
         if (!EXACT) {
             uint32_t lo = t_dirty & ((1u << id) - 1u);
@@ -422,7 +493,7 @@ struct ChainWarp {
         tn = an; tI = aI; tX = aX; tY = aY; tS = aS;
         tBG = aBG; tABG = aABG; tBBG = aBBG;
         t_overflow = false;
-        if (EXACT) tsrc = lane;
+        if (EXACT) trow = arow;
         if (!EXACT) {
             a_dirty = 0u;
             t_dirty = 0u;
@@ -455,6 +526,18 @@ struct ChainWarp {
         if (EXACT) return stat_pdf(s.x, s.pdf, s.L, I);
         return stat_pdf_fast(s.x, s.pdf, s.L, s.inv_dx, I);
     }
+    /* findPDF of two intensities at once: one in each half of the warp */
+    __device__ __forceinline__ void findPDF2(const DevStat &s, float I0, float I1, float &p0, float &p1) const
+    {
+        if (EXACT) {
+            const float v = stat_pdf(s.x, s.pdf, s.L, lane < 16 ? I0 : I1);
+            p0 = __shfl_sync(BAMF_FULL, v, 0);
+            p1 = __shfl_sync(BAMF_FULL, v, 16);
+        } else {
+            p0 = findPDF(s, I0);
+            p1 = findPDF(s, I1);
+        }
+    }
     __device__ __forceinline__ float genRand(const DevStat &s)
     {
         float R = urand();
@@ -478,12 +561,19 @@ struct ChainWarp {
         bool in = false;
         if (lane < an && lane != jj) {
             float dx = aX - xj, dy = aY - yj;
-            float d;
-            if (EXACT)
-                d = (float)sqrt(dadd(dmul((double)dx, (double)dx), dmul((double)dy, (double)dy)));
-            else
-                d = sqrtf(dx * dx + dy * dy);
-            in = d < dmin;
+            if (EXACT) {
+                /* the reference compares (float)sqrt of the double sum; where
+                 * the float sum of squares (three roundings, 1.8e-7) is more
+                 * than 1e-6 from dmin^2 the answer is the same, and only the
+                 * rest, NaN included, pays for FP64 */
+                const float s = dx * dx + dy * dy, q = dmin * dmin;
+                in = q > 1e-30f && s < q * 0.999999f;
+                if (!in && !(q > 1e-30f && s > q * 1.000001f))
+                    in = (float)sqrt(dadd(dmul((double)dx, (double)dx), dmul((double)dy, (double)dy))) < dmin;
+            } else {
+                const float d = sqrtf(dx * dx + dy * dy);
+                in = d < dmin;
+            }
         }
         return __ballot_sync(BAMF_FULL, in);
     }
@@ -532,39 +622,68 @@ struct ChainWarp {
     }
 
     /* ------------------------------------------------------------ model */
-    /* Stencil + Model (:15-59) of a lane-distributed state, into out[]. */
-    __device__ __forceinline__ void model_full(int n, float I, float Xv, float Yv, float BG, float ABG, float BBG,
-                               float *out, float *nx, float *ny)
+    /* Exact mode, Stencil (:15-37): rows of the pool for the emitters in
+     * `todo` (lane k's emitter for bit k) of the state (I, Xv, Yv, row); `keep`
+     * is the row of this lane that must survive, or -1.  Unchanged emitters
+     * keep their rows: the same function of the same inputs, so the same
+     * bits.  One emitter's X + Y entries go over the lanes together; the kept
+     * rows are at most BAMF_NMAX of A's, so BAMF_NMAX are free. */
+    __device__ __forceinline__ void exact_rows(uint32_t todo, int keep, float I, float Xv, float Yv, int &row)
     {
-        int totx = n * X, toty = n * Y;
+        if (todo == 0u) return;
+        uint32_t f0 = ~__reduce_or_sync(BAMF_FULL, keep >= 0 && keep < 32 ? 1u << keep : 0u);
+        uint32_t f1 = ~__reduce_or_sync(BAMF_FULL, keep >= 32 ? 1u << (keep - 32) : 0u);
+        const int XY = X + Y;
 #pragma unroll 1
-        for (int b0 = 0; b0 < totx; b0 += 32) {
-            int item = b0 + lane;
-            int k = min(item / X, n - 1);
-            int x = item - k * X;
-            float Ik = __shfl_sync(BAMF_FULL, I, k);
-            float Xk = __shfl_sync(BAMF_FULL, Xv, k);
-            if (item < totx)
-                nx[k * X + x] = Ik * 0.5f * (MT::erf_(((float)x - Xk + 1.0f) * Cst) -
-                                             MT::erf_(((float)x - Xk) * Cst));
-        }
+        for (; todo; todo &= todo - 1u) {
+            const int k = __ffs(todo) - 1;
+            int r;
+            if (f0) {
+                r = __ffs(f0) - 1;
+                f0 &= f0 - 1u;
+            } else {
+                r = 31 + __ffs(f1);
+                f1 &= f1 - 1u;
+            }
+            if (lane == k) row = r;
+            const float Ik = __shfl_sync(BAMF_FULL, I, k), Xk = __shfl_sync(BAMF_FULL, Xv, k);
+            const float Yk = __shfl_sync(BAMF_FULL, Yv, k);
 #pragma unroll 1
-        for (int b0 = 0; b0 < toty; b0 += 32) {
-            int item = b0 + lane;
-            int k = min(item / Y, n - 1);
-            int y = item - k * Y;
-            float Yk = __shfl_sync(BAMF_FULL, Yv, k);
-            if (item < toty)
-                ny[k * Y + y] = 0.5f * (MT::erf_(((float)y - Yk + 1.0f) * Cst) -
-                                        MT::erf_(((float)y - Yk) * Cst));
+            for (int c = lane; c < XY; c += 32) {
+                const bool isx = c < X;
+                const int cc = isx ? c : c - X;
+                const float mu = isx ? Xk : Yk;
+                const float x1 = ((float)cc - mu + 1.0f) * Cst, x0 = ((float)cc - mu) * Cst;
+                float e1 = pq::erf_try(x1), e0 = pq::erf_try(x0); /* both in flight */
+                if (e1 != e1) e1 = pq::erf_rest(x1);
+                if (e0 != e0) e0 = pq::erf_rest(x0);
+                if (isx) NX[r * X + cc] = Ik * 0.5f * (e1 - e0);
+                else NY[r * Y + cc] = 0.5f * (e1 - e0);
+            }
         }
         __syncwarp();
-        int x = lane / Y, y = lane - (lane / Y) * Y;
-#pragma unroll 1
-        for (int p = lane; p < npix; p += 32) {
-            float m = BG + ABG * (float)x + BBG * (float)y + (scm ? scm[p] : 0.0f);
-            for (int k = 0; k < n; ++k) m += nx[k * X + x] * ny[k * Y + y];
-            out[p] = m;
+    }
+    /* Exact mode, Model (:39-59) of pixels p + STEP j, j < J: the background
+     * plane and sCMOS, then the emitters in slot order, into out; SCORE: the
+     * likelihood-ratio term of each pixel into E.  J independent pixels per
+     * lane keep the row loads and the logarithms in flight (one at a time: 7.2k
+     * cycles per 16x16 proposal, four: 5.4k, eight: 5.0k, but with 16 chains on
+     * an SM, where instruction fetch binds, 24k, 32k and 35k); lanes past the
+     * last pixel store to `sink`, so there is no branch.  (x, y) is this
+     * lane's pixel p, moved on to p + STEP J. */
+    template <int J, bool SCORE>
+    __device__ __forceinline__ void exact_pixels(int p, int &x, int &y, int n, int row, float BG, float ABG, float BBG,
+                                                 float *out, float *sink)
+    {
+        int xs[J], ys[J];
+        float m[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int q = p + STEP * j;
+            const bool in = q < npix;
+            xs[j] = in ? x : 0;
+            ys[j] = in ? y : 0;
+            m[j] = BG + ABG * (float)xs[j] + BBG * (float)ys[j] + scm[in ? q : 0];
             x += px_dx;
             y += px_dy;
             if (y >= Y) {
@@ -572,55 +691,175 @@ struct ChainWarp {
                 x++;
             }
         }
-        __syncwarp();
+#pragma unroll 1
+        for (int k = 0; k < n; ++k) {
+            const int r = __shfl_sync(BAMF_FULL, row, k);
+            const float *nx = NX + r * X, *ny = NY + r * Y;
+#pragma unroll
+            for (int j = 0; j < J; ++j) m[j] += nx[xs[j]] * ny[ys[j]];
+        }
+        uint32_t open = 0u; /* pixels whose quotient or logarithm the quick forms leave open */
+        if (SCORE) {
+            /* all loads before the first store (which may alias them) */
+            float ma[J], d[J], lg[J];
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const int q = p + STEP * j < npix ? p + STEP * j : 0;
+                ma[j] = M[q];
+                d[j] = D[q];
+            }
+#pragma unroll
+            for (int j = 0; j < J; ++j) lg[j] = pq::log_try(pq::div_try(m[j], ma[j]));
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const bool in = p + STEP * j < npix;
+                *(in ? E + p + STEP * j : sink) = ma[j] - m[j] + d[j] * lg[j];
+                if (in && lg[j] != lg[j]) open |= 1u << j;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < J; ++j) *(p + STEP * j < npix ? out + p + STEP * j : sink) = m[j];
+        if (SCORE) {
+#pragma unroll 1
+            for (; open; open &= open - 1u) {
+                const int q = p + STEP * (__ffs(open) - 1);
+                const float mt = out[q];
+                E[q] = M[q] - mt + D[q] * pq::log_slow(mt / M[q]);
+            }
+        }
     }
-
-    /* Exact mode, the proposal's model: as model_full for T, but the
-     * stencil rows of the emitters the proposal left unchanged are copied
-     * from A's rows (the same function of the same inputs, so the same
-     * bits) instead of evaluated again; only changed or new emitters pay
-     * the erf evaluations.  Rows go to NXt / NYt. */
-    __device__ __forceinline__ void model_cached(int n, float I, float Xv, float Yv, float BG, float ABG, float BBG,
-                                                 float *out)
+    /* This warp's share (warp `part` of TEAM) of the model of a state. */
+    template <bool SCORE>
+    __device__ __forceinline__ void exact_share(int part, int n, int row, float BG, float ABG, float BBG, float *out,
+                                                float *sink)
     {
-        int totx = n * X, toty = n * Y;
+        int p = 32 * part + lane, x = p / Y, y = p - x * Y;
+        if (TEAM == 1) {
 #pragma unroll 1
-        for (int b0 = 0; b0 < totx; b0 += 32) {
-            int item = b0 + lane;
-            int k = min(item / X, n - 1);
-            int x = item - k * X;
-            float Ik = __shfl_sync(BAMF_FULL, I, k);
-            float Xk = __shfl_sync(BAMF_FULL, Xv, k);
-            int src = __shfl_sync(BAMF_FULL, tsrc, k);
-            if (item < totx)
-                NXt[k * X + x] = src >= 0 ? NX[src * X + x]
-                                          : Ik * 0.5f * (MT::erf_(((float)x - Xk + 1.0f) * Cst) -
-                                                         MT::erf_(((float)x - Xk) * Cst));
+            for (; p - lane + 64 < npix; p += 4 * STEP) exact_pixels<4, SCORE>(p, x, y, n, row, BG, ABG, BBG, out, sink);
         }
 #pragma unroll 1
-        for (int b0 = 0; b0 < toty; b0 += 32) {
-            int item = b0 + lane;
-            int k = min(item / Y, n - 1);
-            int y = item - k * Y;
-            float Yk = __shfl_sync(BAMF_FULL, Yv, k);
-            int src = __shfl_sync(BAMF_FULL, tsrc, k);
-            if (item < toty)
-                NYt[k * Y + y] = src >= 0 ? NY[src * Y + y]
-                                          : 0.5f * (MT::erf_(((float)y - Yk + 1.0f) * Cst) -
-                                                    MT::erf_(((float)y - Yk) * Cst));
+        for (; p - lane < npix; p += 2 * STEP) exact_pixels<2, SCORE>(p, x, y, n, row, BG, ABG, BBG, out, sink);
+    }
+    /* the team's barrier (CTA barrier 1, all its warps); a CTA is one team */
+    static __device__ __forceinline__ void team_sync()
+    {
+        asm volatile("barrier.sync 1, %0;" ::"n"(STEP) : "memory");
+    }
+    template <bool SCORE>
+    __device__ __forceinline__ void exact_model(int n, int row, float BG, float ABG, float BBG, float *out)
+    {
+        float *sink = (float *)(cl + BAMF_NMAX);
+        if (TEAM > 1) {
+            cmd->row[lane] = row;
+            if (lane == 0) {
+                cmd->ask = SCORE ? TeamCmd::ASK_SCORE : TeamCmd::ASK_MODEL;
+                cmd->X = X;
+                cmd->Y = Y;
+                cmd->n = n;
+                cmd->BG = BG;
+                cmd->ABG = ABG;
+                cmd->BBG = BBG;
+                cmd->D = D;
+                cmd->M = M;
+                cmd->NX = NX;
+                cmd->NY = NY;
+                cmd->scm = scm;
+                cmd->E = E;
+                cmd->out = out;
+                cmd->sink = sink;
+            }
+            team_sync();
+        }
+        exact_share<SCORE>(0, n, row, BG, ABG, BBG, out, sink);
+        if (TEAM > 1) team_sync();
+        else __syncwarp();
+    }
+    /* warps 1 .. TEAM - 1 of a team: serve until its first warp ends */
+    __device__ __forceinline__ void team_serve(int part)
+    {
+        for (;;) {
+            team_sync();
+            const int ask = cmd->ask;
+            if (ask == TeamCmd::ASK_END) return;
+            X = cmd->X;
+            Y = cmd->Y;
+            npix = X * Y;
+            px_dx = STEP / Y;
+            px_dy = STEP - px_dx * Y;
+            D = const_cast<float *>(cmd->D);
+            M = const_cast<float *>(cmd->M);
+            NX = const_cast<float *>(cmd->NX);
+            NY = const_cast<float *>(cmd->NY);
+            scm = cmd->scm;
+            E = cmd->E;
+            if (ask == TeamCmd::ASK_SCORE)
+                exact_share<true>(part, cmd->n, cmd->row[lane], cmd->BG, cmd->ABG, cmd->BBG, cmd->out, cmd->sink);
+            else
+                exact_share<false>(part, cmd->n, cmd->row[lane], cmd->BG, cmd->ABG, cmd->BBG, cmd->out, cmd->sink);
+            team_sync();
+        }
+    }
+    /* Exact mode: the sum of E in pixel order, on every lane.  The additions
+     * are one dependent chain; 16-byte loads one step ahead keep it at the
+     * adder's latency. */
+    __device__ __forceinline__ float exact_sum() const
+    {
+        const float4 *E4 = reinterpret_cast<const float4 *>(E);
+        const int nq = npix >> 2;
+        float t = 0.0f;
+        int q = 0;
+        float4 v[4];
+        if (nq >= 4) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = E4[j];
+        }
+#pragma unroll 1
+        for (; q + 4 <= nq; q += 4) {
+            float4 w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w[j] = E4[min(q + 4 + j, nq - 1)];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) t = t + v[j].x + v[j].y + v[j].z + v[j].w;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = w[j];
+        }
+#pragma unroll 1
+        for (int p = 4 * q; p < npix; ++p) t += E[p];
+        return t;
+    }
+    /* Exact mode: E becomes its running sum, in place (every lane adds the
+     * same chain, lane 0 stores). */
+    __device__ __forceinline__ void exact_scan()
+    {
+        float4 *E4 = reinterpret_cast<float4 *>(E);
+        const int nq = npix >> 2;
+        float t = 0.0f;
+        int q = 0;
+#pragma unroll 1
+        for (; q + 8 <= nq; q += 8) {
+            float4 v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = E4[q + j];
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                t = q + j == 0 ? v[j].x : v[j].x + t;
+                v[j].x = t;
+                v[j].y = t = v[j].y + t;
+                v[j].z = t = v[j].z + t;
+                v[j].w = t = v[j].w + t;
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) E4[q + j] = v[j];
+            }
         }
         __syncwarp();
-        int x = lane / Y, y = lane - (lane / Y) * Y;
+        if (lane == 0) {
 #pragma unroll 1
-        for (int p = lane; p < npix; p += 32) {
-            float m = BG + ABG * (float)x + BBG * (float)y + (scm ? scm[p] : 0.0f);
-            for (int k = 0; k < n; ++k) m += NXt[k * X + x] * NYt[k * Y + y];
-            out[p] = m;
-            x += px_dx;
-            y += px_dy;
-            if (y >= Y) {
-                y -= Y;
-                x++;
+            for (int p = 4 * q; p < npix; ++p) {
+                if (p > 0) E[p] += E[p - 1];
             }
         }
         __syncwarp();
@@ -858,16 +1097,16 @@ struct ChainWarp {
     {
         n_llr++;
         if (EXACT) {
-            if constexpr (NUM) model_num(tn, tI, tX, tY, tBG, tABG, tBBG, Mt);
-            else model_cached(tn, tI, tX, tY, tBG, tABG, tBBG, Mt);
-            for (int p = lane; p < npix; p += 32)
-                E[p] = M[p] - Mt[p] + D[p] * MT::log_(Mt[p] / M[p]);
-            __syncwarp();
-            float tmp = 0.0f;
-            if (lane == 0)
-                for (int p = 0; p < npix; ++p) tmp += E[p];
-            tmp = __shfl_sync(BAMF_FULL, tmp, 0);
-            return MT::exp_(tmp);
+            if constexpr (NUM) {
+                model_num(tn, tI, tX, tY, tBG, tABG, tBBG, Mt);
+                for (int p = lane; p < npix; p += 32)
+                    E[p] = M[p] - Mt[p] + D[p] * MT::log_(Mt[p] / M[p]);
+                __syncwarp();
+            } else {
+                exact_rows(__ballot_sync(BAMF_FULL, lane < tn && trow < 0), lane < an ? arow : -1, tI, tX, tY, trow);
+                exact_model<true>(tn, trow, tBG, tABG, tBBG, Mt);
+            }
+            return MT::exp_(exact_sum());
         } else {
             /* Mt = M + background delta - old stencils of A's changed slots
              *        + new stencils of T's changed slots;
@@ -985,18 +1224,15 @@ struct ChainWarp {
 
     __device__ __forceinline__ void accept_T()
     {
-        if (!EXACT) {
-            commit_fast();
-            if (tBG != aBG) pdf_aBG = findPDF(K->off, tBG);
-        }
+        if (!EXACT) commit_fast();
+        if (tBG != aBG) pdf_aBG = findPDF(K->off, tBG);
         an = tn; aI = tI; aX = tX; aY = tY; aS = tS;
         aBG = tBG; aABG = tABG; aBBG = tBBG;
         if (EXACT) {
             float *t = M;
             M = Mt;
             Mt = t;
-            t = NX; NX = NXt; NXt = t;
-            t = NY; NY = NYt; NYt = t;
+            arow = trow;
         }
     }
 
@@ -1005,7 +1241,10 @@ struct ChainWarp {
     {
         if (EXACT) {
             if constexpr (NUM) model_num(an, aI, aX, aY, aBG, aABG, aBBG, M);
-            else model_full(an, aI, aX, aY, aBG, aABG, aBBG, M, NX, NY);
+            else {
+                exact_rows(__ballot_sync(BAMF_FULL, lane < an), -1, aI, aX, aY, arow);
+                exact_model<false>(an, arow, aBG, aABG, aBBG, M);
+            }
         } else {
             /* with a drift output, a periodic rebuild goes to Mt (free
              * between proposals) first, to measure how far the incrementally
@@ -1037,24 +1276,26 @@ struct ChainWarp {
         bamf_chain *ch = &B->chains[2 * roi + w];
         int e = entries;
         if (e >= ch->capacity_entries) return;
-        if (lane == 0) {
-            ch->N[e] = n; ch->LLR[e] = LLR; ch->PR[e] = PR; ch->JumpType[e] = type;
-            ch->Accepted[e] = acc; ch->BG[e] = BG; ch->ABG[e] = ABG; ch->BBG[e] = BBG;
+        /* the entry's eight fields are consecutive pointers of bamf_chain: lane
+         * k loads the k-th and stores the k-th value */
+        if (lane < 8) {
+            uint32_t v = lane == 0 ? (uint32_t)n : lane == 1 ? __float_as_uint(LLR) : __float_as_uint(PR);
+            v = lane == 3 ? (uint32_t)type : lane == 4 ? (uint32_t)acc : v;
+            v = lane == 5 ? __float_as_uint(BG) : lane == 6 ? __float_as_uint(ABG) : lane == 7 ? __float_as_uint(BBG) : v;
+            reinterpret_cast<uint32_t *const *>(&ch->N)[lane][e] = v;
         }
         int rc = rec_n[w];
         int nrec = n < 1 ? 1 : n;
         if (rc + nrec <= ch->capacity_records) {
-            if (n < 1) {
-                if (lane == 0) {
-                    ch->Index[rc] = e + 1; ch->Photons[rc] = 0.0f; ch->X[rc] = -100.0f;
-                    ch->Y[rc] = -100.0f; ch->Signal[rc] = -1;
-                }
-            } else if (lane < n) {
-                ch->Index[rc + lane] = e + 1;
-                ch->Photons[rc + lane] = I;
-                ch->X[rc + lane] = x + K->p.DriftX;
-                ch->Y[rc + lane] = y + K->p.DriftY;
-                ch->Signal[rc + lane] = s;
+            /* all pointers before the first store (which may alias them) */
+            int32_t *pi = ch->Index + rc + lane, *ps = ch->Signal + rc + lane;
+            float *pp = ch->Photons + rc + lane, *px = ch->X + rc + lane, *py = ch->Y + rc + lane;
+            if (lane < nrec) {
+                *pi = e + 1;
+                *pp = n < 1 ? 0.0f : I;
+                *px = n < 1 ? -100.0f : x + K->p.DriftX;
+                *py = n < 1 ? -100.0f : y + K->p.DriftY;
+                *ps = n < 1 ? -1 : s;
             }
         }
         rec_n[w] = rc + nrec;
@@ -1117,6 +1358,18 @@ struct ChainWarp {
         entries++;
     }
 
+    /* floor(g + 0.5) as the reference forms it, in double.  Below 2^22 the
+     * fraction g - floor(g) is exact in float, or rounds within [1/2, 1] (g in
+     * (-1/2, 0)), so its comparison with 1/2 gives the same integer. */
+    static __device__ __forceinline__ int kround(float g)
+    {
+        if (fabsf(g) < 4194304.0f) {
+            const float f = floorf(g);
+            return (int)f + (g - f >= 0.5f ? 1 : 0);
+        }
+        return (int)floor(dadd((double)g, 0.5));
+    }
+
     /* RJMCMC::update_grids (:1629-1648). */
     __device__ __forceinline__ void update_grids()
     {
@@ -1126,8 +1379,8 @@ struct ChainWarp {
             /* the float sum with 0.5 is exact for |coordinate| < 2^22: fast
              * mode rounds as the reference's double sum does */
             const float gx = (float)Z * (aX + K->p.DriftX), gy = (float)Z * (aY + K->p.DriftY);
-            int x = EXACT ? (int)floor(dadd((double)gx, 0.5)) : (int)floorf(gx + 0.5f);
-            int y = EXACT ? (int)floor(dadd((double)gy, 0.5)) : (int)floorf(gy + 0.5f);
+            int x = EXACT ? kround(gx) : (int)floorf(gx + 0.5f);
+            int y = EXACT ? kround(gy) : (int)floorf(gy + 0.5f);
             float *gb = aS == 1 ? B->pgrid : B->pback;
             if (gb && x >= 0 && x < X * Z && y >= 0 && y < Y * Z && aI > K->p.Icutoff) {
                 /* grid slot (ROIs sharing one accumulate) and column stride */
@@ -1166,9 +1419,11 @@ struct ChainWarp {
         const bamf_mcmc_params &p = K->p;
         if (Ub < 0.25f) {
             type = 2;
-            tBG = tBG + p.BG_std * randn();
-            tABG = tABG + p.ABBG_std * randn();
-            tBBG = tBBG + p.ABBG_std * randn();
+            float g0, g1, g2;
+            randn3(g0, g1, g2);
+            tBG = tBG + p.BG_std * g0;
+            tABG = tABG + p.ABBG_std * g1;
+            tBBG = tBBG + p.ABBG_std * g2;
         } else if (Ub < 0.50f && Ub >= 0.25f) {
             if (an < 2) return ACT_SKIP;
             type = 10;
@@ -1183,17 +1438,19 @@ struct ChainWarp {
                 int aSc = A_S(c);
                 float nX, nY, nI;
                 if (aSc == 1) {
-                    nX = aXc + p.X_stdFg * randn();
-                    nY = aYc + p.X_stdFg * randn();
-                    nI = (I0 / (float)(Np + 1)) * (0.15f * randn() + 1.0f);
-                    IPDFtest = findPDF(K->sig, nI);
-                    IPDF = findPDF(K->sig, aIc);
+                    float g0, g1, g2;
+                    randn3(g0, g1, g2);
+                    nX = aXc + p.X_stdFg * g0;
+                    nY = aYc + p.X_stdFg * g1;
+                    nI = (I0 / (float)(Np + 1)) * (0.15f * g2 + 1.0f);
+                    findPDF2(K->sig, nI, aIc, IPDFtest, IPDF);
                 } else {
-                    nX = aXc + p.X_stdBg * randn();
-                    nY = aYc + p.X_stdBg * randn();
-                    nI = (I0 / (float)(Np + 1)) * (0.15f * randn() + 1.0f);
-                    IPDFtest = findPDF(K->back, nI);
-                    IPDF = findPDF(K->back, aIc);
+                    float g0, g1, g2;
+                    randn3(g0, g1, g2);
+                    nX = aXc + p.X_stdBg * g0;
+                    nY = aYc + p.X_stdBg * g1;
+                    nI = (I0 / (float)(Np + 1)) * (0.15f * g2 + 1.0f);
+                    findPDF2(K->back, nI, aIc, IPDFtest, IPDF);
                 }
                 PrI = PrI * IPDFtest / IPDF;
                 setT(c, nI, nX, nY);
@@ -1229,18 +1486,20 @@ struct ChainWarp {
                 float nI, nX, nY;
                 if (aSc == 1) {
                     cinc(C_N_jumpFg);
-                    nI = cI + p.I_stdFg * randn();
-                    nX = cX + p.X_stdFg * randn();
-                    nY = cY + p.X_stdFg * randn();
-                    IPDFtest = findPDF(K->sig, nI);
-                    IPDF = findPDF(K->sig, aIc);
+                    float g0, g1, g2;
+                    randn3(g0, g1, g2);
+                    nI = cI + p.I_stdFg * g0;
+                    nX = cX + p.X_stdFg * g1;
+                    nY = cY + p.X_stdFg * g2;
+                    findPDF2(K->sig, nI, aIc, IPDFtest, IPDF);
                 } else {
                     cinc(C_N_jumpBg);
-                    nI = cI + p.I_stdBg * randn();
-                    nX = cX + p.X_stdBg * randn();
-                    nY = cY + p.X_stdBg * randn();
-                    IPDFtest = findPDF(K->back, nI);
-                    IPDF = findPDF(K->back, aIc);
+                    float g0, g1, g2;
+                    randn3(g0, g1, g2);
+                    nI = cI + p.I_stdBg * g0;
+                    nX = cX + p.X_stdBg * g1;
+                    nY = cY + p.X_stdBg * g2;
+                    findPDF2(K->back, nI, aIc, IPDFtest, IPDF);
                 }
                 PrI = PrI * IPDFtest / IPDF;
                 setT(c, nI, nX, nY);
@@ -1270,18 +1529,20 @@ struct ChainWarp {
             }
             if (aSn == 1) {
                 cinc(C_N_jumpFg);
-                nI = aIn + p.I_stdFg * randn();
-                nX = aXn + p.X_stdFg * randn();
-                nY = aYn + p.X_stdFg * randn();
-                IPDFtest = findPDF(K->sig, nI);
-                IPDF = findPDF(K->sig, aIn);
+                float g0, g1, g2;
+                randn3(g0, g1, g2);
+                nI = aIn + p.I_stdFg * g0;
+                nX = aXn + p.X_stdFg * g1;
+                nY = aYn + p.X_stdFg * g2;
+                findPDF2(K->sig, nI, aIn, IPDFtest, IPDF);
             } else {
                 cinc(C_N_jumpBg);
-                nI = aIn + p.I_stdBg * randn();
-                nX = aXn + p.X_stdBg * randn();
-                nY = aYn + p.X_stdBg * randn();
-                IPDFtest = findPDF(K->back, nI);
-                IPDF = findPDF(K->back, aIn);
+                float g0, g1, g2;
+                randn3(g0, g1, g2);
+                nI = aIn + p.I_stdBg * g0;
+                nX = aXn + p.X_stdBg * g1;
+                nY = aYn + p.X_stdBg * g2;
+                findPDF2(K->back, nI, aIn, IPDFtest, IPDF);
             }
             PrI = IPDFtest / IPDF;
             setT(nn, nI, nX, nY);
@@ -1305,10 +1566,13 @@ struct ChainWarp {
             if (tABG != aABG) PrBg *= MT::exp_(-(tABG * tABG - aABG * aABG) / 2.0f);
             return LLR * pk_f0 * PrBg;
         }
-        float BgPDF = findPDF(K->off, aBG);
-        float BgPDFtest = findPDF(K->off, tBG);
-        float PrBg = (BgPDFtest / BgPDF) * MT::exp_(-(tBBG * tBBG - aBBG * aBBG) / 2.0f) *
-                     MT::exp_(-(tABG * tABG - aABG * aABG) / 2.0f);
+        float BgPDF = pdf_aBG;
+        float BgPDFtest = tBG == aBG ? pdf_aBG : findPDF(K->off, tBG);
+        /* unchanged slopes: exp(-0) = 1, and the product with 1 is exact */
+        float PrBg = BgPDFtest / BgPDF;
+        const float db = -(tBBG * tBBG - aBBG * aBBG) / 2.0f, da = -(tABG * tABG - aABG * aABG) / 2.0f;
+        if (db != 0.0f) PrBg = PrBg * MT::exp_(db);
+        if (da != 0.0f) PrBg = PrBg * MT::exp_(da);
         return LLR * pk_f0 * PrBg;
     }
 
@@ -1583,9 +1847,7 @@ struct ChainWarp {
                 E[p] = (0.0f > v) ? 0.0f : v;
             }
             __syncwarp();
-            if (lane == 0)
-                for (int p = 1; p < npix; ++p) E[p] += E[p - 1];
-            __syncwarp();
+            exact_scan();
             total = E[npix - 1];
         } else {
             /* Fast: the residual's running sum is never stored.  Lane j sums
@@ -1993,8 +2255,8 @@ struct ChainWarp {
 /* Loads ROI `roi` into a warp's carve-out and sets up its chain (the
  * set-up of cRJMCMC.cpp:103-148).  Returns false, with the ROI's status set,
  * when the ROI does not fit the launch. */
-template <bool EXACT, bool NUM>
-__device__ __forceinline__ bool begin_roi(ChainWarp<EXACT, NUM> &w, const SamplerConsts *Kp, const SamplerBatch &Bt,
+template <bool EXACT, bool NUM, int TEAM>
+__device__ __forceinline__ bool begin_roi(ChainWarp<EXACT, NUM, TEAM> &w, const SamplerConsts *Kp, const SamplerBatch &Bt,
                                           float *sw, int roi)
 {
     const int lane = w.lane;
@@ -2003,10 +2265,9 @@ __device__ __forceinline__ bool begin_roi(ChainWarp<EXACT, NUM> &w, const Sample
     w.X = X;
     w.Y = Y;
     w.npix = X * Y;
-    w.px_dx = 32 / Y;
-    w.px_dy = 32 - (32 / Y) * Y;
-    int npix_max = Bt.side_max * Bt.side_max;
-    int nxs = BAMF_NMAX * Bt.side_max;
+    w.px_dx = w.STEP / Y;
+    w.px_dy = w.STEP - (w.STEP / Y) * Y;
+    int npix_max = EXACT ? exact_npix(Bt.side_max) : Bt.side_max * Bt.side_max;
     w.D = sw;
     w.M = sw + npix_max;
     w.Mt = sw + 2 * npix_max;
@@ -2015,15 +2276,15 @@ __device__ __forceinline__ bool begin_roi(ChainWarp<EXACT, NUM> &w, const Sample
         w.E = sw + 3 * npix_max;
         scm_smem = sw + 4 * npix_max;
         w.NX = sw + 5 * npix_max;
-        w.NY = w.NX + nxs;
-        w.NXt = w.NY + nxs;
-        w.NYt = w.NXt + nxs;
+        w.NY = w.NX + EXACT_ROWS * Bt.side_max;
+        w.ubuf = w.NY + EXACT_ROWS * Bt.side_max;
         w.SXo = w.SYo = w.SXn = w.SYn = nullptr;
-        w.cnt = (int *)(w.NYt + nxs);
+        w.cnt = (int *)(w.ubuf + EXACT_UBUF);
+        w.arow = w.trow = -1;
     } else {
         const int rs = FAST_ROWS * Bt.side_max;
         w.E = nullptr;
-        w.NX = w.NY = w.NXt = w.NYt = nullptr;
+        w.NX = w.NY = w.ubuf = nullptr;
         w.SXo = sw + 3 * npix_max;
         w.SYo = w.SXo + rs;
         w.SXn = w.SYo + rs;
@@ -2082,13 +2343,14 @@ __device__ __forceinline__ bool begin_roi(ChainWarp<EXACT, NUM> &w, const Sample
     }
     w.aBG = Bt.init_bg ? Bt.init_bg[roi] : Kp->bg0;
     if (w.aBG == 0.0f) w.aBG = 1.0f;
-    if (!EXACT) w.pdf_aBG = w.findPDF(Kp->off, w.aBG);
+    w.pdf_aBG = w.findPDF(Kp->off, w.aBG);
     w.aABG = 0.0f;
     w.aBBG = 0.0f;
     w.seed = Kp->seed;
     w.chain = Bt.chain_ids ? Bt.chain_ids[roi] : (uint32_t)roi;
     w.idx = Bt.rng_offset ? Bt.rng_offset[roi] : 0u;
     w.base = w.idx >> 2;
+    if (EXACT) w.idx &= 3u;
     w.refill();
     w.entries = 0;
     w.overflow = 0;
@@ -2104,8 +2366,8 @@ __device__ __forceinline__ bool begin_roi(ChainWarp<EXACT, NUM> &w, const Sample
 }
 
 /* Writes the chain's per-ROI results. */
-template <bool EXACT, bool NUM>
-__device__ __forceinline__ void end_roi(ChainWarp<EXACT, NUM> &w, const SamplerBatch &Bt)
+template <bool EXACT, bool NUM, int TEAM>
+__device__ __forceinline__ void end_roi(ChainWarp<EXACT, NUM, TEAM> &w, const SamplerBatch &Bt)
 {
     const int lane = w.lane, roi = w.roi;
     if (Bt.final_n && lane == 0) Bt.final_n[roi] = w.an;
@@ -2130,7 +2392,8 @@ __device__ __forceinline__ void end_roi(ChainWarp<EXACT, NUM> &w, const SamplerB
     }
     if (lane == 0) {
         if (Bt.n_entries) Bt.n_entries[roi] = w.entries;
-        if (Bt.uniforms_used) Bt.uniforms_used[roi] = w.idx - (Bt.rng_offset ? Bt.rng_offset[roi] : 0u);
+        if (Bt.uniforms_used)
+            Bt.uniforms_used[roi] = (EXACT ? 4u * w.base : 0u) + w.idx - (Bt.rng_offset ? Bt.rng_offset[roi] : 0u);
         if (Bt.overflow) Bt.overflow[roi] = w.overflow;
         if (Bt.llr_evals) Bt.llr_evals[roi] = w.n_llr;
         if (Bt.status) Bt.status[roi] = BAMF_OK;
@@ -2144,7 +2407,7 @@ template <bool EXACT, bool NUM>
 __global__ void __launch_bounds__(128, 4) rjmcmc_kernel(const __grid_constant__ SamplerConsts Kc,
                                                      const __grid_constant__ SamplerBatch Bc)
 {
-    extern __shared__ float smem_raw[];
+    extern __shared__ __align__(16) float smem_raw[];
     const SamplerBatch &Bt = Bc;
     int warp = threadIdx.x >> 5;
     int lane = threadIdx.x & 31;
@@ -2170,6 +2433,50 @@ __global__ void __launch_bounds__(128, 4) rjmcmc_kernel(const __grid_constant__ 
     }
 }
 
+/* Exact sampler for few ROIs: a CTA of TEAM warps runs one chain at a time.
+ * The first warp runs the chain; the others take their share of every
+ * proposal's pixels (the model and the likelihood-ratio terms, 40% of a
+ * chain's time on one warp).  The terms are then added by the first warp in
+ * pixel order, so the chain is the same.  A chain is latency-bound (about
+ * 2,700 dependent warp instructions per jump, a fifth of the issue slots of
+ * its scheduler).  16x16, 3000+3000 jumps, 200 ROIs: 47.0 ms with a warp per
+ * chain, 38.1 ms with teams of four; one ROI: 32.4 and 28.6 ms. */
+template <int TEAM>
+__global__ void __launch_bounds__(32 * TEAM, 2) rjmcmc_kernel_team(const __grid_constant__ SamplerConsts Kc,
+                                                                const __grid_constant__ SamplerBatch Bc)
+{
+    extern __shared__ __align__(16) float smem_raw[];
+    __shared__ TeamCmd cmd;
+    const SamplerBatch &Bt = Bc;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    ChainWarp<true, false, TEAM> w;
+    w.K = &Kc;
+    w.B = &Bc;
+    w.lane = lane;
+    w.cmd = &cmd;
+    if (warp > 0) {
+        w.team_serve(warp);
+        return;
+    }
+    int q_begin = 0, q_end = Bt.n_rois;
+    if (Bt.class_range) {
+        q_begin = Bt.class_range[2 * Bt.cls];
+        q_end = Bt.class_range[2 * Bt.cls + 1];
+    }
+    for (;;) {
+        int slot = 0;
+        if (lane == 0) slot = q_begin + atomicAdd(Bt.queue, 1);
+        slot = __shfl_sync(BAMF_FULL, slot, 0);
+        if (slot >= q_end) break;
+        int roi = Bt.order ? Bt.order[slot] : slot;
+        if (!begin_roi(w, &Kc, Bt, smem_raw, roi)) continue;
+        w.run_chain();
+        end_roi(w, Bt);
+    }
+    if (lane == 0) cmd.ask = TeamCmd::ASK_END;
+    w.team_sync();
+}
+
 /* Move-synchronous persistent sampler (fast arithmetic): the CTA pulls one
  * ROI per warp at a time and its warps run their chains in lockstep, one
  * barrier per jump, with the move type and jump sub-branch shared across the
@@ -2178,7 +2485,7 @@ template <bool NUM, int MIN_CTAS>
 __global__ void __launch_bounds__(MIN_CTAS == 1 ? 32 * BAMF_SYNC_GROUP : 256, MIN_CTAS) rjmcmc_kernel_sync(const __grid_constant__ SamplerConsts Kc,
                                                           const __grid_constant__ SamplerBatch Bc)
 {
-    extern __shared__ float smem_raw[];
+    extern __shared__ __align__(16) float smem_raw[];
     __shared__ int grp_base;
     const SamplerBatch &Bt = Bc;
     const int nwarps = blockDim.x >> 5;

@@ -20,6 +20,9 @@ cudaError_t launch_rjmcmc_fast(const SamplerConsts &K, const SamplerBatch &B, in
 int blocks_per_sm_fast(int side_max, int warps_per_block, int min_ctas, int opt_model);
 cudaError_t launch_rjmcmc_exact(const SamplerConsts &K, const SamplerBatch &B, int side_max, int blocks,
                                 int warps_per_block, cudaStream_t stream);
+/* a team of warps on each chain (Gaussian PSF only): for batches of few ROIs */
+cudaError_t launch_rjmcmc_exact_team(const SamplerConsts &K, const SamplerBatch &B, int side_max, int blocks,
+                                     cudaStream_t stream);
 int blocks_per_sm_exact(int side_max, int warps_per_block, int opt_model);
 
 /* the CTA shape with the most resident chains per SM for a fast launch
