@@ -681,13 +681,17 @@ __global__ void __launch_bounds__(1024) dw_reduce_kernel(const float *__restrict
 }
 
 /* ----------------------------------------------------------------- heads */
-/* Training: one CTA (256 threads, thread = pixel) per ROI: loss, head
+/* One CTA (256 threads, thread = pixel) per ROI.  TRAIN: loss, head
  * gradients (row r of `hrows`, HEAD_NPARAM floats per ROI), dz4 = dL/d(pre-
- * activation of conv4). */
+ * activation of conv4).  INFER: the sampler's birth tables and the count
+ * logits. */
+template <bool TRAIN>
 __global__ void __launch_bounds__(256) head_kernel(const bf16 *__restrict__ a4, int n, const float *__restrict__ P,
                                                    const int32_t *__restrict__ n_em, const float *__restrict__ xyi,
                                                    float inv_batch, float *__restrict__ hrows, bf16 *__restrict__ dz4,
-                                                   float *__restrict__ loss_buf, const int *__restrict__ step_dev)
+                                                   float *__restrict__ loss_buf, const int *__restrict__ step_dev,
+                                                   float *__restrict__ cdf, float *__restrict__ sub,
+                                                   float *__restrict__ cnt_out)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float *H = (float *)smem_raw;             /* [256][HS] */
@@ -773,7 +777,26 @@ __global__ void __launch_bounds__(256) head_kernel(const bf16 *__restrict__ a4, 
     }
     __syncthreads();
     const float inv_sum = 1.0f / sm_sum;
-    /* ---- targets, loss, gradients */
+    if (!TRAIN) {
+        /* pixel probability, inclusive scan over pixels (thread order = p) */
+        float pp = se * inv_sum;
+        float incl = pp;
+        for (int o = 1; o < 32; o <<= 1) {
+            float v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        __syncthreads();
+        if (lane == 31) red[warp] = incl;
+        __syncthreads();
+        float base = 0.0f;
+        for (int k = 0; k < warp; ++k) base += red[k];
+        cdf[(size_t)r * NPX + t] = base + incl;
+        float inv_se = 1.0f / se;
+        for (int s = 0; s < NSUB; ++s) sub[((size_t)r * NPX + t) * NSUB + s] = e[s] * inv_se;
+        if (cnt_out && t < NC) cnt_out[(size_t)r * NC + t] = zc[t];
+        return;
+    }
+    /* ---- training: targets, loss, gradients */
     const int ntrue = n_em[r];
     if (t < BAMF_SYNTH_NMAX) {
         ex[t] = xyi[((size_t)r * BAMF_SYNTH_NMAX + t) * 3 + 0];
@@ -895,281 +918,6 @@ __global__ void __launch_bounds__(256) head_kernel(const bf16 *__restrict__ a4, 
     }
     for (int o = t; o < NC * CH; o += 256) row_wc(hrows, r)[o] = dzc[o / CH] * gmean[o - (o / CH) * CH];
     if (t < NC) row_wc(hrows, r)[NC * CH + t] = dzc[t];
-}
-
-/* ------------------------------------------------------ fused inference */
-/* The whole network on a ROI in one CTA: its activations never leave shared
- * memory.  A persistent CTA of 256 threads (two per SM) keeps the three
- * layers' packed weights resident and takes one ROI per iteration: conv1 (FP32,
- * thread = pixel), three 32 -> 32 convolutions on tcgen05, the heads, and the
- * birth tables written out.
- *
- * One activation buffer, [ci group g][padded x 0..17][padded y 0..17][8 ci]
- * BF16 with zero borders, serves every tap without shifted copies: M tile
- * `mt` is the ROI's half y in [8 mt, 8 mt + 8), its row m the pixel x = m / 8,
- * y = 8 mt + m mod 8, so a core matrix is 8 consecutive y of one x (128
- * contiguous bytes), the next one is one padded column away (SBO = 288), and
- * tap (kx, ky) starts (18 kx + ky) 16-byte rows in.  The epilogue of a layer
- * (bias, ReLU, BF16) writes the next layer's input over it once the layer's
- * MMAs completed.  The sums over channels and taps run in conv_tc_kernel's
- * order, and the heads in head_kernel's, so the tables are the same bits as
- * from the layer-by-layer kernels that training uses.
- *
- * Bound: shared-memory traffic of the 108 MMAs (each reads a 4 KB A tile for
- * 32 columns) and the FP32 heads' issue; packed f32x2 FMAs (two exact FP32
- * results per instruction) halve the latter.  MEASURED_INFER */
-constexpr int IB_G = PS * PS * 16;                 /* bytes of one ci group of the buffer */
-constexpr int IB_BYTES = 4 * IB_G;
-constexpr int INF_W1 = 3 * PKT * 2 + IB_BYTES;     /* byte offsets behind the weights and the buffer */
-constexpr int INF_WL = INF_W1 + 9 * CH * 4;        /* conv1 weights [tap][co] */
-constexpr int INF_BIAS = INF_WL + CH * NSUB * 4;   /* head weights [c][s] */
-constexpr int INF_XP = INF_BIAS + 4 * CH * 4;      /* biases of conv1 .. conv4 */
-constexpr int INF_MBAR = INF_XP + PS * PS * 4;     /* padded conv1 input */
-constexpr size_t SMEM_INFER = INF_MBAR + 16;
-static_assert(INF_W1 % 16 == 0 && INF_XP % 16 == 0 && INF_MBAR % 8 == 0, "shared-memory alignment");
-
-/* two FP32 fused multiply-adds, each rounded as fmaf rounds it */
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
-{
-    float2 d;
-    asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
-        "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
-
-/* 32 bytes of one thread in one store: a whole L2 sector */
-__device__ __forceinline__ void store8(float *p, const float *v)
-{
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
-                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-                 : "memory");
-}
-
-template <bool WIDE>
-__global__ void __launch_bounds__(256, 2) infer_kernel(const float *__restrict__ data, int n, const float *__restrict__ P,
-                                                       const bf16 *__restrict__ Wt, float *__restrict__ cdf,
-                                                       float *__restrict__ sub, float *__restrict__ cnt_out,
-                                                       int *__restrict__ status)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    unsigned char *Ws = smem_raw, *buf = smem_raw + 3 * PKT * 2;
-    float *w1 = (float *)(smem_raw + INF_W1), *wl = (float *)(smem_raw + INF_WL);
-    float *bias = (float *)(smem_raw + INF_BIAS), *xp = (float *)(smem_raw + INF_XP);
-    uint64_t *mbar = (uint64_t *)(smem_raw + INF_MBAR);
-    __shared__ uint32_t tslot;
-    __shared__ __align__(16) float bl[NSUB];
-    __shared__ float Wc[NC * CH], bc[NC];
-    __shared__ float red[8], red2[8], red3[8], gmean[CH], part[8][CH];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    if (warp == 0) bamf::tc::tmem_alloc(&tslot, 64);
-    {
-        const uint4 *src = (const uint4 *)Wt;
-        uint4 *dst = (uint4 *)Ws;
-        for (int i = t; i < 3 * PKT * 2 / 16; i += 256) dst[i] = src[i];
-        const uint4 z = make_uint4(0, 0, 0, 0);
-        for (int i = t; i < IB_BYTES / 16; i += 256) ((uint4 *)buf)[i] = z;
-        for (int i = t; i < 9 * CH; i += 256) w1[i] = P[O_W1 + (i % CH) * 9 + i / CH];
-        for (int i = t; i < CH * NSUB; i += 256) wl[i] = P[O_WL + (i % NSUB) * CH + i / NSUB];
-        for (int i = t; i < 4 * CH; i += 256) {
-            const int l = i / CH;
-            bias[i] = P[(l == 0 ? O_B1 : l == 1 ? O_B2 : l == 2 ? O_B3 : O_B4) + i % CH];
-        }
-        for (int i = t; i < PS * PS; i += 256) xp[i] = 0.0f;
-        for (int i = t; i < NC * CH; i += 256) Wc[i] = P[O_WC + i];
-        if (t < NSUB) bl[t] = P[O_BL + t];
-        if (t < NC) bc[t] = P[O_BC + t];
-    }
-    if (t == 0) bamf::tc::mbar_init(mbar, 1);
-    bamf::tc::fence_before_sync();
-    __syncthreads();
-    bamf::tc::fence_after_sync();
-    const uint32_t tbase = tslot;
-    const uint32_t ws_addr = bamf::tc::smem_addr(Ws), buf_addr = bamf::tc::smem_addr(buf);
-    /* this thread's pixel t in conv1 and the heads, and the pixel of its TMEM
-     * lane in the convolutions' epilogues, as 16-byte rows of a ci group */
-    const int own = ((t >> 4) + 1) * PS + (t & 15) + 1;
-    const int mt = warp >> 2, m = 32 * (warp & 3) + lane;
-    const int epi = ((m >> 3) + 1) * PS + 8 * mt + (m & 7) + 1;
-    uint32_t phase = 0;
-    bool alive = true;
-    float next = blockIdx.x < n ? data[(size_t)blockIdx.x * NPX + t] : 0.0f;
-    for (int r = blockIdx.x; r < n && alive; r += gridDim.x) {
-        /* conv1: normalisation and the 1 -> 32 convolution, as conv1_fwd_kernel */
-        const float v = sqrtf(fmaxf(next, 0.0f) + 0.375f);
-        if (r + (int)gridDim.x < n) next = data[(size_t)(r + gridDim.x) * NPX + t];
-        float s = v;
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) red[warp] = s;
-        __syncthreads();
-        float mean = 0.0f;
-        for (int k = 0; k < 8; ++k) mean += red[k];
-        mean *= (1.0f / NPX);
-        xp[own] = (v - mean) * 0.25f;
-        __syncthreads();
-        {
-            float in[9];
-#pragma unroll
-            for (int k = 0; k < 9; ++k) in[k] = xp[own + (k / 3 - 1) * PS + k % 3 - 1];
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                float2 z[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) z[q] = ((const float2 *)bias)[4 * g + q];
-#pragma unroll
-                for (int k = 0; k < 9; ++k) {
-                    const float2 x2 = make_float2(in[k], in[k]);
-                    const float4 wa = ((const float4 *)w1)[k * (CH / 4) + 2 * g], wb = ((const float4 *)w1)[k * (CH / 4) + 2 * g + 1];
-                    z[0] = fma2(make_float2(wa.x, wa.y), x2, z[0]);
-                    z[1] = fma2(make_float2(wa.z, wa.w), x2, z[1]);
-                    z[2] = fma2(make_float2(wb.x, wb.y), x2, z[2]);
-                    z[3] = fma2(make_float2(wb.z, wb.w), x2, z[3]);
-                }
-                __align__(16) __nv_bfloat162 o[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) o[q] = __floats2bfloat162_rn(fmaxf(z[q].x, 0.0f), fmaxf(z[q].y, 0.0f));
-                *(uint4 *)(buf + g * IB_G + own * 16) = *(const uint4 *)o;
-            }
-        }
-#pragma unroll 1
-        for (int l = 0; l < 3; ++l) {
-            bamf::tc::fence_proxy_async();
-            bamf::tc::fence_before_sync();
-            __syncthreads();
-            bamf::tc::fence_after_sync();
-            if (t == 0) {
-#pragma unroll 1
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t acc = 0;
-#pragma unroll 1
-                    for (int tap = 0; tap < 9; ++tap) {
-                        const int kx = tap / 3, ky = tap - kx * 3;
-#pragma unroll
-                        for (int cb = 0; cb < 2; ++cb) {
-                            const uint32_t a = buf_addr + (2 * cb) * IB_G + (kx * PS + ky + 8 * h) * 16;
-                            const uint32_t b = ws_addr + l * (PKT * 2) + tap * (CH * CH * 2) + (2 * cb) * (CH * 16);
-                            bamf::tc::mma_bf16(tbase + 32 * h, bamf::tc::smem_desc(a, IB_G, PS * 16),
-                                               bamf::tc::smem_desc(b, CH * 16, 128), TC_IDESC, acc);
-                            acc = 1;
-                        }
-                    }
-                }
-                bamf::tc::commit(mbar);
-            }
-            if (!bamf::tc::mbar_wait(mbar, phase, 1u << 24)) {
-                if (t == 0) atomicExch(status, 1);
-                alive = false;
-            }
-            phase ^= 1u;
-            bamf::tc::fence_after_sync();
-            /* a thread that gave up leaves with all the others: the MMAs may
-             * still be reading the buffer */
-            if (!__syncthreads_and(alive)) {
-                alive = false;
-                break;
-            }
-            float d[32];
-            bamf::tc::tmem_ld32(tbase + ((uint32_t)((warp & 3) * 32) << 16) + 32 * mt, d);
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                const float4 ba = ((const float4 *)bias)[(l + 1) * (CH / 4) + 2 * g], bb = ((const float4 *)bias)[(l + 1) * (CH / 4) + 2 * g + 1];
-                __align__(16) __nv_bfloat162 o[4];
-                o[0] = __floats2bfloat162_rn(fmaxf(d[8 * g] + ba.x, 0.0f), fmaxf(d[8 * g + 1] + ba.y, 0.0f));
-                o[1] = __floats2bfloat162_rn(fmaxf(d[8 * g + 2] + ba.z, 0.0f), fmaxf(d[8 * g + 3] + ba.w, 0.0f));
-                o[2] = __floats2bfloat162_rn(fmaxf(d[8 * g + 4] + bb.x, 0.0f), fmaxf(d[8 * g + 5] + bb.y, 0.0f));
-                o[3] = __floats2bfloat162_rn(fmaxf(d[8 * g + 6] + bb.z, 0.0f), fmaxf(d[8 * g + 7] + bb.w, 0.0f));
-                *(uint4 *)(buf + g * IB_G + epi * 16) = *(const uint4 *)o;
-            }
-        }
-        if (!alive) break;
-        __syncthreads();
-        /* heads, as head_kernel: thread = pixel, a4 from the buffer */
-        float2 z[NSUB / 2];
-#pragma unroll
-        for (int k = 0; k < NSUB / 2; ++k) z[k] = ((const float2 *)bl)[k];
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            const uint4 u = *(const uint4 *)(buf + g * IB_G + own * 16);
-            const __nv_bfloat162 *h2 = (const __nv_bfloat162 *)&u;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const float2 hp = __bfloat1622float2(h2[e >> 1]);
-                const float h = e & 1 ? hp.y : hp.x;
-                const float4 *wc = (const float4 *)wl + (8 * g + e) * (NSUB / 4);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float4 w = wc[k];
-                    z[2 * k] = fma2(make_float2(w.x, w.y), make_float2(h, h), z[2 * k]);
-                    z[2 * k + 1] = fma2(make_float2(w.z, w.w), make_float2(h, h), z[2 * k + 1]);
-                }
-            }
-        }
-        float mx = -INFINITY;
-#pragma unroll
-        for (int k = 0; k < NSUB / 2; ++k) mx = fmaxf(mx, fmaxf(z[k].x, z[k].y));
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) red[warp] = mx;
-        if (cnt_out) { /* mean of a4 over pixels: channel lane, pixels warp, warp + 8, ... */
-            const bf16 *hc = (const bf16 *)(buf + (lane >> 3) * IB_G) + (lane & 7);
-            float sacc = 0.0f;
-#pragma unroll 4
-            for (int p = warp; p < NPX; p += 8) sacc += __bfloat162float(hc[(((p >> 4) + 1) * PS + (p & 15) + 1) * 8]);
-            part[warp][lane] = sacc;
-        }
-        __syncthreads();
-        mx = red[0];
-#pragma unroll
-        for (int k = 1; k < 8; ++k) mx = fmaxf(mx, red[k]);
-        if (cnt_out && t < CH) {
-            float sacc = 0.0f;
-            for (int k = 0; k < 8; ++k) sacc += part[k][t];
-            gmean[t] = sacc * (1.0f / NPX);
-        }
-        float e[NSUB], se = 0.0f;
-#pragma unroll
-        for (int k = 0; k < NSUB; ++k) {
-            e[k] = expf((k & 1 ? z[k >> 1].y : z[k >> 1].x) - mx);
-            se += e[k];
-        }
-        float tot = se;
-        for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-        if (lane == 0) red2[warp] = tot;
-        __syncthreads();
-        if (cnt_out && t < NC) {
-            float c = bc[t];
-            for (int k = 0; k < CH; ++k) c += Wc[t * CH + k] * gmean[k];
-            cnt_out[(size_t)r * NC + t] = c;
-        }
-        float sum = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) sum += red2[k];
-        const float pp = se * (1.0f / sum);
-        float incl = pp;
-        for (int o = 1; o < 32; o <<= 1) {
-            const float u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
-        }
-        if (lane == 31) red3[warp] = incl;
-        __syncthreads();
-        float base = 0.0f;
-        for (int k = 0; k < warp; ++k) base += red3[k];
-        cdf[(size_t)r * NPX + t] = base + incl;
-        const float inv_se = 1.0f / se;
-#pragma unroll
-        for (int k = 0; k < NSUB; ++k) e[k] *= inv_se;
-        float *dst = sub + ((size_t)r * NPX + t) * NSUB;
-        if (WIDE) {
-            store8(dst, e);
-            store8(dst + 8, e + 8);
-        } else {
-#pragma unroll
-            for (int k = 0; k < NSUB; ++k) dst[k] = e[k];
-        }
-    }
-    bamf::tc::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) bamf::tc::tmem_dealloc(tbase, 64);
 }
 
 /* --------------------------------------------------------- start states */
@@ -1332,11 +1080,9 @@ cudaError_t set_attrs()
         return e;
     if ((e = cudaFuncSetAttribute(conv_dw_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_DW)))
         return e;
-    if ((e = cudaFuncSetAttribute(head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_HEAD)))
+    if ((e = cudaFuncSetAttribute(head_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_HEAD)))
         return e;
-    if ((e = cudaFuncSetAttribute(infer_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_INFER)))
-        return e;
-    if ((e = cudaFuncSetAttribute(infer_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_INFER)))
+    if ((e = cudaFuncSetAttribute(head_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_HEAD)))
         return e;
     g_attr_done = true;
     return cudaSuccess;
@@ -1368,8 +1114,8 @@ bamf_status forward(bamf_cnn *net, const float *data, int n, cudaStream_t s)
 /* loss and gradients (accumulated into G) of the batch whose forward ran */
 bamf_status backward(bamf_cnn *net, const int32_t *n_em, const float *xyi, int n, float inv_batch, cudaStream_t s)
 {
-    head_kernel<<<n, 256, SMEM_HEAD, s>>>(net->a[3], n, net->P, n_em, xyi, inv_batch, net->hpart, net->dzA,
-                                                net->loss, net->step);
+    head_kernel<true><<<n, 256, SMEM_HEAD, s>>>(net->a[3], n, net->P, n_em, xyi, inv_batch, net->hpart, net->dzA,
+                                                net->loss, net->step, nullptr, nullptr, nullptr);
     bf16 *dz = net->dzA, *dzn = net->dzB;
     for (int l = 2; l >= 0; --l) {
         /* layer l+2: input a[l], output a[l+1]; dz = dL/dz_{l+2} */
@@ -1651,11 +1397,16 @@ extern "C" bamf_status bamf_cnn_infer(bamf_cnn *net, const float *data, int n, f
                                       float *count_logits, void *stream)
 {
     if (!net || n < 0 || (n > 0 && (!data || !cdf || !sub))) return BAMF_ERR_INVALID_ARG;
-    if (n == 0) return BAMF_OK;
-    /* 32-byte stores need the table at a 32-byte boundary */
-    const auto kernel = ((uintptr_t)sub & 31) == 0 ? infer_kernel<true> : infer_kernel<false>;
-    kernel<<<grid_for(n, 2, net->sms), 256, SMEM_INFER, (cudaStream_t)stream>>>(data, n, net->P, net->Wf, cdf, sub,
-                                                                                count_logits, net->tc_status);
-    CK(cudaGetLastError());
+    cudaStream_t s = (cudaStream_t)stream;
+    for (int b0 = 0; b0 < n; b0 += MAX_BATCH) {
+        int m = std::min(MAX_BATCH, n - b0);
+        bamf_status r = forward(net, data + (size_t)b0 * NPX, m, s);
+        if (r) return r;
+        head_kernel<false><<<m, 256, SMEM_HEAD, s>>>(net->a[3], m, net->P, nullptr, nullptr, 0.0f, nullptr, nullptr,
+                                                     nullptr, nullptr, cdf + (size_t)b0 * NPX,
+                                                     sub + (size_t)b0 * NPX * NSUB,
+                                                     count_logits ? count_logits + (size_t)b0 * NC : nullptr);
+        CK(cudaGetLastError());
+    }
     return BAMF_OK;
 }
