@@ -681,17 +681,13 @@ __global__ void __launch_bounds__(1024) dw_reduce_kernel(const float *__restrict
 }
 
 /* ----------------------------------------------------------------- heads */
-/* One CTA (256 threads, thread = pixel) per ROI.  TRAIN: loss, head
+/* Training: one CTA (256 threads, thread = pixel) per ROI: loss, head
  * gradients (row r of `hrows`, HEAD_NPARAM floats per ROI), dz4 = dL/d(pre-
- * activation of conv4).  INFER: the sampler's birth tables and the count
- * logits. */
-template <bool TRAIN>
+ * activation of conv4). */
 __global__ void __launch_bounds__(256) head_kernel(const bf16 *__restrict__ a4, int n, const float *__restrict__ P,
                                                    const int32_t *__restrict__ n_em, const float *__restrict__ xyi,
                                                    float inv_batch, float *__restrict__ hrows, bf16 *__restrict__ dz4,
-                                                   float *__restrict__ loss_buf, const int *__restrict__ step_dev,
-                                                   float *__restrict__ cdf, float *__restrict__ sub,
-                                                   float *__restrict__ cnt_out)
+                                                   float *__restrict__ loss_buf, const int *__restrict__ step_dev)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float *H = (float *)smem_raw;             /* [256][HS] */
@@ -777,26 +773,7 @@ __global__ void __launch_bounds__(256) head_kernel(const bf16 *__restrict__ a4, 
     }
     __syncthreads();
     const float inv_sum = 1.0f / sm_sum;
-    if (!TRAIN) {
-        /* pixel probability, inclusive scan over pixels (thread order = p) */
-        float pp = se * inv_sum;
-        float incl = pp;
-        for (int o = 1; o < 32; o <<= 1) {
-            float v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        __syncthreads();
-        if (lane == 31) red[warp] = incl;
-        __syncthreads();
-        float base = 0.0f;
-        for (int k = 0; k < warp; ++k) base += red[k];
-        cdf[(size_t)r * NPX + t] = base + incl;
-        float inv_se = 1.0f / se;
-        for (int s = 0; s < NSUB; ++s) sub[((size_t)r * NPX + t) * NSUB + s] = e[s] * inv_se;
-        if (cnt_out && t < NC) cnt_out[(size_t)r * NC + t] = zc[t];
-        return;
-    }
-    /* ---- training: targets, loss, gradients */
+    /* ---- targets, loss, gradients */
     const int ntrue = n_em[r];
     if (t < BAMF_SYNTH_NMAX) {
         ex[t] = xyi[((size_t)r * BAMF_SYNTH_NMAX + t) * 3 + 0];
@@ -918,6 +895,340 @@ __global__ void __launch_bounds__(256) head_kernel(const bf16 *__restrict__ a4, 
     }
     for (int o = t; o < NC * CH; o += 256) row_wc(hrows, r)[o] = dzc[o / CH] * gmean[o - (o / CH) * CH];
     if (t < NC) row_wc(hrows, r)[NC * CH + t] = dzc[t];
+}
+
+/* ------------------------------------------------------ fused inference */
+/* The whole network on a ROI without leaving the SM.  A persistent CTA keeps
+ * the packed weights of the three convolutions resident and runs GROUPS groups
+ * of 256 threads; a group takes one ROI per iteration: conv1 (FP32), three 32 ->
+ * 32 convolutions and the 1x1 head on tcgen05, the birth tables written out.
+ *
+ * One activation buffer per group, [ci group g][padded x 0..17][padded y
+ * 0..17][8 ci] BF16 with zero borders, serves every tap without shifted copies:
+ * M tile `mt` is the ROI's half y in [8 mt, 8 mt + 8), its row m the pixel x = m
+ * / 8, y = 8 mt + m mod 8, so a core matrix is 8 consecutive y of one x (128
+ * contiguous bytes), the next one is one padded column away (SBO = 288), and
+ * tap (kx, ky) starts (18 kx + ky) 16-byte rows in.  The epilogue of a layer
+ * (bias, ReLU, BF16) writes the next layer's input over it once the layer's
+ * MMAs completed.  The sums over channels and taps run in conv_tc_kernel's
+ * order, so a1..a4 are the same bits as from the kernels that training uses.
+ *
+ * The 1x1 head keeps FP32 weights: each is the exact sum of three BF16 parts
+ * (8 significant bits each), a4 is BF16, so loc = a4 Wl^T is three exact-product
+ * GEMMs with FP32 accumulation, one MMA of N = 48 per 16 channels, whose
+ * results are added smallest first.  On 50,000 ROIs the tables' error against
+ * 64 bits (3.2e-3, from the BF16 activations) is the same as with FP32 FMAs.
+ *
+ * Bound: shared memory.  Each of the 108 convolution MMAs reads a 4 KB A tile
+ * and 1 KB of weights for 32 columns, 40 cycles of the SM's 128 bytes/cycle;
+ * a 16-byte broadcast load takes 4 of them, so conv1 gives a thread 4 pixels x
+ * 8 channels (18 weight loads instead of 72 for one pixel x 32).  Four groups
+ * on an SM (two CTAs of two) overlap one's MMAs with the others' epilogues.
+ * 50,000 ROIs: 3.78 ms as five launches per 4096 ROIs, 1.93 ms with the heads in
+ * FP32 FMAs and one thread building every descriptor, 1.53 with this conv1 and
+ * head, 1.32 with the warp-uniform issue, 1.26 with GROUPS = 2 instead of 1;
+ * 0.74 ms is 108 x 40 + 4 x 44 cycles per ROI and SM. */
+constexpr int IB_G = PS * PS * 16;                 /* bytes of one ci group of the buffer */
+constexpr int IB_BYTES = 4 * IB_G;
+constexpr int INF_GROUPS = 2;
+constexpr int IH_N = 3 * NSUB;                     /* head columns: three parts of 16 sub-cells */
+constexpr int IH_BYTES = 4 * IH_N * 16;            /* [ci group][48][8 ci] */
+/* byte offsets: convolution weights, head weights, conv1 weights [tap][co],
+ * biases of conv1 .. conv4, then per group buffer, conv1 input, reductions */
+constexpr int INF_WH = 3 * PKT * 2;
+constexpr int INF_W1 = INF_WH + IH_BYTES;
+constexpr int INF_BIAS = INF_W1 + 9 * CH * 4;
+constexpr int INF_GRP = INF_BIAS + 4 * CH * 4;
+struct alignas(16) InferGroup {
+    unsigned char buf[IB_BYTES];
+    float xp[PS * PS];
+    float se[NPX];
+    float part[8][CH];
+    float gmean[CH], red[8], red2[8], red3[8];
+    uint64_t mbar;
+    int dead;
+};
+constexpr size_t SMEM_INFER = INF_GRP + INF_GROUPS * sizeof(InferGroup);
+constexpr int INF_TMEM = 128; /* columns per group: 64 of a convolution, then 96 of the head over them */
+constexpr uint32_t IH_IDESC = bamf::tc::idesc_bf16_f32(128, IH_N);
+static_assert(INF_W1 % 16 == 0 && INF_GRP % 16 == 0, "shared-memory alignment");
+
+/* two FP32 fused multiply-adds, each rounded as fmaf rounds it */
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    float2 d;
+    asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+        "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+
+/* 32 bytes of one thread in one store: a whole L2 sector */
+__device__ __forceinline__ void store8(float *p, const float *v)
+{
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+
+__device__ __forceinline__ uint4 relu_bf16(const float (&v)[8])
+{
+    __align__(16) __nv_bfloat162 o[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) o[q] = __floats2bfloat162_rn(fmaxf(v[2 * q], 0.0f), fmaxf(v[2 * q + 1], 0.0f));
+    return *(const uint4 *)o;
+}
+
+template <bool WIDE>
+__global__ void __launch_bounds__(256 * INF_GROUPS, 2) infer_kernel(
+    const float *__restrict__ data, int n, const float *__restrict__ P, const bf16 *__restrict__ Wt,
+    float *__restrict__ cdf, float *__restrict__ sub, float *__restrict__ cnt_out, int *__restrict__ status)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float *w1 = (float *)(smem_raw + INF_W1), *bias = (float *)(smem_raw + INF_BIAS);
+    __shared__ uint32_t tslot;
+    __shared__ float Wc[NC * CH], bc[NC], bl[NSUB];
+    const int t = threadIdx.x % 256, lane = t & 31;
+    /* warp-uniform, and known to be */
+    const int wid = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), grp = wid >> 3, warp = wid & 7;
+    InferGroup &G = ((InferGroup *)(smem_raw + INF_GRP))[grp];
+    unsigned char *const buf = G.buf;
+    if (threadIdx.x < 32) bamf::tc::tmem_alloc(&tslot, INF_TMEM * INF_GROUPS);
+    {
+        const int nt = 256 * INF_GROUPS, i0 = threadIdx.x;
+        for (int i = i0; i < 3 * PKT * 2 / 16; i += nt) ((uint4 *)smem_raw)[i] = ((const uint4 *)Wt)[i];
+        for (int i = i0; i < CH * NSUB; i += nt) {
+            const int s = i / CH, c = i - s * CH;
+            bf16 *w = (bf16 *)(smem_raw + INF_WH) + (c >> 3) * (IH_N * 8) + s * 8 + (c & 7);
+            float v = P[O_WL + i];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const bf16 h = __float2bfloat16_rn(v);
+                w[k * NSUB * 8] = h;
+                v -= __bfloat162float(h); /* exact */
+            }
+        }
+        for (int i = i0; i < 9 * CH; i += nt) w1[i] = P[O_W1 + (i % CH) * 9 + i / CH];
+        for (int i = i0; i < 4 * CH; i += nt) {
+            const int l = i / CH;
+            bias[i] = P[(l == 0 ? O_B1 : l == 1 ? O_B2 : l == 2 ? O_B3 : O_B4) + i % CH];
+        }
+        for (int i = i0; i < NC * CH; i += nt) Wc[i] = P[O_WC + (i % NC) * CH + i / NC];
+        if (i0 < NSUB) bl[i0] = P[O_BL + i0];
+        if (i0 < NC) bc[i0] = P[O_BC + i0];
+        const uint4 z = make_uint4(0, 0, 0, 0);
+        for (int i = t; i < IB_BYTES / 16; i += 256) ((uint4 *)buf)[i] = z;
+        for (int i = t; i < PS * PS; i += 256) G.xp[i] = 0.0f;
+    }
+    if (t == 0) {
+        bamf::tc::mbar_init(&G.mbar, 1);
+        G.dead = 0;
+    }
+    bamf::tc::fence_before_sync();
+    __syncthreads();
+    bamf::tc::fence_after_sync();
+    const auto group_sync = [&]() { asm volatile("barrier.sync %0, 256;" ::"r"(1 + grp) : "memory"); };
+    const uint32_t tbase = __shfl_sync(0xffffffffu, tslot, 0) + INF_TMEM * grp;
+    const uint64_t ad0 = bamf::tc::smem_desc(bamf::tc::smem_addr(buf), IB_G, PS * 16);
+    const uint64_t bd0 = bamf::tc::smem_desc(bamf::tc::smem_addr(smem_raw), CH * 16, 128);
+    const uint64_t hd0 = bamf::tc::smem_desc(bamf::tc::smem_addr(smem_raw) + INF_WH, IH_N * 16, 128);
+    /* this thread's pixel in the convolutions' epilogues and the head (its TMEM
+     * lane's), and that pixel's 16-byte row of a ci group */
+    const int mt = warp >> 2, m = 32 * (warp & 3) + lane;
+    const int pe = 16 * (m >> 3) + 8 * mt + (m & 7);
+    const int epi = ((pe >> 4) + 1) * PS + (pe & 15) + 1;
+    const uint32_t tlane = tbase + ((uint32_t)((warp & 3) * 32) << 16);
+    uint32_t phase = 0;
+    const int stride = gridDim.x * INF_GROUPS, r0 = blockIdx.x * INF_GROUPS + grp;
+    float next = r0 < n ? data[(size_t)r0 * NPX + t] : 0.0f;
+    /* every thread of the group waits for the group's MMAs; false (for all)
+     * when the wait ran out */
+    const auto mma_done = [&]() {
+        if (!bamf::tc::mbar_wait(&G.mbar, phase, 1u << 24)) {
+            G.dead = 1;
+            atomicExch(status, 1);
+        }
+        phase ^= 1u;
+        bamf::tc::fence_after_sync();
+    };
+    const auto mma_ready = [&]() {
+        bamf::tc::fence_proxy_async();
+        bamf::tc::fence_before_sync();
+        group_sync();
+        bamf::tc::fence_after_sync();
+    };
+    for (int r = r0; r < n; r += stride) {
+        /* conv1: the normalisation as conv1_fwd_kernel's (thread = pixel) */
+        const float v = sqrtf(fmaxf(next, 0.0f) + 0.375f);
+        if (r + stride < n) next = data[(size_t)(r + stride) * NPX + t];
+        float s = v;
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) G.red[warp] = s;
+        group_sync();
+        float mean = 0.0f;
+        for (int k = 0; k < 8; ++k) mean += G.red[k];
+        mean *= (1.0f / NPX);
+        G.xp[((t >> 4) + 1) * PS + (t & 15) + 1] = (v - mean) * 0.25f;
+        group_sync();
+        {
+            /* this thread: channels 8 g .. 8 g + 7 of the pixels y = lane & 15,
+             * x = x0 + 2 j */
+            const int g = warp & 3, y = lane & 15, x0 = 8 * (warp >> 2) + (lane >> 4);
+            float2 z[4][4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 b = ((const float2 *)bias)[4 * g + q];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) z[j][q] = b;
+            }
+            float in[9][3]; /* padded rows x0 .. x0 + 8 of columns y .. y + 2 */
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+#pragma unroll
+                for (int ky = 0; ky < 3; ++ky) in[k][ky] = G.xp[(x0 + k) * PS + y + ky];
+#pragma unroll
+            for (int tap = 0; tap < 9; ++tap) {
+                const float4 wa = ((const float4 *)w1)[tap * (CH / 4) + 2 * g];
+                const float4 wb = ((const float4 *)w1)[tap * (CH / 4) + 2 * g + 1];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 x2 = make_float2(in[2 * j + tap / 3][tap % 3], in[2 * j + tap / 3][tap % 3]);
+                    z[j][0] = fma2(make_float2(wa.x, wa.y), x2, z[j][0]);
+                    z[j][1] = fma2(make_float2(wa.z, wa.w), x2, z[j][1]);
+                    z[j][2] = fma2(make_float2(wb.x, wb.y), x2, z[j][2]);
+                    z[j][3] = fma2(make_float2(wb.z, wb.w), x2, z[j][3]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float o[8] = {z[j][0].x, z[j][0].y, z[j][1].x, z[j][1].y,
+                                    z[j][2].x, z[j][2].y, z[j][3].x, z[j][3].y};
+                *(uint4 *)(buf + g * IB_G + ((x0 + 2 * j + 1) * PS + y + 1) * 16) = relu_bf16(o);
+            }
+        }
+#pragma unroll 1
+        for (int l = 0; l < 3; ++l) {
+            mma_ready();
+            if (warp == 0) {
+                /* descriptors by adding to the first one's address field (no
+                 * carry out of it: shared memory is below 2^18 bytes) */
+                const uint64_t bd = bd0 + (uint32_t)l * (PKT * 2 / 16);
+                const uint32_t one = bamf::tc::elect_one();
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int tap = 0; tap < 9; ++tap)
+#pragma unroll
+                        for (int cb = 0; cb < 2; ++cb)
+                            bamf::tc::mma_bf16_warp(
+                                tbase + 32 * h, ad0 + (2 * cb * IB_G + (tap / 3 * PS + tap % 3 + 8 * h) * 16) / 16,
+                                bd + (tap * (CH * CH * 2) + 2 * cb * (CH * 16)) / 16, TC_IDESC, tap + cb > 0 ? 1u : 0u,
+                                one);
+                if (one) bamf::tc::commit(&G.mbar);
+            }
+            mma_done();
+            float d[32];
+            bamf::tc::tmem_ld32(tlane + 32 * mt, d);
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const float4 ba = ((const float4 *)bias)[(l + 1) * (CH / 4) + 2 * g];
+                const float4 bb = ((const float4 *)bias)[(l + 1) * (CH / 4) + 2 * g + 1];
+                const float o[8] = {d[8 * g] + ba.x,     d[8 * g + 1] + ba.y, d[8 * g + 2] + ba.z, d[8 * g + 3] + ba.w,
+                                    d[8 * g + 4] + bb.x, d[8 * g + 5] + bb.y, d[8 * g + 6] + bb.z, d[8 * g + 7] + bb.w};
+                *(uint4 *)(buf + g * IB_G + epi * 16) = relu_bf16(o);
+            }
+        }
+        mma_ready();
+        if (warp == 0) {
+            const uint32_t one = bamf::tc::elect_one();
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int cb = 0; cb < 2; ++cb)
+                    bamf::tc::mma_bf16_warp(tbase + IH_N * h, ad0 + (2 * cb * IB_G + (PS + 1 + 8 * h) * 16) / 16,
+                                            hd0 + 2 * cb * IH_N, IH_IDESC, (uint32_t)cb, one);
+            if (one) bamf::tc::commit(&G.mbar);
+        }
+        if (cnt_out) { /* mean of a4 over pixels: channel lane, pixels warp, warp + 8, ... */
+            const bf16 *hc = (const bf16 *)(buf + (lane >> 3) * IB_G) + (lane & 7);
+            float sacc = 0.0f;
+#pragma unroll
+            for (int p = warp; p < NPX; p += 8) sacc += __bfloat162float(hc[(((p >> 4) + 1) * PS + (p & 15) + 1) * 8]);
+            G.part[warp][lane] = sacc;
+        }
+        mma_done();
+        float e[NSUB];
+        {
+            float d[32], d3[16];
+            bamf::tc::tmem_ld32(tlane + IH_N * mt, d);
+            bamf::tc::tmem_ld16(tlane + IH_N * mt + 32, d3);
+#pragma unroll
+            for (int k = 0; k < NSUB; ++k) e[k] = ((d3[k] + d[16 + k]) + d[k]) + bl[k];
+        }
+        float mx = -INFINITY;
+#pragma unroll
+        for (int k = 0; k < NSUB; ++k) mx = fmaxf(mx, e[k]);
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (lane == 0) G.red[warp] = mx;
+        group_sync();
+        if (G.dead) break; /* set before this barrier, seen by the whole group */
+        mx = G.red[0];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) mx = fmaxf(mx, G.red[k]);
+        if (cnt_out && t < CH) {
+            float sacc = 0.0f;
+            for (int k = 0; k < 8; ++k) sacc += G.part[k][t];
+            G.gmean[t] = sacc * (1.0f / NPX);
+        }
+        float se = 0.0f;
+#pragma unroll
+        for (int k = 0; k < NSUB; ++k) {
+            e[k] = expf(e[k] - mx);
+            se += e[k];
+        }
+        G.se[pe] = se;
+        const float inv_se = 1.0f / se;
+#pragma unroll
+        for (int k = 0; k < NSUB; ++k) e[k] *= inv_se;
+        float *dst = sub + ((size_t)r * NPX + pe) * NSUB;
+        if (WIDE) {
+            store8(dst, e);
+            store8(dst + 8, e + 8);
+        } else {
+#pragma unroll
+            for (int k = 0; k < NSUB; ++k) dst[k] = e[k];
+        }
+        group_sync();
+        /* the running sum over pixels, thread = pixel */
+        se = G.se[t];
+        float tot = se;
+        for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+        if (lane == 0) G.red2[warp] = tot;
+        group_sync();
+        float sum = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sum += G.red2[k];
+        float incl = se * (1.0f / sum);
+        for (int o = 1; o < 32; o <<= 1) {
+            const float u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) G.red3[warp] = incl;
+        group_sync();
+        float base = 0.0f;
+        for (int k = 0; k < warp; ++k) base += G.red3[k];
+        cdf[(size_t)r * NPX + t] = base + incl;
+        if (cnt_out && warp == 7 && lane < NC) {
+            float c = bc[lane];
+#pragma unroll
+            for (int k = 0; k < CH; ++k) c += Wc[k * NC + lane] * G.gmean[k];
+            cnt_out[(size_t)r * NC + lane] = c;
+        }
+    }
+    bamf::tc::fence_before_sync();
+    __syncthreads();
+    if (threadIdx.x < 32) bamf::tc::tmem_dealloc(tslot, INF_TMEM * INF_GROUPS);
 }
 
 /* --------------------------------------------------------- start states */
@@ -1080,9 +1391,11 @@ cudaError_t set_attrs()
         return e;
     if ((e = cudaFuncSetAttribute(conv_dw_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_DW)))
         return e;
-    if ((e = cudaFuncSetAttribute(head_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_HEAD)))
+    if ((e = cudaFuncSetAttribute(head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_HEAD)))
         return e;
-    if ((e = cudaFuncSetAttribute(head_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_HEAD)))
+    if ((e = cudaFuncSetAttribute(infer_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_INFER)))
+        return e;
+    if ((e = cudaFuncSetAttribute(infer_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_INFER)))
         return e;
     g_attr_done = true;
     return cudaSuccess;
@@ -1114,8 +1427,8 @@ bamf_status forward(bamf_cnn *net, const float *data, int n, cudaStream_t s)
 /* loss and gradients (accumulated into G) of the batch whose forward ran */
 bamf_status backward(bamf_cnn *net, const int32_t *n_em, const float *xyi, int n, float inv_batch, cudaStream_t s)
 {
-    head_kernel<true><<<n, 256, SMEM_HEAD, s>>>(net->a[3], n, net->P, n_em, xyi, inv_batch, net->hpart, net->dzA,
-                                                net->loss, net->step, nullptr, nullptr, nullptr);
+    head_kernel<<<n, 256, SMEM_HEAD, s>>>(net->a[3], n, net->P, n_em, xyi, inv_batch, net->hpart, net->dzA,
+                                                net->loss, net->step);
     bf16 *dz = net->dzA, *dzn = net->dzB;
     for (int l = 2; l >= 0; --l) {
         /* layer l+2: input a[l], output a[l+1]; dz = dL/dz_{l+2} */
@@ -1397,16 +1710,11 @@ extern "C" bamf_status bamf_cnn_infer(bamf_cnn *net, const float *data, int n, f
                                       float *count_logits, void *stream)
 {
     if (!net || n < 0 || (n > 0 && (!data || !cdf || !sub))) return BAMF_ERR_INVALID_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    for (int b0 = 0; b0 < n; b0 += MAX_BATCH) {
-        int m = std::min(MAX_BATCH, n - b0);
-        bamf_status r = forward(net, data + (size_t)b0 * NPX, m, s);
-        if (r) return r;
-        head_kernel<false><<<m, 256, SMEM_HEAD, s>>>(net->a[3], m, net->P, nullptr, nullptr, 0.0f, nullptr, nullptr,
-                                                     nullptr, nullptr, cdf + (size_t)b0 * NPX,
-                                                     sub + (size_t)b0 * NPX * NSUB,
-                                                     count_logits ? count_logits + (size_t)b0 * NC : nullptr);
-        CK(cudaGetLastError());
-    }
+    if (n == 0) return BAMF_OK;
+    /* 32-byte stores need the table at a 32-byte boundary */
+    const auto kernel = ((uintptr_t)sub & 31) == 0 ? infer_kernel<true> : infer_kernel<false>;
+    kernel<<<grid_for((n + INF_GROUPS - 1) / INF_GROUPS, 2, net->sms), 256 * INF_GROUPS, SMEM_INFER, (cudaStream_t)stream>>>(data, n, net->P, net->Wf, cdf, sub,
+                                                                                count_logits, net->tc_status);
+    CK(cudaGetLastError());
     return BAMF_OK;
 }
