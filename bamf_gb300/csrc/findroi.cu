@@ -44,36 +44,36 @@
 
 namespace {
 
-/* rb0 = RN(1/b0); the fused filter divides by b0 through rb0 (div_fast)
- * for |q| in [lo, hi], and with IEEE division elsewhere (lo = +inf: never
- * through rb0). */
+/* rb0 + rb1 = 1/b0 (two floats); the filter divides by b0 through them
+ * (div_fast) for |q| in [lo, hi], and with IEEE division elsewhere (lo = +inf:
+ * never through them). */
 struct Coef {
-    float b0, b1, b2, b3, B, rb0, lo, hi;
+    float b0, b1, b2, b3, B, rb0, rb1, lo, hi;
 };
 
-/* Division by the constant b0 with one multiply and two FMAs (Markstein,
- * "Computation of elementary functions on the IBM RISC System/6000
- * processor", IBM J. Res. Dev. 34(1), 1990): q0 = RN(q*rb0), the residual
- * b0*q0 - q in one FMA, the corrected quotient RN(q0 - residual*rb0); a zero
- * q keeps its sign.  The sequence is invariant under scaling q by a power of
+/* Division by the constant b0 as a product with 1/b0 held in two floats
+ * (N. Brisebarre and J.-M. Muller, "Correctly rounded multiplication by
+ * arbitrary precision constants", IEEE Trans. Computers 57(2), 2008): RN(q rb0 +
+ * RN(q rb1)), two operations instead of Markstein's three (a recurrence step
+ * is a chain of them).  The sequence is invariant under scaling q by a power of
  * two while no intermediate leaves the normal range, which holds for |q| in
- * [2^-100, 2^100] and b0 in [2^-20, 2^20]; so it equals RN(q/b0) on that whole
- * range iff it does for the 2^23 significands of [1, 2), which
- * fast_division_exact checks on the host, once per divisor. */
-__host__ __device__ __forceinline__ float div_fast(float q, float b0, float rb0)
+ * [2^-125 / |rb1|, 2^100] (at most, 2^-100) and b0 in [2^-20, 2^20]; so it equals
+ * RN(q/b0) on that whole range iff it does for the 2^23 significands of [1, 2),
+ * which fast_division_exact checks on the host, once per divisor.  It did for
+ * every width from 0.6 to 6.0 in steps of 0.1. */
+__host__ __device__ __forceinline__ float div_fast(float q, float rb0, float rb1)
 {
 #ifdef __CUDA_ARCH__
-    const float q0 = __fmul_rn(q, rb0);
-    return __fmaf_rn(-__fmaf_rn(b0, q0, -q), rb0, q0);
+    return __fmaf_rn(q, rb0, __fmul_rn(q, rb1));
 #else
-    const float q0 = q * rb0;
-    return std::fma(-std::fma(b0, q0, -q), rb0, q0);
+    return std::fma(q, rb0, q * rb1);
 #endif
 }
 
-bool fast_division_exact(float b0, float rb0)
+bool fast_division_exact(float b0, float rb0, float rb1)
 {
     if (!(std::fabs(b0) >= 0x1p-20f && std::fabs(b0) <= 0x1p20f)) return false;
+    if (!(rb1 == 0.0f || std::fabs(rb1) >= 0x1p-60f)) return false;
     static std::mutex mu;
     static std::vector<std::pair<float, bool>> seen;
     std::lock_guard<std::mutex> lock(mu);
@@ -88,7 +88,7 @@ bool fast_division_exact(float b0, float rb0)
                 const uint32_t bits = 0x3f800000u | m;
                 float q;
                 std::memcpy(&q, &bits, sizeof q);
-                const float want = q / b0, got = div_fast(q, b0, rb0);
+                const float want = q / b0, got = div_fast(q, rb0, rb1);
                 if (std::memcmp(&want, &got, sizeof got) != 0) ok = false;
             }
         });
@@ -111,10 +111,12 @@ Coef iir_coef(double Sigma)
     double B2 = -1.4281 * Qq - 1.26661 * Qqq;
     double B3 = 0.422205 * Qqq;
     double B = 1 - (B1 + B2 + B3) / B0;
-    Coef c{(float)B0, (float)B1, (float)B2, (float)B3, (float)B, 0.0f, INFINITY, 0.0f};
+    Coef c{(float)B0, (float)B1, (float)B2, (float)B3, (float)B, 0.0f, 0.0f, INFINITY, 0.0f};
     c.rb0 = 1.0f / c.b0;
-    if (fast_division_exact(c.b0, c.rb0)) {
-        c.lo = 0x1p-100f;
+    c.rb1 = (float)(1.0 / (double)c.b0 - (double)c.rb0);
+    if (fast_division_exact(c.b0, c.rb0, c.rb1)) {
+        /* q rb1 stays normal */
+        c.lo = c.rb1 == 0.0f ? 0x1p-100f : std::ldexp(1.0f, std::max(-100, -125 - std::ilogb(c.rb1)));
         c.hi = 0x1p100f;
     }
     return c;
@@ -130,191 +132,34 @@ __device__ __forceinline__ float iir_step(float w0, float w1, float w2, float w3
     return __fmaf_rn(w0, c.B, __fdiv_rn(iir_q(w1, w2, w3, c), c.b0));
 }
 
-/* Pass 1: one thread per (frame, row) runs the row's recurrence for both
- * sigmas, in the reference's sequential order.  Rows are contiguous, so the
- * warp moves its 32 rows through shared memory in chunks of 32 columns: a
- * [32][33] tile is loaded with 128-byte row segments (coalesced), each
- * thread walks its own tile row (stride 33: conflict-free), and the
- * results leave the same way.  The forward results go to out_a/out_b and
- * come back chunk by chunk, last chunk first, for the backward pass; the
- * grid is persistent with ROWS_CTAS_PER_SM CTAs per SM so that the rows in
- * flight (and their forward results) stay within L2. */
-constexpr int ROWS_WARPS = 3;
-constexpr int ROWS_CTAS_PER_SM = 5;
-
-__global__ void __launch_bounds__(32 * ROWS_WARPS) rows_kernel(const float *__restrict__ in,
-                                                               float *__restrict__ out_a,
-                                                               float *__restrict__ out_b, int X, int Y,
-                                                               int Z, Coef ca, Coef cb)
-{
-    __shared__ float tile[ROWS_WARPS][3][32][33];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float(*ti)[33] = tile[warp][0];
-    float(*ta_)[33] = tile[warp][1];
-    float(*tb_)[33] = tile[warp][2];
-    const int64_t nrows = (int64_t)Y * Z;
-    const int64_t ngroups = (nrows + 31) / 32;
-    const int nch = (X + 31) / 32;
-    for (int64_t g = (int64_t)blockIdx.x * ROWS_WARPS + warp; g < ngroups; g += (int64_t)gridDim.x * ROWS_WARPS) {
-        const int64_t row0 = g * 32;
-        const int rows_here = (int)min((int64_t)32, nrows - row0);
-        const bool mine = lane < rows_here;
-        float a1 = 0.0f, a2 = 0.0f, a3 = 0.0f, b1 = 0.0f, b2 = 0.0f, b3 = 0.0f;
-        for (int c = 0; c < nch; ++c) {
-            const int c0 = c * 32, w = min(32, X - c0);
-            for (int r = 0; r < rows_here; ++r)
-                if (lane < w) ti[r][lane] = in[(row0 + r) * X + c0 + lane];
-            __syncwarp();
-            if (mine) {
-                if (c == 0) {
-                    a1 = a2 = a3 = ti[lane][0];
-                    b1 = b2 = b3 = ti[lane][0];
-                }
-                for (int j = 0; j < w; ++j) {
-                    float w0 = ti[lane][j];
-                    float ta = iir_step(w0, a1, a2, a3, ca);
-                    float tb = iir_step(w0, b1, b2, b3, cb);
-                    ta_[lane][j] = ta;
-                    tb_[lane][j] = tb;
-                    a3 = a2; a2 = a1; a1 = ta;
-                    b3 = b2; b2 = b1; b1 = tb;
-                }
-            }
-            __syncwarp();
-            for (int r = 0; r < rows_here; ++r)
-                if (lane < w) {
-                    out_a[(row0 + r) * X + c0 + lane] = ta_[r][lane];
-                    out_b[(row0 + r) * X + c0 + lane] = tb_[r][lane];
-                }
-            __syncwarp();
-        }
-        for (int c = nch - 1; c >= 0; --c) {
-            const int c0 = c * 32, w = min(32, X - c0);
-            for (int r = 0; r < rows_here; ++r)
-                if (lane < w) {
-                    ta_[r][lane] = out_a[(row0 + r) * X + c0 + lane];
-                    tb_[r][lane] = out_b[(row0 + r) * X + c0 + lane];
-                }
-            __syncwarp();
-            if (mine) {
-                if (c == nch - 1) {
-                    a1 = a2 = a3 = ta_[lane][w - 1];
-                    b1 = b2 = b3 = tb_[lane][w - 1];
-                }
-                for (int j = w - 1; j >= 0; --j) {
-                    float ta = iir_step(ta_[lane][j], a1, a2, a3, ca);
-                    float tb = iir_step(tb_[lane][j], b1, b2, b3, cb);
-                    ta_[lane][j] = ta;
-                    tb_[lane][j] = tb;
-                    a3 = a2; a2 = a1; a1 = ta;
-                    b3 = b2; b2 = b1; b1 = tb;
-                }
-            }
-            __syncwarp();
-            for (int r = 0; r < rows_here; ++r)
-                if (lane < w) {
-                    out_a[(row0 + r) * X + c0 + lane] = ta_[r][lane];
-                    out_b[(row0 + r) * X + c0 + lane] = tb_[r][lane];
-                }
-            __syncwarp();
-        }
-    }
-}
-
-/* Pass 2: one thread per (frame, column): column filters of both images in
- * place, then dog = a - b written over a. */
-__global__ void __launch_bounds__(128) cols_kernel(float *__restrict__ a, float *__restrict__ b,
-                                                   int X, int Y, int Z, Coef ca, Coef cb)
-{
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)X * Z) return;
-    int64_t z = t / X, c = t - z * X;
-    float *pa = a + z * (int64_t)X * Y + c, *pb = b + z * (int64_t)X * Y + c;
-    float a1, a2, a3, b1, b2, b3;
-    a1 = a2 = a3 = pa[0];
-    b1 = b2 = b3 = pb[0];
-    /* the loads of a block of COLS_PF rows are issued before its
-     * recurrence steps (they do not depend on it), hiding their latency */
-    constexpr int COLS_PF = 8;
-    int i = 0;
-    for (; i + COLS_PF <= Y; i += COLS_PF) {
-        float va[COLS_PF], vb[COLS_PF];
-#pragma unroll
-        for (int u = 0; u < COLS_PF; ++u) {
-            va[u] = pa[(int64_t)(i + u) * X];
-            vb[u] = pb[(int64_t)(i + u) * X];
-        }
-#pragma unroll
-        for (int u = 0; u < COLS_PF; ++u) {
-            float ta = iir_step(va[u], a1, a2, a3, ca);
-            float tb = iir_step(vb[u], b1, b2, b3, cb);
-            pa[(int64_t)(i + u) * X] = ta;
-            pb[(int64_t)(i + u) * X] = tb;
-            a3 = a2; a2 = a1; a1 = ta;
-            b3 = b2; b2 = b1; b1 = tb;
-        }
-    }
-    for (; i < Y; ++i) {
-        float ta = iir_step(pa[(int64_t)i * X], a1, a2, a3, ca);
-        float tb = iir_step(pb[(int64_t)i * X], b1, b2, b3, cb);
-        pa[(int64_t)i * X] = ta;
-        pb[(int64_t)i * X] = tb;
-        a3 = a2; a2 = a1; a1 = ta;
-        b3 = b2; b2 = b1; b1 = tb;
-    }
-    a1 = a2 = a3 = pa[(int64_t)(Y - 1) * X];
-    b1 = b2 = b3 = pb[(int64_t)(Y - 1) * X];
-    i = Y - 1;
-    for (; i - COLS_PF + 1 >= 0; i -= COLS_PF) {
-        float va[COLS_PF], vb[COLS_PF];
-#pragma unroll
-        for (int u = 0; u < COLS_PF; ++u) {
-            va[u] = pa[(int64_t)(i - u) * X];
-            vb[u] = pb[(int64_t)(i - u) * X];
-        }
-#pragma unroll
-        for (int u = 0; u < COLS_PF; ++u) {
-            float ta = iir_step(va[u], a1, a2, a3, ca);
-            float tb = iir_step(vb[u], b1, b2, b3, cb);
-            pa[(int64_t)(i - u) * X] = __fsub_rn(ta, tb); /* kernel_subtract */
-            a3 = a2; a2 = a1; a1 = ta;
-            b3 = b2; b2 = b1; b1 = tb;
-        }
-    }
-    for (; i >= 0; --i) {
-        float ta = iir_step(pa[(int64_t)i * X], a1, a2, a3, ca);
-        float tb = iir_step(pb[(int64_t)i * X], b1, b2, b3, cb);
-        pa[(int64_t)i * X] = __fsub_rn(ta, tb); /* kernel_subtract */
-        a3 = a2; a2 = a1; a1 = ta;
-        b3 = b2; b2 = b1; b1 = tb;
-    }
-}
-
-/* Passes 1 and 2 fused, for whole frames (frames of up to FF_MAX_SLOT
- * pixels per intermediate image; larger frames take rows_kernel +
- * cols_kernel).  One CTA owns one frame at a time, persistent over the
- * stack, and keeps the frame's two intermediate images in its own slot of
- * `scratch`: column-major, pixel (r, j) at j*YP + r with YP = Y rounded up to
- * 32, 2*X*YP floats.  The grid's slots together stay within L2, so only the
- * frames are read from DRAM and only the DoG is written.  The recurrences
- * run exactly as in rows_kernel / cols_kernel (bit-identical results):
- *   rows, forward:  thread r walks its row through shared-memory chunks of
- *                   FF_CW columns (cp.async, double-buffered) and writes each
- *                   output to the slot (consecutive r: coalesced)
- *   rows, backward: the slot's chunks come back through shared memory, last
- *                   first; outputs overwrite the forward ones in place
- *   cols, forward:  tiles of FF_CW rows x FF_T columns, [column][FF_TS]:
- *                   thread c walks column c in float4 steps (conflict-free),
- *                   results go back into the tile and the tile to the slot
+/* Passes 1 and 2, the row and the column recurrences, run in the reference's
+ * order.  A warp's chunks and tiles are its own, staged by cp.async one ahead:
+ *   rows, forward:  a row walks through chunks of FF_CW columns and writes each
+ *                   output to the frame's slot of `scratch` (column-major, YP = Y
+ *                   rounded up to 32 rows per column)
+ *   rows, backward: the slot's chunks come back, last first; outputs
+ *                   overwrite the forward ones in place
+ *   cols, forward:  tiles of FF_CW rows: a column walks in float4 steps
+ *                   (conflict-free), results go back into the tile and the
+ *                   tile to the slot
  *   cols, backward: the same, last tile first, the DoG written to `dog` in
- *                   frame layout (consecutive c: coalesced) */
-constexpr int FF_T = 256;   /* threads: rows of a row group / columns of a column group */
+ *                   frame layout
+ * A step is a chain of five dependent operations.  What it takes: filter_kernel
+ * (stacks) keeps both sigmas on a lane, two chains in flight per lane and 8
+ * warps per SM; filter_rows_kernel + filter_cols_kernel (few frames, where the
+ * chain's latency is all there is) put one recurrence on a lane and spread a
+ * frame over the SMs.  Neither packed f32x2 operations (three 64-bit operands
+ * issue every 3.3 cycles, slower than two scalar FMAs) nor 16 warps of one
+ * recurrence per lane made the stacks faster: the slot's 1.8 MB each way per 256 x
+ * 256 frame, at about 60 bytes per cycle and SM, adds to the arithmetic. */
+constexpr int FF_R = 16;    /* rows (columns) per warp */
 constexpr int FF_CW = 32;   /* columns per row-pass chunk, rows per column-pass tile */
-constexpr int FF_TS = 36;   /* tile row stride in floats: 16-byte rows, float4 reads conflict-free */
-constexpr size_t FF_MAX_SLOT = 80 * 1024; /* pixels per image in a slot (X * YP) */
-/* per warp: the largest phase, two buffers of column tiles [sigma][32 columns][FF_TS] */
-constexpr int FF_WARP_FLOATS = 2 * 2 * 32 * FF_TS;
-constexpr int FF_SMEM_FLOATS = (FF_T / 32) * FF_WARP_FLOATS;
+constexpr int FF_TS = 36;   /* row stride of an input chunk, column stride of a tile: float4 reads conflict-free */
+constexpr size_t FF_MAX_SLOT = 80 * 1024; /* pixels in a slot of filter_kernel (X * YP) */
+constexpr size_t FF_SPLIT_BYTES = (size_t)96 << 20; /* slots of the two-kernel form: within L2 */
+/* per warp, in floats: the largest phase, two buffers of column tiles */
+constexpr int FF_WARP_FLOATS = 2 * 2 * FF_R * FF_TS;
+static_assert(FF_WARP_FLOATS >= 2 * FF_R * FF_TS && FF_WARP_FLOATS >= 2 * FF_CW * 2 * FF_R, "the other phases fit");
 
 /* L2 eviction priorities: the frames and the DoG stream through L2 once
  * (evict first); the slots are reused all the time (evict last) and are
@@ -354,14 +199,14 @@ __device__ __forceinline__ void cp_wait_prev() { asm volatile("cp.async.wait_gro
 
 __device__ __forceinline__ void st_hint(float *g, float v, uint64_t pol)
 {
-    asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(g), "f"(v), "l"(pol));
+    asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(g), "f"(v), "l"(pol) : "memory");
 }
 
 /* st_hint at g + OFF bytes, the offset folded into the address */
 template <int OFF>
 __device__ __forceinline__ void st_hint_at(float *g, float v, uint64_t pol)
 {
-    asm volatile("st.global.L2::cache_hint.f32 [%0+%3], %1, %2;" ::"l"(g), "f"(v), "l"(pol), "n"(OFF));
+    asm volatile("st.global.L2::cache_hint.f32 [%0+%3], %1, %2;" ::"l"(g), "f"(v), "l"(pol), "n"(OFF) : "memory");
 }
 
 /* v0..v3 to g[0], g[stride], g[2 stride], g[3 stride]; with the stride
@@ -385,13 +230,275 @@ __device__ __forceinline__ void st_hint_4(float *g, int stride, float v0, float 
 __device__ __forceinline__ void st4_hint(float *g, float4 v, uint64_t pol)
 {
     asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(g), "f"(v.x), "f"(v.y),
-                 "f"(v.z), "f"(v.w), "l"(pol));
+                 "f"(v.z), "f"(v.w), "l"(pol)
+                 : "memory");
 }
 
 __device__ __forceinline__ void discard_line(const float *g)
 {
     asm volatile("discard.global.L2 [%0], 128;" ::"l"(g) : "memory");
 }
+
+/* minimum / maximum of three; a NaN operand is ignored */
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+/* the last three outputs of one recurrence */
+struct Iir {
+    float w1, w2, w3;
+    __device__ __forceinline__ void init(float v) { w1 = w2 = w3 = v; }
+    /* one step, IEEE division */
+    __device__ __forceinline__ float step(float x, const Coef &c)
+    {
+        const float o = iir_step(x, w1, w2, w3, c);
+        w3 = w2;
+        w2 = w1;
+        w1 = o;
+        return o;
+    }
+};
+
+static __device__ __noinline__ float4 steps4_ieee(Iir s, float4 x, Coef c)
+{
+    float4 y;
+    y.x = s.step(x.x, c);
+    y.y = s.step(x.y, c);
+    y.z = s.step(x.z, c);
+    y.w = s.step(x.w, c);
+    return y;
+}
+
+/* Four steps in processing order, x.x first, the division by b0 through rb0.
+ * A block in which any q left [lo, hi] is redone with IEEE division, so every
+ * output is the one iir_step gives; a NaN q passes the test and gives the NaN
+ * that IEEE division would. */
+__device__ __forceinline__ float4 steps4(Iir &s, const Coef &c, float4 x)
+{
+    const float q0 = iir_q(s.w1, s.w2, s.w3, c);
+    float4 y;
+    y.x = __fmaf_rn(x.x, c.B, div_fast(q0, c.rb0, c.rb1));
+    const float q1 = iir_q(y.x, s.w1, s.w2, c);
+    y.y = __fmaf_rn(x.y, c.B, div_fast(q1, c.rb0, c.rb1));
+    const float q2 = iir_q(y.y, y.x, s.w1, c);
+    y.z = __fmaf_rn(x.z, c.B, div_fast(q2, c.rb0, c.rb1));
+    const float q3 = iir_q(y.z, y.y, y.x, c);
+    y.w = __fmaf_rn(x.w, c.B, div_fast(q3, c.rb0, c.rb1));
+    const float mn = min3(fminf(fabsf(q0), fabsf(q1)), fabsf(q2), fabsf(q3));
+    const float mx = max3(fmaxf(fabsf(q0), fabsf(q1)), fabsf(q2), fabsf(q3));
+    if (!(mn >= c.lo && mx <= c.hi)) y = steps4_ieee(s, x, c);
+    s.w1 = y.w;
+    s.w2 = y.z;
+    s.w3 = y.y;
+    return y;
+}
+
+/* The warp's rows rg .. rg + 15 of the frame `fin`, forward and backward, into the
+ * slot S.  Every shared-memory index, also of values loaded ahead and not used,
+ * lies inside the warp's part. */
+template <bool VEC>
+__device__ __forceinline__ void filter_rows(const float *__restrict__ fin, float *S, int X, int Y, int YP, int rg,
+                                            float *wsm, const Coef &c, uint64_t pf, uint64_t pl)
+{
+    const int lane = threadIdx.x & 31, r = lane & 15, sg = lane >> 4;
+    const int nch = (X + FF_CW - 1) / FF_CW;
+    const int nr = min(FF_R, Y - rg);
+    const bool mine = r < nr;
+    Iir s;
+    s.init(0.0f);
+    /* ---- forward: input chunk [row][FF_TS] */
+    auto stage_in = [&](int ch, float *buf) {
+        const int c0 = ch * FF_CW, w = min(FF_CW, X - c0);
+        if (VEC) {
+            const int p = lane & 7;
+            if (4 * p < w)
+                for (int i = lane >> 3; i < nr; i += 4)
+                    cp_async16(buf + i * FF_TS + 4 * p, fin + (size_t)(rg + i) * X + c0 + 4 * p, pf);
+        } else if (lane < w) {
+            for (int i = 0; i < nr; ++i) cp_async4(buf + i * FF_TS + lane, fin + (size_t)(rg + i) * X + c0 + lane, pf);
+        }
+    };
+    stage_in(0, wsm);
+    cp_commit();
+    for (int ch = 0; ch < nch; ++ch) {
+        if (ch + 1 < nch) stage_in(ch + 1, wsm + ((ch + 1) & 1) * FF_R * FF_TS);
+        cp_commit();
+        cp_wait_prev();
+        __syncwarp();
+        const float *ti = wsm + (ch & 1) * FF_R * FF_TS + r * FF_TS;
+        const int c0 = ch * FF_CW, w = min(FF_CW, X - c0);
+        if (mine) {
+            if (ch == 0) s.init(ti[0]);
+            float *ps = S + (size_t)(2 * c0 + sg) * YP + rg + r;
+            int j = 0;
+            float4 v = *reinterpret_cast<const float4 *>(ti);
+#pragma unroll 2
+            for (; j + 4 <= w; j += 4) {
+                const float4 x = v;
+                v = *reinterpret_cast<const float4 *>(ti + j + 4); /* the next block's (a row has FF_TS floats) */
+                const float4 y = steps4(s, c, x);
+                st_hint_4<0>(ps + (size_t)(2 * j) * YP, 2 * YP, y.x, y.y, y.z, y.w, pl);
+            }
+            for (; j < w; ++j) st_hint(ps + (size_t)(2 * j) * YP, s.step(ti[j], c), pl);
+        }
+        __syncwarp(); /* buffer ch & 1 is restaged for chunk ch + 2; the slot stores are seen */
+    }
+    /* ---- backward: the warp's rows of the slot's chunks, [column][sigma][16] */
+    constexpr int BUF = FF_CW * 2 * FF_R;
+    auto stage_f = [&](int ch, float *buf) {
+        const int c0 = ch * FF_CW, w = min(FF_CW, X - c0), p = lane & 3;
+        if (4 * p < nr)
+            for (int k = lane >> 2; k < 2 * w; k += 8) /* k = 2 column + sigma */
+                cp_async16(buf + k * FF_R + 4 * p, S + (size_t)(2 * c0 + k) * YP + rg + 4 * p, pl);
+    };
+    stage_f(nch - 1, wsm);
+    cp_commit();
+    for (int ci = 0; ci < nch; ++ci) {
+        const int ch = nch - 1 - ci;
+        if (ch > 0) stage_f(ch - 1, wsm + ((ci + 1) & 1) * BUF);
+        cp_commit();
+        cp_wait_prev();
+        __syncwarp();
+        const float *f = wsm + (ci & 1) * BUF + lane;
+        const int c0 = ch * FF_CW, w = min(FF_CW, X - c0);
+        if (mine) {
+            if (ci == 0) s.init(f[(w - 1) * 32]);
+            float *ps = S + (size_t)(2 * c0 + sg) * YP + rg + r;
+            int j = w;
+            for (; j & 3; --j) st_hint(ps + (size_t)(2 * (j - 1)) * YP, s.step(f[(j - 1) * 32], c), pl);
+            const float *fn = f + max(j - 4, 0) * 32;
+            float4 v = make_float4(fn[96], fn[64], fn[32], fn[0]);
+#pragma unroll 2
+            for (j -= 4; j >= 0; j -= 4) {
+                const float4 x = v;
+                fn = f + max(j - 4, 0) * 32;
+                v = make_float4(fn[96], fn[64], fn[32], fn[0]);
+                const float4 y = steps4(s, c, x);
+                st_hint_4<0>(ps + (size_t)(2 * j) * YP, 2 * YP, y.w, y.z, y.y, y.x, pl);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+/* The warp's columns cg .. cg + 15 of a frame, from the slot, the DoG to dogz. */
+__device__ __forceinline__ void filter_cols(float *S, float *__restrict__ dogz, int X, int Y, int YP, int cg,
+                                            float *wsm, const Coef &c, uint64_t pf, uint64_t pl)
+{
+    const int lane = threadIdx.x & 31, col = lane & 15, sg = lane >> 4;
+    const int nq = (Y + FF_CW - 1) / FF_CW;
+    constexpr int TBUF = 2 * FF_R * FF_TS;
+    const int nc = min(FF_R, X - cg);
+    const bool mine = col < nc;
+    auto stage_t = [&](int q, float *buf) {
+        const int p = lane & 7;
+        for (int k = lane >> 3; k < 2 * nc; k += 4) /* k = 2 column + sigma */
+            cp_async16(buf + k * FF_TS + 4 * p, S + (size_t)(2 * cg + k) * YP + q * FF_CW + 4 * p, pl);
+    };
+    const int own = (2 * col + sg) * FF_TS;
+    Iir s;
+    s.init(0.0f);
+    /* ---- forward */
+    stage_t(0, wsm);
+    cp_commit();
+    for (int q = 0; q < nq; ++q) {
+        if (q + 1 < nq) stage_t(q + 1, wsm + ((q + 1) & 1) * TBUF);
+        cp_commit();
+        cp_wait_prev();
+        __syncwarp();
+        float *buf = wsm + (q & 1) * TBUF, *t = buf + own;
+        const int nr = min(FF_CW, Y - q * FF_CW);
+        if (mine) {
+            if (q == 0) s.init(t[0]);
+            int i = 0;
+            float4 v = *reinterpret_cast<const float4 *>(t);
+#pragma unroll 2
+            for (; i + 4 <= nr; i += 4) {
+                const float4 x = v;
+                v = *reinterpret_cast<const float4 *>(t + i + 4); /* (a column has FF_TS floats) */
+                *reinterpret_cast<float4 *>(t + i) = steps4(s, c, x);
+            }
+            for (; i < nr; ++i) t[i] = s.step(t[i], c);
+        }
+        __syncwarp();
+        {
+            const int p = lane & 7;
+            for (int k = lane >> 3; k < 2 * nc; k += 4)
+                st4_hint(S + (size_t)(2 * cg + k) * YP + q * FF_CW + 4 * p,
+                         *reinterpret_cast<const float4 *>(buf + k * FF_TS + 4 * p), pl);
+        }
+        __syncwarp(); /* buffer q & 1 is restaged for tile q + 2; the slot stores are seen */
+    }
+    /* ---- backward, DoG out: the whole warp takes the steps (a lane without a
+     * column repeats the last one's), because the halves exchange outputs */
+    const int rd = (2 * min(col, nc - 1) + sg) * FF_TS;
+    stage_t(nq - 1, wsm);
+    cp_commit();
+    for (int qi = 0; qi < nq; ++qi) {
+        const int q = nq - 1 - qi;
+        if (q > 0) stage_t(q - 1, wsm + ((qi + 1) & 1) * TBUF);
+        cp_commit();
+        cp_wait_prev();
+        __syncwarp();
+        const float *t = wsm + (qi & 1) * TBUF + rd;
+        const int nr = min(FF_CW, Y - q * FF_CW);
+        if (qi == 0) s.init(t[nr - 1]);
+        float *pd = dogz + (size_t)q * FF_CW * X + cg + col;
+        /* this lane's output and the other sigma's: sigma 1 minus sigma 2 */
+        auto diff = [&](float v) {
+            const float o = __shfl_xor_sync(0xffffffffu, v, 16);
+            return sg == 0 ? __fsub_rn(v, o) : __fsub_rn(o, v);
+        };
+        int i = nr;
+        for (; i & 3; --i) {
+            const float d = diff(s.step(t[i - 1], c));
+            if (mine && sg == 0) st_hint(pd + (size_t)(i - 1) * X, d, pf);
+        }
+        float4 v = *reinterpret_cast<const float4 *>(t + max(i - 4, 0));
+#pragma unroll 2
+        for (i -= 4; i >= 0; i -= 4) {
+            const float4 x = make_float4(v.w, v.z, v.y, v.x);
+            v = *reinterpret_cast<const float4 *>(t + max(i - 4, 0));
+            const float4 y = steps4(s, c, x);
+            /* rows i + 3, i + 2, i + 1, i: the halves store two of them each */
+            const float d3 = diff(y.x), d2 = diff(y.y), d1 = diff(y.z), d0 = diff(y.w);
+            if (mine) {
+                float *g = pd + (size_t)(i + sg) * X;
+                st_hint(g, sg == 0 ? d0 : d1, pf);
+                st_hint(g + 2 * (size_t)X, sg == 0 ? d2 : d3, pf);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+/* the coefficients of this lane's sigma */
+__device__ __forceinline__ Coef lane_coef(const Coef &a, const Coef &b)
+{
+    const bool first = (threadIdx.x & 16) == 0;
+    return Coef{first ? a.b0 : b.b0, first ? a.b1 : b.b1, first ? a.b2 : b.b2,   first ? a.b3 : b.b3,
+                first ? a.B : b.B,   first ? a.rb0 : b.rb0, first ? a.rb1 : b.rb1, first ? a.lo : b.lo, first ? a.hi : b.hi};
+}
+
+/* Both passes of whole frames, for stacks that give every SM a frame or
+ * nearly: a persistent CTA of 8 warps owns one frame at a time and one slot (two
+ * images, sigma 1 then sigma 2, column-major), a lane a row (column) with both
+ * sigmas' recurrences.  The grid's slots together stay within L2, so only the
+ * frames are read from DRAM and only the DoG is written.  findROI of 2000 frames
+ * of 256 x 256: 1.70 ms with the three-operation division, 1.68 with this. */
+constexpr int FW_T = 256; /* threads: rows of a row group / columns of a column group */
+/* per warp: the largest phase, two buffers of column tiles [sigma][32 columns][FF_TS] */
+constexpr int FW_FLOATS = 2 * 2 * 32 * FF_TS;
+constexpr int FW_SMEM_FLOATS = (FW_T / 32) * FW_FLOATS;
 
 struct IirState {
     float w1, w2, w3;
@@ -409,32 +516,34 @@ struct IirState {
         push(o);
         return o;
     }
-    /* one step, division through rb0; `slow` records a q outside [lo, hi] */
-    __device__ __forceinline__ float step_fast(float w0, const Coef &c, bool &slow)
+    /* one step, division through rb0 and rb1; q0 its numerator */
+    __device__ __forceinline__ float step_fast(float w0, const Coef &c, float &q0)
     {
-        const float q = iir_q(w1, w2, w3, c);
-        slow |= !(fabsf(q) >= c.lo && fabsf(q) <= c.hi);
-        const float o = __fmaf_rn(w0, c.B, div_fast(q, c.b0, c.rb0));
+        q0 = iir_q(w1, w2, w3, c);
+        const float o = __fmaf_rn(w0, c.B, div_fast(q0, c.rb0, c.rb1));
         push(o);
         return o;
     }
 };
 
 /* Four steps of both recurrences, inputs xa / xb to outputs ya / yb in
- * processing order.  A block in which any q left [lo, hi] is redone from
+ * processing order (steps4 for one recurrence).  A block in which any q left [lo, hi] is redone from
  * its saved state with IEEE division, so every output is the one iir_step
  * gives. */
-__device__ __forceinline__ void steps4(IirState &a, IirState &b, const Coef &ca, const Coef &cb,
+__device__ __forceinline__ void steps4x2(IirState &a, IirState &b, const Coef &ca, const Coef &cb,
                                        const float (&xa)[4], const float (&xb)[4], float (&ya)[4], float (&yb)[4])
 {
     const IirState a0 = a, b0 = b;
-    bool slow = false;
+    float mn = INFINITY, mx = 0.0f;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-        ya[u] = a.step_fast(xa[u], ca, slow);
-        yb[u] = b.step_fast(xb[u], cb, slow);
+        float qa, qb;
+        ya[u] = a.step_fast(xa[u], ca, qa);
+        yb[u] = b.step_fast(xb[u], cb, qb);
+        mn = min3(mn, fabsf(qa), fabsf(qb));
+        mx = max3(mx, fabsf(qa), fabsf(qb));
     }
-    if (slow) {
+    if (!(mn >= fmaxf(ca.lo, cb.lo) && mx <= fminf(ca.hi, cb.hi))) {
         a = a0;
         b = b0;
 #pragma unroll
@@ -447,7 +556,7 @@ __device__ __forceinline__ void steps4(IirState &a, IirState &b, const Coef &ca,
 
 /* F > 0: frames of F x F pixels (YP = F), the strides compile-time */
 template <bool VEC, int F>
-__global__ void __launch_bounds__(FF_T, 1) filter_kernel(const float *__restrict__ in, float *__restrict__ dog,
+__global__ void __launch_bounds__(FW_T, 1) filter_kernel(const float *__restrict__ in, float *__restrict__ dog,
                                                          float *__restrict__ scratch, int X_, int Y_, int Z, int YP_,
                                                          Coef ca, Coef cb)
 {
@@ -457,12 +566,12 @@ __global__ void __launch_bounds__(FF_T, 1) filter_kernel(const float *__restrict
     const uint64_t pf = l2_evict_first(), pl = l2_evict_last();
     const size_t img = (size_t)X * YP;
     float *FA = scratch + (size_t)blockIdx.x * 2 * img, *FB = FA + img;
-    float *wsm = fsm + warp * FF_WARP_FLOATS; /* this warp's chunks and tiles */
+    float *wsm = fsm + warp * FW_FLOATS; /* this warp's chunks and tiles */
     const int nch = (X + FF_CW - 1) / FF_CW, nq = (Y + FF_CW - 1) / FF_CW;
     for (int z = blockIdx.x; z < Z; z += gridDim.x) {
         const float *fin = in + (size_t)z * X * Y;
-        /* rows: the warp's 32 rows of each group of FF_T */
-        for (int rg = 32 * warp; rg < Y; rg += FF_T) {
+        /* rows: the warp's 32 rows of each group of FW_T */
+        for (int rg = 32 * warp; rg < Y; rg += FW_T) {
             const int nr = min(32, Y - rg), r = rg + lane;
             const bool mine = lane < nr;
             IirState a, b;
@@ -500,7 +609,7 @@ __global__ void __launch_bounds__(FF_T, 1) filter_kernel(const float *__restrict
                             const float4 v = *reinterpret_cast<const float4 *>(ti + j4);
                             const float x[4] = {v.x, v.y, v.z, v.w};
                             float ya[4], yb[4];
-                            steps4(a, b, ca, cb, x, x, ya, yb);
+                            steps4x2(a, b, ca, cb, x, x, ya, yb);
                             st_hint_4<F>(pa + (size_t)j4 * YP, YP, ya[0], ya[1], ya[2], ya[3], pl);
                             st_hint_4<F>(pb + (size_t)j4 * YP, YP, yb[0], yb[1], yb[2], yb[3], pl);
                         }
@@ -549,7 +658,7 @@ __global__ void __launch_bounds__(FF_T, 1) filter_kernel(const float *__restrict
                             const float xb[4] = {fb[(j4 + 3) * 32], fb[(j4 + 2) * 32], fb[(j4 + 1) * 32],
                                                  fb[j4 * 32]};
                             float ya[4], yb[4];
-                            steps4(a, b, ca, cb, xa, xb, ya, yb);
+                            steps4x2(a, b, ca, cb, xa, xb, ya, yb);
                             st_hint_4<F>(pa + (size_t)j4 * YP, YP, ya[3], ya[2], ya[1], ya[0], pl);
                             st_hint_4<F>(pb + (size_t)j4 * YP, YP, yb[3], yb[2], yb[1], yb[0], pl);
                         }
@@ -564,10 +673,10 @@ __global__ void __launch_bounds__(FF_T, 1) filter_kernel(const float *__restrict
             }
         }
         __syncthreads(); /* every row of the frame is in the slot */
-        /* columns: the warp's 32 columns of each group of FF_T, tiles
+        /* columns: the warp's 32 columns of each group of FW_T, tiles
          * [sigma][column][FF_TS] of FF_CW rows */
         constexpr int TBUF = 2 * 32 * FF_TS;
-        for (int cg = 32 * warp; cg < X; cg += FF_T) {
+        for (int cg = 32 * warp; cg < X; cg += FW_T) {
             const int nc = min(32, X - cg), col = cg + lane;
             const bool mine = lane < nc;
             auto stage_t = [&](int q, float *buf) {
@@ -602,7 +711,7 @@ __global__ void __launch_bounds__(FF_T, 1) filter_kernel(const float *__restrict
                             const float4 vb = *reinterpret_cast<const float4 *>(tb + i4);
                             const float xa[4] = {va.x, va.y, va.z, va.w}, xb[4] = {vb.x, vb.y, vb.z, vb.w};
                             float ya[4], yb[4];
-                            steps4(a, b, ca, cb, xa, xb, ya, yb);
+                            steps4x2(a, b, ca, cb, xa, xb, ya, yb);
                             *reinterpret_cast<float4 *>(ta + i4) = make_float4(ya[0], ya[1], ya[2], ya[3]);
                             *reinterpret_cast<float4 *>(tb + i4) = make_float4(yb[0], yb[1], yb[2], yb[3]);
                         }
@@ -648,7 +757,7 @@ __global__ void __launch_bounds__(FF_T, 1) filter_kernel(const float *__restrict
                             const float4 vb = *reinterpret_cast<const float4 *>(tb + i4);
                             const float xa[4] = {va.w, va.z, va.y, va.x}, xb[4] = {vb.w, vb.z, vb.y, vb.x};
                             float ya[4], yb[4];
-                            steps4(a, b, ca, cb, xa, xb, ya, yb);
+                            steps4x2(a, b, ca, cb, xa, xb, ya, yb);
                             st_hint_4<F>(pd + (size_t)i4 * X, X, __fsub_rn(ya[3], yb[3]), __fsub_rn(ya[2], yb[2]),
                                          __fsub_rn(ya[1], yb[1]), __fsub_rn(ya[0], yb[0]), pf);
                         }
@@ -662,11 +771,32 @@ __global__ void __launch_bounds__(FF_T, 1) filter_kernel(const float *__restrict
         }
         __syncthreads(); /* every read of the slot is done */
         /* the frame's slot is dead: drop its lines without writing them back */
-        for (size_t off = (size_t)threadIdx.x * 32; off < 2 * img; off += (size_t)FF_T * 32) discard_line(FA + off);
+        for (size_t off = (size_t)threadIdx.x * 32; off < 2 * img; off += (size_t)FW_T * 32) discard_line(FA + off);
         __syncthreads();
     }
 }
 
+
+/* The passes as two kernels, for few frames (a CTA per frame would leave SMs
+ * without work) and for frames too large for a slot in L2: one warp per CTA
+ * runs a row group (column group) of a frame, a slot per frame. */
+template <bool VEC>
+__global__ void __launch_bounds__(32) filter_rows_kernel(const float *__restrict__ in, float *__restrict__ scratch,
+                                                         int X, int Y, int YP, Coef ca, Coef cb)
+{
+    extern __shared__ __align__(16) float fsm[];
+    float *S = scratch + (size_t)blockIdx.y * 2 * X * YP;
+    filter_rows<VEC>(in + (size_t)blockIdx.y * X * Y, S, X, Y, YP, FF_R * blockIdx.x, fsm, lane_coef(ca, cb),
+                        l2_evict_first(), l2_evict_last());
+}
+__global__ void __launch_bounds__(32) filter_cols_kernel(float *__restrict__ dog, float *__restrict__ scratch, int X,
+                                                         int Y, int YP, Coef ca, Coef cb)
+{
+    extern __shared__ __align__(16) float fsm[];
+    float *S = scratch + (size_t)blockIdx.y * 2 * X * YP;
+    filter_cols(S, dog + (size_t)blockIdx.y * X * Y, X, Y, YP, FF_R * blockIdx.x, fsm, lane_coef(ca, cb),
+                   l2_evict_first(), l2_evict_last());
+}
 
 /* Passes 3 and 4, fused: kernel_maxX (window max along rows with floor
  * minval, +max / -max) then kernel_maxY (window max of |.| along columns,
@@ -1346,10 +1476,7 @@ namespace {
  * the frames are first copied from there in chunks of chunk_frames on the
  * workspace's copy stream, and each chunk's filters start on `s` as soon as
  * its copy has landed (the filters are frame-local, so a chunk is filtered
- * exactly as inside the whole stack).  Frames whose two intermediate images
- * fit a slot take the fused filter (one slot per CTA, one CTA per SM, the
- * slots in ws->b); larger frames take rows_kernel + cols_kernel (the second
- * image in ws->b).  after_chunk, when given, is called with the number of
+ * exactly as inside the whole stack).  The slots are in ws->b.  after_chunk, when given, is called with the number of
  * frames filtered so far after each chunk's launches. */
 bamf_status run_filter(bamf_findroi_ws *ws, const float *host_frames, int chunk_frames, const float *frames,
                        int KX, int KY, int zsize, double sigma1, double sigma2, float *dog, cudaStream_t s,
@@ -1360,15 +1487,25 @@ bamf_status run_filter(bamf_findroi_ws *ws, const float *host_frames, int chunk_
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int step = host_frames ? std::max(1, chunk_frames) : zsize;
-    const int64_t plane = (int64_t)KX * KY, n = plane * zsize;
+    const int64_t plane = (int64_t)KX * KY;
     const int YP = (KY + FF_CW - 1) / FF_CW * FF_CW;
-    const bool fused = (size_t)KX * YP <= FF_MAX_SLOT;
+    const size_t slot_bytes = (size_t)2 * KX * YP * sizeof(float);
+    /* a CTA per frame (filter_kernel) once half the SMs get one (findROI of 90
+     * frames of 256 x 256: 242 us); else (60 frames: 211 us against 221, one 250 x
+     * 190 frame 172 against 199, five 400 x 400 frames 212 against 381), and for
+     * frames whose slots would not stay in L2 one per SM, a warp per CTA, on
+     * as many frames at a time as FF_SPLIT_BYTES of slots hold, and at least
+     * as many as give every SM eight warps (600 frames of 320 x 320: 1.11 ms; 1.45
+     * as one launch over the stack with IEEE divisions) */
+    const bool fused = (size_t)KX * YP <= FF_MAX_SLOT && 2 * std::min(step, zsize) >= sms;
     const int ff_grid = std::min(step, sms);
-    const size_t b_bytes = fused ? (size_t)ff_grid * 2 * KX * YP * sizeof(float) : n * sizeof(float);
-    if (!ws->b.ensure(b_bytes)) return BAMF_ERR_CUDA;
+    const int groups = (std::min(KX, KY) + FF_R - 1) / FF_R;
+    const int per = std::min(std::min(step, 65535),
+                             std::max((int)(FF_SPLIT_BYTES / slot_bytes), (8 * sms + groups - 1) / groups));
+    if (!ws->b.ensure(slot_bytes * (size_t)(fused ? ff_grid : std::min(per, zsize)))) return BAMF_ERR_CUDA;
     float *Bb = (float *)ws->b.p;
     const bool vec = KX % 4 == 0 && (reinterpret_cast<uintptr_t>(frames) & 15) == 0;
-    const size_t ff_smem = (size_t)FF_SMEM_FLOATS * sizeof(float);
+    const size_t ff_smem = (size_t)FW_SMEM_FLOATS * sizeof(float);
     /* 256 x 256 frames (the common camera region) have their own build */
     auto ff = vec ? (KX == 256 && KY == 256 ? filter_kernel<true, 256> : filter_kernel<true, 0>)
                   : filter_kernel<false, 0>;
@@ -1395,14 +1532,16 @@ bamf_status run_filter(bamf_findroi_ws *ws, const float *host_frames, int chunk_
         }
         if (fused) {
             const unsigned grid = (unsigned)std::min(zc, ff_grid);
-            ff<<<grid, FF_T, ff_smem, s>>>(frames + off, dog + off, Bb, KX, KY, zc, YP, ca, cb);
+            ff<<<grid, FW_T, ff_smem, s>>>(frames + off, dog + off, Bb, KX, KY, zc, YP, ca, cb);
         } else {
-            const int64_t nrows = (int64_t)KY * zc, ncols = (int64_t)KX * zc;
-            const int64_t groups = (nrows + 31) / 32;
-            const unsigned grid = (unsigned)std::max<int64_t>(
-                1, std::min<int64_t>((groups + ROWS_WARPS - 1) / ROWS_WARPS, (int64_t)sms * ROWS_CTAS_PER_SM));
-            rows_kernel<<<grid, 32 * ROWS_WARPS, 0, s>>>(frames + off, dog + off, Bb + off, KX, KY, zc, ca, cb);
-            cols_kernel<<<(unsigned)((ncols + 127) / 128), 128, 0, s>>>(dog + off, Bb + off, KX, KY, zc, ca, cb);
+            constexpr size_t smem = FF_WARP_FLOATS * sizeof(float);
+            for (int f0 = 0; f0 < zc; f0 += per) {
+                const unsigned fr = (unsigned)std::min(per, zc - f0);
+                const int64_t o = off + f0 * plane;
+                (vec ? filter_rows_kernel<true> : filter_rows_kernel<false>)<<<dim3((KY + FF_R - 1) / FF_R, fr), 32, smem, s>>>(
+                    frames + o, Bb, KX, KY, YP, ca, cb);
+                filter_cols_kernel<<<dim3((KX + FF_R - 1) / FF_R, fr), 32, smem, s>>>(dog + o, Bb, KX, KY, YP, ca, cb);
+            }
         }
         if (after_chunk) {
             const bamf_status r = (*after_chunk)(z0 + zc);
@@ -1589,7 +1728,7 @@ __global__ void division_check_kernel(Coef c, unsigned long long *bad_in_range, 
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (1ull << 32); i += stride) {
         const float q = __uint_as_float((unsigned)i);
-        const float want = __fdiv_rn(q, c.b0), got = div_fast(q, c.b0, c.rb0);
+        const float want = __fdiv_rn(q, c.b0), got = div_fast(q, c.rb0, c.rb1);
         if (__float_as_uint(want) != __float_as_uint(got) && !(isnan(want) && isnan(got))) {
             ++n_all;
             if (fabsf(q) >= c.lo && fabsf(q) <= c.hi) ++n_in;

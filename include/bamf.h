@@ -612,8 +612,8 @@ bamf_status bamf_find_roi_dog_device(bamf_findroi_ws *ws, const float *frames, i
                                      int zsize, double sigma1, double sigma2, float *dog, void *stream);
 
 /* The filters divide by the recurrence constant b0 with one multiply and
- * two FMAs through RN(1/b0) (Markstein's method) where |q| lies in
- * [2^-100, 2^100], after the host has checked, once per b0, that this equals
+ * one FMA through 1/b0 held in two floats (Brisebarre and Muller's method)
+ * where |q| lies in about [2^-91, 2^100], after the host has checked, once per b0, that this equals
  * IEEE division over the 2^23 significands of [1, 2) (the method is
  * scale-invariant on that range); elsewhere, and for a b0 that fails the
  * check, they use IEEE division.  For the b0 of filter width `sigma`:
