@@ -294,7 +294,7 @@ extern "C" bamf_status bamf_rjmcmc_batch_device_noalloc(const bamf_roi_batch *ro
         Bc.side_max = std::min(class_side(c), side_max);
         int wpb = 4, mc = 2;
         int per_sm = exact ? blocks_per_sm_exact(Bc.side_max, wpb, K.opt_model)
-                           : best_fast_shape(Bc.side_max, K.opt_model, &wpb, &mc);
+                           : best_fast_shape(Bc.side_max, K.opt_model, n, sms, &wpb, &mc);
         if (per_sm < 1) return BAMF_ERR_TOO_LARGE;
         int blocks = std::min((n + wpb - 1) / wpb, per_sm * sms);
         cudaError_t e = exact ? launch_rjmcmc_exact(K, Bc, Bc.side_max, blocks, wpb, s)

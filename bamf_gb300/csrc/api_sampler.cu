@@ -301,7 +301,7 @@ static bamf_status launch_batch(bamf_workspace *ws, const SamplerConsts &K, Samp
          * schedulers twice; beyond, a warp per chain keeps more chains going). */
         const bool team = exact && K.opt_model == 0 && B.n_rois <= 2 * sms;
         if (exact) wpb = pick_wpb_exact(Bc.side_max, B.n_rois <= 4 * sms, K.opt_model, &per_sm);
-        else per_sm = best_fast_shape(Bc.side_max, K.opt_model, &wpb, &mc);
+        else per_sm = best_fast_shape(Bc.side_max, K.opt_model, B.n_rois, sms, &wpb, &mc);
         if (per_sm < 1) return BAMF_ERR_TOO_LARGE;
         const int tw = ws->tuned_wpb[exact ? 0 : 1][c], tm = exact ? 0 : ws->tuned_min_ctas[c];
         if (tw > 0 && !team) {

@@ -46,8 +46,37 @@ int blocks_per_sm_fast(int side_max, int warps_per_block, int min_ctas, int opt_
                           : occupancy_fast_gauss(smem, 32 * warps_per_block, min_ctas);
 }
 
-int best_fast_shape(int side_max, int opt_model, int *warps_per_block, int *min_ctas)
+/* A batch of n ROIs with w chains resident per SM, in units of a round of 16:
+ * the first round costs `a` (it holds the brightest ROIs), later ones 0.77 a, a
+ * last one that is not full 0.25 a more; less than one round costs between 0.68
+ * and 1 of it.  Fitted to batches of 2,400 to 10,000 ROIs of 8, 16 and 24 px:
+ * within 8%. */
+static float batch_cost(int n, int sms, int w, float a)
 {
+    const float x = (float)n / (float)(w * sms);
+    if (x <= 1.0f) return a * (0.68f + 0.32f * x);
+    const float frac = x - floorf(x);
+    return a * (1.0f + 0.77f * (x - 1.0f) + (frac > 0.02f ? 0.25f : 0.0f));
+}
+
+int best_fast_shape(int side_max, int opt_model, int n_rois, int sms, int *warps_per_block, int *min_ctas)
+{
+    /* A batch that one CTA per SM can hold: the fewest chains per CTA that do,
+     * on the register budget without spills.  Chains of a CTA wait for each
+     * other at every jump, and an SM's instruction cache serves one or a few
+     * move streams either way (500 + 500 jumps of uneven ROIs, us, with 1 / 2 / 4 /
+     * 8 chains per CTA against the shapes with the most resident chains: 64
+     * ROIs 4759 / 5076 / 5468 / 6000 against 7006, 300 ROIs 5606 / 5347 / 5703 /
+     * 6213 against 7753, 1216 ROIs 10827 / 9254 / 7530 / 6716 against 8772). */
+    for (int w = 1; w <= 8; w *= 2)
+        if (n_rois <= w * sms) {
+            const int per = blocks_per_sm_fast(side_max, w, 2, opt_model);
+            if (per > 0) {
+                *warps_per_block = w;
+                *min_ctas = 2;
+                return per;
+            }
+        }
     int best_w = 0, best_wpb = 8, best_mc = 2, best_per = 0;
     const int cand[3] = {8, 4, 2};
     for (int mc = 2; mc <= 3; ++mc)
@@ -70,6 +99,18 @@ int best_fast_shape(int side_max, int opt_model, int *warps_per_block, int *min_
             best_mc = 1;
             best_per = per;
         }
+    }
+    /* Two CTAs of 8 on the larger register budget run a round in 1 / 1.42 of the
+     * time of three on the smaller (8 to 12 px, one CTA of 24: 1 / 1.25), so which
+     * is faster depends on how full the last round is (16 px, 250 + 250 jumps:
+     * 2432 ROIs 3260 us against 3922, 3380: 5250 against 4636, 5000: 6422 against
+     * 7219, 7300: 8285 against 8224; uneven sides, 10,000: 11.6 ms against 12.5). */
+    const int per2 = blocks_per_sm_fast(side_max, 8, 2, opt_model);
+    if (per2 * 8 >= 16 && best_w > per2 * 8 &&
+        batch_cost(n_rois, sms, per2 * 8, 1.0f) < batch_cost(n_rois, sms, best_w, best_mc == 1 ? 1.25f : 1.42f)) {
+        best_wpb = 8;
+        best_mc = 2;
+        best_per = per2;
     }
     *warps_per_block = best_wpb;
     *min_ctas = best_mc;

@@ -25,10 +25,13 @@ cudaError_t launch_rjmcmc_exact_team(const SamplerConsts &K, const SamplerBatch 
                                      cudaStream_t stream);
 int blocks_per_sm_exact(int side_max, int warps_per_block, int opt_model);
 
-/* the CTA shape with the most resident chains per SM for a fast launch
- * (ties: the larger register budget per thread, then more chains per CTA;
- * up to side 12, a whole move-stream group per CTA when it keeps as many) */
-int best_fast_shape(int side_max, int opt_model, int *warps_per_block, int *min_ctas);
+/* the CTA shape for a fast launch of a batch of n_rois: few ROIs, one CTA per
+ * SM; else the shape with the most resident chains per SM (ties: the larger
+ * register budget per thread, then more chains per CTA; up to side 12, a whole
+ * move-stream group per CTA when it keeps as many) or two CTAs of 8, whichever
+ * takes the batch's rounds of resident chains faster.  Returns the CTAs per SM,
+ * 0 when none fits. */
+int best_fast_shape(int side_max, int opt_model, int n_rois, int sms, int *warps_per_block, int *min_ctas);
 
 /* per translation unit */
 cudaError_t launch_fast_gauss(const SamplerConsts &K, const SamplerBatch &B, size_t smem, int blocks, int threads,
