@@ -16,7 +16,9 @@
  *     broadcasts are needed and the warp never diverges there;
  *   - uniforms come from the chain's Philox stream (include/bamf_philox.h):
  *     each lane generates one 4-word block, 32 blocks = 128 uniforms per
- *     refill, and a draw is one shuffle.
+ *     refill, kept as floats in shared memory; a draw is one broadcast load.
+ *   - what is the same on every lane anyway is done for two or three arguments
+ *     at once, one per part of the warp: Irwin-Hall draws, prior lookups.
  *
  * Two instantiations (template parameter EXACT):
  *   EXACT = true  (sampler_exact.cu, built with -fmad=false): the reference's
@@ -76,24 +78,25 @@ struct SMath<false> {
  * proposal model Mt, per-pixel work E, sCMOS (each rounded up to 16 bytes,
  * for the vector loads of the serial sums), a pool of 2 x 32 stencil rows
  * NX/NY shared by A and T, 128 buffered uniforms.
- * Fast: D, M, Mt and the compact stencil rows SXo/SYo (old, of A) and
- * SXn/SYn (new, of T); log2 M is recomputed in each likelihood pass (the
+ * Fast: D, M, Mt, the compact stencil rows SXo/SYo (old, of A) and SXn/SYn (new,
+ * of T), the buffered uniforms and the shared draws of the next jumps; log2 M is recomputed in each likelihood pass (the
  * SFU has room; the smaller carve-out keeps 3 CTAs of 8 chains resident
  * up to 24x24 ROIs); sCMOS is read from global memory at model rebuilds
- * only.  Both: counters and the neighbour pick list. */
+ * only.  Both: the neighbour pick list. */
 /* Fast mode keeps stencil rows only for the emitters a proposal changes:
  * up to FAST_ROWS old rows (A) and FAST_ROWS new rows (T); larger proposals
  * (rare: a jump of a cluster of more than 4 emitters) and periodic rebuilds
  * stream the model one emitter at a time. */
 #define FAST_ROWS 4
 #define EXACT_ROWS (2 * BAMF_NMAX) /* stencil rows of the exact sampler's pool */
-#define EXACT_UBUF 128
+#define UBUF 128      /* buffered uniforms */
+#define MOVE_AHEAD 32 /* jumps whose shared move draws are formed together (fast) */
 __host__ __device__ inline int exact_npix(int side_max) { return (side_max * side_max + 3) & ~3; }
 __host__ __device__ inline int warp_smem_floats(int side_max, bool exact)
 {
     int npix = side_max * side_max, nxs = BAMF_NMAX * side_max;
-    return exact ? 5 * exact_npix(side_max) + 4 * nxs + EXACT_UBUF + C_COUNT + BAMF_NMAX + 2
-                 : 3 * npix + 4 * FAST_ROWS * side_max + C_COUNT + BAMF_NMAX + 2; /* D M Mt SXo SYo SXn SYn */
+    return exact ? 5 * exact_npix(side_max) + 4 * nxs + UBUF + BAMF_NMAX + 2 + 2
+                 : (3 * npix + 4 * FAST_ROWS * side_max + 3 & ~3) + UBUF + 2 * MOVE_AHEAD + BAMF_NMAX;
 }
 
 /* double helpers that nvcc may not contract */
@@ -197,27 +200,19 @@ static __device__ __noinline__ float stat_rand(const float *__restrict__ ux, con
     return (__ldg(&ux[hi - 1]) * (uc1 - R) + __ldg(&ux[hi]) * (R - uc0)) / (uc1 - uc0);
 }
 
-/* Fast-mode Irwin-Hall draw: lanes 0..11 fetch uniforms idx..idx+11 of the
- * warp's buffered Philox blocks (lane l holds block base+l in r0..r3) and
- * add them in a butterfly.  Call with the whole warp and the 12 draws inside
- * the buffer. */
-static __device__ __noinline__ float irwin_hall12(uint32_t idx, uint32_t base, uint32_t r0, uint32_t r1,
-                                           uint32_t r2, uint32_t r3, int lane)
+/* Fast-mode Irwin-Hall draws: the 12 uniforms from u (the warp's buffer) on
+ * lanes 0..11 of each half of the warp, added in a butterfly; STEP = 12 gives
+ * the upper half the next twelve, so that a warp makes two draws at once.  Call
+ * with the whole warp. */
+template <int STEP>
+static __device__ __noinline__ float irwin_hall12(const float *u, int lane)
 {
-    uint32_t my = idx + (uint32_t)(lane & 15);
-    int src = (int)((my >> 2) - base) & 31;
-    uint32_t v0 = __shfl_sync(0xffffffffu, r0, src);
-    uint32_t v1 = __shfl_sync(0xffffffffu, r1, src);
-    uint32_t v2 = __shfl_sync(0xffffffffu, r2, src);
-    uint32_t v3 = __shfl_sync(0xffffffffu, r3, src);
-    uint32_t c = my & 3u;
-    uint32_t v = c == 0 ? v0 : (c == 1 ? v1 : (c == 2 ? v2 : v3));
-    float u = (lane & 15) < 12 ? bamf_u31_to_float(v >> 1) : 0.0f;
-    u += __shfl_xor_sync(0xffffffffu, u, 1);
-    u += __shfl_xor_sync(0xffffffffu, u, 2);
-    u += __shfl_xor_sync(0xffffffffu, u, 4);
-    u += __shfl_xor_sync(0xffffffffu, u, 8);
-    return u - 6.0f;
+    float v = (lane & 15) < 12 ? u[(lane & 15) + STEP * (lane >> 4)] : 0.0f;
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    return v - 6.0f;
 }
 
 /* Uniform in [0, 1) shared by the warps of a CTA in move-synchronous mode:
@@ -311,14 +306,16 @@ struct ChainWarp {
      * the row of this lane's emitter of A / of T (an emitter T left unchanged
      * keeps A's row; -1: changed or new, not evaluated yet) */
     int arow, trow;
-    float *ubuf; /* exact mode: uniforms base * 4 .. base * 4 + 127 */
+    float *ubuf; /* uniforms base * 4 .. base * 4 + 127 of the stream */
+    float *ahead; /* fast mode: the shared draws of MOVE_AHEAD jumps: move, then sub-branch */
     float *SXo, *SYo, *SXn, *SYn; /* fast mode: compact stencil rows */
     const float *scm; /* sCMOS: shared memory (exact) or global/null (fast) */
     /* sampled PSF (OptModel 1): [P0 y][P1 x][P2 y-sub][P3 x-sub], y fastest;
      * null for the Gaussian model */
     const float *psf;
     int pn0, pn01, pn012, ptot, pos;
-    int *cnt, *cl;
+    int cnt; /* lane k: counter k */
+    int *cl;
     int rec_n[2];
     /* current state A (lane j = slot j) */
     int an;
@@ -333,8 +330,7 @@ struct ChainWarp {
     bool t_overflow;
     /* uniform stream */
     uint32_t seed, chain, base;
-    uint32_t idx;            /* exact mode: next uniform of ubuf, else of the stream */
-    uint32_t r0, r1, r2, r3; /* fast mode: this lane's block of the buffer */
+    uint32_t idx; /* next uniform of ubuf */
     /* phase */
     int is_burnin;
     float P[8];
@@ -352,87 +348,69 @@ struct ChainWarp {
     /* ---------------------------------------------------------- RNG */
     __device__ __forceinline__ void refill()
     {
-        if (EXACT) {
-            /* block numbers wrap where a 32-bit stream index wraps */
-            const uint4 b = philox_block((base + (uint32_t)lane) & 0x3fffffffu, seed, chain);
-            __syncwarp();
-            reinterpret_cast<float4 *>(ubuf)[lane] =
-                make_float4(bamf_u31_to_float(b.x >> 1), bamf_u31_to_float(b.y >> 1), bamf_u31_to_float(b.z >> 1),
-                            bamf_u31_to_float(b.w >> 1));
-            __syncwarp();
-            return;
+        /* block numbers wrap where a 32-bit stream index wraps */
+        const uint4 b = philox_block((base + (uint32_t)lane) & 0x3fffffffu, seed, chain);
+        __syncwarp();
+        reinterpret_cast<float4 *>(ubuf)[lane] =
+            make_float4(bamf_u31_to_float(b.x >> 1), bamf_u31_to_float(b.y >> 1), bamf_u31_to_float(b.z >> 1),
+                        bamf_u31_to_float(b.w >> 1));
+        __syncwarp();
+    }
+    /* the next n uniforms into the buffer (n <= 36): it then starts at the block
+     * of the next one */
+    __device__ __forceinline__ void ensure(uint32_t n)
+    {
+        if (idx + n > (uint32_t)UBUF) {
+            base += idx >> 2;
+            idx &= 3u;
+            refill();
         }
-        uint4 b = philox_block(base + (uint32_t)lane, seed, chain);
-        r0 = b.x; r1 = b.y; r2 = b.z; r3 = b.w;
     }
     __device__ __forceinline__ float urand()
     {
-        if (EXACT) {
-            if (idx >= (uint32_t)EXACT_UBUF) {
-                base += EXACT_UBUF / 4;
-                idx = 0u;
-                refill();
-            }
-            return ubuf[idx++];
-        }
-        uint32_t blk = idx >> 2;
-        if (blk - base >= 32u) {
-            base = blk;
-            refill();
-        }
-        uint32_t c = idx & 3u;
-        uint32_t v = c == 0 ? r0 : (c == 1 ? r1 : (c == 2 ? r2 : r3));
-        v = __shfl_sync(BAMF_FULL, v, (int)(blk - base));
-        idx++;
-        return bamf_u31_to_float(v >> 1);
+        ensure(1u);
+        return ubuf[idx++];
     }
     /* Irwin-Hall sum of 12 uniforms (LibRJMCMCreturn.hpp:23-26).  Exact
-     * mode adds them in draw order; fast mode has lanes 0..11 fetch the 12
-     * draws at once and adds them in a butterfly (same distribution, other
-     * rounding). */
+     * mode adds them in draw order; fast mode in a butterfly over 12 lanes
+     * (same distribution, other rounding). */
     __device__ __forceinline__ float randn()
     {
+        ensure(12u);
+        float t = 0;
         if (EXACT) {
-            float t = 0;
-            if (idx + 12u <= (uint32_t)EXACT_UBUF) { /* all twelve buffered: loads in flight together */
-                const float *u = ubuf + idx;
+            const float *u = ubuf + idx;
 #pragma unroll
-                for (int k = 0; k < 12; ++k) t = t + u[k];
-                idx += 12u;
-            } else {
-#pragma unroll 1
-                for (int k = 0; k < 12; ++k) t = t + urand();
-            }
-            return t - 6.0f;
+            for (int k = 0; k < 12; ++k) t = t + u[k];
+            t = t - 6.0f;
+        } else {
+            t = irwin_hall12<0>(ubuf + idx, lane);
         }
-        if (((idx + 11u) >> 2) - base >= 32u) {
-            base = idx >> 2;
-            refill();
-        }
-        float u = irwin_hall12(idx, base, r0, r1, r2, r3, lane);
         idx += 12u;
-        return u;
+        return t;
     }
 
-    /* Three consecutive randn().  Exact mode:
-     * lane k adds the k-th draw's twelve uniforms, in draw order. */
+    /* Three consecutive randn().  Exact mode: lane k adds the k-th draw's twelve
+     * uniforms, in draw order.  Fast mode: two at once in the warp's halves. */
     __device__ __forceinline__ void randn3(float &a, float &b, float &c)
     {
-        if (EXACT && idx + 36u <= (uint32_t)EXACT_UBUF) {
+        ensure(36u);
+        if (EXACT) {
             const float *u = ubuf + idx + 12 * min(lane, 2);
             float t = 0;
 #pragma unroll
             for (int k = 0; k < 12; ++k) t = t + u[k];
             t = t - 6.0f;
-            idx += 36u;
             a = __shfl_sync(BAMF_FULL, t, 0);
             b = __shfl_sync(BAMF_FULL, t, 1);
             c = __shfl_sync(BAMF_FULL, t, 2);
         } else {
-            a = randn();
-            b = randn();
-            c = randn();
+            const float t = irwin_hall12<12>(ubuf + idx, lane);
+            a = __shfl_sync(BAMF_FULL, t, 0);
+            b = __shfl_sync(BAMF_FULL, t, 16);
+            c = irwin_hall12<0>(ubuf + idx + 24, lane);
         }
+        idx += 36u;
     }
 
     /* ------------------------------------------------------ lane access */
@@ -501,7 +479,7 @@ struct ChainWarp {
     }
     __device__ __forceinline__ void cinc(int k)
     {
-        if (lane == 0) cnt[k]++;
+        if (lane == k) cnt++;
     }
 
     /* Emitters::test (:492-514) with Bnd_out cast to int. */
@@ -529,14 +507,9 @@ struct ChainWarp {
     /* findPDF of two intensities at once: one in each half of the warp */
     __device__ __forceinline__ void findPDF2(const DevStat &s, float I0, float I1, float &p0, float &p1) const
     {
-        if (EXACT) {
-            const float v = stat_pdf(s.x, s.pdf, s.L, lane < 16 ? I0 : I1);
-            p0 = __shfl_sync(BAMF_FULL, v, 0);
-            p1 = __shfl_sync(BAMF_FULL, v, 16);
-        } else {
-            p0 = findPDF(s, I0);
-            p1 = findPDF(s, I1);
-        }
+        const float v = findPDF(s, lane < 16 ? I0 : I1);
+        p0 = __shfl_sync(BAMF_FULL, v, 0);
+        p1 = __shfl_sync(BAMF_FULL, v, 16);
     }
     __device__ __forceinline__ float genRand(const DevStat &s)
     {
@@ -553,6 +526,10 @@ struct ChainWarp {
     {
         return normpdf_f<EXACT>(x, u, s);
     }
+
+    /* a / b for 0 <= a <= 32, 1 <= b <= 64 (fast mode): (a + 1/2) / b is at least
+     * 1/128 from an integer, far more than the reciprocal's error */
+    static __device__ __forceinline__ int small_div(int a, float rb) { return (int)(((float)a + 0.5f) * rb); }
 
     /* ------------------------------------------------ neighbour search */
     __device__ __forceinline__ uint32_t near_mask(int jj, float dmin) const
@@ -874,8 +851,9 @@ struct ChainWarp {
         const int XY = X + Y, nr = na + nt;
         /* G rows per 32-lane pass when a row (X + Y entries) fits in 32
          * lanes, else one row at a time over ceil(XY / 32) passes */
-        const int G = XY <= 32 ? 32 / XY : 1;
-        const int rg = XY <= 32 ? lane / XY : 0;
+        const float rXY = __frcp_rn((float)XY);
+        const int G = XY <= 32 ? small_div(32, rXY) : 1;
+        const int rg = XY <= 32 ? small_div(lane, rXY) : 0;
         const int c0 = XY <= 32 ? lane - rg * XY : lane;
 #pragma unroll 1
         for (int r0 = 0; r0 < nr; r0 += G) {
@@ -1163,7 +1141,8 @@ struct ChainWarp {
                      * -SYo, new with +SYn); each lane holds its first four
                      * weights in registers. */
                     const int h = y1 - y0 + 1;
-                    const int yl = y0 + lane % h, xo = lane / h, R = 32 / h;
+                    const float rh = __frcp_rn((float)h);
+                    const int xo = small_div(lane, rh), yl = y0 + lane - xo * h, R = small_div(32, rh);
                     float w[4];
                     const float *sx[4];
 #pragma unroll
@@ -1213,7 +1192,9 @@ struct ChainWarp {
     {
         const int x0 = llr_box & 255, x1 = (llr_box >> 8) & 255, y0 = (llr_box >> 16) & 255, y1 = llr_box >> 24;
         if (x0 <= x1) {
-            const int h = y1 - y0 + 1, R = 32 / h, yy = y0 + lane % h, xo = lane / h;
+            const int h = y1 - y0 + 1;
+            const float rh = __frcp_rn((float)h);
+            const int xo = small_div(lane, rh), yy = y0 + lane - xo * h, R = small_div(32, rh);
             if (xo < R) {
 #pragma unroll 1
                 for (int xx = x0 + xo; xx <= x1; xx += R) M[yy + Y * xx] = Mt[yy + Y * xx];
@@ -2215,8 +2196,15 @@ struct ChainWarp {
                 for (int k = 0; k < 8; ++k) P[k] = is_burnin ? p.P_Burnin[k] : Pt[k];
             }
             if (!active) continue;
-            float t = shared_uniform(K->seed, grp, (uint32_t)n, 0u);
-            shared_ub = shared_uniform(K->seed, grp, (uint32_t)n, 1u);
+            /* the next jumps' shared draws, a lane each */
+            if ((n & (MOVE_AHEAD - 1)) == 0) {
+                __syncwarp();
+                ahead[lane] = shared_uniform(K->seed, grp, (uint32_t)(n + lane), 0u);
+                ahead[MOVE_AHEAD + lane] = shared_uniform(K->seed, grp, (uint32_t)(n + lane), 1u);
+                __syncwarp();
+            }
+            const float t = ahead[n & (MOVE_AHEAD - 1)];
+            shared_ub = ahead[MOVE_AHEAD + (n & (MOVE_AHEAD - 1))];
             step(K->PVB, is_burnin ? K->PVB : K->PVT, t);
             if (++since_rebuild == 512) {
                 rebuild_model();
@@ -2279,19 +2267,21 @@ __device__ __forceinline__ bool begin_roi(ChainWarp<EXACT, NUM, TEAM> &w, const 
         w.NY = w.NX + EXACT_ROWS * Bt.side_max;
         w.ubuf = w.NY + EXACT_ROWS * Bt.side_max;
         w.SXo = w.SYo = w.SXn = w.SYn = nullptr;
-        w.cnt = (int *)(w.ubuf + EXACT_UBUF);
+        w.cl = (int *)(w.ubuf + UBUF);
+        w.ahead = nullptr;
         w.arow = w.trow = -1;
     } else {
         const int rs = FAST_ROWS * Bt.side_max;
         w.E = nullptr;
-        w.NX = w.NY = w.ubuf = nullptr;
+        w.NX = w.NY = nullptr;
         w.SXo = sw + 3 * npix_max;
         w.SYo = w.SXo + rs;
         w.SXn = w.SYo + rs;
         w.SYn = w.SXn + rs;
-        w.cnt = (int *)(w.SYn + rs);
+        w.ubuf = sw + ((3 * npix_max + 4 * rs + 3) & ~3);
+        w.ahead = w.ubuf + UBUF;
+        w.cl = (int *)(w.ahead + 2 * MOVE_AHEAD);
     }
-    w.cl = w.cnt + C_COUNT;
     int n0 = Bt.init_n ? Bt.init_n[roi] : 0;
     bool ok = X >= 1 && Y >= 1 && X <= Bt.side_max && Y <= Bt.side_max && n0 <= BAMF_NMAX;
     if (!ok) {
@@ -2305,11 +2295,11 @@ __device__ __forceinline__ bool begin_roi(ChainWarp<EXACT, NUM, TEAM> &w, const 
         if (EXACT) scm_smem[p] = scm_src ? scm_src[p] : 0.0f;
     }
     w.scm = EXACT ? scm_smem : scm_src;
-    if (lane < C_COUNT) {
-        int k = lane;
-        bool isN = (k <= C_N_death) || (k >= C_N_jumpFg && k <= C_N_deathFg) ||
-                   (k >= C_N_jumpBg && k <= C_N_deathBg);
-        w.cnt[k] = isN ? 1 : 0;
+    {
+        const int k = lane;
+        const bool isN = (k <= C_N_death) || (k >= C_N_jumpFg && k <= C_N_deathFg) ||
+                         (k >= C_N_jumpBg && k <= C_N_deathBg);
+        w.cnt = isN ? 1 : 0;
     }
     float s = Bt.psf_sigma ? Bt.psf_sigma[roi] : Kp->p.PSFsigma;
     w.sigma = s;
@@ -2350,7 +2340,7 @@ __device__ __forceinline__ bool begin_roi(ChainWarp<EXACT, NUM, TEAM> &w, const 
     w.chain = Bt.chain_ids ? Bt.chain_ids[roi] : (uint32_t)roi;
     w.idx = Bt.rng_offset ? Bt.rng_offset[roi] : 0u;
     w.base = w.idx >> 2;
-    if (EXACT) w.idx &= 3u;
+    w.idx &= 3u;
     w.refill();
     w.entries = 0;
     w.overflow = 0;
@@ -2382,8 +2372,8 @@ __device__ __forceinline__ void end_roi(ChainWarp<EXACT, NUM, TEAM> &w, const Sa
         fs[4 + 3 * BAMF_NMAX + lane] = lane < w.an ? (float)w.aS : 0.0f;
     }
     __syncwarp();
-    if (Bt.counters)
-        for (int k = lane; k < C_COUNT; k += 32) Bt.counters[(size_t)roi * C_COUNT + k] = w.cnt[k];
+    static_assert(C_COUNT <= 32, "a lane per counter");
+    if (Bt.counters && lane < C_COUNT) Bt.counters[(size_t)roi * C_COUNT + lane] = w.cnt;
     if (Bt.chains && lane == 0) {
         Bt.chains[2 * roi].n_entries = min(w.entries, Bt.chains[2 * roi].capacity_entries);
         Bt.chains[2 * roi + 1].n_entries = min(w.entries, Bt.chains[2 * roi + 1].capacity_entries);
@@ -2393,7 +2383,7 @@ __device__ __forceinline__ void end_roi(ChainWarp<EXACT, NUM, TEAM> &w, const Sa
     if (lane == 0) {
         if (Bt.n_entries) Bt.n_entries[roi] = w.entries;
         if (Bt.uniforms_used)
-            Bt.uniforms_used[roi] = (EXACT ? 4u * w.base : 0u) + w.idx - (Bt.rng_offset ? Bt.rng_offset[roi] : 0u);
+            Bt.uniforms_used[roi] = 4u * w.base + w.idx - (Bt.rng_offset ? Bt.rng_offset[roi] : 0u);
         if (Bt.overflow) Bt.overflow[roi] = w.overflow;
         if (Bt.llr_evals) Bt.llr_evals[roi] = w.n_llr;
         if (Bt.status) Bt.status[roi] = BAMF_OK;
