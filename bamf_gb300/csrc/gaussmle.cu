@@ -4,13 +4,9 @@
  * with GPUgaussLib.cuh:14-258 and MatInvLib.h:15-75) for sm_103a.
  *
  * A group of 8 lanes per fit (one thread per fit in the reference).  The model
- * is separable: the integrated PSF along x depends only on the column ii
- * and along y only on the row jj, and so do the x/y derivative factors up to
- * the final multiply by the other axis's PSF.  Those per-axis terms are
- * computed once per Newton iteration (2*sz values instead of sz^2), which
- * leaves every per-pixel value bit for bit what the direct evaluation gives.
- * The O(sz^4) start-up filter uses a table of the sz*2-1 distinct Gaussian
- * weights for the same reason.
+ * is separable (gaussmle_axis.cuh): the integrated PSF and its derivatives are
+ * evaluated once per pixel edge and axis and Newton iteration, and the start-up
+ * filter is two passes of one-dimensional sums (O(sz^3) instead of O(sz^4)).
  * Output layout as the reference: param-major P[Nfits*k + i], k = 0..3 for
  * (x along the contiguous axis, y, N, bg), CRLB likewise, LogLikelihood[i].
  */
@@ -18,191 +14,149 @@
 
 #include "bamf.h"
 #include "frontend_launch.h"
+#include "gaussmle_axis.cuh"
 
 namespace {
 
 constexpr int MAXSZ = GAUSS_MLE_MAX_SIZE; /* IMSZBIG of definitions.h: largest fit window */
-#define MLE_PI 3.141592f         /* definitions.h:13 */
+constexpr int GROUP_FITS_PER_BLOCK = 16;  /* 128 threads */
 
-/* kernel_IntGauss1D (GPUgaussLib.cuh:14-24) */
-__device__ __forceinline__ float int_gauss(int ii, float x, float sigma)
+/* A CTA's shared memory in floats: the staged ROIs, per fit the filter's first
+ * pass and the edge and axis rows, then the filter's tables and pixel p -> (ii,
+ * jj) as ii << 8 | jj (no division in the pixel loops).  Axis rows first: they
+ * are read 16 bytes at a time. */
+constexpr int AXIS_FLOATS = 2 * 4 * MAXSZ + 2 * 2 * (MAXSZ + 2);
+__host__ __device__ inline int mle_smem_floats(int sz)
 {
-    const float norm = 1.0f / 2.0f / sigma / sigma;
-    return 1.0f / 2.0f * (erff((ii - x + 1.0f) * sqrtf(norm)) - erff((ii - x) * sqrtf(norm)));
-}
-
-/* the part of kernel_DerivativeIntGauss1D (:67-87) before "* PSFother" */
-__device__ __forceinline__ void dgauss_axis(int ii, float x, float sigma, float N, float *d1, float *d2)
-{
-    float u = (ii + 1.0f - x) / sigma, v = (ii - x) / sigma;
-    float a = expf(-1.0f / 2.0f * (u * u));
-    float b = expf(-1.0f / 2.0f * (v * v));
-    *d1 = -N / sqrtf(2.0f * MLE_PI) / sigma * (a - b);
-    *d2 = -N / sqrtf(2.0f * MLE_PI) / (sigma * sigma * sigma) * ((ii + 1.0f - x) * a - (ii - x) * b);
-}
-
-/* One fit per group of GL lanes (GL = 8: four fits per warp), ROIs staged
- * through shared memory with coalesced loads (the reference reads each ROI
- * per thread, uncoalesced).  Lane l of a group owns pixels l, l + GL, ...;
- * the centre of mass,
- * the start-up filter's positions, the Newton sums and the Fisher
- * information are lane partial sums (or maxima / minima) combined by
- * butterfly shuffles within the group, so every lane of the group holds
- * the same totals and the same theta.  The per-axis PSF and derivative
- * terms of an iteration are computed one value per lane into the group's
- * shared-memory rows.  The group's first lane inverts the 4 x 4 Fisher
- * matrix (MatInvLib.h:15-75) and writes the fit.  The reference's formulas
- * throughout; only the order of the pixel sums differs from its serial
- * loops. */
-constexpr int GL = 8;
-constexpr int GROUP_FITS_PER_BLOCK = 16; /* 128 threads */
-
-__device__ __forceinline__ float group_sum(float v)
-{
-#pragma unroll
-    for (int o = GL / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    return GROUP_FITS_PER_BLOCK * (AXIS_FLOATS + 2 * sz * sz) + 3 * MAXSZ + sz * sz;
 }
 
 /* The nblk (<= GROUP_FITS_PER_BLOCK) fits from ROI `first` of `data`, by
  * the whole CTA; parameter k of fit i to P[stride * k + i] and CRLB alike,
  * the log-likelihood to LL[i].  Every thread returns here (lanes other than
- * a group's first return early). */
-__device__ __forceinline__ void mle_xynb_block(const float *__restrict__ data, float sigma, int sz, int iterations,
+ * a group's first return early).  Lane l of a group owns pixels l, l + GL, ...:
+ * the Newton sums and the Fisher information are lane partial sums; the sums
+ * of an iteration are scattered over the group (group_sum_pairs), so that each
+ * parameter's quotient and update run once, on its own two lanes.  SZ > 0 fixes
+ * sz: the pixels' values and offsets then stay in registers.
+ *
+ * Issue-bound.  79,787 fits of 7x7, 10 iterations: 256 us with both edges
+ * of every index evaluated, the two-dimensional filter and all four updates on
+ * every lane, 143 us with these, 125 us with the quick reciprocal. */
+template <int SZ>
+__device__ __forceinline__ void mle_xynb_block(const float *__restrict__ data, float sigma, int sz_, int iterations,
                                                float *__restrict__ P, float *__restrict__ CRLB,
                                                float *__restrict__ LL, int64_t stride, int64_t first, int nblk)
 {
-    extern __shared__ float sm[];
-    const int npx = sz * sz;
-    /* coalesced staging of this block's ROIs; per fit 6 axis rows and the
-     * start-up filter's weight table behind them */
-    float *axis_all = sm + GROUP_FITS_PER_BLOCK * npx;
-    /* pixel p -> (ii, jj) as ii << 8 | jj, once per block (no division in the
-     * pixel loops) */
-    int *pix = (int *)(axis_all + GROUP_FITS_PER_BLOCK * 8 * MAXSZ);
-    for (int i = threadIdx.x; i < nblk * npx; i += blockDim.x) sm[i] = data[first * npx + i];
+    extern __shared__ __align__(16) float sm[];
+    const int sz = SZ > 0 ? SZ : sz_, npx = sz * sz;
+    float *rois = sm + GROUP_FITS_PER_BLOCK * AXIS_FLOATS;
+    float *tmps = rois + GROUP_FITS_PER_BLOCK * npx;
+    float *w = tmps + GROUP_FITS_PER_BLOCK * npx, *norm = w + 2 * MAXSZ;
+    int *pix = (int *)(norm + MAXSZ);
+    for (int i = threadIdx.x; i < nblk * npx; i += blockDim.x) rois[i] = data[first * npx + i];
     for (int q = threadIdx.x; q < npx; q += blockDim.x) pix[q] = (q / sz) << 8 | (q % sz);
+    filter_tables(w, norm, sz, sigma);
     __syncthreads();
     const int g = threadIdx.x / GL, l = threadIdx.x % GL;
     /* a group past the batch's end fits the block's first ROI again (its
      * lanes take part in the warp's shuffles) and writes nothing */
     const bool active = g < nblk;
-    const float *d = sm + (active ? g : 0) * npx;
-    float *px = axis_all + g * 6 * MAXSZ, *py = px + MAXSZ, *dx1 = py + MAXSZ, *dx2 = dx1 + MAXSZ,
-          *dy1 = dx2 + MAXSZ, *dy2 = dy1 + MAXSZ;
+    const float *d = rois + (active ? g : 0) * npx;
+    float4 *xr = (float4 *)(sm + g * AXIS_FLOATS), *yr = xr + MAXSZ; /* {PSF, d1, d2, 0} per index */
+    float2 *xe = (float2 *)(yr + MAXSZ), *ye = xe + MAXSZ + 2;
     const int64_t fit = first + g;
-
     float theta[4];
-    const float maxjump[4] = {1e0f, 1e0f, 1e2f, 2e0f};
-    /* kernel_CenterofMass2D (GPUgaussLib.cuh:207-227) */
-    float tx = 0.0f, ty = 0.0f, ts = 0.0f;
-    for (int p = l; p < npx; p += GL) {
-        const int ii = pix[p] >> 8, jj = pix[p] & 255; /* pixel d[sz*jj + ii] */
-        const float v = d[sz * jj + ii];
-        tx += v * ii;
-        ty += v * jj;
-        ts += v;
-    }
-    tx = group_sum(tx);
-    ty = group_sum(ty);
-    ts = group_sum(ts);
-    theta[0] = tx / ts;
-    theta[1] = ty / ts;
-    /* kernel_GaussFMaxMin2D (:230-258): each lane filters its positions,
-     * with the group's table of the 2 sz - 1 distinct Gaussian weights */
-    float *w = axis_all + GROUP_FITS_PER_BLOCK * 6 * MAXSZ + g * (2 * MAXSZ);
     {
-        const float norm = 1.0f / 2.0f / sigma / sigma;
-        for (int q = l - (sz - 1); q <= sz - 1; q += GL) w[q + sz - 1] = expf(-(float)(q * q) * norm);
+        float nmax, bg;
+        start_values<SZ>(d, tmps + g * npx, w, norm, pix, sz, l, &theta[0], &theta[1], &nmax, &bg);
+        theta[3] = bg;
+        theta[2] = fmaxf(0.0f, (nmax - bg) * 2 * 2 * MLE_PI * sigma * sigma);
     }
-    __syncwarp();
-    float Nmax = 0.0f, MinBG = 10e10f;
-    for (int pos = l; pos < npx; pos += GL) {
-        const int kk = pix[pos] >> 8, ll = pix[pos] & 255;
-        float fp = 0.0f, sum = 0.0f;
-        for (int ii = 0; ii < sz; ii++)
-            for (int jj = 0; jj < sz; jj++) {
-                const float ww = w[ii - kk + sz - 1] * w[ll - jj + sz - 1];
-                fp += ww * d[ii * sz + jj];
-                sum += ww;
-            }
-        fp /= sum;
-        Nmax = fmaxf(Nmax, fp);
-        MinBG = fminf(MinBG, fp);
-    }
+    const float inv_s = 1.0f / sigma, erf_s = sqrtf(1.0f / 2.0f / sigma / sigma);
+    const float k1 = -1.0f / sqrtf(2.0f * MLE_PI) / sigma, k2 = -1.0f / sqrtf(2.0f * MLE_PI) / (sigma * sigma * sigma);
+    /* this lane's pixels: value, and (ii, jj) */
+    constexpr int NP = SZ > 0 ? (SZ * SZ + GL - 1) / GL : 1;
+    float dv[NP];
+    int at[NP];
 #pragma unroll
-    for (int o = GL / 2; o > 0; o >>= 1) {
-        Nmax = fmaxf(Nmax, __shfl_xor_sync(0xffffffffu, Nmax, o));
-        MinBG = fminf(MinBG, __shfl_xor_sync(0xffffffffu, MinBG, o));
+    for (int t = 0; t < (SZ > 0 ? NP : 0); ++t) {
+        const int p = min(l + GL * t, npx - 1);
+        at[t] = pix[p];
+        dv[t] = d[sz * (at[t] & 255) + (at[t] >> 8)];
     }
-    theta[3] = MinBG;
-    theta[2] = fmaxf(0.0f, (Nmax - theta[3]) * 2 * 2 * MLE_PI * sigma * sigma);
 
     for (int kk = 0; kk <= iterations; kk++) {
         /* the axis terms of theta (after the last iteration: for the Fisher
          * information) */
+        axis_edges(xe, sz, theta[0], inv_s, erf_s, l);
+        axis_edges(ye, sz, theta[1], inv_s, erf_s, l);
+        __syncwarp();
+        const float n1 = k1 * theta[2], n2 = k2 * theta[2];
         for (int q = l; q < sz; q += GL) {
-            px[q] = int_gauss(q, theta[0], sigma);
-            py[q] = int_gauss(q, theta[1], sigma);
-            dgauss_axis(q, theta[0], sigma, theta[2], &dx1[q], &dx2[q]);
-            dgauss_axis(q, theta[1], sigma, theta[2], &dy1[q], &dy2[q]);
+            const float2 x0 = xe[q], x1 = xe[q + 1], y0 = ye[q], y1 = ye[q + 1];
+            const float ux = (float)q - theta[0], uy = (float)q - theta[1];
+            xr[q] = make_float4(0.5f * (x1.x - x0.x), n1 * (x1.y - x0.y), n2 * ((ux + 1.0f) * x1.y - ux * x0.y), 0.0f);
+            yr[q] = make_float4(0.5f * (y1.x - y0.x), n1 * (y1.y - y0.y), n2 * ((uy + 1.0f) * y1.y - uy * y0.y), 0.0f);
         }
         __syncwarp();
         if (kk == iterations) break;
         float num[4] = {0.0f, 0.0f, 0.0f, 0.0f}, den[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        for (int p = l; p < npx; p += GL) {
-            const int ii = pix[p] >> 8, jj = pix[p] & 255;
-            const float PSFx = px[ii], PSFy = py[jj];
-            const float model = theta[3] + theta[2] * PSFx * PSFy;
-            const float data_v = d[sz * jj + ii];
-            float dudt[4], d2udt2[4];
-            dudt[0] = dx1[ii] * PSFy;
-            d2udt2[0] = dx2[ii] * PSFy;
-            dudt[1] = dy1[jj] * PSFx;
-            d2udt2[1] = dy2[jj] * PSFx;
-            dudt[2] = PSFx * PSFy;
-            d2udt2[2] = 0.0f;
-            dudt[3] = 1.0f;
-            d2udt2[3] = 0.0f;
+        auto pixel = [&](int ij, float data_v) {
+            const float4 ax = xr[ij >> 8], ay = yr[ij & 255];
+            const float psf = ax.x * ay.x, model = theta[3] + theta[2] * psf;
+            const float u0 = ax.y * ay.x, u1 = ay.y * ax.x;
             float cf = 0.0f, df = 0.0f;
             if (model > 10e-3f) {
-                const float r = __frcp_rn(model); /* data/model, data/model^2 as products */
+                /* data/model, data/model^2 as products (beyond 1e37, as at infinity, both
+                 * vanish against the rest) */
+                const float r = recip(fminf(model, 1e37f));
                 cf = data_v * r - 1;
                 df = data_v * r * r;
             }
             cf = fminf(cf, 10e4f);
             df = fminf(df, 10e4f);
-            for (int q = 0; q < 4; q++) {
-                num[q] += dudt[q] * cf;
-                den[q] += d2udt2[q] * cf - (dudt[q] * dudt[q]) * df;
-            }
+            num[0] += u0 * cf;
+            num[1] += u1 * cf;
+            num[2] += psf * cf;
+            num[3] += cf;
+            den[0] = fmaf(ax.z * ay.x, cf, fmaf(-(u0 * u0), df, den[0]));
+            den[1] = fmaf(ay.z * ax.x, cf, fmaf(-(u1 * u1), df, den[1]));
+            den[2] = fmaf(-(psf * psf), df, den[2]);
+            den[3] -= df;
+        };
+        if (SZ > 0) {
+#pragma unroll
+            for (int t = 0; t < NP; ++t)
+                if (l + GL * t < npx) pixel(at[t], dv[t]);
+        } else {
+            for (int p = l; p < npx; p += GL) pixel(pix[p], d[sz * (pix[p] & 255) + (pix[p] >> 8)]);
         }
-        for (int q = 0; q < 4; q++) {
-            num[q] = group_sum(num[q]);
-            den[q] = group_sum(den[q]);
-        }
-        __syncwarp(); /* every lane has read the axis rows before they change */
-        theta[0] -= fminf(fmaxf(num[0] / den[0], -maxjump[0]), maxjump[0]);
-        theta[1] -= fminf(fmaxf(num[1] / den[1], -maxjump[1]), maxjump[1]);
-        theta[2] -= fminf(fmaxf(num[2] / den[2], -theta[2]), theta[2]);
-        theta[3] -= fminf(fmaxf(num[3] / den[3], -theta[3]), theta[3]);
-        theta[2] = fmaxf(theta[2], 1.0f);
-        theta[3] = fmaxf(theta[3], 0.01f);
+        group_sum_pairs(num, den, l);
+        /* parameter k = l >> 1: steps bounded by 1 (positions) or by its value */
+        const int k = l >> 1;
+        const float th = k == 0 ? theta[0] : k == 1 ? theta[1] : k == 2 ? theta[2] : theta[3];
+        const float jump = k < 2 ? 1.0f : th;
+        float nt = th - fminf(fmaxf(num[0] / den[0], -jump), jump);
+        if (k == 2) nt = fmaxf(nt, 1.0f);
+        if (k == 3) nt = fmaxf(nt, 0.01f);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) theta[q] = __shfl_sync(0xffffffffu, nt, 2 * q, GL);
     }
 
     /* Fisher information (10 distinct entries) and log-likelihood
      * (cuda_gaussMLEv2.cu:104-130) */
     float F[10] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     float Div = 0.0f;
-    for (int p = l; p < npx; p += GL) {
-        const int ii = pix[p] >> 8, jj = pix[p] & 255;
-        const float PSFx = px[ii], PSFy = py[jj];
-        const float model = theta[3] + theta[2] * PSFx * PSFy;
-        const float data_v = d[sz * jj + ii];
-        const float dudt[4] = {dx1[ii] * PSFy, dy1[jj] * PSFx, PSFx * PSFy, 1.0f};
-        const float rm = __frcp_rn(model);
+    auto fisher = [&](int ij, float data_v) {
+        const float4 ax = xr[ij >> 8], ay = yr[ij & 255];
+        const float psf = ax.x * ay.x, model = theta[3] + theta[2] * psf;
+        const float dudt[4] = {ax.y * ay.x, ay.y * ax.x, psf, 1.0f};
+        const float rm = model > 10e-3f && model < 1e37f ? recip(model) : 1.0f / model;
         int e = 0;
+#pragma unroll
         for (int a = 0; a < 4; a++)
+#pragma unroll
             for (int b = a; b < 4; b++) F[e++] += dudt[b] * dudt[a] * rm;
         if (model > 0) {
             if (data_v > 0)
@@ -210,6 +164,12 @@ __device__ __forceinline__ void mle_xynb_block(const float *__restrict__ data, f
             else
                 Div += -model;
         }
+    };
+    if (SZ > 0) {
+#pragma unroll 1
+        for (int p = l; p < npx; p += GL) fisher(pix[p], d[sz * (pix[p] & 255) + (pix[p] >> 8)]);
+    } else {
+        for (int p = l; p < npx; p += GL) fisher(pix[p], d[sz * (pix[p] & 255) + (pix[p] >> 8)]);
     }
     for (int e = 0; e < 10; ++e) F[e] = group_sum(F[e]);
     Div = group_sum(Div);
@@ -266,18 +226,20 @@ __device__ __forceinline__ void mle_xynb_block(const float *__restrict__ data, f
     LL[fit] = Div;
 }
 
+template <int SZ>
 __global__ void __launch_bounds__(GL * GROUP_FITS_PER_BLOCK) mle_xynb_group_kernel(
     const float *__restrict__ data, float sigma, int sz, int iterations,
     float *__restrict__ P, float *__restrict__ CRLB, float *__restrict__ LL, int nfits)
 {
     const int64_t first = (int64_t)blockIdx.x * GROUP_FITS_PER_BLOCK;
-    mle_xynb_block(data, sigma, sz, iterations, P, CRLB, LL, nfits, first,
+    mle_xynb_block<SZ>(data, sigma, sz, iterations, P, CRLB, LL, nfits, first,
                    (int)min((int64_t)GROUP_FITS_PER_BLOCK, (int64_t)nfits - first));
 }
 
 /* The fits of ROIs [range[0], min(range[1], capacity)) of a stack whose
  * range is known only on the device: blocks of GROUP_FITS_PER_BLOCK fits,
  * grid-stride. */
+template <int SZ>
 __global__ void __launch_bounds__(GL * GROUP_FITS_PER_BLOCK) mle_xynb_range_kernel(
     const float *__restrict__ data, float sigma, int sz, int iterations, float *__restrict__ P,
     float *__restrict__ CRLB, float *__restrict__ LL, int64_t stride, const int64_t *__restrict__ range,
@@ -286,17 +248,21 @@ __global__ void __launch_bounds__(GL * GROUP_FITS_PER_BLOCK) mle_xynb_range_kern
     const int64_t f0 = range[0], f1 = min(range[1], capacity);
     for (int64_t first = f0 + (int64_t)blockIdx.x * GROUP_FITS_PER_BLOCK; first < f1;
          first += (int64_t)gridDim.x * GROUP_FITS_PER_BLOCK) {
-        mle_xynb_block(data, sigma, sz, iterations, P, CRLB, LL, stride, first,
-                       (int)min((int64_t)GROUP_FITS_PER_BLOCK, f1 - first));
+        mle_xynb_block<SZ>(data, sigma, sz, iterations, P, CRLB, LL, stride, first,
+                           (int)min((int64_t)GROUP_FITS_PER_BLOCK, f1 - first));
         __syncthreads(); /* the staged ROIs and axis rows are rewritten for the next fits */
     }
 }
 
 }  // namespace
 
-static size_t gauss_mle_smem_bytes(int sz)
+/* dynamic shared memory of a launch; above 48 KB (sz > 16) it is asked for */
+template <typename Kern>
+static bool gauss_mle_smem(Kern kern, int sz, size_t *bytes)
 {
-    return ((size_t)GROUP_FITS_PER_BLOCK * (sz * sz + 8 * MAXSZ) + (size_t)sz * sz) * sizeof(float);
+    *bytes = (size_t)mle_smem_floats(sz) * sizeof(float);
+    return *bytes <= 48 * 1024 ||
+           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*bytes) == cudaSuccess;
 }
 
 bamf_status launch_gauss_mle_range(const float *rois, int sz, float psf_sigma, int iterations, float *params,
@@ -304,7 +270,14 @@ bamf_status launch_gauss_mle_range(const float *rois, int sz, float psf_sigma, i
                                    int64_t capacity, int blocks, cudaStream_t stream)
 {
     if (sz < 1 || sz > MAXSZ || iterations < 0 || blocks < 1) return BAMF_ERR_INVALID_ARG;
-    mle_xynb_range_kernel<<<blocks, GL * GROUP_FITS_PER_BLOCK, gauss_mle_smem_bytes(sz), stream>>>(
+    /* 7 and 8 px are findROI's and findPriors' boxes */
+    const auto kern = sz == 7 ? mle_xynb_range_kernel<7> : sz == 8 ? mle_xynb_range_kernel<8> : mle_xynb_range_kernel<0>;
+    size_t smem;
+    if (!gauss_mle_smem(kern, sz, &smem)) {
+        cudaGetLastError();
+        return BAMF_ERR_CUDA;
+    }
+    kern<<<blocks, GL * GROUP_FITS_PER_BLOCK, smem, stream>>>(
         rois, psf_sigma, sz, iterations, params, crlb, loglik, stride, range, capacity);
     return cudaGetLastError() == cudaSuccess ? BAMF_OK : BAMF_ERR_CUDA;
 }
@@ -318,9 +291,14 @@ extern "C" bamf_status bamf_gauss_mle_device(const float *rois, int sz, int nfit
     if (sz > MAXSZ) return BAMF_ERR_TOO_LARGE;
     if (nfits == 0) return BAMF_OK;
     /* a group of GL lanes per fit: 16 fits per CTA of 128 threads */
-    size_t smem = gauss_mle_smem_bytes(sz);
+    const auto kern = sz == 7 ? mle_xynb_group_kernel<7> : sz == 8 ? mle_xynb_group_kernel<8> : mle_xynb_group_kernel<0>;
+    size_t smem;
+    if (!gauss_mle_smem(kern, sz, &smem)) {
+        cudaGetLastError();
+        return BAMF_ERR_CUDA;
+    }
     int blocks = (nfits + GROUP_FITS_PER_BLOCK - 1) / GROUP_FITS_PER_BLOCK;
-    mle_xynb_group_kernel<<<blocks, GL * GROUP_FITS_PER_BLOCK, smem, (cudaStream_t)stream>>>(
+    kern<<<blocks, GL * GROUP_FITS_PER_BLOCK, smem, (cudaStream_t)stream>>>(
         rois, psf_sigma, sz, iterations, params, crlb, loglik, nfits);
     return cudaGetLastError() == cudaSuccess ? BAMF_OK : BAMF_ERR_CUDA;
 }
