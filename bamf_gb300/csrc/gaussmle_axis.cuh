@@ -129,4 +129,63 @@ __device__ __forceinline__ void start_values(const float *d, float *tmp, const f
     *fmin_ = mn;
 }
 
+/* The CRLB, the diagonal of the inverse of the Fisher matrix with the distinct
+ * entries F (row by row): LU without pivoting in the order of kernel_MatInvN
+ * (MatInvLib.h:15-75).  Every lane factors; lane num < NV solves for unit vector
+ * num and returns its element num (the reference solves them one by one). */
+template <int NV>
+__device__ __forceinline__ float inverse_diagonal(const float (&F)[NV * (NV + 1) / 2], int num)
+{
+    float M[NV][NV]; /* row, column */
+    int e = 0;
+#pragma unroll
+    for (int a = 0; a < NV; a++)
+#pragma unroll
+        for (int b = a; b < NV; b++) {
+            M[a][b] = M[b][a] = F[e];
+            ++e;
+        }
+    float rd[NV]; /* 1 / M[i][i] */
+#pragma unroll
+    for (int jj = 0; jj < NV; jj++) {
+#pragma unroll
+        for (int ii = 1; ii < NV; ii++) {
+            float t = 0.0f;
+#pragma unroll
+            for (int q = 0; q < NV; q++)
+                if (q < ii && q < jj) t += M[ii][q] * M[q][jj];
+            if (ii <= jj) M[ii][jj] -= t;
+        }
+        rd[jj] = 1 / M[jj][jj];
+#pragma unroll
+        for (int ii = 1; ii < NV; ii++)
+            if (ii > jj) {
+                float t = 0.0f;
+#pragma unroll
+                for (int q = 0; q < NV; q++)
+                    if (q < jj) t += M[ii][q] * M[q][jj];
+                M[ii][jj] = rd[jj] * (M[ii][jj] - t);
+            }
+    }
+    float y[NV], x[NV], out = 0.0f;
+#pragma unroll
+    for (int ii = 0; ii < NV; ii++) {
+        float t = 0.0f;
+#pragma unroll
+        for (int q = 0; q < NV; q++)
+            if (q < ii) t += M[ii][q] * y[q];
+        y[ii] = (ii == num ? 1.0f : 0.0f) - t;
+    }
+#pragma unroll
+    for (int ii = NV - 1; ii >= 0; ii--) {
+        float t = 0.0f;
+#pragma unroll
+        for (int q = 0; q < NV; q++)
+            if (q > ii) t += M[ii][q] * x[q];
+        x[ii] = ii == NV - 1 ? y[ii] / M[ii][ii] : rd[ii] * (y[ii] - t);
+        if (ii == num) out = x[ii];
+    }
+    return out;
+}
+
 }  // namespace

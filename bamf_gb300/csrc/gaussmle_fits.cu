@@ -7,14 +7,14 @@
  * optimised kernel (gaussmle.cu).
  *
  * One group of 8 lanes per fit (four fits per warp), the block's ROIs staged
- * through shared memory with coalesced loads; lane l of a group evaluates
- * pixels l, l + 8, ..., and the group's partial sums (centre of mass,
- * Newton numerators and denominators, Fisher information, log-likelihood)
- * and the start-up filter's maximum and minimum are combined by butterfly
- * shuffles, so all lanes of a group carry the same parameters.  Parameters
- * theta: 0 = position along the contiguous
- * ROI axis (MATLAB rows: Results.Y), 1 = the other axis (Results.X),
- * 2 = photons, 3 = background, then
+ * through shared memory; lane l of a group evaluates pixels l, l + 8, ....  As in
+ * the Basic kernel the model's axis terms, the start filter and the sums are
+ * those of gaussmle_axis.cuh.  Issue-bound: 20,000 Sigma fits of 8x8, 20
+ * iterations, took 389 us with every pixel evaluating both axes' functions at
+ * both edges (8 erf, 8 exp and 20 divisions), 148 us with the axis rows.
+ *
+ * Parameters theta: 0 = position along the contiguous ROI axis (MATLAB rows:
+ * Results.Y), 1 = the other axis (Results.X), 2 = photons, 3 = background, then
  *   Sigma:   4 = sigma of a symmetric PSF
  *   Z:       4 = z of an astigmatic PSF, sigma_a = sigma_a0 sqrt(alpha_a(z)),
  *            alpha_a(z) = 1 + (z'/d)^2 + A_a (z'/d)^3 + B_a (z'/d)^4 with
@@ -31,45 +31,16 @@
 #include <cuda_runtime.h>
 
 #include "bamf.h"
+#include "gaussmle_axis.cuh"
 
 namespace {
 
 constexpr int MAXSZ = 21;
 constexpr int FITS_PER_BLOCK = 16; /* fits per CTA, 8 lanes each */
-#define MLE_PI 3.141592f
 
 struct ZPar {
     float sx, sy, Ax, Ay, Bx, By, gamma, d;
 };
-
-__device__ __forceinline__ float int_gauss(int ii, float x, float sigma)
-{
-    const float norm = 1.0f / 2.0f / sigma / sigma;
-    return 1.0f / 2.0f * (erff((ii - x + 1.0f) * sqrtf(norm)) - erff((ii - x) * sqrtf(norm)));
-}
-
-/* kernel_DerivativeIntGauss1D (GPUgaussLib.cuh:67-87) */
-__device__ __forceinline__ void d_gauss(int ii, float x, float sigma, float N, float other, float *d1, float *d2)
-{
-    float a = expf(-1.0f / 2.0f * ((ii + 1.0f - x) / sigma) * ((ii + 1.0f - x) / sigma));
-    float b = expf(-1.0f / 2.0f * ((ii - x) / sigma) * ((ii - x) / sigma));
-    *d1 = -N / sqrtf(2.0f * MLE_PI) / sigma * (a - b) * other;
-    if (d2) *d2 = -N / sqrtf(2.0f * MLE_PI) / (sigma * sigma * sigma) * ((ii + 1.0f - x) * a - (ii - x) * b) * other;
-}
-
-/* kernel_DerivativeIntGauss1DSigma (:90-110) */
-__device__ __forceinline__ void d_gauss_sigma(int ii, float x, float S, float N, float other, float *d1, float *d2)
-{
-    float u = ii - x + 1.0f, v = ii - x;
-    float a = expf(-1.0f / 2.0f * (u / S) * (u / S));
-    float b = expf(-1.0f / 2.0f * (v / S) * (v / S));
-    float g = -N / sqrtf(2.0f * MLE_PI) / S / S * (a * u - b * v) * other;
-    *d1 = g;
-    if (d2) {
-        float S5 = S * S * S * S * S;
-        *d2 = -2.0f / S * g - N / sqrtf(2.0f * MLE_PI) / S5 * (a * u * u * u - b * v * v * v) * other;
-    }
-}
 
 /* kernel_alpha and its z-derivatives (:25-57) */
 __device__ __forceinline__ float alpha_z(float z, float A, float B, float d)
@@ -86,70 +57,29 @@ __device__ __forceinline__ float d2alpha_z(float z, float A, float B, float d)
     return 2.0f / (d * d) + 6.0f * A * z / (d * d * d) + 12.0f * B * z * z / (d * d * d * d);
 }
 
-/* model terms of pixel (ii, jj): PSF along both axes, dudt, d2udt2 */
-template <int FIT>
-__device__ __forceinline__ void pixel(int ii, int jj, const float *th, float sigma, const ZPar &z, float *px,
-                                      float *py, float *du, float *d2u)
-{
-    if (FIT == BAMF_FIT_BASIC || FIT == BAMF_FIT_SIGMA || FIT == BAMF_FIT_SIGMAYX) {
-        float s0 = FIT == BAMF_FIT_BASIC ? sigma : th[4];
-        float s1 = FIT == BAMF_FIT_SIGMAYX ? th[5] : s0;
-        float PSFx = int_gauss(ii, th[0], s0), PSFy = int_gauss(jj, th[1], s1);
-        d_gauss(ii, th[0], s0, th[2], PSFy, &du[0], d2u ? &d2u[0] : nullptr);
-        d_gauss(jj, th[1], s1, th[2], PSFx, &du[1], d2u ? &d2u[1] : nullptr);
-        if (FIT == BAMF_FIT_SIGMA) {
-            float a, b, c, e;
-            d_gauss_sigma(ii, th[0], s0, th[2], PSFy, &a, &b);
-            d_gauss_sigma(jj, th[1], s0, th[2], PSFx, &c, &e);
-            du[4] = a + c;
-            if (d2u) d2u[4] = b + e;
-        }
-        if (FIT == BAMF_FIT_SIGMAYX) {
-            d_gauss_sigma(ii, th[0], s0, th[2], PSFy, &du[4], d2u ? &d2u[4] : nullptr);
-            d_gauss_sigma(jj, th[1], s1, th[2], PSFx, &du[5], d2u ? &d2u[5] : nullptr);
-        }
-        *px = PSFx;
-        *py = PSFy;
-    } else { /* Z: kernel_DerivativeIntGauss2Dz (:135-205) */
-        float zz = th[4];
-        float ax = alpha_z(zz - z.gamma, z.Ax, z.Bx, z.d), ay = alpha_z(zz + z.gamma, z.Ay, z.By, z.d);
-        float Sx = z.sx * sqrtf(ax), Sy = z.sy * sqrtf(ay);
-        float PSFx = int_gauss(ii, th[0], Sx), PSFy = int_gauss(jj, th[1], Sy);
-        float ddx, ddy, dSx, dSy, ddSx, ddSy;
-        d_gauss(ii, th[0], Sx, th[2], PSFy, &du[0], &ddx);
-        d_gauss(jj, th[1], Sy, th[2], PSFx, &du[1], &ddy);
-        d_gauss_sigma(ii, th[0], Sx, th[2], PSFy, &dSx, &ddSx);
-        d_gauss_sigma(jj, th[1], Sy, th[2], PSFx, &dSy, &ddSy);
-        float dSax = z.sx / 2.0f / sqrtf(ax), dSay = z.sy / 2.0f / sqrtf(ay);
-        float dzx = dalpha_z(zz - z.gamma, z.Ax, z.Bx, z.d), dzy = dalpha_z(zz + z.gamma, z.Ay, z.By, z.d);
-        float dSdzx = dSax * dzx, dSdzy = dSay * dzy;
-        du[4] = dSx * dSdzx + dSy * dSdzy;
-        if (d2u) {
-            d2u[0] = ddx;
-            d2u[1] = ddy;
-            float d2Sax = -z.sx / 4.0f / (ax * sqrtf(ax)), d2Say = -z.sy / 4.0f / (ay * sqrtf(ay));
-            float ddSddzx = d2Sax * dzx * dzx + dSax * d2alpha_z(zz - z.gamma, z.Ax, z.Bx, z.d);
-            float ddSddzy = d2Say * dzy * dzy + dSay * d2alpha_z(zz + z.gamma, z.Ay, z.By, z.d);
-            d2u[4] = ddSx * (dSdzx * dSdzx) + dSx * ddSddzx + ddSy * (dSdzy * dSdzy) + dSy * ddSddzy;
-        }
-        *px = PSFx;
-        *py = PSFy;
-    }
-    du[2] = *px * *py;
-    du[3] = 1.0f;
-    if (d2u) {
-        d2u[2] = 0.0f;
-        d2u[3] = 0.0f;
-    }
-}
+/* axis_rows: the terms of every index along one axis: the PSF; the first and
+ * second derivative by the position (kernel_DerivativeIntGauss1D,
+ * GPUgaussLib.cuh:67-87) and by the width (kernel_DerivativeIntGauss1DSigma,
+ * :90-110), up to the other axis's PSF. */
+/* shared memory of a fit in floats: two axes of {PSF, d1, d2, s1} rows, the edges,
+ * the s2 rows */
+constexpr int AXIS_FLOATS = 2 * 4 * MAXSZ + 2 * 2 * (MAXSZ + 2) + 2 * (MAXSZ + 1);
+static_assert(AXIS_FLOATS % 4 == 0, "16-byte rows");
 
-constexpr int GL = 8; /* lanes per fit: four fits per warp */
-
-__device__ __forceinline__ float group_sum(float v)
+__device__ __forceinline__ void axis_rows(float4 *row, float *row2, float2 *edge, int sz, float c, float S, float N,
+                                          bool width, int l)
 {
-#pragma unroll
-    for (int o = GL / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    axis_edges(edge, sz, c, 1.0f / S, sqrtf(1.0f / 2.0f / S / S), l);
+    __syncwarp();
+    const float k = N / sqrtf(2.0f * MLE_PI) / S; /* N / sqrt(2 pi) / S */
+    const float k2 = k / S, k3 = k2 / S, k5 = k3 / S / S, m2 = 2.0f / S;
+    for (int q = l; q < sz; q += GL) {
+        const float2 e0 = edge[q], e1 = edge[q + 1];
+        const float v = (float)q - c, u = v + 1.0f;
+        const float au = u * e1.y, bv = v * e0.y, g = -k2 * (au - bv);
+        row[q] = make_float4(0.5f * (e1.x - e0.x), -k * (e1.y - e0.y), -k3 * (au - bv), g);
+        if (width) row2[q] = -m2 * g - k5 * (au * u * u - bv * v * v);
+    }
 }
 
 template <int FIT, bool SCMOS>
@@ -159,22 +89,28 @@ __global__ void __launch_bounds__(GL * FITS_PER_BLOCK) mle_fit_kernel(
     float *__restrict__ CRLB, float *__restrict__ LL, int nfits)
 {
     constexpr int NV = FIT == BAMF_FIT_BASIC ? 4 : (FIT == BAMF_FIT_SIGMAYX ? 6 : 5);
-    extern __shared__ float sm[];
+    constexpr bool WIDTH = FIT != BAMF_FIT_BASIC;
+    extern __shared__ __align__(16) float sm[];
     const int npx = sz * sz;
     const int64_t first = (int64_t)blockIdx.x * FITS_PER_BLOCK;
     const int nblk = (int)min((int64_t)FITS_PER_BLOCK, (int64_t)nfits - first);
-    /* staged ROIs, then per fit the start-up filter's weight table, then the
-     * pixel -> (ii, jj) table (ii << 8 | jj) */
-    float *wt = sm + FITS_PER_BLOCK * npx;
-    int *pix = (int *)(wt + FITS_PER_BLOCK * (2 * MAXSZ));
-    for (int i = threadIdx.x; i < nblk * npx; i += blockDim.x) sm[i] = data[first * npx + i];
+    /* per fit the axis rows, then the staged ROIs, the filter's first pass, its
+     * tables, and pixel -> (ii, jj) (ii << 8 | jj) */
+    float *rois = sm + FITS_PER_BLOCK * AXIS_FLOATS, *tmps = rois + FITS_PER_BLOCK * npx;
+    float *w = tmps + FITS_PER_BLOCK * npx, *norm = w + 2 * MAXSZ;
+    int *pix = (int *)(norm + MAXSZ);
+    for (int i = threadIdx.x; i < nblk * npx; i += blockDim.x) rois[i] = data[first * npx + i];
     for (int q = threadIdx.x; q < npx; q += blockDim.x) pix[q] = (q / sz) << 8 | (q % sz);
+    filter_tables(w, norm, sz, FIT == BAMF_FIT_Z ? zp.sx : sigma);
     __syncthreads();
     const int g = threadIdx.x / GL, l = threadIdx.x % GL;
     /* a group past the batch's end fits the block's first ROI again (its
      * lanes take part in the warp's shuffles) and writes nothing */
     const bool active = g < nblk;
-    const float *d = sm + (active ? g : 0) * npx;
+    const float *d = rois + (active ? g : 0) * npx;
+    float4 *xr = (float4 *)(sm + g * AXIS_FLOATS), *yr = xr + MAXSZ;
+    float2 *xe = (float2 *)(yr + MAXSZ), *ye = xe + MAXSZ + 2;
+    float *x2 = (float *)(ye + MAXSZ + 2), *y2 = x2 + MAXSZ + 1;
     const int64_t fit = first + (active ? g : 0);
     float c0 = 0.0f, c1 = 0.0f;
     if (SCMOS) {
@@ -183,103 +119,135 @@ __global__ void __launch_bounds__(GL * FITS_PER_BLOCK) mle_fit_kernel(
     }
 
     float th[6];
-    float maxjump[6] = {1e0f, 1e0f, 1e2f, 2e0f, FIT == BAMF_FIT_SIGMA ? 5e-1f : 1e-1f, 1e-1f};
-    /* kernel_CenterofMass2D (GPUgaussLib.cuh:207-227): lane partial sums */
-    float tx = 0.0f, ty = 0.0f, ts = 0.0f;
-    for (int p = l; p < npx; p += GL) {
-        const int ii = pix[p] >> 8, jj = pix[p] & 255;
-        const float v = d[sz * jj + ii];
-        tx += v * ii;
-        ty += v * jj;
-        ts += v;
-    }
-    th[0] = group_sum(tx) / group_sum(ts);
-    th[1] = group_sum(ty) / group_sum(ts);
-    /* kernel_GaussFMaxMin2D (:230-258): each lane filters its positions with
-     * the group's table of the distinct weights */
-    const float s_init = FIT == BAMF_FIT_Z ? zp.sx : sigma;
-    float *w = wt + g * (2 * MAXSZ);
     {
-        const float norm = 1.0f / 2.0f / s_init / s_init;
-        for (int q = l - (sz - 1); q <= sz - 1; q += GL) w[q + sz - 1] = expf(-(float)(q * q) * norm);
-    }
-    __syncwarp();
-    float Nmax = 0.0f, MinBG = 10e10f;
-    for (int pos = l; pos < npx; pos += GL) {
-        const int kk = pix[pos] >> 8, ll = pix[pos] & 255;
-        float fp = 0.0f, sum = 0.0f;
-        for (int ii = 0; ii < sz; ii++)
-            for (int jj = 0; jj < sz; jj++) {
-                float ww = w[ii - kk + sz - 1] * w[ll - jj + sz - 1];
-                fp += ww * d[ii * sz + jj];
-                sum += ww;
-            }
-        fp /= sum;
-        Nmax = fmaxf(Nmax, fp);
-        MinBG = fminf(MinBG, fp);
-    }
-#pragma unroll
-    for (int o = GL / 2; o > 0; o >>= 1) {
-        Nmax = fmaxf(Nmax, __shfl_xor_sync(0xffffffffu, Nmax, o));
-        MinBG = fminf(MinBG, __shfl_xor_sync(0xffffffffu, MinBG, o));
-    }
-    th[3] = MinBG;
-    if (FIT == BAMF_FIT_Z) {
-        th[2] = fmaxf(0.0f, (Nmax - th[3]) * 2 * MLE_PI * zp.sx * zp.sy * sqrtf(2.0f));
-        th[4] = 0.0f; /* z0: gaussMLE.m passes zeros */
-    } else {
-        th[2] = fmaxf(0.0f, (Nmax - th[3]) * 2 * 2 * MLE_PI * sigma * sigma);
-        th[4] = sigma;
+        float nmax, bg;
+        start_values<0>(d, tmps + g * npx, w, norm, pix, sz, l, &th[0], &th[1], &nmax, &bg);
+        th[3] = bg;
+        if (FIT == BAMF_FIT_Z) {
+            th[2] = fmaxf(0.0f, (nmax - bg) * 2 * MLE_PI * zp.sx * zp.sy * sqrtf(2.0f));
+            th[4] = 0.0f; /* z0: gaussMLE.m passes zeros */
+        } else {
+            th[2] = fmaxf(0.0f, (nmax - bg) * 2 * 2 * MLE_PI * sigma * sigma);
+            th[4] = sigma;
+        }
         th[5] = sigma;
     }
 
+    /* Z (kernel_DerivativeIntGauss2Dz, :135-205): the widths of both axes and
+     * their first two derivatives by z */
+    float zx1 = 0.0f, zx2 = 0.0f, zy1 = 0.0f, zy2 = 0.0f;
+    auto axes = [&]() {
+        float sx = FIT == BAMF_FIT_BASIC ? sigma : th[4], sy = FIT == BAMF_FIT_SIGMAYX ? th[5] : sx;
+        if (FIT == BAMF_FIT_Z) {
+            const float zz = th[4], zm = zz - zp.gamma, zpl = zz + zp.gamma;
+            const float ax = alpha_z(zm, zp.Ax, zp.Bx, zp.d), ay = alpha_z(zpl, zp.Ay, zp.By, zp.d);
+            const float rx = sqrtf(ax), ry = sqrtf(ay);
+            const float dax = dalpha_z(zm, zp.Ax, zp.Bx, zp.d), day = dalpha_z(zpl, zp.Ay, zp.By, zp.d);
+            sx = zp.sx * rx;
+            sy = zp.sy * ry;
+            const float px = zp.sx / 2.0f / rx, py = zp.sy / 2.0f / ry;
+            zx1 = px * dax;
+            zy1 = py * day;
+            zx2 = -zp.sx / 4.0f / (ax * rx) * dax * dax + px * d2alpha_z(zm, zp.Ax, zp.Bx, zp.d);
+            zy2 = -zp.sy / 4.0f / (ay * ry) * day * day + py * d2alpha_z(zpl, zp.Ay, zp.By, zp.d);
+        }
+        axis_rows(xr, x2, xe, sz, th[0], sx, th[2], WIDTH, l);
+        axis_rows(yr, y2, ye, sz, th[1], sy, th[2], WIDTH, l);
+        __syncwarp();
+    };
+    /* derivatives of the model at a pixel; d2u null: first ones only */
+    auto pixel = [&](int ii, int jj, float *psf, float *du, float *d2u) {
+        const float4 ax = xr[ii], ay = yr[jj];
+        *psf = ax.x * ay.x;
+        du[0] = ax.y * ay.x;
+        du[1] = ay.y * ax.x;
+        du[2] = *psf;
+        du[3] = 1.0f;
+        const float sx1 = ax.w * ay.x, sy1 = ay.w * ax.x;
+        if (FIT == BAMF_FIT_SIGMA) du[4] = sx1 + sy1;
+        if (FIT == BAMF_FIT_SIGMAYX) {
+            du[4] = sx1;
+            du[5] = sy1;
+        }
+        if (FIT == BAMF_FIT_Z) du[4] = sx1 * zx1 + sy1 * zy1;
+        if (d2u) {
+            d2u[0] = ax.z * ay.x;
+            d2u[1] = ay.z * ax.x;
+            d2u[2] = 0.0f;
+            d2u[3] = 0.0f;
+            if (WIDTH) {
+                const float sx2 = x2[ii] * ay.x, sy2 = y2[jj] * ax.x;
+                if (FIT == BAMF_FIT_SIGMA) d2u[4] = sx2 + sy2;
+                if (FIT == BAMF_FIT_SIGMAYX) {
+                    d2u[4] = sx2;
+                    d2u[5] = sy2;
+                }
+                if (FIT == BAMF_FIT_Z) d2u[4] = sx2 * (zx1 * zx1) + sx1 * zx2 + sy2 * (zy1 * zy1) + sy1 * zy2;
+            }
+        }
+    };
+
     for (int kk = 0; kk < iterations; kk++) {
+        axes();
         float num[6] = {0, 0, 0, 0, 0, 0}, den[6] = {0, 0, 0, 0, 0, 0};
         for (int p = l; p < npx; p += GL) {
             const int ii = pix[p] >> 8, jj = pix[p] & 255;
-            float PSFx, PSFy, du[6], d2u[6];
-            pixel<FIT>(ii, jj, th, sigma, zp, &PSFx, &PSFy, du, d2u);
-            float model = th[3] + th[2] * PSFx * PSFy;
+            float psf, du[6], d2u[6];
+            pixel(ii, jj, &psf, du, d2u);
+            float model = th[3] + th[2] * psf;
             float dv = d[sz * jj + ii];
             float cf = 0.0f, df = 0.0f;
             if (SCMOS) {
                 int gi = (int)((c1 + jj) * mapsz + c0 + ii);
                 gi = min(max(gi, 0), mapsz * mapsz - 1); /* corners outside the map: edge value */
                 const float gRp = gmap[gi];
-                if (model > 10e-3f) cf = (dv - model) / (model + gRp);
-                if (model > 10e-3f) df = (dv + gRp) / ((model + gRp) * (model + gRp));
-            } else {
-                if (model > 10e-3f) cf = dv / model - 1;
-                if (model > 10e-3f) df = dv / (model * model);
+                if (model > 10e-3f) {
+                    cf = (dv - model) / (model + gRp);
+                    df = (dv + gRp) / ((model + gRp) * (model + gRp));
+                }
+            } else if (model > 10e-3f) {
+                const float r = recip(fminf(model, 1e37f));
+                cf = dv * r - 1;
+                df = dv * r * r;
             }
             cf = fminf(cf, 10e4f);
             df = fminf(df, 10e4f);
+#pragma unroll
             for (int q = 0; q < NV; q++) {
                 num[q] += du[q] * cf;
-                den[q] += d2u[q] * cf - (du[q] * du[q]) * df;
+                den[q] = fmaf(d2u[q], cf, fmaf(-(du[q] * du[q]), df, den[q]));
             }
         }
-        for (int q = 0; q < NV; q++) {
+        /* parameters 0..3 on lane pairs, 4 and 5 on every lane */
+#pragma unroll
+        for (int q = 4; q < NV; q++) {
             num[q] = group_sum(num[q]);
             den[q] = group_sum(den[q]);
         }
-        th[0] -= fminf(fmaxf(num[0] / den[0], -maxjump[0]), maxjump[0]);
-        th[1] -= fminf(fmaxf(num[1] / den[1], -maxjump[1]), maxjump[1]);
-        th[2] -= fminf(fmaxf(num[2] / den[2], -th[2]), th[2]);
-        th[3] -= fminf(fmaxf(num[3] / den[3], -th[3]), th[3]);
-        if (FIT == BAMF_FIT_SIGMA || FIT == BAMF_FIT_SIGMAYX) th[4] -= fminf(fmaxf(num[4] / den[4], -th[4]), th[4]);
-        if (FIT == BAMF_FIT_SIGMAYX) th[5] -= fminf(fmaxf(num[5] / den[5], -th[5]), th[5]);
-        if (FIT == BAMF_FIT_Z) th[4] -= fminf(fmaxf(num[4] / den[4], -maxjump[4]), maxjump[4]);
-        th[2] = fmaxf(th[2], 1.0f);
-        th[3] = fmaxf(th[3], 0.01f);
+        {
+            float n4[4] = {num[0], num[1], num[2], num[3]}, d4[4] = {den[0], den[1], den[2], den[3]};
+            group_sum_pairs(n4, d4, l);
+            const int k = l >> 1;
+            const float t = k == 0 ? th[0] : k == 1 ? th[1] : k == 2 ? th[2] : th[3];
+            const float jump = k < 2 ? 1.0f : t;
+            float nt = t - fminf(fmaxf(n4[0] / d4[0], -jump), jump);
+            if (k == 2) nt = fmaxf(nt, 1.0f);
+            if (k == 3) nt = fmaxf(nt, 0.01f);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) th[q] = __shfl_sync(0xffffffffu, nt, 2 * q, GL);
+        }
         if (FIT == BAMF_FIT_SIGMA || FIT == BAMF_FIT_SIGMAYX) {
+            th[4] -= fminf(fmaxf(num[4] / den[4], -th[4]), th[4]);
             th[4] = fmaxf(th[4], 0.5f);
             th[4] = fminf(th[4], sz / 2.0f);
         }
         if (FIT == BAMF_FIT_SIGMAYX) {
+            th[5] -= fminf(fmaxf(num[5] / den[5], -th[5]), th[5]);
             th[5] = fmaxf(th[5], 0.5f);
             th[5] = fminf(th[5], sz / 2.0f);
         }
+        if (FIT == BAMF_FIT_Z) th[4] -= fminf(fmaxf(num[4] / den[4], -1e-1f), 1e-1f);
+        __syncwarp(); /* every lane has read the axis rows before they change */
     }
     /* the reference's CRLB / log-likelihood pass uses the variance-gain
      * ratio left from the last pixel of the last iteration, (sz-1, sz-1) */
@@ -293,18 +261,22 @@ __global__ void __launch_bounds__(GL * FITS_PER_BLOCK) mle_fit_kernel(
      * log-likelihood */
     constexpr int NF = NV * (NV + 1) / 2;
     float F[NF];
+#pragma unroll
     for (int q = 0; q < NF; ++q) F[q] = 0.0f;
     float Div = 0.0f;
+    axes();
     for (int p = l; p < npx; p += GL) {
         const int ii = pix[p] >> 8, jj = pix[p] & 255;
-        float PSFx, PSFy, du[6];
-        pixel<FIT>(ii, jj, th, sigma, zp, &PSFx, &PSFy, du, nullptr);
-        float model = th[3] + th[2] * PSFx * PSFy;
+        float psf, du[6];
+        pixel(ii, jj, &psf, du, nullptr);
+        float model = th[3] + th[2] * psf;
         float dv = d[sz * jj + ii];
-        float den = SCMOS ? model + gR : model;
+        const float rd = 1.0f / (SCMOS ? model + gR : model);
         int e = 0;
+#pragma unroll
         for (int a = 0; a < NV; a++)
-            for (int b = a; b < NV; b++) F[e++] += du[b] * du[a] / den;
+#pragma unroll
+            for (int b = a; b < NV; b++) F[e++] += du[b] * du[a] * rd;
         if (SCMOS) {
             if (model + gR > 0) {
                 if (dv + gR > 0)
@@ -319,65 +291,27 @@ __global__ void __launch_bounds__(GL * FITS_PER_BLOCK) mle_fit_kernel(
                 Div += -model;
         }
     }
+#pragma unroll
     for (int q = 0; q < NF; ++q) F[q] = group_sum(F[q]);
     Div = group_sum(Div);
-    if (l != 0 || !active) return;
-    float M[NV * NV];
-    {
-        int e = 0;
-        for (int a = 0; a < NV; a++)
-            for (int b = a; b < NV; b++) {
-                M[a * NV + b] = F[e];
-                M[b * NV + a] = F[e];
-                ++e;
-            }
+    const float crlb = inverse_diagonal<NV>(F, l);
+    if (!active) return;
+    float t = th[0];
+#pragma unroll
+    for (int k = 1; k < NV; k++)
+        if (l == k) t = th[k];
+    if (l < NV) {
+        P[(int64_t)nfits * l + fit] = t;
+        CRLB[(int64_t)nfits * l + fit] = crlb;
     }
-    /* inverse by LU without pivoting (the order of MatInvLib.h:15-75),
-     * diagonal only */
-    float Minv[NV * NV], yy[NV], tmp1 = 0.0f;
-    for (int jj = 0; jj < NV; jj++) {
-        for (int ii = 1; ii <= jj; ii++) {
-            for (int q = 0; q <= ii - 1; q++) tmp1 += M[ii + q * NV] * M[q + jj * NV];
-            M[ii + jj * NV] -= tmp1;
-            tmp1 = 0.0f;
-        }
-        for (int ii = jj + 1; ii < NV; ii++) {
-            if (jj > 0) {
-                for (int q = 0; q <= jj - 1; q++) tmp1 += M[ii + q * NV] * M[q + jj * NV];
-                M[ii + jj * NV] = (1 / M[jj + jj * NV]) * (M[ii + jj * NV] - tmp1);
-                tmp1 = 0.0f;
-            } else {
-                M[ii + jj * NV] = (1 / M[jj + jj * NV]) * M[ii + jj * NV];
-            }
-        }
-    }
-    for (int num = 0; num < NV; num++) {
-        yy[0] = num == 0 ? 1.0f : 0.0f;
-        for (int ii = 1; ii < NV; ii++) {
-            float b = ii == num ? 1.0f : 0.0f;
-            for (int q = 0; q <= ii - 1; q++) tmp1 += M[ii + q * NV] * yy[q];
-            yy[ii] = b - tmp1;
-            tmp1 = 0.0f;
-        }
-        Minv[NV - 1 + num * NV] = yy[NV - 1] / M[(NV - 1) + (NV - 1) * NV];
-        for (int ii = NV - 2; ii >= 0; ii--) {
-            for (int q = ii + 1; q < NV; q++) tmp1 += M[ii + q * NV] * Minv[q + num * NV];
-            Minv[ii + num * NV] = (1 / M[ii + ii * NV]) * (yy[ii] - tmp1);
-            tmp1 = 0.0f;
-        }
-    }
-    for (int k = 0; k < NV; k++) {
-        P[(int64_t)nfits * k + fit] = th[k];
-        CRLB[(int64_t)nfits * k + fit] = Minv[k * NV + k];
-    }
-    LL[fit] = Div;
+    if (l == 0) LL[fit] = Div;
 }
 
 template <int FIT, bool SCMOS>
 cudaError_t launch(const float *rois, int sz, int nfits, float sigma, const ZPar &zp, const float *coords,
                    const float *gmap, int mapsz, int iterations, float *P, float *C, float *L, cudaStream_t s)
 {
-    size_t smem = ((size_t)FITS_PER_BLOCK * (sz * sz + 2 * MAXSZ) + (size_t)sz * sz) * sizeof(float);
+    size_t smem = ((size_t)FITS_PER_BLOCK * (AXIS_FLOATS + 2 * sz * sz) + 3 * MAXSZ + (size_t)sz * sz) * sizeof(float);
     if (smem > 48 * 1024) {
         cudaError_t e =
             cudaFuncSetAttribute(mle_fit_kernel<FIT, SCMOS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
