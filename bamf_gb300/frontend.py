@@ -54,9 +54,9 @@ def _declare():
     L.bamf_gauss_mle_host.argtypes = [pf, C.c_int, C.c_int, C.c_float, C.c_int, pf, pf, pf]
     L.bamf_gauss_mle_nparams.restype = C.c_int
     L.bamf_gauss_mle_nparams.argtypes = [C.c_int]
-    L.bamf_gauss_mle_fit_host.restype = C.c_int
-    L.bamf_gauss_mle_fit_host.argtypes = [pf, C.c_int, C.c_int, C.c_int, C.c_float, C.c_void_p, pf, pf, C.c_int,
-                                          C.c_int, pf, pf, pf]
+    for fn in (L.bamf_gauss_mle_fit_host, L.bamf_gauss_mle_fit_host_planes):
+        fn.restype = C.c_int
+        fn.argtypes = [pf, C.c_int, C.c_int, C.c_int, C.c_float, C.c_void_p, pf, pf, C.c_int, C.c_int, pf, pf, pf]
     L._frontend_declared = True
     return L
 
@@ -127,7 +127,10 @@ def gaussMLE(Data, FitType: str = "Basic", CameraType: str = "CCD", Sigma=1.3, *
     if d.ndim == 2:
         d = d[:, :, None]
     sz, _, n = d.shape
-    flat = np.ascontiguousarray(d.ravel(order="F"))
+    # a C-ordered array goes to the device as it lies and is reordered there
+    planes = d.flags.c_contiguous and not d.flags.f_contiguous
+    flat = d if planes else np.ascontiguousarray(d.ravel(order="F"))
+    fit_host = L.bamf_gauss_mle_fit_host_planes if planes else L.bamf_gauss_mle_fit_host
     sig = np.atleast_1d(np.asarray(Sigma, np.float64))
     zf = None
     var = corners = None
@@ -150,11 +153,11 @@ def gaussMLE(Data, FitType: str = "Basic", CameraType: str = "CCD", Sigma=1.3, *
     CR = np.zeros(npar * n, np.float32)
     LL = np.zeros(n, np.float32)
     msz = int(np.sqrt(var.size)) if var is not None else 0
-    abi.check(L.bamf_gauss_mle_fit_host(abi.fptr(flat), sz, n, FIT_TYPES[FitType], float(np.mean(sig)),
-                                        C.byref(zf) if zf is not None else None,
-                                        abi.fptr(corners) if corners is not None else None,
-                                        abi.fptr(var) if var is not None else None, msz, int(Iterations),
-                                        abi.fptr(P), abi.fptr(CR), abi.fptr(LL)), "bamf_gauss_mle_fit_host")
+    abi.check(fit_host(abi.fptr(flat), sz, n, FIT_TYPES[FitType], float(np.mean(sig)),
+                       C.byref(zf) if zf is not None else None,
+                       abi.fptr(corners) if corners is not None else None,
+                       abi.fptr(var) if var is not None else None, msz, int(Iterations),
+                       abi.fptr(P), abi.fptr(CR), abi.fptr(LL)), "bamf_gauss_mle_fit_host")
     P = P.reshape(npar, n).T
     CR = CR.reshape(npar, n).T
     # a negative CRLB diagonal (an ill-conditioned fit) gives NaN here where

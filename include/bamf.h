@@ -674,6 +674,12 @@ bamf_status bamf_gauss_mle_fit_device(const float *rois, int sz, int nfits, int 
 bamf_status bamf_gauss_mle_fit_host(const float *rois, int sz, int nfits, int fit_type, float psf_sigma,
                                     const bamf_zfit *zfit, const float *box_corners, const float *var_gain_map,
                                     int map_size, int iterations, float *params, float *crlb, float *loglik);
+/* the same fits of ROIs that lie pixel by pixel, as a C-ordered array (sz, sz, nfits)
+ * does: pixel (row a, column b) of fit i at planes[(a * sz + b) * nfits + i] */
+bamf_status bamf_gauss_mle_fit_host_planes(const float *planes, int sz, int nfits, int fit_type, float psf_sigma,
+                                           const bamf_zfit *zfit, const float *box_corners,
+                                           const float *var_gain_map, int map_size, int iterations, float *params,
+                                           float *crlb, float *loglik);
 
 /* ------------------------------------------------------------------ */
 /* Measurement helpers                                                  */

@@ -187,3 +187,16 @@ def test_fit_types_of_every_window(cuda_lib, fit, camera, sz):
         assert good.mean() > 0.9
         assert np.quantile(np.abs(SE[good] ** 2 / CR[good] - 1), 0.99) < 1e-3
         assert np.quantile(np.abs(res["LogLikelihood"] - LL) / np.maximum(np.abs(LL), 1.0), 0.99) < 1e-3
+
+
+@pytest.mark.parametrize("sz,n", [(1, 1), (2, 1), (5, 31), (6, 32), (7, 33), (21, 65)])
+def test_fits_do_not_depend_on_the_memory_order(cuda_lib, sz, n):
+    from bamf_gb300 import frontend
+    rois = np.random.default_rng(sz).poisson(20.0, (sz, sz, n)).astype(np.float32)
+    a = frontend.gaussMLE(np.asfortranarray(rois), "Sigma", "CCD", 1.3, Iterations=2)
+    wide = np.zeros((sz, sz + 1, n + 2), np.float32)
+    wide[:, 1:, 1:-1] = rois
+    for other in (rois, rois.astype(np.float64), wide[:, 1:, 1:-1]):
+        b = frontend.gaussMLE(other, "Sigma", "CCD", 1.3, Iterations=2)
+        for k in a:
+            np.testing.assert_array_equal(a[k], b[k])
