@@ -1,15 +1,16 @@
 /*
  * cnn.cu - the learned birth proposal (include/bamf_cnn.h): synthetic ROI
- * generator, the network's forward and backward kernels, Adam, a CUDA-graph
- * training step, and inference into the sampler's LEARNED birth tables.
+ * generator, the network's forward (net_kernel, for training and for
+ * inference into the sampler's LEARNED birth tables) and backward kernels,
+ * Adam, and a CUDA-graph training step.
  *
  * Layouts.  Activations are channels-last BF16, [roi][p][32] with pixel
- * p = y + 16 x.  The three 32 -> 32 convolutions (forward and input
- * gradient) run on the 5th-generation tensor cores (tcgen05.mma from
- * shared-memory descriptors into TMEM, conv_tc_kernel): per ROI an implicit
+ * p = y + 16 x.  The three 32 -> 32 convolutions (forward in net_kernel,
+ * input gradient in conv_tc_kernel) run on the 5th-generation tensor cores
+ * (tcgen05.mma from shared-memory descriptors into TMEM): per ROI an implicit
  * GEMM with M = 256 pixels (two tiles of 128), N = 32, K = 9 taps x 32
- * channels.  The input gradient of a convolution is the same kernel run with
- * the taps flipped and the channel roles swapped (packed once per step).
+ * channels.  The input gradient is the convolution with the taps flipped and
+ * the channel roles swapped (packed once per step).
  * The weight gradient is a GEMM with K = the pixels of every ROI of the
  * CTA, also on tcgen05, with MN-major operands so that the channels-last
  * activations stage without a transpose (conv_dw_tc_kernel).
@@ -182,44 +183,6 @@ __global__ void pack_kernel(const float *__restrict__ P, bf16 *__restrict__ Wf, 
 }
 
 /* --------------------------------------------------------------- conv1 */
-/* x0 normalisation and the 1 -> 32 convolution (FP32), one CTA per ROI. */
-__global__ void conv1_fwd_kernel(const float *__restrict__ data, int n, const float *__restrict__ P,
-                                 float *__restrict__ x0, bf16 *__restrict__ a1)
-{
-    __shared__ float xp[PS * PS];
-    __shared__ float w[288 + 32];
-    __shared__ float red[8];
-    int r = blockIdx.x, t = threadIdx.x;
-    if (r >= n) return;
-    for (int i = t; i < 320; i += blockDim.x) w[i] = P[O_W1 + i];
-    for (int i = t; i < PS * PS; i += blockDim.x) xp[i] = 0.0f;
-    float v = sqrtf(fmaxf(data[(size_t)r * NPX + t], 0.0f) + 0.375f);
-    float s = v;
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((t & 31) == 0) red[t >> 5] = s;
-    __syncthreads();
-    float mean = 0.0f;
-    for (int k = 0; k < 8; ++k) mean += red[k];
-    mean *= (1.0f / NPX);
-    float xv = (v - mean) * 0.25f;
-    int x = t / S, y = t - (t / S) * S;
-    xp[(x + 1) * PS + (y + 1)] = xv;
-    if (x0) x0[(size_t)r * NPX + t] = xv;
-    __syncthreads();
-    float in[9];
-    for (int kx = 0; kx < 3; ++kx)
-        for (int ky = 0; ky < 3; ++ky) in[kx * 3 + ky] = xp[(x + kx) * PS + (y + ky)];
-    __align__(16) bf16 o[CH];
-    for (int co = 0; co < CH; ++co) {
-        float z = w[288 + co];
-        for (int tp = 0; tp < 9; ++tp) z += w[co * 9 + tp] * in[tp];
-        o[co] = __float2bfloat16_rn(fmaxf(z, 0.0f));
-    }
-    uint4 *dst = (uint4 *)(a1 + ((size_t)r * NPX + t) * CH);
-    const uint4 *src = (const uint4 *)o;
-    for (int q = 0; q < 4; ++q) dst[q] = src[q];
-}
-
 /* dW1, db1 from dz1 (= dL/d pre-activation of conv1) and x0: each CTA's
  * sums over its ROIs into row blockIdx.x of `rows` (C1_NPARAM floats).  Warp w
  * owns output channels 4w .. 4w + 3 (all 9 taps and the bias), lane l the
@@ -292,8 +255,7 @@ __global__ void __launch_bounds__(256) conv1_bwd_kernel(const float *__restrict_
 }
 
 /* -------------------------------------------------- 32 -> 32 convolution */
-/* MODE 0: out = relu(conv(in, W) + bias).  MODE 1 (input gradient):
- * out = conv(in, W) * (mask > 0).  On the 5th-generation tensor cores: per
+/* Input gradient: out = conv(in, W) * (mask > 0).  On the 5th-generation tensor cores: per
  * ROI an implicit GEMM D[pixel][co] = sum over 9 taps of A_tap[pixel][ci]
  * B_tap[co][ci], M = 256 pixels as two tiles of 128, N = 32, K = 32 per tap
  * as two MMAs of 16: 36 tcgen05.mma (BF16 x BF16 -> FP32) issued by one
@@ -314,9 +276,7 @@ constexpr int TC_COPY = 4 * TC_GSTRIDE;            /* bytes of one shifted copy 
 constexpr size_t SMEM_TC = (size_t)PKT * 2 + 3 * TC_COPY + 16;
 constexpr uint32_t TC_IDESC = bamf::tc::idesc_bf16_f32(128, 32);
 
-template <int MODE>
 __global__ void __launch_bounds__(128) conv_tc_kernel(const bf16 *__restrict__ in, const bf16 *__restrict__ Wt,
-                                                      const float *__restrict__ bias,
                                                       const bf16 *__restrict__ mask, bf16 *__restrict__ out, int n,
                                                       int *__restrict__ status)
 {
@@ -399,16 +359,14 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(const bf16 *__restrict__ i
         }
         const int rn = r + gridDim.x;
         if (rn < n) load(rn);
-        /* MODE 1: this thread's two pixels of the ReLU mask, loaded while
+        /* this thread's two pixels of the ReLU mask, loaded while
          * the MMAs run */
         uint4 mk[2][4];
-        if (MODE == 1) {
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-                const uint4 *ms = (const uint4 *)(mask + ((size_t)r * NPX + 128 * mt + t) * CH);
+        for (int mt = 0; mt < 2; ++mt) {
+            const uint4 *ms = (const uint4 *)(mask + ((size_t)r * NPX + 128 * mt + t) * CH);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) mk[mt][q] = ms[q];
-            }
+            for (int q = 0; q < 4; ++q) mk[mt][q] = ms[q];
         }
         const bool ok = bamf::tc::mbar_wait(mbar, phase, 1u << 24);
         phase ^= 1u;
@@ -424,21 +382,14 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(const bf16 *__restrict__ i
                 const int p = 128 * mt + t;
                 const size_t off = ((size_t)r * NPX + p) * CH;
                 __align__(16) __nv_bfloat162 o[16];
-                if (MODE == 0) {
+                __align__(16) uint4 m4[4];
 #pragma unroll
-                    for (int c = 0; c < 16; ++c)
-                        o[c] = __floats2bfloat162_rn(fmaxf(v[2 * c] + bias[2 * c], 0.0f),
-                                                     fmaxf(v[2 * c + 1] + bias[2 * c + 1], 0.0f));
-                } else {
-                    __align__(16) uint4 m4[4];
+                for (int q = 0; q < 4; ++q) m4[q] = mt == 0 ? mk[0][q] : mk[1][q];
+                const __nv_bfloat162 *m2 = (const __nv_bfloat162 *)m4;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) m4[q] = mt == 0 ? mk[0][q] : mk[1][q];
-                    const __nv_bfloat162 *m2 = (const __nv_bfloat162 *)m4;
-#pragma unroll
-                    for (int c = 0; c < 16; ++c)
-                        o[c] = __floats2bfloat162_rn(__bfloat162float(m2[c].x) > 0.0f ? v[2 * c] : 0.0f,
-                                                     __bfloat162float(m2[c].y) > 0.0f ? v[2 * c + 1] : 0.0f);
-                }
+                for (int c = 0; c < 16; ++c)
+                    o[c] = __floats2bfloat162_rn(__bfloat162float(m2[c].x) > 0.0f ? v[2 * c] : 0.0f,
+                                                 __bfloat162float(m2[c].y) > 0.0f ? v[2 * c + 1] : 0.0f);
                 uint4 *dst = (uint4 *)(out + off);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) dst[q] = ((uint4 *)o)[q];
@@ -897,8 +848,10 @@ __global__ void __launch_bounds__(256) head_kernel(const bf16 *__restrict__ a4, 
     if (t < NC) row_wc(hrows, r)[NC * CH + t] = dzc[t];
 }
 
-/* ------------------------------------------------------ fused inference */
-/* The whole network on a ROI without leaving the SM.  A persistent CTA keeps
+/* ------------------------------------------------------ fused forward */
+/* The whole network on a ROI without leaving the SM (NET_TRAIN: up to a4, the
+ * activations also written out for the backward kernels, 1024 ROIs in 44 us
+ * for 72 us of four kernels).  A persistent CTA keeps
  * the packed weights of the three convolutions resident and runs GROUPS groups
  * of 256 threads; a group takes one ROI per iteration: conv1 (FP32), three 32 ->
  * 32 convolutions and the 1x1 head on tcgen05, the birth tables written out.
@@ -910,8 +863,7 @@ __global__ void __launch_bounds__(256) head_kernel(const bf16 *__restrict__ a4, 
  * contiguous bytes), the next one is one padded column away (SBO = 288), and
  * tap (kx, ky) starts (18 kx + ky) 16-byte rows in.  The epilogue of a layer
  * (bias, ReLU, BF16) writes the next layer's input over it once the layer's
- * MMAs completed.  The sums over channels and taps run in conv_tc_kernel's
- * order, so a1..a4 are the same bits as from the kernels that training uses.
+ * MMAs completed.
  *
  * The 1x1 head keeps FP32 weights: each is the exact sum of three BF16 parts
  * (8 significant bits each), a4 is BF16, so loc = a4 Wl^T is three exact-product
@@ -980,10 +932,18 @@ __device__ __forceinline__ uint4 relu_bf16(const float (&v)[8])
     return *(const uint4 *)o;
 }
 
-template <bool WIDE>
-__global__ void __launch_bounds__(256 * INF_GROUPS, 2) infer_kernel(
+/* what training keeps of a forward pass: x0 [roi][p], a1..a4 [roi][p][32] */
+struct Kept {
+    float *x0;
+    bf16 *a[4];
+};
+enum NetMode { NET_INFER, NET_INFER_WIDE, NET_TRAIN }; /* WIDE: `sub` at a 32-byte boundary */
+
+template <int MODE>
+__global__ void __launch_bounds__(256 * INF_GROUPS, 2) net_kernel(
     const float *__restrict__ data, int n, const float *__restrict__ P, const bf16 *__restrict__ Wt,
-    float *__restrict__ cdf, float *__restrict__ sub, float *__restrict__ cnt_out, int *__restrict__ status)
+    float *__restrict__ cdf, float *__restrict__ sub, float *__restrict__ cnt_out, Kept kept,
+    int *__restrict__ status)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float *w1 = (float *)(smem_raw + INF_W1), *bias = (float *)(smem_raw + INF_BIAS);
@@ -1059,17 +1019,20 @@ __global__ void __launch_bounds__(256 * INF_GROUPS, 2) infer_kernel(
         bamf::tc::fence_after_sync();
     };
     for (int r = r0; r < n; r += stride) {
-        /* conv1: the normalisation as conv1_fwd_kernel's (thread = pixel) */
+        /* conv1: the normalisation, thread = pixel */
         const float v = sqrtf(fmaxf(next, 0.0f) + 0.375f);
         if (r + stride < n) next = data[(size_t)(r + stride) * NPX + t];
         float s = v;
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) G.red[warp] = s;
         group_sync();
+        if (MODE == NET_TRAIN && G.dead) break; /* set before this barrier, seen by the whole group */
         float mean = 0.0f;
         for (int k = 0; k < 8; ++k) mean += G.red[k];
         mean *= (1.0f / NPX);
-        G.xp[((t >> 4) + 1) * PS + (t & 15) + 1] = (v - mean) * 0.25f;
+        const float xv = (v - mean) * 0.25f;
+        G.xp[((t >> 4) + 1) * PS + (t & 15) + 1] = xv;
+        if (MODE == NET_TRAIN) kept.x0[(size_t)r * NPX + t] = xv;
         group_sync();
         {
             /* this thread: channels 8 g .. 8 g + 7 of the pixels y = lane & 15,
@@ -1104,7 +1067,10 @@ __global__ void __launch_bounds__(256 * INF_GROUPS, 2) infer_kernel(
             for (int j = 0; j < 4; ++j) {
                 const float o[8] = {z[j][0].x, z[j][0].y, z[j][1].x, z[j][1].y,
                                     z[j][2].x, z[j][2].y, z[j][3].x, z[j][3].y};
-                *(uint4 *)(buf + g * IB_G + ((x0 + 2 * j + 1) * PS + y + 1) * 16) = relu_bf16(o);
+                const uint4 u = relu_bf16(o);
+                *(uint4 *)(buf + g * IB_G + ((x0 + 2 * j + 1) * PS + y + 1) * 16) = u;
+                if (MODE == NET_TRAIN)
+                    ((uint4 *)kept.a[0])[((size_t)r * NPX + (x0 + 2 * j) * S + y) * 4 + g] = u;
             }
         }
 #pragma unroll 1
@@ -1130,15 +1096,21 @@ __global__ void __launch_bounds__(256 * INF_GROUPS, 2) infer_kernel(
             mma_done();
             float d[32];
             bamf::tc::tmem_ld32(tlane + 32 * mt, d);
+            uint4 *keep = MODE == NET_TRAIN
+                              ? (uint4 *)(l == 0 ? kept.a[1] : l == 1 ? kept.a[2] : kept.a[3]) + ((size_t)r * NPX + pe) * 4
+                              : nullptr;
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
                 const float4 ba = ((const float4 *)bias)[(l + 1) * (CH / 4) + 2 * g];
                 const float4 bb = ((const float4 *)bias)[(l + 1) * (CH / 4) + 2 * g + 1];
                 const float o[8] = {d[8 * g] + ba.x,     d[8 * g + 1] + ba.y, d[8 * g + 2] + ba.z, d[8 * g + 3] + ba.w,
                                     d[8 * g + 4] + bb.x, d[8 * g + 5] + bb.y, d[8 * g + 6] + bb.z, d[8 * g + 7] + bb.w};
-                *(uint4 *)(buf + g * IB_G + epi * 16) = relu_bf16(o);
+                const uint4 u = relu_bf16(o);
+                if (MODE != NET_TRAIN || l < 2) *(uint4 *)(buf + g * IB_G + epi * 16) = u;
+                if (MODE == NET_TRAIN) keep[g] = u;
             }
         }
+        if (MODE == NET_TRAIN) continue;
         mma_ready();
         if (warp == 0) {
             const uint32_t one = bamf::tc::elect_one();
@@ -1192,7 +1164,7 @@ __global__ void __launch_bounds__(256 * INF_GROUPS, 2) infer_kernel(
 #pragma unroll
         for (int k = 0; k < NSUB; ++k) e[k] *= inv_se;
         float *dst = sub + ((size_t)r * NPX + pe) * NSUB;
-        if (WIDE) {
+        if (MODE == NET_INFER_WIDE) {
             store8(dst, e);
             store8(dst + 8, e + 8);
         } else {
@@ -1385,18 +1357,14 @@ cudaError_t set_attrs()
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (g_attr_done) return cudaSuccess;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(conv_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_TC)))
-        return e;
-    if ((e = cudaFuncSetAttribute(conv_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_TC)))
+    if ((e = cudaFuncSetAttribute(conv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_TC)))
         return e;
     if ((e = cudaFuncSetAttribute(conv_dw_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_DW)))
         return e;
     if ((e = cudaFuncSetAttribute(head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_HEAD)))
         return e;
-    if ((e = cudaFuncSetAttribute(infer_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_INFER)))
-        return e;
-    if ((e = cudaFuncSetAttribute(infer_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_INFER)))
-        return e;
+    for (const auto kernel : {net_kernel<NET_INFER>, net_kernel<NET_INFER_WIDE>, net_kernel<NET_TRAIN>})
+        if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_INFER))) return e;
     g_attr_done = true;
     return cudaSuccess;
 }
@@ -1412,14 +1380,15 @@ cudaError_t set_attrs()
 
 int grid_for(int n, int per_sm, int sms) { return std::max(1, std::min(n, per_sm * sms)); }
 
+/* CTAs of net_kernel: a ROI per group, two CTAs per SM */
+int net_grid(int n, int sms) { return grid_for((n + INF_GROUPS - 1) / INF_GROUPS, 2, sms); }
+
 /* forward of a batch of n <= capacity ROIs from data, activations kept */
 bamf_status forward(bamf_cnn *net, const float *data, int n, cudaStream_t s)
 {
-    conv1_fwd_kernel<<<n, 256, 0, s>>>(data, n, net->P, net->x0, net->a[0]);
-    for (int l = 0; l < 3; ++l)
-        conv_tc_kernel<0><<<grid_for(n, 3, net->sms), 128, SMEM_TC, s>>>(net->a[l], net->Wf + l * PKT,
-                                                                         net->P + O_B[l], nullptr, net->a[l + 1], n,
-                                                                         net->tc_status);
+    const Kept kept = {net->x0, {net->a[0], net->a[1], net->a[2], net->a[3]}};
+    net_kernel<NET_TRAIN><<<net_grid(n, net->sms), 256 * INF_GROUPS, SMEM_INFER, s>>>(
+        data, n, net->P, net->Wf, nullptr, nullptr, nullptr, kept, net->tc_status);
     CK(cudaGetLastError());
     return BAMF_OK;
 }
@@ -1435,8 +1404,8 @@ bamf_status backward(bamf_cnn *net, const int32_t *n_em, const float *xyi, int n
         const int gdw = grid_for(n, 2, net->sms);
         conv_dw_tc_kernel<<<gdw, 128, SMEM_DW, s>>>(net->a[l], dz, n, net->dwpart, net->tc_status);
         dw_reduce_kernel<<<(DW_PART + 31) / 32, 1024, 0, s>>>(net->dwpart, gdw, net->G + O_W[l], net->G + O_B[l]);
-        conv_tc_kernel<1><<<grid_for(n, 3, net->sms), 128, SMEM_TC, s>>>(dz, net->Wb + l * PKT, nullptr,
-                                                                         net->a[l], dzn, n, net->tc_status);
+        conv_tc_kernel<<<grid_for(n, 3, net->sms), 128, SMEM_TC, s>>>(dz, net->Wb + l * PKT, net->a[l], dzn, n,
+                                                                      net->tc_status);
         bf16 *tmp = dz;
         dz = dzn;
         dzn = tmp;
@@ -1712,9 +1681,9 @@ extern "C" bamf_status bamf_cnn_infer(bamf_cnn *net, const float *data, int n, f
     if (!net || n < 0 || (n > 0 && (!data || !cdf || !sub))) return BAMF_ERR_INVALID_ARG;
     if (n == 0) return BAMF_OK;
     /* 32-byte stores need the table at a 32-byte boundary */
-    const auto kernel = ((uintptr_t)sub & 31) == 0 ? infer_kernel<true> : infer_kernel<false>;
-    kernel<<<grid_for((n + INF_GROUPS - 1) / INF_GROUPS, 2, net->sms), 256 * INF_GROUPS, SMEM_INFER, (cudaStream_t)stream>>>(data, n, net->P, net->Wf, cdf, sub,
-                                                                                count_logits, net->tc_status);
+    const auto kernel = ((uintptr_t)sub & 31) == 0 ? net_kernel<NET_INFER_WIDE> : net_kernel<NET_INFER>;
+    kernel<<<net_grid(n, net->sms), 256 * INF_GROUPS, SMEM_INFER, (cudaStream_t)stream>>>(
+        data, n, net->P, net->Wf, cdf, sub, count_logits, Kept{}, net->tc_status);
     CK(cudaGetLastError());
     return BAMF_OK;
 }
