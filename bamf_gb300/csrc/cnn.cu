@@ -49,8 +49,6 @@ constexpr int C1_NPARAM = O_W2;            /* W1, B1 */
 constexpr int HS = CH + 4;                 /* head kernel: floats per pixel row of H (16-byte rows) */
 /* the WC part of ROI r's head-gradient row */
 __device__ __forceinline__ float *row_wc(float *rows, int r) { return rows + (size_t)r * HEAD_NPARAM + (O_WC - O_WL); }
-constexpr int O_W[3] = {O_W2, O_W3, O_W4};
-constexpr int O_B[3] = {O_B2, O_B3, O_B4};
 constexpr int PKT = 9 * CH * CH; /* tensor-core operand weights of one layer */
 
 typedef __nv_bfloat16 bf16;
@@ -431,7 +429,7 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(const bf16 *__restrict__ i
  * pixel (t & 7) + 8 (t >> 5) + 32 k, channel group (t >> 3) & 3: the 8 lanes
  * of a 16-byte store phase write 8 consecutive pixels of one block, one
  * shared-memory bank group each.  Each CTA writes its partial sums (D, then
- * the 32 bias sums) to its own slice of `part`, coalesced; dw_reduce_kernel
+ * the 32 bias sums) to its own slice of `part`, coalesced; reduce_kernel
  * adds the slices in a fixed order (no atomics, the same bits every run).
  * The mbarrier wait is bounded; a timeout is recorded in *status, the CTA
  * writes zeros, frees its TMEM and returns. */
@@ -575,58 +573,163 @@ __global__ void __launch_bounds__(128) conv_dw_tc_kernel(const bf16 *__restrict_
 }
 
 /* Column sums of a row-major [nrows][width] array of partial sums, in a
- * fixed order (no atomics: the same bits every run).  A CTA of 32 warps owns
- * 32 consecutive columns (lane = column, coalesced): warp w adds rows w,
- * w + 32, ... into four interleaved accumulators; then warp 0 adds the 32
- * warp sums in order.  The result is valid in warp 0. */
+ * fixed order (no atomics: the same bits every run).  A CTA of 8 warps owns 32
+ * consecutive columns (lane = column, coalesced) and adds 32 strands of rows, w,
+ * w + 32, ... into four interleaved accumulators each, four strands per warp (so
+ * that 16 loads are in flight and every CTA of a step is resident at once); then
+ * warp 0 adds the 32 sums in order.  The result is valid in warp 0. */
+constexpr int RED_THREADS = 256;
 __device__ __forceinline__ float column_sum(const float *__restrict__ part, int nrows, int width, int j,
                                             float (*red)[33])
 {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f; /* four loads in flight */
+    constexpr int RW = RED_THREADS / 32, SV = 32 / RW;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float a[SV][4];
+#pragma unroll
+    for (int v = 0; v < SV; ++v)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) a[v][k] = 0.0f;
     if (j < width) {
-        int c = w;
-        for (; c + 96 < nrows; c += 128) {
-            a0 += part[(size_t)c * width + j];
-            a1 += part[(size_t)(c + 32) * width + j];
-            a2 += part[(size_t)(c + 64) * width + j];
-            a3 += part[(size_t)(c + 96) * width + j];
+        const float *p = part + j;
+        int base = 0;
+        for (; base + 128 <= nrows; base += 128)
+#pragma unroll
+            for (int v = 0; v < SV; ++v)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) a[v][k] += p[(size_t)(base + warp + RW * v + 32 * k) * width];
+        if (base < nrows) {
+            float f[SV][4];
+#pragma unroll
+            for (int v = 0; v < SV; ++v)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int c = base + warp + RW * v + 32 * k;
+                    f[v][k] = c < nrows ? p[(size_t)c * width] : 0.0f;
+                }
+#pragma unroll
+            for (int v = 0; v < SV; ++v) {
+                const bool whole = base + warp + RW * v + 96 < nrows;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    a[v][k] += whole || k == 0 ? f[v][k] : 0.0f;
+                    if (k > 0) a[v][0] += whole ? 0.0f : f[v][k];
+                }
+            }
         }
-        for (; c < nrows; c += 32) a0 += part[(size_t)c * width + j];
     }
-    red[w][lane] = (a0 + a1) + (a2 + a3);
+#pragma unroll
+    for (int v = 0; v < SV; ++v) red[warp + RW * v][lane] = (a[v][0] + a[v][1]) + (a[v][2] + a[v][3]);
     __syncthreads();
     float sum = 0.0f;
-    if (w == 0)
+    if (warp == 0)
+#pragma unroll
         for (int k = 0; k < 32; ++k) sum += red[k][lane];
     return sum;
 }
 
-/* out[j] += sum over rows of part[row][j], j < width */
-__global__ void __launch_bounds__(1024) reduce_rows_kernel(const float *__restrict__ part, int nrows, int width,
-                                                           float *__restrict__ out)
-{
-    __shared__ float red[32][33];
-    const int j = blockIdx.x * 32 + (threadIdx.x & 31);
-    const float sum = column_sum(part, nrows, width, j, red);
-    if (threadIdx.x < 32 && j < width) out[j] += sum;
-}
+/* The backward kernels' partial sums, and what a training step does with them. */
+struct Partials {
+    const float *head; /* [nhead][HEAD_NPARAM] */
+    const float *c1;   /* [nc1][C1_NPARAM] */
+    const float *dw;   /* three layers of [ndw][DW_PART], layer l at l * dw_pitch */
+    size_t dw_pitch;
+    int nhead, nc1, ndw;
+};
+struct Optimiser {
+    float *P, *m, *v;
+    bf16 *Wf, *Wb;
+    int *step;      /* the step being taken; incremented by the last CTA */
+    unsigned *done; /* CTAs that have finished; left at zero */
+    int steps_total;
+    float lr0;
+};
+/* CTAs of 32 columns: the head's first (their rows, one per ROI, take longest) */
+constexpr int RB_HEAD = (HEAD_NPARAM + 31) / 32, RB_C1 = (C1_NPARAM + 31) / 32, RB_DW = (DW_PART + 31) / 32;
+constexpr int RB_ALL = RB_HEAD + RB_C1 + 3 * RB_DW;
 
-/* dW[co][ci][3 kx + ky] += sum over CTAs of part[cta][(32 kx + co) * 96 +
- * 32 ky + ci], db[c] += sum of part[cta][96 * 96 + c] */
-__global__ void __launch_bounds__(1024) dw_reduce_kernel(const float *__restrict__ part, int nparts,
-                                                         float *__restrict__ dW, float *__restrict__ db)
+/* Every parameter's gradient from the partial sums, in one launch.  ADAM: the
+ * parameter's Adam update and its BF16 copies for the tensor cores at once;
+ * else grad[j] = the sum.  Bound by latency: of the 34 MB of partial sums (in
+ * L2) the longest chain is a warp's n / 32 rows.  A step of 1024 ROIs ran five
+ * reductions, Adam, the packing and the step count as eight launches, 50 us;
+ * this one takes 13 (28 with a strand per warp of 1024 threads, 19 with two). */
+template <bool ADAM>
+__global__ void __launch_bounds__(RED_THREADS) reduce_kernel(Partials pt, float *__restrict__ grad, Optimiser opt)
 {
     __shared__ float red[32][33];
-    const int j = blockIdx.x * 32 + (threadIdx.x & 31);
-    const float sum = column_sum(part, nparts, DW_PART, j, red);
-    if (threadIdx.x < 32 && j < DW_PART) {
-        if (j < 96 * 96) {
-            const int col = j / 96, row = j - col * 96;
-            const int kx = col >> 5, co = col & 31, ky = row >> 5, ci = row & 31;
-            dW[(co * CH + ci) * 9 + 3 * kx + ky] += sum;
+    const int lane = threadIdx.x & 31;
+    int b = blockIdx.x, l = 0, nrows, width;
+    const float *part;
+    if (b < RB_HEAD) {
+        part = pt.head, nrows = pt.nhead, width = HEAD_NPARAM;
+    } else if (b < RB_HEAD + RB_C1) {
+        b -= RB_HEAD;
+        part = pt.c1, nrows = pt.nc1, width = C1_NPARAM;
+    } else {
+        b -= RB_HEAD + RB_C1;
+        l = b / RB_DW;
+        b -= l * RB_DW;
+        part = pt.dw + l * pt.dw_pitch, nrows = pt.ndw, width = DW_PART;
+    }
+    const int j = b * 32 + lane;
+    const bool mine = threadIdx.x < 32 && j < width;
+    /* the parameter, and a convolution weight's place in the packed operands */
+    int i, of = -1, ob = -1;
+    if (width == HEAD_NPARAM) {
+        i = O_WL + j;
+    } else if (width == C1_NPARAM) {
+        i = O_W1 + j;
+    } else if (j < 96 * 96) {
+        /* column 32 kx + co, row 32 ky + ci of conv_dw_tc_kernel's D */
+        const int col = j / 96, row = j - col * 96;
+        const int kx = col >> 5, co = col & 31, ky = row >> 5, ci = row & 31, tap = 3 * kx + ky;
+        i = (l == 0 ? O_W2 : l == 1 ? O_W3 : O_W4) + (co * CH + ci) * 9 + tap;
+        of = l * PKT + tap * (CH * CH) + (ci >> 3) * (CH * 8) + co * 8 + (ci & 7);
+        ob = l * PKT + (8 - tap) * (CH * CH) + (co >> 3) * (CH * 8) + ci * 8 + (co & 7);
+    } else {
+        i = (l == 0 ? O_B2 : l == 1 ? O_B3 : O_B4) + j - 96 * 96;
+    }
+    /* Adam's inputs, loaded while the sums run */
+    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    float p = 0.0f, m = 0.0f, v = 0.0f, lr = 0.0f, c1 = 0.0f, c2 = 0.0f;
+    int step = 0;
+    if (ADAM) {
+        step = *opt.step;
+        if (mine) {
+            p = opt.P[i];
+            m = opt.m[i];
+            v = opt.v[i];
+            const float frac = opt.steps_total > 1 ? (float)step / (float)(opt.steps_total - 1) : 0.0f;
+            lr = opt.lr0 * (1.0f - 0.9f * fminf(frac, 1.0f));
+            const float t = (float)(step + 1);
+            c1 = 1.0f - powf(b1, t);
+            c2 = 1.0f - powf(b2, t);
+        }
+    }
+    const float g = column_sum(part, nrows, width, j, red);
+    if (mine) {
+        if (ADAM) {
+            const float mi = b1 * m + (1.0f - b1) * g;
+            const float vi = b2 * v + (1.0f - b2) * g * g;
+            opt.m[i] = mi;
+            opt.v[i] = vi;
+            const float mh = mi / c1, vh = vi / c2;
+            p -= lr * mh / (sqrtf(vh) + eps);
+            opt.P[i] = p;
+            if (of >= 0) {
+                opt.Wf[of] = __float2bfloat16_rn(p);
+                opt.Wb[ob] = __float2bfloat16_rn(p);
+            }
         } else {
-            db[j - 96 * 96] += sum;
+            grad[i] = g;
+        }
+    }
+    if (ADAM && threadIdx.x == 0) {
+        /* every CTA has read *step before it counts itself */
+        __threadfence();
+        if (atomicAdd(opt.done, 1u) == gridDim.x - 1) {
+            *opt.done = 0;
+            *opt.step = step + 1;
         }
     }
 }
@@ -804,7 +907,7 @@ __global__ void __launch_bounds__(256) head_kernel(const bf16 *__restrict__ a4, 
         for (int qd = 0; qd < 4; ++qd) dst[qd] = src[qd];
     }
     /* head parameter gradients of this ROI, in the parameter order from O_WL
-     * (WL, BL, WC, BC), into its row of `hrows` (one row per ROI; reduce_rows_kernel
+     * (WL, BL, WC, BC), into its row of `hrows` (one row per ROI; reduce_kernel
      * adds the rows).  dWL[s][c] = sum over pixels of DZ[p][s] H[p][c] and
      * dBL[s] = sum of DZ[p][s]: thread t owns the 2 x 4 block (s0, c0) of
      * tile t & 63 over the pixel quarter t >> 6; the four quarters are added
@@ -1283,30 +1386,7 @@ __global__ void __launch_bounds__(256) init_kernel(const float *__restrict__ cdf
     if (t == 0) init_n[r] = n0;
 }
 
-/* ------------------------------------------------------------------ Adam */
-__global__ void adam_kernel(float *__restrict__ P, float *__restrict__ G, float *__restrict__ m,
-                            float *__restrict__ v, const int *__restrict__ step_dev, int steps_total, float lr0)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NPARAM) return;
-    int step = *step_dev;
-    float frac = steps_total > 1 ? (float)step / (float)(steps_total - 1) : 0.0f;
-    float lr = lr0 * (1.0f - 0.9f * fminf(frac, 1.0f));
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    float g = G[i];
-    float mi = b1 * m[i] + (1.0f - b1) * g;
-    float vi = b2 * v[i] + (1.0f - b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    float t = (float)(step + 1);
-    float mh = mi / (1.0f - powf(b1, t));
-    float vh = vi / (1.0f - powf(b2, t));
-    P[i] -= lr * mh / (sqrtf(vh) + eps);
-    G[i] = 0.0f;
-}
-
-__global__ void step_inc_kernel(int *step_dev) { *step_dev += 1; }
-
+/* ---------------------------------------------------- training examples */
 /* Training batch `step` from caller-provided examples: ROI b of the batch is
  * example (step * batch + b) mod n_examples; counts clipped to the target
  * capacity.  One CTA of NPX threads per ROI. */
@@ -1335,8 +1415,9 @@ struct bamf_cnn {
     float *gdata = nullptr, *gxyi = nullptr;
     int32_t *gn = nullptr;
     int *step = nullptr;
+    unsigned *done = nullptr; /* reduce_kernel's count of finished CTAs */
     int *tc_status = nullptr; /* set by a convolution whose tensor-core wait timed out */
-    float *dwpart = nullptr;  /* per-CTA partial weight gradients, 2 CTAs per SM */
+    float *dwpart = nullptr;  /* per-CTA partial weight gradients, three layers, 2 CTAs per SM */
     float *hpart = nullptr;   /* per-ROI head gradients (MAX_BATCH rows) */
     float *c1part = nullptr;  /* per-CTA conv1 gradients, 4 CTAs per SM */
     float *loss = nullptr;
@@ -1393,29 +1474,26 @@ bamf_status forward(bamf_cnn *net, const float *data, int n, cudaStream_t s)
     return BAMF_OK;
 }
 
-/* loss and gradients (accumulated into G) of the batch whose forward ran */
-bamf_status backward(bamf_cnn *net, const int32_t *n_em, const float *xyi, int n, float inv_batch, cudaStream_t s)
+/* loss and gradients' partial sums of the batch whose forward ran */
+Partials backward(bamf_cnn *net, const int32_t *n_em, const float *xyi, int n, float inv_batch, cudaStream_t s)
 {
+    const Partials pt = {net->hpart, net->c1part, net->dwpart, (size_t)2 * net->sms * DW_PART,
+                         n, grid_for(n, 4, net->sms), grid_for(n, 2, net->sms)};
     head_kernel<<<n, 256, SMEM_HEAD, s>>>(net->a[3], n, net->P, n_em, xyi, inv_batch, net->hpart, net->dzA,
                                                 net->loss, net->step);
     bf16 *dz = net->dzA, *dzn = net->dzB;
     for (int l = 2; l >= 0; --l) {
         /* layer l+2: input a[l], output a[l+1]; dz = dL/dz_{l+2} */
-        const int gdw = grid_for(n, 2, net->sms);
-        conv_dw_tc_kernel<<<gdw, 128, SMEM_DW, s>>>(net->a[l], dz, n, net->dwpart, net->tc_status);
-        dw_reduce_kernel<<<(DW_PART + 31) / 32, 1024, 0, s>>>(net->dwpart, gdw, net->G + O_W[l], net->G + O_B[l]);
+        conv_dw_tc_kernel<<<pt.ndw, 128, SMEM_DW, s>>>(net->a[l], dz, n, net->dwpart + l * pt.dw_pitch,
+                                                       net->tc_status);
         conv_tc_kernel<<<grid_for(n, 3, net->sms), 128, SMEM_TC, s>>>(dz, net->Wb + l * PKT, net->a[l], dzn, n,
                                                                       net->tc_status);
         bf16 *tmp = dz;
         dz = dzn;
         dzn = tmp;
     }
-    reduce_rows_kernel<<<(HEAD_NPARAM + 31) / 32, 1024, 0, s>>>(net->hpart, n, HEAD_NPARAM, net->G + O_WL);
-    const int g1 = grid_for(n, 4, net->sms);
-    conv1_bwd_kernel<<<g1, 256, 0, s>>>(net->x0, dz, n, net->c1part);
-    reduce_rows_kernel<<<(C1_NPARAM + 31) / 32, 1024, 0, s>>>(net->c1part, g1, C1_NPARAM, net->G + O_W1);
-    CK(cudaGetLastError());
-    return BAMF_OK;
+    conv1_bwd_kernel<<<pt.nc1, 256, 0, s>>>(net->x0, dz, n, net->c1part);
+    return pt;
 }
 
 bamf_status pack(bamf_cnn *net, cudaStream_t s)
@@ -1445,7 +1523,7 @@ extern "C" void bamf_cnn_destroy(bamf_cnn *net)
     if (!net) return;
     void *ps[] = {net->P, net->G, net->M, net->V, net->Wf, net->Wb, net->x0, net->a[0], net->a[1], net->a[2],
                   net->a[3], net->dzA, net->dzB, net->gdata, net->gxyi, net->gn, net->step, net->loss,
-                  net->tc_status, net->dwpart, net->hpart, net->c1part};
+                  net->tc_status, net->dwpart, net->hpart, net->c1part, net->done};
     for (void *p : ps)
         if (p) cudaFree(p);
     delete net;
@@ -1466,14 +1544,15 @@ extern "C" bamf_status bamf_cnn_create(bamf_cnn **out, uint32_t seed)
               cudaMalloc(&net->M, NPARAM * 4) == cudaSuccess && cudaMalloc(&net->V, NPARAM * 4) == cudaSuccess &&
               cudaMalloc(&net->Wf, 3 * PKT * 2) == cudaSuccess && cudaMalloc(&net->Wb, 3 * PKT * 2) == cudaSuccess &&
               cudaMalloc(&net->tc_status, sizeof(int)) == cudaSuccess &&
-              cudaMalloc(&net->dwpart, (size_t)2 * net->sms * DW_PART * 4) == cudaSuccess &&
+              cudaMalloc(&net->dwpart, (size_t)3 * 2 * net->sms * DW_PART * 4) == cudaSuccess &&
               cudaMalloc(&net->hpart, B * HEAD_NPARAM * 4) == cudaSuccess &&
               cudaMalloc(&net->c1part, (size_t)4 * net->sms * C1_NPARAM * 4) == cudaSuccess &&
               cudaMalloc(&net->x0, B * NPX * 4) == cudaSuccess && cudaMalloc(&net->dzA, B * NPX * CH * 2) == cudaSuccess &&
               cudaMalloc(&net->dzB, B * NPX * CH * 2) == cudaSuccess &&
               cudaMalloc(&net->gdata, B * NPX * 4) == cudaSuccess &&
               cudaMalloc(&net->gxyi, B * BAMF_SYNTH_NMAX * 3 * 4) == cudaSuccess &&
-              cudaMalloc(&net->gn, B * 4) == cudaSuccess && cudaMalloc(&net->step, sizeof(int)) == cudaSuccess;
+              cudaMalloc(&net->gn, B * 4) == cudaSuccess && cudaMalloc(&net->step, sizeof(int)) == cudaSuccess &&
+              cudaMalloc(&net->done, sizeof(unsigned)) == cudaSuccess;
     for (int l = 0; l < 4 && ok; ++l) ok = cudaMalloc(&net->a[l], B * NPX * CH * 2) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
@@ -1501,6 +1580,7 @@ extern "C" bamf_status bamf_cnn_create(bamf_cnn **out, uint32_t seed)
     bool ok2 = cudaMemcpy(net->P, h.data(), NPARAM * 4, cudaMemcpyHostToDevice) == cudaSuccess &&
                cudaMemset(net->G, 0, NPARAM * 4) == cudaSuccess && cudaMemset(net->M, 0, NPARAM * 4) == cudaSuccess &&
                cudaMemset(net->V, 0, NPARAM * 4) == cudaSuccess && cudaMemset(net->step, 0, sizeof(int)) == cudaSuccess &&
+               cudaMemset(net->done, 0, sizeof(unsigned)) == cudaSuccess &&
                cudaMemset(net->tc_status, 0, sizeof(int)) == cudaSuccess;
     if (!ok2 || pack(net, nullptr) != BAMF_OK || cudaDeviceSynchronize() != cudaSuccess) {
         cudaGetLastError();
@@ -1562,14 +1642,14 @@ extern "C" bamf_status bamf_cnn_loss_grad(bamf_cnn *net, const float *data, cons
     CK(cudaMemcpy(&saved, net->step, sizeof(int), cudaMemcpyDeviceToHost));
     CK(cudaMemset(net->step, 0, sizeof(int)));
     CK(cudaMemset(net->loss, 0, sizeof(float)));
-    CK(cudaMemset(net->G, 0, NPARAM * 4));
     if ((r = forward(net, data, n, nullptr))) return r;
-    if ((r = backward(net, n_em, xyi, n, 1.0f / (float)n, nullptr))) return r;
+    const Partials pt = backward(net, n_em, xyi, n, 1.0f / (float)n, nullptr);
+    reduce_kernel<false><<<RB_ALL, RED_THREADS>>>(pt, net->G, Optimiser{});
+    CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
     if ((r = check_tc(net))) return r;
     if (loss) CK(cudaMemcpy(loss, net->loss, sizeof(float), cudaMemcpyDeviceToHost));
     if (grad) CK(cudaMemcpy(grad, net->G, NPARAM * 4, cudaMemcpyDeviceToHost));
-    CK(cudaMemset(net->G, 0, NPARAM * 4));
     CK(cudaMemcpy(net->step, &saved, sizeof(int), cudaMemcpyHostToDevice));
     return BAMF_OK;
 }
@@ -1590,7 +1670,6 @@ static bamf_status train_graph(bamf_cnn *net, int steps, int batch, float lr, fl
     do {
         if (cudaMemsetAsync(net->step, 0, sizeof(int), s) != cudaSuccess ||
             cudaMemsetAsync(net->loss, 0, (size_t)steps * sizeof(float), s) != cudaSuccess ||
-            cudaMemsetAsync(net->G, 0, NPARAM * 4, s) != cudaSuccess ||
             cudaMemsetAsync(net->M, 0, NPARAM * 4, s) != cudaSuccess ||
             cudaMemsetAsync(net->V, 0, NPARAM * 4, s) != cudaSuccess) {
             res = BAMF_ERR_CUDA;
@@ -1602,13 +1681,12 @@ static bamf_status train_graph(bamf_cnn *net, int steps, int batch, float lr, fl
         }
         produce(s);
         bamf_status r1 = forward(net, net->gdata, batch, s);
-        bamf_status r2 = r1 ? r1 : backward(net, net->gn, net->gxyi, batch, 1.0f / (float)batch, s);
-        adam_kernel<<<(NPARAM + 255) / 256, 256, 0, s>>>(net->P, net->G, net->M, net->V, net->step, steps, lr);
-        pack_kernel<<<(3 * 9 * CH * CH + 255) / 256, 256, 0, s>>>(net->P, net->Wf, net->Wb);
-        step_inc_kernel<<<1, 1, 0, s>>>(net->step);
-        cudaError_t ec = cudaStreamEndCapture(s, &graph);
-        if (r2 || ec != cudaSuccess) {
-            res = r2 ? r2 : BAMF_ERR_CUDA;
+        const Partials pt = backward(net, net->gn, net->gxyi, batch, 1.0f / (float)batch, s);
+        const Optimiser opt = {net->P, net->M, net->V, net->Wf, net->Wb, net->step, net->done, steps, lr};
+        reduce_kernel<true><<<RB_ALL, RED_THREADS, 0, s>>>(pt, nullptr, opt);
+        const cudaError_t el = cudaGetLastError(), ec = cudaStreamEndCapture(s, &graph);
+        if (r1 || el != cudaSuccess || ec != cudaSuccess) {
+            res = r1 ? r1 : BAMF_ERR_CUDA;
             break;
         }
         if (cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {
