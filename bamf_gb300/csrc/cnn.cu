@@ -5,15 +5,11 @@
  * Adam, and a CUDA-graph training step.
  *
  * Layouts.  Activations are channels-last BF16, [roi][p][32] with pixel
- * p = y + 16 x.  The three 32 -> 32 convolutions (forward in net_kernel,
- * input gradient in conv_tc_kernel) run on the 5th-generation tensor cores
- * (tcgen05.mma from shared-memory descriptors into TMEM): per ROI an implicit
- * GEMM with M = 256 pixels (two tiles of 128), N = 32, K = 9 taps x 32
- * channels.  The input gradient is the convolution with the taps flipped and
- * the channel roles swapped (packed once per step).
- * The weight gradient is a GEMM with K = the pixels of every ROI of the
- * CTA, also on tcgen05, with MN-major operands so that the channels-last
- * activations stage without a transpose (conv_dw_tc_kernel).
+ * p = y + 16 x.  The three 32 -> 32 convolutions run on the 5th-generation
+ * tensor cores (tcgen05.mma from shared-memory descriptors into TMEM): the
+ * forward pass in net_kernel, the input and weight gradients in
+ * conv_bwd_kernel, per ROI implicit GEMMs over its 256 pixels whose operands
+ * are the channels-last rows as they lie, without a transpose.
  */
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -252,244 +248,107 @@ __global__ void __launch_bounds__(256) conv1_bwd_kernel(const float *__restrict_
     }
 }
 
-/* -------------------------------------------------- 32 -> 32 convolution */
-/* Input gradient: out = conv(in, W) * (mask > 0).  On the 5th-generation tensor cores: per
- * ROI an implicit GEMM D[pixel][co] = sum over 9 taps of A_tap[pixel][ci]
- * B_tap[co][ci], M = 256 pixels as two tiles of 128, N = 32, K = 32 per tap
- * as two MMAs of 16: 36 tcgen05.mma (BF16 x BF16 -> FP32) issued by one
- * thread into TMEM (64 columns), completion through an mbarrier, epilogue
- * from tcgen05.ld.
+/* ------------------------------------ backward of a 32 -> 32 convolution */
+/* One layer: from act (the layer's input) and dz (dL/d pre-activation of its
+ * output), the input gradient masked by the input's ReLU,
+ *   out[p][ci] = (act[p][ci] > 0) * sum over taps and co of
+ *                dz[p + tap][co] Wb_tap[ci][co],
+ * (Wb: taps flipped, pack_kernel), and the weight and bias gradients
+ *   dW[co][ci][tap] = sum over ROIs and pixels p of act[p + tap][ci] dz[p][co],
+ * tap = 3 kx + ky the shift (kx - 1, ky - 1) in (x, y).
  *
- * A operands straight from shared memory: the ROI is staged as three copies
- * shifted by ky - 1 along y, each [ci group g][padded x 0..17][y 0..15][8 ci]
- * BF16, so that for tap (kx, ky) the 128 rows of M tile t (pixels p = 128 t
- * + m, x = p / 16, y = p mod 16) are 16-byte rows at consecutive addresses
- * from (8 t + kx) * 16 rows into copy ky: K-major core matrices with SBO =
- * 128 B and LBO = one ci group.  Borders stay zero.  One ROI per iteration
- * of a persistent CTA of 128 threads (thread m owns pixels m and 128 + m in
- * the epilogue).  The mbarrier wait is bounded; a timeout is recorded in
- * *status and the kernel frees its TMEM and returns. */
-constexpr int TC_GSTRIDE = PS * S * 16;            /* bytes of one ci group of one copy */
-constexpr int TC_COPY = 4 * TC_GSTRIDE;            /* bytes of one shifted copy */
-constexpr size_t SMEM_TC = (size_t)PKT * 2 + 3 * TC_COPY + 16;
-constexpr uint32_t TC_IDESC = bamf::tc::idesc_bf16_f32(128, 32);
-
-__global__ void __launch_bounds__(128) conv_tc_kernel(const bf16 *__restrict__ in, const bf16 *__restrict__ Wt,
-                                                      const bf16 *__restrict__ mask, bf16 *__restrict__ out, int n,
-                                                      int *__restrict__ status)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    unsigned char *Ws = smem_raw;                    /* [9][4][32][8] bf16 */
-    unsigned char *Cp = smem_raw + PKT * 2;          /* 3 copies */
-    uint64_t *mbar = (uint64_t *)(Cp + 3 * TC_COPY);
-    __shared__ uint32_t tslot;
-    const int t = threadIdx.x, warp = t >> 5;
-    if (warp == 0) bamf::tc::tmem_alloc(&tslot, 64);
-    {
-        const uint4 *src = (const uint4 *)Wt;
-        uint4 *dst = (uint4 *)Ws;
-        for (int i = t; i < PKT * 2 / 16; i += blockDim.x) dst[i] = src[i];
-        const uint4 z = make_uint4(0, 0, 0, 0);
-        uint4 *cc = (uint4 *)Cp;
-        for (int i = t; i < 3 * TC_COPY / 16; i += blockDim.x) cc[i] = z;
-    }
-    if (t == 0) bamf::tc::mbar_init(mbar, 1);
-    bamf::tc::fence_before_sync();
-    __syncthreads();
-    bamf::tc::fence_after_sync();
-    const uint32_t tbase = tslot;
-    const uint32_t ws_addr = bamf::tc::smem_addr(Ws), cp_addr = bamf::tc::smem_addr(Cp);
-    uint32_t phase = 0;
-    bool alive = true;
-    /* each thread carries 8 of the ROI's 1024 16-byte chunks (8 channels of
-     * one pixel): pixels (t & 7) + 8 (t >> 5) + 32 k, channel group
-     * (t >> 3) & 3, so that the 8 lanes of a 16-byte store phase write 8
-     * consecutive pixels of one group (one bank group each); the next ROI's
-     * chunks are loaded while the current ROI's MMAs run, and staged once
-     * they completed */
-    constexpr int CPT = NPX * 4 / 128;
-    const int cg = (t >> 3) & 3, p0 = (t & 7) + 8 * (t >> 5);
-    uint4 pre[CPT];
-    auto load = [&](int r) {
-        const uint4 *src = (const uint4 *)(in + (size_t)r * NPX * CH);
-#pragma unroll
-        for (int k = 0; k < CPT; ++k) pre[k] = src[(p0 + 32 * k) * 4 + cg];
-    };
-    /* each chunk goes to the three shifted copies where it lands inside */
-    auto stage = [&]() {
-#pragma unroll
-        for (int k = 0; k < CPT; ++k) {
-            const int p = p0 + 32 * k, g = cg, x = p >> 4, y = p & 15;
-#pragma unroll
-            for (int ky = 0; ky < 3; ++ky) {
-                const int yo = y - ky + 1;
-                if (yo >= 0 && yo < S)
-                    *(uint4 *)(Cp + ky * TC_COPY + g * TC_GSTRIDE + ((x + 1) * S + yo) * 16) = pre[k];
-            }
-        }
-    };
-    if (blockIdx.x < n) {
-        load(blockIdx.x);
-        stage();
-    }
-    for (int r = blockIdx.x; r < n && alive; r += gridDim.x) {
-        bamf::tc::fence_proxy_async();
-        bamf::tc::fence_before_sync();
-        __syncthreads();
-        bamf::tc::fence_after_sync();
-        if (t == 0) {
-            uint32_t acc = 0;
-#pragma unroll 1
-            for (int mt = 0; mt < 2; ++mt) {
-                acc = 0;
-                for (int tap = 0; tap < 9; ++tap) {
-                    const int kx = tap / 3, ky = tap - kx * 3;
-                    for (int cb = 0; cb < 2; ++cb) {
-                        const uint32_t a = cp_addr + ky * TC_COPY + (2 * cb) * TC_GSTRIDE + (8 * mt + kx) * S * 16;
-                        const uint32_t b = ws_addr + tap * (CH * CH * 2) + (2 * cb) * (CH * 16);
-                        bamf::tc::mma_bf16(tbase + 32 * mt, bamf::tc::smem_desc(a, TC_GSTRIDE, 128),
-                                           bamf::tc::smem_desc(b, CH * 16, 128), TC_IDESC, acc);
-                        acc = 1;
-                    }
-                }
-            }
-            bamf::tc::commit(mbar);
-        }
-        const int rn = r + gridDim.x;
-        if (rn < n) load(rn);
-        /* this thread's two pixels of the ReLU mask, loaded while
-         * the MMAs run */
-        uint4 mk[2][4];
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-            const uint4 *ms = (const uint4 *)(mask + ((size_t)r * NPX + 128 * mt + t) * CH);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) mk[mt][q] = ms[q];
-        }
-        const bool ok = bamf::tc::mbar_wait(mbar, phase, 1u << 24);
-        phase ^= 1u;
-        bamf::tc::fence_after_sync();
-        if (!ok) {
-            if (t == 0) atomicExch(status, 1);
-            alive = false;
-        } else {
-#pragma unroll 1
-            for (int mt = 0; mt < 2; ++mt) {
-                float v[32];
-                bamf::tc::tmem_ld32(tbase + ((uint32_t)(warp * 32) << 16) + 32 * mt, v);
-                const int p = 128 * mt + t;
-                const size_t off = ((size_t)r * NPX + p) * CH;
-                __align__(16) __nv_bfloat162 o[16];
-                __align__(16) uint4 m4[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) m4[q] = mt == 0 ? mk[0][q] : mk[1][q];
-                const __nv_bfloat162 *m2 = (const __nv_bfloat162 *)m4;
-#pragma unroll
-                for (int c = 0; c < 16; ++c)
-                    o[c] = __floats2bfloat162_rn(__bfloat162float(m2[c].x) > 0.0f ? v[2 * c] : 0.0f,
-                                                 __bfloat162float(m2[c].y) > 0.0f ? v[2 * c + 1] : 0.0f);
-                uint4 *dst = (uint4 *)(out + off);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) dst[q] = ((uint4 *)o)[q];
-            }
-        }
-        bamf::tc::fence_before_sync();
-        __syncthreads(); /* TMEM read and copies consumed before the next ROI */
-        bamf::tc::fence_after_sync();
-        alive = __syncthreads_and(alive);
-        if (alive && rn < n) stage();
-    }
-    bamf::tc::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) bamf::tc::tmem_dealloc(tbase, 64);
-}
-
-/* Weight and bias gradient of a 32 -> 32 convolution on the tensor cores:
- * dW[co][ci][tap] += sum over ROIs and pixels p of act[p + tap][ci] dz[p][co]
- * with tap = 3 kx + ky the shift (kx - 1, ky - 1) in (x, y).  Substituting
- * q = p + 16 (kx - 1) (the x shift moves a pixel index by 16),
- *   D[(ky, ci)][(kx, co)] = sum over q in [0, 256) of
- *                           A[(ky, ci)][q] * B[(kx, co)][q],
- *   A[(ky, ci)][q] = act[q + ky - 1][ci] (zero where y(q) + ky - 1 leaves
- *                    the ROI),
- *   B[(kx, co)][q] = dz[q - 16 (kx - 1)][co] (zero outside the ROI),
- * an M = 128 (96 rows (ky, ci), the last 32 rows ignored) x N = 96 x K = 256
- * GEMM per ROI: 16 tcgen05.mma of K = 16, accumulated in TMEM over all ROIs
- * of the CTA (column 32 kx + co).
+ * A persistent CTA takes one ROI per iteration and stages dz once, [padded x][co
+ * group g][padded y][8 co], and act as three copies shifted along y, [x][ky][ci
+ * group g][y][8 ci], copy ky holding act[y + ky - 1] at y.  A 16-byte chunk of the
+ * channels-last tensors (8 channels of one pixel) is a row of a core matrix in
+ * both products, K-major in the first, MN-major in the second:
+ *   input gradient: D[pixel][ci], 18 MMAs of 128 x 32 x 16 for each half y in [8
+ *     h, 8 h + 8) of the ROI: a core matrix is 8 y of one x and g, the next 8 rows
+ *     are the next x, tap (kx, ky) starts kx columns and ky rows in.
+ *   weight gradient: D[(ky, ci)][(j, co)] += sum over y of act[x][y + ky - 1][ci]
+ *     dz[x - 1 + j][y][co], j = 2 - kx, one MMA of 128 x 96 x 16 for each x: the
+ *     columns of dz lie 4 groups apart, so the rows 32 j + co of B are one stride
+ *     and the shift in x costs nothing; rows 96..127 of A are the column after
+ *     (in bounds, ignored).  It stays in TMEM over all ROIs of the CTA.
+ * The next ROI's chunks are loaded into registers while the MMAs run; the input
+ * gradient's epilogue and the bias gradient's sums run during the weight
+ * gradient's MMAs.  Each CTA writes its partial sums (D, then the 32 bias sums) to
+ * its own slice of `part`; reduce_kernel adds the slices in a fixed order (no
+ * atomics, the same bits every run).
  *
- * Both operands MN-major, so that a 16-byte chunk of the channels-last
- * tensors (8 channels of one pixel) is one row of a core matrix and staging
- * is plain 16-byte copies: A as three y-shifted copies of act, B as three
- * x-shifted copies of dz, core matrix (k group j, row block 4 s + g) at
- * j * 1536 + (4 s + g) * 128 (s = ky for A, kx for B).  The ignored rows
- * 96..127 of A read the next k group's rows (in bounds: B follows A).  One
- * ROI per iteration of a persistent CTA of 128 threads, the next ROI's
- * chunks loaded into registers while the MMAs run; the bias gradient (sum of
- * dz over pixels) is formed from the staged chunks.  A lane's chunks are
- * pixel (t & 7) + 8 (t >> 5) + 32 k, channel group (t >> 3) & 3: the 8 lanes
- * of a 16-byte store phase write 8 consecutive pixels of one block, one
- * shared-memory bank group each.  Each CTA writes its partial sums (D, then
- * the 32 bias sums) to its own slice of `part`, coalesced; reduce_kernel
- * adds the slices in a fixed order (no atomics, the same bits every run).
- * The mbarrier wait is bounded; a timeout is recorded in *status, the CTA
+ * Bound by shared memory: 36 MMAs of 40 cycles and 16 of 56 a ROI, 2340 cycles
+ * (two CTAs per SM: 8.6 us for 1024 ROIs).  Measured 24 us for 1024 ROIs, which are
+ * three or four a CTA, so that the first one's loads and the last one's epilogue
+ * stand out; as two kernels, each with its own staging, 38 us.
+ *
+ * The mbarrier waits are bounded; a timeout is recorded in *status, the CTA
  * writes zeros, frees its TMEM and returns. */
-constexpr int DW_KS = 12 * 128;                /* bytes of one k group (8 pixels) */
-constexpr int DW_PART = 96 * 96 + CH;          /* floats of one CTA's partial sums */
-constexpr int DW_ABYTES = 32 * DW_KS;          /* 256 pixels */
-constexpr size_t SMEM_DW = (size_t)2 * DW_ABYTES + 16;
+constexpr int BW_AG = S * 16;                    /* bytes of a group of act: 16 y of 8 channels */
+constexpr int BW_ACOL = 12 * BW_AG;              /* an x column of the three copies of act */
+constexpr int BW_DG = PS * 16;                   /* a group of dz */
+constexpr int BW_DCOL = 4 * BW_DG;               /* an x column of dz */
+constexpr int BW_ACT = PKT * 2;                  /* offsets: weights, act, dz, barriers */
+constexpr int BW_DZ = BW_ACT + S * BW_ACOL + 4 * BW_AG;
+constexpr int BW_BAR = BW_DZ + PS * BW_DCOL;
+constexpr size_t SMEM_BW = BW_BAR + 2 * sizeof(uint64_t);
+constexpr int BW_THREADS = 256;
+constexpr int BW_TMEM = 256;                     /* columns: 96 of dW, 2 x 32 of the input gradient */
+constexpr int DW_PART = 96 * 96 + CH;            /* floats of one CTA's partial sums */
+constexpr uint32_t TC_IDESC = bamf::tc::idesc_bf16_f32(128, 32);
 constexpr uint32_t DW_IDESC = bamf::tc::idesc_bf16_f32_mn(128, 96);
+static_assert(BW_ACT % 16 == 0 && BW_DZ % 16 == 0 && BW_BAR % 16 == 0, "shared-memory alignment");
 
-__global__ void __launch_bounds__(128) conv_dw_tc_kernel(const bf16 *__restrict__ act, const bf16 *__restrict__ dz,
-                                                         int n, float *__restrict__ part, int *__restrict__ status)
+__global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const bf16 *__restrict__ act,
+                                                                 const bf16 *__restrict__ dz,
+                                                                 const bf16 *__restrict__ Wt, int n,
+                                                                 bf16 *__restrict__ out, float *__restrict__ part,
+                                                                 int *__restrict__ status)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    unsigned char *As = smem_raw;
-    unsigned char *Bs = smem_raw + DW_ABYTES;
-    uint64_t *mbar = (uint64_t *)(Bs + DW_ABYTES);
+    unsigned char *const As = smem_raw + BW_ACT, *const Ds = smem_raw + BW_DZ;
+    uint64_t *const bar_in = (uint64_t *)(smem_raw + BW_BAR), *const bar_w = bar_in + 1;
     __shared__ uint32_t tslot;
-    const int t = threadIdx.x, warp = t >> 5;
-    if (warp == 0) bamf::tc::tmem_alloc(&tslot, 128);
-    {
-        const uint4 z = make_uint4(0, 0, 0, 0);
-        uint4 *dst = (uint4 *)smem_raw;
-        for (int i = t; i < 2 * DW_ABYTES / 16; i += blockDim.x) dst[i] = z;
-    }
-    if (t == 0) bamf::tc::mbar_init(mbar, 1);
-    bamf::tc::fence_before_sync();
-    __syncthreads();
-    bamf::tc::fence_after_sync();
-    const uint32_t tbase = tslot;
-    const uint32_t a_addr = bamf::tc::smem_addr(As), b_addr = bamf::tc::smem_addr(Bs);
-    /* each thread carries 8 of the ROI's 1024 chunks of act and of dz */
-    constexpr int CPT = NPX * 4 / 128;
-    const int g = (t >> 3) & 3, p0 = (t & 7) + 8 * (t >> 5);
+    __shared__ float bred[4][CH];
+    const int t = threadIdx.x, lane = t & 31;
+    const int warp = __shfl_sync(0xffffffffu, t >> 5, 0); /* warp-uniform, and known to be */
+    if (warp == 0) bamf::tc::tmem_alloc(&tslot, BW_TMEM);
+    /* chunk k of this thread: pixel p0 + 64 k, channel group g; the 8 lanes of a
+     * 16-byte store phase write 8 consecutive y of one group */
+    constexpr int CPT = NPX * 4 / BW_THREADS;
+    const int g = (t >> 3) & 3, p0 = (t & 7) + 8 * warp;
     uint4 pa[CPT], pd[CPT];
     float bsum[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) bsum[c] = 0.0f;
-    auto load = [&](int r) {
-        const uint4 *sa = (const uint4 *)(act + (size_t)r * NPX * CH);
-        const uint4 *sd = (const uint4 *)(dz + (size_t)r * NPX * CH);
+    const auto load = [&](int r) {
+        const uint4 *sa = (const uint4 *)(act + (size_t)r * NPX * CH) + p0 * 4 + g;
+        const uint4 *sd = (const uint4 *)(dz + (size_t)r * NPX * CH) + p0 * 4 + g;
 #pragma unroll
         for (int k = 0; k < CPT; ++k) {
-            pa[k] = sa[(p0 + 32 * k) * 4 + g];
-            pd[k] = sd[(p0 + 32 * k) * 4 + g];
+            pa[k] = sa[64 * 4 * k];
+            pd[k] = sd[64 * 4 * k];
         }
     };
-    auto stage = [&]() {
+    const auto stage = [&]() {
 #pragma unroll
         for (int k = 0; k < CPT; ++k) {
-            const int p = p0 + 32 * k, y = p & 15;
+            const int p = p0 + 64 * k, x = p >> 4, y = p & 15;
+            *(uint4 *)(Ds + (x + 1) * BW_DCOL + g * BW_DG + (y + 1) * 16) = pd[k];
 #pragma unroll
-            for (int sh = 0; sh < 3; ++sh) {
-                const int yq = y - sh + 1, qa = p - sh + 1; /* A[(sh, .)][qa] = act[p] */
-                if (yq >= 0 && yq < S)
-                    *(uint4 *)(As + (qa >> 3) * DW_KS + (4 * sh + g) * 128 + (qa & 7) * 16) = pa[k];
-                const int qb = p + 16 * (sh - 1); /* B[(sh, .)][qb] = dz[p] */
-                if (qb >= 0 && qb < NPX)
-                    *(uint4 *)(Bs + (qb >> 3) * DW_KS + (4 * sh + g) * 128 + (qb & 7) * 16) = pd[k];
+            for (int ky = 0; ky < 3; ++ky) {
+                const int yo = y - ky + 1;
+                if (yo >= 0 && yo < S) *(uint4 *)(As + x * BW_ACOL + (4 * ky + g) * BW_AG + yo * 16) = pa[k];
             }
-            const __nv_bfloat162 *h = (const __nv_bfloat162 *)&pd[k];
+        }
+    };
+    /* warps 4..7: a group's 8 channels over the pixels (t & 7) + 8 (warp - 4) + 32 k */
+    const auto bias_sums = [&]() {
+        const int pb = p0 - 32;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int p = pb + 32 * k;
+            const uint4 u = *(const uint4 *)(Ds + ((p >> 4) + 1) * BW_DCOL + g * BW_DG + ((p & 15) + 1) * 16);
+            const __nv_bfloat162 *h = (const __nv_bfloat162 *)&u;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const float2 f = __bfloat1622float2(h[c]);
@@ -498,57 +357,107 @@ __global__ void __launch_bounds__(128) conv_dw_tc_kernel(const bf16 *__restrict_
             }
         }
     };
+    if ((int)blockIdx.x < n) load(blockIdx.x);
+    {
+        for (int i = t; i < PKT * 2 / 16; i += BW_THREADS) ((uint4 *)smem_raw)[i] = ((const uint4 *)Wt)[i];
+        const uint4 z = make_uint4(0, 0, 0, 0);
+        for (int i = t; i < (BW_BAR - BW_ACT) / 16; i += BW_THREADS) ((uint4 *)As)[i] = z;
+    }
+    if (t == 0) {
+        bamf::tc::mbar_init(bar_in, 1);
+        bamf::tc::mbar_init(bar_w, 1);
+    }
+    bamf::tc::fence_before_sync();
+    __syncthreads();
+    bamf::tc::fence_after_sync();
+    const uint32_t tw = __shfl_sync(0xffffffffu, tslot, 0), tin = tw + 96;
+    const uint64_t wd = bamf::tc::smem_desc(bamf::tc::smem_addr(smem_raw), CH * 16, 128);
+    const uint64_t dk = bamf::tc::smem_desc(bamf::tc::smem_addr(Ds), BW_DG, BW_DCOL);
+    const uint64_t am = bamf::tc::smem_desc(bamf::tc::smem_addr(As), 128, BW_AG);
+    const uint64_t dm = bamf::tc::smem_desc(bamf::tc::smem_addr(Ds) + 16, 128, BW_DG);
+    /* this thread's pixel of the input gradient: row m of half h */
+    const int h = warp >> 2, m = 32 * (warp & 3) + lane, ex = m >> 3, ey = 8 * h + (m & 7);
+    const uint32_t tlane = (uint32_t)((warp & 3) * 32) << 16;
     bool alive = true, first = true;
     uint32_t phase = 0;
-    if (blockIdx.x < n) {
-        load(blockIdx.x);
-        stage();
-    }
+    if ((int)blockIdx.x < n) stage();
     for (int r = blockIdx.x; r < n && alive; r += gridDim.x) {
         bamf::tc::fence_proxy_async();
         bamf::tc::fence_before_sync();
         __syncthreads();
         bamf::tc::fence_after_sync();
-        if (t == 0) {
-#pragma unroll 1
-            for (int sk = 0; sk < 16; ++sk)
-                bamf::tc::mma_bf16(tbase, bamf::tc::smem_desc(a_addr + 2 * sk * DW_KS, DW_KS, 128),
-                                   bamf::tc::smem_desc(b_addr + 2 * sk * DW_KS, DW_KS, 128), DW_IDESC,
-                                   (first && sk == 0) ? 0u : 1u);
-            bamf::tc::commit(mbar);
+        if (warp == 0) {
+            /* descriptors by adding to the address field (no carry out of it:
+             * shared memory is below 2^18 bytes) */
+            const uint32_t one = bamf::tc::elect_one();
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+                for (int tap = 0; tap < 9; ++tap)
+#pragma unroll
+                    for (int cb = 0; cb < 2; ++cb)
+                        bamf::tc::mma_bf16_warp(
+                            tin + 32 * hh,
+                            dk + (tap / 3 * BW_DCOL + 2 * cb * BW_DG + tap % 3 * 16 + 128 * hh) / 16,
+                            wd + (tap * (CH * CH * 2) + 2 * cb * (CH * 16)) / 16, TC_IDESC, tap + cb > 0 ? 1u : 0u,
+                            one);
+            if (one) bamf::tc::commit(bar_in);
+#pragma unroll
+            for (int x = 0; x < S; ++x)
+                bamf::tc::mma_bf16_warp(tw, am + x * BW_ACOL / 16, dm + x * BW_DCOL / 16, DW_IDESC,
+                                        first && x == 0 ? 0u : 1u, one);
+            if (one) bamf::tc::commit(bar_w);
         }
         first = false;
         const int rn = r + gridDim.x;
         if (rn < n) load(rn);
-        const bool ok = bamf::tc::mbar_wait(mbar, phase, 1u << 24);
+        if (warp >= 4) bias_sums();
+        bool ok = bamf::tc::mbar_wait(bar_in, phase, 1u << 24);
+        bamf::tc::fence_after_sync();
+        if (ok) {
+            float v[32];
+            bamf::tc::tmem_ld32(tin + 32 * h + tlane, v);
+            uint4 *dst = (uint4 *)(out + ((size_t)r * NPX + 16 * ex + ey) * CH);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint4 mk = *(const uint4 *)(As + ex * BW_ACOL + (4 + q) * BW_AG + ey * 16);
+                const __nv_bfloat162 *m2 = (const __nv_bfloat162 *)&mk;
+                __align__(16) __nv_bfloat162 o[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    o[c] = __floats2bfloat162_rn(__bfloat162float(m2[c].x) > 0.0f ? v[8 * q + 2 * c] : 0.0f,
+                                                 __bfloat162float(m2[c].y) > 0.0f ? v[8 * q + 2 * c + 1] : 0.0f);
+                dst[q] = *(const uint4 *)o;
+            }
+        }
+        ok = bamf::tc::mbar_wait(bar_w, phase, 1u << 24) && ok;
         phase ^= 1u;
         bamf::tc::fence_after_sync();
         if (!ok) {
-            if (t == 0) atomicExch(status, 1);
+            atomicExch(status, 1);
             alive = false;
         }
         bamf::tc::fence_before_sync();
-        __syncthreads(); /* the MMAs have read the tiles before they are restaged */
-        bamf::tc::fence_after_sync();
+        /* the MMAs and the epilogue have read the tiles before they are restaged */
         alive = __syncthreads_and(alive);
+        bamf::tc::fence_after_sync();
         if (alive && rn < n) stage();
     }
-    if (blockIdx.x < n) {
+    if ((int)blockIdx.x < n) {
         float *mine = part + (size_t)blockIdx.x * DW_PART;
-        if (warp < 3) {
-            /* warp ky, lane ci: D[(ky, ci)][(kx, co)] in column 32 kx + co,
-             * stored at (32 kx + co) * 96 + 32 ky + ci */
+        if ((warp & 3) < 3) {
+            /* lane 32 ky + ci, column 32 j + co, stored at (32 j + co) * 96 + 32 ky + ci */
 #pragma unroll 1
-            for (int kx = 0; kx < 3; ++kx) {
+            for (int j = h; j < 3; j += 2) {
                 float v[32];
                 if (alive) {
-                    bamf::tc::tmem_ld32(tbase + ((uint32_t)(warp * 32) << 16) + 32 * kx, v);
+                    bamf::tc::tmem_ld32(tw + 32 * j + tlane, v);
                 } else {
 #pragma unroll
                     for (int co = 0; co < CH; ++co) v[co] = 0.0f;
                 }
 #pragma unroll
-                for (int co = 0; co < CH; ++co) mine[(32 * kx + co) * 96 + t] = v[co];
+                for (int co = 0; co < CH; ++co) mine[(32 * j + co) * 96 + m] = v[co];
             }
         }
         /* bias: lanes with equal (lane >> 3) hold the same 8 channels */
@@ -560,16 +469,15 @@ __global__ void __launch_bounds__(128) conv_dw_tc_kernel(const bf16 *__restrict_
             v += __shfl_xor_sync(0xffffffffu, v, 4);
             bsum[c] = v;
         }
-        __shared__ float bred[4][CH];
-        if ((t & 7) == 0)
+        if (warp >= 4 && (t & 7) == 0)
 #pragma unroll
-            for (int c = 0; c < 8; ++c) bred[warp][8 * g + c] = bsum[c];
+            for (int c = 0; c < 8; ++c) bred[warp - 4][8 * g + c] = bsum[c];
         __syncthreads();
         if (t < CH) mine[96 * 96 + t] = alive ? (bred[0][t] + bred[1][t]) + (bred[2][t] + bred[3][t]) : 0.0f;
     }
     bamf::tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) bamf::tc::tmem_dealloc(tbase, 128);
+    if (warp == 0) bamf::tc::tmem_dealloc(tw, BW_TMEM);
 }
 
 /* Column sums of a row-major [nrows][width] array of partial sums, in a
@@ -680,9 +588,9 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_kernel(Partials pt, float 
     } else if (width == C1_NPARAM) {
         i = O_W1 + j;
     } else if (j < 96 * 96) {
-        /* column 32 kx + co, row 32 ky + ci of conv_dw_tc_kernel's D */
+        /* column 32 (2 - kx) + co, row 32 ky + ci of conv_bwd_kernel's D */
         const int col = j / 96, row = j - col * 96;
-        const int kx = col >> 5, co = col & 31, ky = row >> 5, ci = row & 31, tap = 3 * kx + ky;
+        const int kx = 2 - (col >> 5), co = col & 31, ky = row >> 5, ci = row & 31, tap = 3 * kx + ky;
         i = (l == 0 ? O_W2 : l == 1 ? O_W3 : O_W4) + (co * CH + ci) * 9 + tap;
         of = l * PKT + tap * (CH * CH) + (ci >> 3) * (CH * 8) + co * 8 + (ci & 7);
         ob = l * PKT + (8 - tap) * (CH * CH) + (co >> 3) * (CH * 8) + ci * 8 + (co & 7);
@@ -1438,9 +1346,7 @@ cudaError_t set_attrs()
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (g_attr_done) return cudaSuccess;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(conv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_TC)))
-        return e;
-    if ((e = cudaFuncSetAttribute(conv_dw_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_DW)))
+    if ((e = cudaFuncSetAttribute(conv_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BW)))
         return e;
     if ((e = cudaFuncSetAttribute(head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_HEAD)))
         return e;
@@ -1484,10 +1390,8 @@ Partials backward(bamf_cnn *net, const int32_t *n_em, const float *xyi, int n, f
     bf16 *dz = net->dzA, *dzn = net->dzB;
     for (int l = 2; l >= 0; --l) {
         /* layer l+2: input a[l], output a[l+1]; dz = dL/dz_{l+2} */
-        conv_dw_tc_kernel<<<pt.ndw, 128, SMEM_DW, s>>>(net->a[l], dz, n, net->dwpart + l * pt.dw_pitch,
-                                                       net->tc_status);
-        conv_tc_kernel<<<grid_for(n, 3, net->sms), 128, SMEM_TC, s>>>(dz, net->Wb + l * PKT, net->a[l], dzn, n,
-                                                                      net->tc_status);
+        conv_bwd_kernel<<<pt.ndw, BW_THREADS, SMEM_BW, s>>>(net->a[l], dz, net->Wb + l * PKT, n, dzn,
+                                                            net->dwpart + l * pt.dw_pitch, net->tc_status);
         bf16 *tmp = dz;
         dz = dzn;
         dzn = tmp;
