@@ -42,7 +42,6 @@ static_assert(O_B1 == O_W1 + 288 && O_BC + NC == NPARAM, "conv1 block and head l
 constexpr int HEAD_NPARAM = NPARAM - O_WL; /* WL, BL, WC, BC: the heads' parameters, contiguous */
 static_assert(O_BL == O_WL + NSUB * CH && O_WC == O_BL + NSUB && O_BC == O_WC + NC * CH, "head layout");
 constexpr int C1_NPARAM = O_W2;            /* W1, B1 */
-constexpr int HS = CH + 4;                 /* head kernel: floats per pixel row of H (16-byte rows) */
 /* the WC part of ROI r's head-gradient row */
 __device__ __forceinline__ float *row_wc(float *rows, int r) { return rows + (size_t)r * HEAD_NPARAM + (O_WC - O_WL); }
 constexpr int PKT = 9 * CH * CH; /* tensor-core operand weights of one layer */
@@ -643,221 +642,286 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_kernel(Partials pt, float 
 }
 
 /* ----------------------------------------------------------------- heads */
-/* Training: one CTA (256 threads, thread = pixel) per ROI: loss, head
- * gradients (row r of `hrows`, HEAD_NPARAM floats per ROI), dz4 = dL/d(pre-
- * activation of conv4). */
-__global__ void __launch_bounds__(256) head_kernel(const bf16 *__restrict__ a4, int n, const float *__restrict__ P,
-                                                   const int32_t *__restrict__ n_em, const float *__restrict__ xyi,
-                                                   float inv_batch, float *__restrict__ hrows, bf16 *__restrict__ dz4,
-                                                   float *__restrict__ loss_buf, const int *__restrict__ step_dev)
+/* Training: one CTA of 128 threads per ROI: loss, head gradients (row r of
+ * `hrows`, HEAD_NPARAM floats per ROI: WL, BL, WC, BC), dz4 = dL/d(pre-activation of
+ * conv4).  Three products of 131072 FP32 multiply-adds a ROI; as a 16-byte
+ * shared-memory load takes 4 cycles of the SM whether or not its lanes share
+ * addresses, their tiles are 4 pixels x 8 sub-cells (loc), 4 pixels x 16 channels
+ * (dz4) and, a quarter of the pixels per warp, 4 sub-cells x 4 channels (dWL) per
+ * thread, with a4 kept in BF16.  Bound by
+ * issue (27,000 warp instructions a ROI, 12,300 of them multiply-adds): 1024 ROIs
+ * took 53 us with a pixel per thread, 42 with these tiles. */
+constexpr int HD_THREADS = 128;
+constexpr int HD_H = CH + 8;    /* bf16 per pixel row of H, floats per pixel row of D: */
+constexpr int HD_D = NSUB + 4;  /* 80 bytes, 8 rows in distinct banks */
+__device__ __forceinline__ float bf_lo(uint32_t u) { return __uint_as_float(u << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
+
+__global__ void __launch_bounds__(HD_THREADS, 5) head_kernel(const bf16 *__restrict__ a4, int n,
+                                                             const float *__restrict__ P,
+                                                             const int32_t *__restrict__ n_em,
+                                                             const float *__restrict__ xyi, float inv_batch,
+                                                             float *__restrict__ hrows, bf16 *__restrict__ dz4,
+                                                             float *__restrict__ loss_buf,
+                                                             const int *__restrict__ step_dev)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float *H = (float *)smem_raw;             /* [256][HS] */
-    float *DZ = H + NPX * HS;                 /* [256][17] */
+    __shared__ __align__(16) bf16 H[NPX * HD_H];
+    __shared__ __align__(16) float D[NPX * HD_D]; /* loc, then dL/dloc */
     __shared__ __align__(16) float Wl[NSUB * CH];
+    __shared__ __align__(16) float dg[CH];
     __shared__ float bl[NSUB], Wc[NC * CH], bc[NC];
-    __shared__ float red[8], gmean[CH], part[8][CH], zc[NC], dzc[NC], dg[CH];
+    __shared__ float part[8][CH], gmean[CH], dzc[NC], red[8], wmax[4];
     __shared__ float ex[BAMF_SYNTH_NMAX], ey[BAMF_SYNTH_NMAX];
-    __shared__ float sm_max, sm_sum, loss_loc_sh;
+    __shared__ float lcnt_sh, lsum[4];
     const int r = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    if (r >= n) return;
-    for (int i = t; i < NSUB * CH; i += 256) Wl[i] = P[O_WL + i];
-    for (int i = t; i < NC * CH; i += 256) Wc[i] = P[O_WC + i];
+    for (int i = t; i < NPX * 4; i += HD_THREADS)
+        *(uint4 *)(H + (i >> 2) * HD_H + (i & 3) * 8) = ((const uint4 *)(a4 + (size_t)r * NPX * CH))[i];
+    ((float4 *)Wl)[t] = make_float4(P[O_WL + 4 * t], P[O_WL + 4 * t + 1], P[O_WL + 4 * t + 2], P[O_WL + 4 * t + 3]);
+    for (int i = t; i < NC * CH; i += HD_THREADS) Wc[i] = P[O_WC + i];
     if (t < NSUB) bl[t] = P[O_BL + t];
     if (t < NC) bc[t] = P[O_BC + t];
-    float h[CH];
-    {
-        const uint4 *src = (const uint4 *)(a4 + ((size_t)r * NPX + t) * CH);
-        for (int qd = 0; qd < 4; ++qd) {
-            uint4 u = src[qd];
-            const bf16 *b = (const bf16 *)&u;
-            for (int e = 0; e < 8; ++e) h[qd * 8 + e] = __bfloat162float(b[e]);
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < CH / 4; ++q)
-        ((float4 *)H)[t * (HS / 4) + q] = make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
-    __syncthreads();
-    float z[NSUB];
-    float mx = -INFINITY;
-    for (int s = 0; s < NSUB; ++s) {
-        float v = bl[s];
-#pragma unroll
-        for (int q = 0; q < CH / 4; ++q) {
-            const float4 w = ((const float4 *)Wl)[s * (CH / 4) + q];
-            v += w.x * h[4 * q];
-            v += w.y * h[4 * q + 1];
-            v += w.z * h[4 * q + 2];
-            v += w.w * h[4 * q + 3];
-        }
-        z[s] = v;
-        mx = fmaxf(mx, v);
-    }
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) red[warp] = mx;
-    /* count head: mean of a4 over pixels */
-    {
-        int c = t & 31, grp = t >> 5;
-        float sacc = 0.0f;
-        for (int p = grp; p < NPX; p += 8) sacc += H[p * HS + c];
-        part[grp][c] = sacc;
-    }
-    __syncthreads();
-    if (t == 0) {
-        float m = red[0];
-        for (int k = 1; k < 8; ++k) m = fmaxf(m, red[k]);
-        sm_max = m;
-    }
-    if (t < CH) {
-        float sacc = 0.0f;
-        for (int k = 0; k < 8; ++k) sacc += part[k][t];
-        gmean[t] = sacc * (1.0f / NPX);
-    }
-    __syncthreads();
-    float e[NSUB], se = 0.0f;
-    for (int s = 0; s < NSUB; ++s) {
-        e[s] = expf(z[s] - sm_max);
-        se += e[s];
-    }
-    float tot = se;
-    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    if (lane == 0) red[warp] = tot;
-    if (t < NC) {
-        float v = bc[t];
-        for (int c = 0; c < CH; ++c) v += Wc[t * CH + c] * gmean[c];
-        zc[t] = v;
-    }
-    __syncthreads();
-    if (t == 0) {
-        float sacc = 0.0f;
-        for (int k = 0; k < 8; ++k) sacc += red[k];
-        sm_sum = sacc;
-    }
-    __syncthreads();
-    const float inv_sum = 1.0f / sm_sum;
-    /* ---- targets, loss, gradients */
-    const int ntrue = n_em[r];
     if (t < BAMF_SYNTH_NMAX) {
         ex[t] = xyi[((size_t)r * BAMF_SYNTH_NMAX + t) * 3 + 0];
         ey[t] = xyi[((size_t)r * BAMF_SYNTH_NMAX + t) * 3 + 1];
     }
-    if (t == 0) loss_loc_sh = 0.0f;
+    const int ntrue = n_em[r];
     __syncthreads();
-    const int px = t / S, py = t - (t / S) * S;
-    float tgt[NSUB];
-    for (int s = 0; s < NSUB; ++s) tgt[s] = 0.0f;
+    { /* loc = Wl a4 + bl */
+        const int s0 = 8 * (lane >> 4), q0 = 64 * warp + (lane & 15); /* pixels q0 + 16 j */
+        float z[4][8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) z[j][s] = bl[s0 + s];
+#pragma unroll 1
+        for (int c8 = 0; c8 < CH; c8 += 8) {
+            uint4 u[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) u[j] = *(const uint4 *)(H + (q0 + 16 * j) * HD_H + c8);
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                float hv[4][4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t a = hf ? u[j].z : u[j].x, b = hf ? u[j].w : u[j].y;
+                    hv[j][0] = bf_lo(a);
+                    hv[j][1] = bf_hi(a);
+                    hv[j][2] = bf_lo(b);
+                    hv[j][3] = bf_hi(b);
+                }
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    const float4 w = *(const float4 *)(Wl + (s0 + s) * CH + c8 + 4 * hf);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        z[j][s] += w.x * hv[j][0];
+                        z[j][s] += w.y * hv[j][1];
+                        z[j][s] += w.z * hv[j][2];
+                        z[j][s] += w.w * hv[j][3];
+                    }
+                }
+            }
+        }
+        float mx = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float4 *row = (float4 *)(D + (q0 + 16 * j) * HD_D + s0);
+            row[0] = make_float4(z[j][0], z[j][1], z[j][2], z[j][3]);
+            row[1] = make_float4(z[j][4], z[j][5], z[j][6], z[j][7]);
+#pragma unroll
+            for (int s = 0; s < 8; ++s) mx = fmaxf(mx, z[j][s]);
+        }
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (lane == 0) wmax[warp] = mx;
+    }
+    /* count head: mean of a4 over pixels (channel lane, pixels k, k + 8, ...) */
+#pragma unroll
+    for (int k = warp; k < 8; k += 4) {
+        float sacc = 0.0f;
+#pragma unroll 8
+        for (int p = k; p < NPX; p += 8) sacc += __bfloat162float(H[p * HD_H + lane]);
+        part[k][lane] = sacc;
+    }
+    __syncthreads();
+    const float mx = fmaxf(fmaxf(wmax[0], wmax[1]), fmaxf(wmax[2], wmax[3]));
+    /* softmax over all sub-cells: thread = pixels t and t + 128 */
+    float e[2][NSUB];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        float se = 0.0f;
+#pragma unroll
+        for (int q = 0; q < NSUB / 4; ++q) {
+            const float4 z = *(const float4 *)(D + (t + 128 * j) * HD_D + 4 * q);
+            e[j][4 * q] = expf(z.x - mx);
+            e[j][4 * q + 1] = expf(z.y - mx);
+            e[j][4 * q + 2] = expf(z.z - mx);
+            e[j][4 * q + 3] = expf(z.w - mx);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) se += e[j][4 * q + k];
+        }
+        for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
+        if (lane == 0) red[warp + 4 * j] = se;
+    }
+    if (warp == 3) { /* count head: logits, loss, gradients */
+        float g = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) g += part[k][lane];
+        gmean[lane] = g * (1.0f / NPX);
+        __syncwarp();
+        float zc = -INFINITY;
+        if (lane < NC) {
+            zc = bc[lane];
+            for (int c = 0; c < CH; ++c) zc += Wc[lane * CH + c] * gmean[c];
+        }
+        float m = zc;
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const float ec = lane < NC ? expf(zc - m) : 0.0f;
+        float sacc = 0.0f;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) sacc += __shfl_sync(0xffffffffu, ec, c);
+        const int cls = min(ntrue, NC - 1);
+        if (lane == cls) lcnt_sh = -(zc - m - logf(sacc));
+        if (lane < NC) dzc[lane] = (ec / sacc - (lane == cls ? 1.0f : 0.0f)) * inv_batch;
+        __syncwarp();
+        float v = 0.0f;
+        for (int c = 0; c < NC; ++c) v += Wc[c * CH + lane] * dzc[c];
+        dg[lane] = v * (1.0f / NPX);
+    }
+    __syncthreads();
+    float sum = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sum += red[k];
+    const float inv_sum = 1.0f / sum, logS = logf(sum) + mx;
+    /* targets, loss, dL/dloc */
     int nin = 0;
+    uint64_t tg[2][2] = {{0, 0}, {0, 0}}; /* emitters per sub-cell of the two pixels, 8 bits each */
     for (int k = 0; k < ntrue; ++k) {
-        float X = ex[k], Y = ey[k];
+        const float X = ex[k], Y = ey[k];
         if (!(X >= 0.0f && X < (float)S && Y >= 0.0f && Y < (float)S)) continue;
         nin++;
-        int cx = min((int)X, S - 1), cy = min((int)Y, S - 1);
-        if (cx == px && cy == py) {
-            int s = min((int)((Y - (float)cy) * 4.0f), 3) + 4 * min((int)((X - (float)cx) * 4.0f), 3);
-            tgt[s] += 1.0f;
-        }
-    }
-    const float wloc = nin > 0 ? 1.0f / (float)nin : 0.0f;
-    float lloc = 0.0f;
-    const float logS = logf(sm_sum) + sm_max;
-    for (int s = 0; s < NSUB; ++s) {
-        if (tgt[s] > 0.0f) lloc -= tgt[s] * wloc * (z[s] - logS);
-        float d = (e[s] * inv_sum - tgt[s] * wloc) * (nin > 0 ? inv_batch : 0.0f);
-        DZ[t * (NSUB + 1) + s] = d;
-    }
-    for (int o = 16; o > 0; o >>= 1) lloc += __shfl_xor_sync(0xffffffffu, lloc, o);
-    if (lane == 0) atomicAdd(&loss_loc_sh, lloc);
-    if (t == 0) {
-        float m = zc[0];
-        for (int c = 1; c < NC; ++c) m = fmaxf(m, zc[c]);
-        float sacc = 0.0f;
-        for (int c = 0; c < NC; ++c) sacc += expf(zc[c] - m);
-        int cls = min(ntrue, NC - 1);
-        float lcnt = -(zc[cls] - m - logf(sacc));
-        for (int c = 0; c < NC; ++c) dzc[c] = (expf(zc[c] - m) / sacc - (c == cls ? 1.0f : 0.0f)) * inv_batch;
-        red[0] = lcnt;
-    }
-    __syncthreads();
-    if (t == 0) {
-        float l = (loss_loc_sh + red[0]) * inv_batch;
-        atomicAdd(&loss_buf[step_dev ? *step_dev : 0], l);
-    }
-    if (t < CH) {
-        float v = 0.0f;
-        for (int c = 0; c < NC; ++c) v += Wc[c * CH + t] * dzc[c];
-        dg[t] = v * (1.0f / NPX);
-    }
-    __syncthreads();
-    /* dz4 of this pixel */
-    {
-        float dzr[NSUB];
+        const int cx = min((int)X, S - 1), cy = min((int)Y, S - 1), p = cx * S + cy;
+        const int s = min((int)((Y - (float)cy) * 4.0f), 3) + 4 * min((int)((X - (float)cx) * 4.0f), 3);
+        const uint64_t one = 1ull << (8 * (s & 7));
 #pragma unroll
-        for (int k = 0; k < NSUB; ++k) dzr[k] = DZ[t * (NSUB + 1) + k];
-        __align__(16) bf16 o[CH];
-#pragma unroll
-        for (int q = 0; q < CH / 4; ++q) {
-            float v0 = dg[4 * q], v1 = dg[4 * q + 1], v2 = dg[4 * q + 2], v3 = dg[4 * q + 3];
-#pragma unroll
-            for (int k = 0; k < NSUB; ++k) {
-                const float4 w = ((const float4 *)Wl)[k * (CH / 4) + q];
-                v0 += dzr[k] * w.x;
-                v1 += dzr[k] * w.y;
-                v2 += dzr[k] * w.z;
-                v3 += dzr[k] * w.w;
+        for (int j = 0; j < 2; ++j)
+            if (p == t + 128 * j) {
+                tg[j][0] += s < 8 ? one : 0;
+                tg[j][1] += s < 8 ? 0 : one;
             }
-            o[4 * q] = __float2bfloat16_rn(h[4 * q] > 0.0f ? v0 : 0.0f);
-            o[4 * q + 1] = __float2bfloat16_rn(h[4 * q + 1] > 0.0f ? v1 : 0.0f);
-            o[4 * q + 2] = __float2bfloat16_rn(h[4 * q + 2] > 0.0f ? v2 : 0.0f);
-            o[4 * q + 3] = __float2bfloat16_rn(h[4 * q + 3] > 0.0f ? v3 : 0.0f);
-        }
-        uint4 *dst = (uint4 *)(dz4 + ((size_t)r * NPX + t) * CH);
-        const uint4 *src = (const uint4 *)o;
-        for (int qd = 0; qd < 4; ++qd) dst[qd] = src[qd];
     }
-    /* head parameter gradients of this ROI, in the parameter order from O_WL
-     * (WL, BL, WC, BC), into its row of `hrows` (one row per ROI; reduce_kernel
-     * adds the rows).  dWL[s][c] = sum over pixels of DZ[p][s] H[p][c] and
-     * dBL[s] = sum of DZ[p][s]: thread t owns the 2 x 4 block (s0, c0) of
-     * tile t & 63 over the pixel quarter t >> 6; the four quarters are added
-     * through shared memory (over H, once every thread has read it). */
+    const float wloc = nin > 0 ? 1.0f / (float)nin : 0.0f, scale = nin > 0 ? inv_batch : 0.0f;
+    float lloc[2] = {0.0f, 0.0f};
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        float *row = D + (t + 128 * j) * HD_D;
+        if (tg[j][0] | tg[j][1]) {
+#pragma unroll
+            for (int s = 0; s < NSUB; ++s) {
+                const float tgt = (float)(uint32_t)(tg[j][s >> 3] >> (8 * (s & 7)) & 255u);
+                if (tgt > 0.0f) lloc[j] -= tgt * wloc * (row[s] - logS);
+                e[j][s] = (e[j][s] * inv_sum - tgt * wloc) * scale;
+            }
+        } else {
+#pragma unroll
+            for (int s = 0; s < NSUB; ++s) e[j][s] = e[j][s] * inv_sum * scale;
+        }
+#pragma unroll
+        for (int q = 0; q < NSUB / 4; ++q)
+            *(float4 *)(row + 4 * q) = make_float4(e[j][4 * q], e[j][4 * q + 1], e[j][4 * q + 2], e[j][4 * q + 3]);
+    }
     {
-        const int tile = t & 63, quarter = t >> 6;
-        const int s0 = 2 * (tile >> 3), c0 = 4 * (tile & 7);
-        float g0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, g1[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gb0 = 0.0f, gb1 = 0.0f;
+        float l = lloc[0] + lloc[1];
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if (lane == 0) lsum[warp] = l;
+    }
+    __syncthreads();
+    if (t == 0)
+        atomicAdd(&loss_buf[*step_dev], (((lsum[0] + lsum[1]) + (lsum[2] + lsum[3])) + lcnt_sh) * inv_batch);
+    { /* dz4: pixels q0 + 16 j, channels c0 .. c0 + 15 */
+        const int c0 = 16 * (lane & 1), q0 = 64 * warp + (lane >> 1);
+        float v[4][16];
+#pragma unroll
+        for (int c = 0; c < 16; c += 4) {
+            const float4 b = *(const float4 *)(dg + c0 + c);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[j][c] = b.x;
+                v[j][c + 1] = b.y;
+                v[j][c + 2] = b.z;
+                v[j][c + 3] = b.w;
+            }
+        }
+#pragma unroll 1
+        for (int k4 = 0; k4 < NSUB; k4 += 4) {
+            float d[4][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) *(float4 *)d[j] = *(const float4 *)(D + (q0 + 16 * j) * HD_D + k4);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int c = 0; c < 16; c += 4) {
+                    const float4 w = *(const float4 *)(Wl + (k4 + k) * CH + c0 + c);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        v[j][c] += d[j][k] * w.x;
+                        v[j][c + 1] += d[j][k] * w.y;
+                        v[j][c + 2] += d[j][k] * w.z;
+                        v[j][c + 3] += d[j][k] * w.w;
+                    }
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int p = q0 + 16 * j;
+            uint4 *dst = (uint4 *)(dz4 + ((size_t)r * NPX + p) * CH + c0);
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                const uint4 u = *(const uint4 *)(H + p * HD_H + c0 + 8 * hf);
+                const uint32_t hw[4] = {u.x, u.y, u.z, u.w};
+                __align__(16) __nv_bfloat162 o[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    o[k] = __floats2bfloat162_rn(bf_lo(hw[k]) > 0.0f ? v[j][8 * hf + 2 * k] : 0.0f,
+                                                 bf_hi(hw[k]) > 0.0f ? v[j][8 * hf + 2 * k + 1] : 0.0f);
+                dst[hf] = *(const uint4 *)o;
+            }
+        }
+    }
+    /* dWL[s][c] = sum over pixels of D[p][s] H[p][c] and dBL[s] = sum of D[p][s]: warp
+     * w adds the pixels 64 w .. 64 w + 63, lane the 4 x 4 block (s0, c0); the four
+     * warps' sums are added through shared memory (over D, once it has been read) */
+    {
+        const int s0 = 4 * (lane >> 3), c0 = 4 * (lane & 7);
+        float g[4][4] = {}, gb[4] = {};
 #pragma unroll 4
-        for (int p = 64 * quarter; p < 64 * quarter + 64; ++p) {
-            const float4 hv = ((const float4 *)H)[p * (HS / 4) + (c0 >> 2)];
-            const float d0 = DZ[p * (NSUB + 1) + s0], d1 = DZ[p * (NSUB + 1) + s0 + 1];
-            g0[0] += d0 * hv.x;
-            g0[1] += d0 * hv.y;
-            g0[2] += d0 * hv.z;
-            g0[3] += d0 * hv.w;
-            g1[0] += d1 * hv.x;
-            g1[1] += d1 * hv.y;
-            g1[2] += d1 * hv.z;
-            g1[3] += d1 * hv.w;
-            gb0 += d0;
-            gb1 += d1;
+        for (int p = 64 * warp; p < 64 * warp + 64; ++p) {
+            const uint2 u = *(const uint2 *)(H + p * HD_H + c0);
+            const float4 d4 = *(const float4 *)(D + p * HD_D + s0);
+            const float hv[4] = {bf_lo(u.x), bf_hi(u.x), bf_lo(u.y), bf_hi(u.y)}, d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                gb[a] += d[a];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) g[a][k] += d[a] * hv[k];
+            }
         }
         __syncthreads();
-        constexpr int QW = NSUB * CH + NSUB; /* one quarter's WL and BL sums */
-        float *red = H + quarter * QW;
+        constexpr int QW = NSUB * CH + NSUB; /* one warp's WL and BL sums */
+        float *q = D + warp * QW;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            red[s0 * CH + c0 + k] = g0[k];
-            red[(s0 + 1) * CH + c0 + k] = g1[k];
-        }
-        if ((tile & 7) == 0) {
-            red[NSUB * CH + s0] = gb0;
-            red[NSUB * CH + s0 + 1] = gb1;
+        for (int a = 0; a < 4; ++a) {
+            *(float4 *)(q + (s0 + a) * CH + c0) = make_float4(g[a][0], g[a][1], g[a][2], g[a][3]);
+            if ((lane & 7) == 0) q[NSUB * CH + s0 + a] = gb[a];
         }
         __syncthreads();
         float *row = hrows + (size_t)r * HEAD_NPARAM;
-        for (int o = t; o < QW; o += 256) row[o] = (H[o] + H[QW + o]) + (H[2 * QW + o] + H[3 * QW + o]);
+        for (int o = t; o < QW; o += HD_THREADS) row[o] = (D[o] + D[QW + o]) + (D[2 * QW + o] + D[3 * QW + o]);
     }
-    for (int o = t; o < NC * CH; o += 256) row_wc(hrows, r)[o] = dzc[o / CH] * gmean[o - (o / CH) * CH];
+    for (int o = t; o < NC * CH; o += HD_THREADS) row_wc(hrows, r)[o] = dzc[o / CH] * gmean[o - (o / CH) * CH];
     if (t < NC) row_wc(hrows, r)[NC * CH + t] = dzc[t];
 }
+static_assert(4 * (NSUB * CH + NSUB) <= NPX * HD_D && NSUB * CH == 4 * HD_THREADS && BAMF_SYNTH_NMAX <= HD_THREADS,
+              "head_kernel's shared memory and loads");
 
 /* ------------------------------------------------------ fused forward */
 /* The whole network on a ROI without leaving the SM (NET_TRAIN: up to a4, the
@@ -1339,16 +1403,12 @@ namespace {
 std::mutex g_attr_mutex;
 bool g_attr_done = false;
 
-const size_t SMEM_HEAD = (size_t)(NPX * HS + NPX * (NSUB + 1)) * sizeof(float);
-
 cudaError_t set_attrs()
 {
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (g_attr_done) return cudaSuccess;
     cudaError_t e;
     if ((e = cudaFuncSetAttribute(conv_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BW)))
-        return e;
-    if ((e = cudaFuncSetAttribute(head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_HEAD)))
         return e;
     for (const auto kernel : {net_kernel<NET_INFER>, net_kernel<NET_INFER_WIDE>, net_kernel<NET_TRAIN>})
         if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_INFER))) return e;
@@ -1385,8 +1445,8 @@ Partials backward(bamf_cnn *net, const int32_t *n_em, const float *xyi, int n, f
 {
     const Partials pt = {net->hpart, net->c1part, net->dwpart, (size_t)2 * net->sms * DW_PART,
                          n, grid_for(n, 4, net->sms), grid_for(n, 2, net->sms)};
-    head_kernel<<<n, 256, SMEM_HEAD, s>>>(net->a[3], n, net->P, n_em, xyi, inv_batch, net->hpart, net->dzA,
-                                                net->loss, net->step);
+    head_kernel<<<n, HD_THREADS, 0, s>>>(net->a[3], n, net->P, n_em, xyi, inv_batch, net->hpart, net->dzA, net->loss,
+                                         net->step);
     bf16 *dz = net->dzA, *dzn = net->dzB;
     for (int l = 2; l >= 0; --l) {
         /* layer l+2: input a[l], output a[l+1]; dz = dL/dz_{l+2} */
