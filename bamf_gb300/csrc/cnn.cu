@@ -247,8 +247,8 @@ __global__ void __launch_bounds__(256) conv1_bwd_kernel(const float *__restrict_
     }
 }
 
-/* ------------------------------------ backward of a 32 -> 32 convolution */
-/* One layer: from act (the layer's input) and dz (dL/d pre-activation of its
+/* ------------------------------------ backward of the 32 -> 32 convolutions */
+/* Per layer, last one first: from act (the layer's input) and dz (dL/d pre-activation of its
  * output), the input gradient masked by the input's ReLU,
  *   out[p][ci] = (act[p][ci] > 0) * sum over taps and co of
  *                dz[p + tap][co] Wb_tap[ci][co],
@@ -256,7 +256,9 @@ __global__ void __launch_bounds__(256) conv1_bwd_kernel(const float *__restrict_
  *   dW[co][ci][tap] = sum over ROIs and pixels p of act[p + tap][ci] dz[p][co],
  * tap = 3 kx + ky the shift (kx - 1, ky - 1) in (x, y).
  *
- * A persistent CTA takes one ROI per iteration and stages dz once, [padded x][co
+ * As a layer needs nothing of other ROIs, a persistent CTA runs its ROIs through
+ * all three layers, one ROI per iteration, dz going back and forth between two
+ * buffers of which it reads only what it wrote itself.  It stages dz once, [padded x][co
  * group g][padded y][8 co], and act as three copies shifted along y, [x][ky][ci
  * group g][y][8 ci], copy ky holding act[y + ky - 1] at y.  A 16-byte chunk of the
  * channels-last tensors (8 channels of one pixel) is a row of a core matrix in
@@ -276,9 +278,10 @@ __global__ void __launch_bounds__(256) conv1_bwd_kernel(const float *__restrict_
  * atomics, the same bits every run).
  *
  * Bound by shared memory: 36 MMAs of 40 cycles and 16 of 56 a ROI, 2340 cycles
- * (two CTAs per SM: 8.6 us for 1024 ROIs).  Measured 24 us for 1024 ROIs, which are
- * three or four a CTA, so that the first one's loads and the last one's epilogue
- * stand out; as two kernels, each with its own staging, 38 us.
+ * and layer (two CTAs per SM: 26 us for 1024 ROIs).  1024 ROIs are three or four a
+ * CTA, so what a launch costs before its first MMA (2.6 to 4 us of allocation, first
+ * loads and cold instructions) stands out: two kernels per layer, each with its own
+ * staging, took 115 us, one per layer 72, this one 64.
  *
  * The mbarrier waits are bounded; a timeout is recorded in *status, the CTA
  * writes zeros, frees its TMEM and returns. */
@@ -297,11 +300,15 @@ constexpr uint32_t TC_IDESC = bamf::tc::idesc_bf16_f32(128, 32);
 constexpr uint32_t DW_IDESC = bamf::tc::idesc_bf16_f32_mn(128, 96);
 static_assert(BW_ACT % 16 == 0 && BW_DZ % 16 == 0 && BW_BAR % 16 == 0, "shared-memory alignment");
 
-__global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const bf16 *__restrict__ act,
-                                                                 const bf16 *__restrict__ dz,
-                                                                 const bf16 *__restrict__ Wt, int n,
-                                                                 bf16 *__restrict__ out, float *__restrict__ part,
-                                                                 int *__restrict__ status)
+struct Backward {
+    const bf16 *act[3]; /* the layers' inputs */
+    bf16 *dz[2];        /* dL/dz of the last layer in dz[0]; layers 2, 1, 0 leave theirs in dz[1], [0], [1] */
+    const bf16 *Wb;     /* packed weights, three layers */
+    float *part;        /* layer l's slices at l * pitch */
+    size_t pitch;
+};
+
+__global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const Backward bw, int n, int *__restrict__ status)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char *const As = smem_raw + BW_ACT, *const Ds = smem_raw + BW_DZ;
@@ -317,16 +324,18 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const bf16 *__r
     const int g = (t >> 3) & 3, p0 = (t & 7) + 8 * warp;
     uint4 pa[CPT], pd[CPT];
     float bsum[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) bsum[c] = 0.0f;
-    const auto load = [&](int r) {
-        const uint4 *sa = (const uint4 *)(act + (size_t)r * NPX * CH) + p0 * 4 + g;
-        const uint4 *sd = (const uint4 *)(dz + (size_t)r * NPX * CH) + p0 * 4 + g;
+    const auto load = [&](int l, int r) {
+        const uint4 *sa = (const uint4 *)(bw.act[l] + (size_t)r * NPX * CH) + p0 * 4 + g;
+        const uint4 *sd = (const uint4 *)(bw.dz[l & 1] + (size_t)r * NPX * CH) + p0 * 4 + g;
 #pragma unroll
         for (int k = 0; k < CPT; ++k) {
             pa[k] = sa[64 * 4 * k];
-            pd[k] = sd[64 * 4 * k];
+            pd[k] = __ldcg(sd + 64 * 4 * k); /* written by this kernel: not through the read-only path */
         }
+    };
+    const auto weights = [&](int l) {
+        for (int i = t; i < PKT * 2 / 16; i += BW_THREADS)
+            ((uint4 *)smem_raw)[i] = ((const uint4 *)(bw.Wb + l * PKT))[i];
     };
     const auto stage = [&]() {
 #pragma unroll
@@ -356,9 +365,10 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const bf16 *__r
             }
         }
     };
-    if ((int)blockIdx.x < n) load(blockIdx.x);
+    const int r0 = blockIdx.x;
+    load(2, r0);
+    weights(2);
     {
-        for (int i = t; i < PKT * 2 / 16; i += BW_THREADS) ((uint4 *)smem_raw)[i] = ((const uint4 *)Wt)[i];
         const uint4 z = make_uint4(0, 0, 0, 0);
         for (int i = t; i < (BW_BAR - BW_ACT) / 16; i += BW_THREADS) ((uint4 *)As)[i] = z;
     }
@@ -377,102 +387,115 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const bf16 *__r
     /* this thread's pixel of the input gradient: row m of half h */
     const int h = warp >> 2, m = 32 * (warp & 3) + lane, ex = m >> 3, ey = 8 * h + (m & 7);
     const uint32_t tlane = (uint32_t)((warp & 3) * 32) << 16;
-    bool alive = true, first = true;
+    bool alive = true;
     uint32_t phase = 0;
-    if ((int)blockIdx.x < n) stage();
-    for (int r = blockIdx.x; r < n && alive; r += gridDim.x) {
-        bamf::tc::fence_proxy_async();
-        bamf::tc::fence_before_sync();
-        __syncthreads();
-        bamf::tc::fence_after_sync();
-        if (warp == 0) {
-            /* descriptors by adding to the address field (no carry out of it:
-             * shared memory is below 2^18 bytes) */
-            const uint32_t one = bamf::tc::elect_one();
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh)
-#pragma unroll
-                for (int tap = 0; tap < 9; ++tap)
-#pragma unroll
-                    for (int cb = 0; cb < 2; ++cb)
-                        bamf::tc::mma_bf16_warp(
-                            tin + 32 * hh,
-                            dk + (tap / 3 * BW_DCOL + 2 * cb * BW_DG + tap % 3 * 16 + 128 * hh) / 16,
-                            wd + (tap * (CH * CH * 2) + 2 * cb * (CH * 16)) / 16, TC_IDESC, tap + cb > 0 ? 1u : 0u,
-                            one);
-            if (one) bamf::tc::commit(bar_in);
-#pragma unroll
-            for (int x = 0; x < S; ++x)
-                bamf::tc::mma_bf16_warp(tw, am + x * BW_ACOL / 16, dm + x * BW_DCOL / 16, DW_IDESC,
-                                        first && x == 0 ? 0u : 1u, one);
-            if (one) bamf::tc::commit(bar_w);
-        }
-        first = false;
-        const int rn = r + gridDim.x;
-        if (rn < n) load(rn);
-        if (warp >= 4) bias_sums();
-        bool ok = bamf::tc::mbar_wait(bar_in, phase, 1u << 24);
-        bamf::tc::fence_after_sync();
-        if (ok) {
-            float v[32];
-            bamf::tc::tmem_ld32(tin + 32 * h + tlane, v);
-            uint4 *dst = (uint4 *)(out + ((size_t)r * NPX + 16 * ex + ey) * CH);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint4 mk = *(const uint4 *)(As + ex * BW_ACOL + (4 + q) * BW_AG + ey * 16);
-                const __nv_bfloat162 *m2 = (const __nv_bfloat162 *)&mk;
-                __align__(16) __nv_bfloat162 o[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    o[c] = __floats2bfloat162_rn(__bfloat162float(m2[c].x) > 0.0f ? v[8 * q + 2 * c] : 0.0f,
-                                                 __bfloat162float(m2[c].y) > 0.0f ? v[8 * q + 2 * c + 1] : 0.0f);
-                dst[q] = *(const uint4 *)o;
-            }
-        }
-        ok = bamf::tc::mbar_wait(bar_w, phase, 1u << 24) && ok;
-        phase ^= 1u;
-        bamf::tc::fence_after_sync();
-        if (!ok) {
-            atomicExch(status, 1);
-            alive = false;
-        }
-        bamf::tc::fence_before_sync();
-        /* the MMAs and the epilogue have read the tiles before they are restaged */
-        alive = __syncthreads_and(alive);
-        bamf::tc::fence_after_sync();
-        if (alive && rn < n) stage();
-    }
-    if ((int)blockIdx.x < n) {
-        float *mine = part + (size_t)blockIdx.x * DW_PART;
-        if ((warp & 3) < 3) {
-            /* lane 32 ky + ci, column 32 j + co, stored at (32 j + co) * 96 + 32 ky + ci */
 #pragma unroll 1
-            for (int j = h; j < 3; j += 2) {
-                float v[32];
-                if (alive) {
-                    bamf::tc::tmem_ld32(tw + 32 * j + tlane, v);
-                } else {
+    for (int l = 2; l >= 0; --l) {
+        bool first = true;
 #pragma unroll
-                    for (int co = 0; co < CH; ++co) v[co] = 0.0f;
-                }
+        for (int c = 0; c < 8; ++c) bsum[c] = 0.0f;
+        bf16 *const out = bw.dz[~l & 1];
+        stage();
+        for (int r = r0; r < n && alive; r += gridDim.x) {
+            bamf::tc::fence_proxy_async();
+            bamf::tc::fence_before_sync();
+            __syncthreads();
+            bamf::tc::fence_after_sync();
+            if (warp == 0) {
+                /* descriptors by adding to the address field (no carry out of it:
+                 * shared memory is below 2^18 bytes) */
+                const uint32_t one = bamf::tc::elect_one();
 #pragma unroll
-                for (int co = 0; co < CH; ++co) mine[(32 * j + co) * 96 + m] = v[co];
+                for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+                    for (int tap = 0; tap < 9; ++tap)
+#pragma unroll
+                        for (int cb = 0; cb < 2; ++cb)
+                            bamf::tc::mma_bf16_warp(
+                                tin + 32 * hh,
+                                dk + (tap / 3 * BW_DCOL + 2 * cb * BW_DG + tap % 3 * 16 + 128 * hh) / 16,
+                                wd + (tap * (CH * CH * 2) + 2 * cb * (CH * 16)) / 16, TC_IDESC, tap + cb > 0 ? 1u : 0u,
+                                one);
+                if (one) bamf::tc::commit(bar_in);
+#pragma unroll
+                for (int x = 0; x < S; ++x)
+                    bamf::tc::mma_bf16_warp(tw, am + x * BW_ACOL / 16, dm + x * BW_DCOL / 16, DW_IDESC,
+                                            first && x == 0 ? 0u : 1u, one);
+                if (one) bamf::tc::commit(bar_w);
             }
-        }
-        /* bias: lanes with equal (lane >> 3) hold the same 8 channels */
+            first = false;
+            const int rn = r + gridDim.x;
+            if (rn < n) load(l, rn);
+            if (warp >= 4) bias_sums();
+            bool ok = bamf::tc::mbar_wait(bar_in, phase, 1u << 24);
+            bamf::tc::fence_after_sync();
+            if (ok) {
+                float v[32];
+                bamf::tc::tmem_ld32(tin + 32 * h + tlane, v);
+                uint4 *dst = (uint4 *)(out + ((size_t)r * NPX + 16 * ex + ey) * CH);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            float v = bsum[c];
-            v += __shfl_xor_sync(0xffffffffu, v, 1);
-            v += __shfl_xor_sync(0xffffffffu, v, 2);
-            v += __shfl_xor_sync(0xffffffffu, v, 4);
-            bsum[c] = v;
-        }
-        if (warp >= 4 && (t & 7) == 0)
+                for (int q = 0; q < 4; ++q) {
+                    const uint4 mk = *(const uint4 *)(As + ex * BW_ACOL + (4 + q) * BW_AG + ey * 16);
+                    const __nv_bfloat162 *m2 = (const __nv_bfloat162 *)&mk;
+                    __align__(16) __nv_bfloat162 o[4];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) bred[warp - 4][8 * g + c] = bsum[c];
-        __syncthreads();
-        if (t < CH) mine[96 * 96 + t] = alive ? (bred[0][t] + bred[1][t]) + (bred[2][t] + bred[3][t]) : 0.0f;
+                    for (int c = 0; c < 4; ++c)
+                        o[c] = __floats2bfloat162_rn(__bfloat162float(m2[c].x) > 0.0f ? v[8 * q + 2 * c] : 0.0f,
+                                                     __bfloat162float(m2[c].y) > 0.0f ? v[8 * q + 2 * c + 1] : 0.0f);
+                    dst[q] = *(const uint4 *)o;
+                }
+            }
+            ok = bamf::tc::mbar_wait(bar_w, phase, 1u << 24) && ok;
+            phase ^= 1u;
+            bamf::tc::fence_after_sync();
+            if (!ok) {
+                atomicExch(status, 1);
+                alive = false;
+            }
+            bamf::tc::fence_before_sync();
+            /* the MMAs and the epilogue have read the tiles before they are restaged */
+            alive = __syncthreads_and(alive);
+            bamf::tc::fence_after_sync();
+            if (alive && rn < n) stage();
+        }
+        /* every MMA of the layer is done and every row of dz written: the next layer's
+         * first ROI and weights, and this one's sums */
+        if (l > 0) {
+            load(l - 1, r0);
+            weights(l - 1);
+        }
+        {
+            float *mine = bw.part + l * bw.pitch + (size_t)blockIdx.x * DW_PART;
+            if ((warp & 3) < 3) {
+                /* lane 32 ky + ci, column 32 j + co, stored at (32 j + co) * 96 + 32 ky + ci */
+#pragma unroll 1
+                for (int j = h; j < 3; j += 2) {
+                    float v[32];
+                    if (alive) {
+                        bamf::tc::tmem_ld32(tw + 32 * j + tlane, v);
+                    } else {
+#pragma unroll
+                        for (int co = 0; co < CH; ++co) v[co] = 0.0f;
+                    }
+#pragma unroll
+                    for (int co = 0; co < CH; ++co) mine[(32 * j + co) * 96 + m] = v[co];
+                }
+            }
+            /* bias: lanes with equal (lane >> 3) hold the same 8 channels */
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                float v = bsum[c];
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+                v += __shfl_xor_sync(0xffffffffu, v, 4);
+                bsum[c] = v;
+            }
+            if (warp >= 4 && (t & 7) == 0)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) bred[warp - 4][8 * g + c] = bsum[c];
+            __syncthreads();
+            if (t < CH) mine[96 * 96 + t] = alive ? (bred[0][t] + bred[1][t]) + (bred[2][t] + bred[3][t]) : 0.0f;
+        }
     }
     bamf::tc::fence_before_sync();
     __syncthreads();
@@ -1447,16 +1470,9 @@ Partials backward(bamf_cnn *net, const int32_t *n_em, const float *xyi, int n, f
                          n, grid_for(n, 4, net->sms), grid_for(n, 2, net->sms)};
     head_kernel<<<n, HD_THREADS, 0, s>>>(net->a[3], n, net->P, n_em, xyi, inv_batch, net->hpart, net->dzA, net->loss,
                                          net->step);
-    bf16 *dz = net->dzA, *dzn = net->dzB;
-    for (int l = 2; l >= 0; --l) {
-        /* layer l+2: input a[l], output a[l+1]; dz = dL/dz_{l+2} */
-        conv_bwd_kernel<<<pt.ndw, BW_THREADS, SMEM_BW, s>>>(net->a[l], dz, net->Wb + l * PKT, n, dzn,
-                                                            net->dwpart + l * pt.dw_pitch, net->tc_status);
-        bf16 *tmp = dz;
-        dz = dzn;
-        dzn = tmp;
-    }
-    conv1_bwd_kernel<<<pt.nc1, 256, 0, s>>>(net->x0, dz, n, net->c1part);
+    const Backward bw = {{net->a[0], net->a[1], net->a[2]}, {net->dzA, net->dzB}, net->Wb, net->dwpart, pt.dw_pitch};
+    conv_bwd_kernel<<<pt.ndw, BW_THREADS, SMEM_BW, s>>>(bw, n, net->tc_status);
+    conv1_bwd_kernel<<<pt.nc1, 256, 0, s>>>(net->x0, net->dzB, n, net->c1part);
     return pt;
 }
 
