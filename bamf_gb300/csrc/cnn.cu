@@ -281,7 +281,8 @@ __global__ void __launch_bounds__(256) conv1_bwd_kernel(const float *__restrict_
  * and layer (two CTAs per SM: 26 us for 1024 ROIs).  1024 ROIs are three or four a
  * CTA, so what a launch costs before its first MMA (2.6 to 4 us of allocation, first
  * loads and cold instructions) stands out: two kernels per layer, each with its own
- * staging, took 115 us, one per layer 72, this one 64.
+ * staging, took 115 us, one per layer 72, this one 64, and 58 with the weights as
+ * one bulk copy under the rest of the prologue.
  *
  * The mbarrier waits are bounded; a timeout is recorded in *status, the CTA
  * writes zeros, frees its TMEM and returns. */
@@ -292,7 +293,7 @@ constexpr int BW_DCOL = 4 * BW_DG;               /* an x column of dz */
 constexpr int BW_ACT = PKT * 2;                  /* offsets: weights, act, dz, barriers */
 constexpr int BW_DZ = BW_ACT + S * BW_ACOL + 4 * BW_AG;
 constexpr int BW_BAR = BW_DZ + PS * BW_DCOL;
-constexpr size_t SMEM_BW = BW_BAR + 2 * sizeof(uint64_t);
+constexpr size_t SMEM_BW = BW_BAR + 3 * sizeof(uint64_t);
 constexpr int BW_THREADS = 256;
 constexpr int BW_TMEM = 256;                     /* columns: 96 of dW, 2 x 32 of the input gradient */
 constexpr int DW_PART = 96 * 96 + CH;            /* floats of one CTA's partial sums */
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const Backward 
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char *const As = smem_raw + BW_ACT, *const Ds = smem_raw + BW_DZ;
-    uint64_t *const bar_in = (uint64_t *)(smem_raw + BW_BAR), *const bar_w = bar_in + 1;
+    uint64_t *const bar_in = (uint64_t *)(smem_raw + BW_BAR), *const bar_w = bar_in + 1, *const bar_wt = bar_in + 2;
     __shared__ uint32_t tslot;
     __shared__ float bred[4][CH];
     const int t = threadIdx.x, lane = t & 31;
@@ -325,18 +326,16 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const Backward 
     uint4 pa[CPT], pd[CPT];
     float bsum[8];
     const auto load = [&](int l, int r) {
-        const uint4 *sa = (const uint4 *)(bw.act[l] + (size_t)r * NPX * CH) + p0 * 4 + g;
-        const uint4 *sd = (const uint4 *)(bw.dz[l & 1] + (size_t)r * NPX * CH) + p0 * 4 + g;
+        const bf16 *act = l == 2 ? bw.act[2] : l == 1 ? bw.act[1] : bw.act[0], *dz = l == 1 ? bw.dz[1] : bw.dz[0];
+        const uint4 *sa = (const uint4 *)(act + (size_t)r * NPX * CH) + p0 * 4 + g;
+        const uint4 *sd = (const uint4 *)(dz + (size_t)r * NPX * CH) + p0 * 4 + g;
 #pragma unroll
         for (int k = 0; k < CPT; ++k) {
             pa[k] = sa[64 * 4 * k];
             pd[k] = __ldcg(sd + 64 * 4 * k); /* written by this kernel: not through the read-only path */
         }
     };
-    const auto weights = [&](int l) {
-        for (int i = t; i < PKT * 2 / 16; i += BW_THREADS)
-            ((uint4 *)smem_raw)[i] = ((const uint4 *)(bw.Wb + l * PKT))[i];
-    };
+
     const auto stage = [&]() {
 #pragma unroll
         for (int k = 0; k < CPT; ++k) {
@@ -367,14 +366,15 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const Backward 
     };
     const int r0 = blockIdx.x;
     load(2, r0);
-    weights(2);
-    {
-        const uint4 z = make_uint4(0, 0, 0, 0);
-        for (int i = t; i < (BW_BAR - BW_ACT) / 16; i += BW_THREADS) ((uint4 *)As)[i] = z;
-    }
     if (t == 0) {
         bamf::tc::mbar_init(bar_in, 1);
         bamf::tc::mbar_init(bar_w, 1);
+        bamf::tc::mbar_init(bar_wt, 1);
+        bamf::tc::bulk_load(smem_raw, bw.Wb + 2 * PKT, PKT * 2, bar_wt);
+    }
+    {
+        const uint4 z = make_uint4(0, 0, 0, 0);
+        for (int i = t; i < (BW_BAR - BW_ACT) / 16; i += BW_THREADS) ((uint4 *)As)[i] = z;
     }
     bamf::tc::fence_before_sync();
     __syncthreads();
@@ -394,8 +394,13 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const Backward 
         bool first = true;
 #pragma unroll
         for (int c = 0; c < 8; ++c) bsum[c] = 0.0f;
-        bf16 *const out = bw.dz[~l & 1];
+        bf16 *const out = l == 1 ? bw.dz[0] : bw.dz[1];
         stage();
+        if (!bamf::tc::mbar_wait(bar_wt, l & 1, 1u << 24)) { /* the layer's weights */
+            atomicExch(status, 1);
+            alive = false;
+        }
+        alive = __syncthreads_and(alive);
         for (int r = r0; r < n && alive; r += gridDim.x) {
             bamf::tc::fence_proxy_async();
             bamf::tc::fence_before_sync();
@@ -462,7 +467,7 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const Backward 
          * first ROI and weights, and this one's sums */
         if (l > 0) {
             load(l - 1, r0);
-            weights(l - 1);
+            if (t == 0) bamf::tc::bulk_load(smem_raw, bw.Wb + (l - 1) * PKT, PKT * 2, bar_wt);
         }
         {
             float *mine = bw.part + l * bw.pitch + (size_t)blockIdx.x * DW_PART;
@@ -948,7 +953,7 @@ static_assert(4 * (NSUB * CH + NSUB) <= NPX * HD_D && NSUB * CH == 4 * HD_THREAD
 
 /* ------------------------------------------------------ fused forward */
 /* The whole network on a ROI without leaving the SM (NET_TRAIN: up to a4, the
- * activations also written out for the backward kernels, 1024 ROIs in 44 us
+ * activations also written out for the backward kernels, 1024 ROIs in 37 us
  * for 72 us of four kernels).  A persistent CTA keeps
  * the packed weights of the three convolutions resident and runs GROUPS groups
  * of 256 threads; a group takes one ROI per iteration: conv1 (FP32), three 32 ->
@@ -976,7 +981,9 @@ static_assert(4 * (NSUB * CH + NSUB) <= NPX * HD_D && NSUB * CH == 4 * HD_THREAD
  * on an SM (two CTAs of two) overlap one's MMAs with the others' epilogues.
  * 50,000 ROIs: 3.78 ms as five launches per 4096 ROIs, 1.93 ms with the heads in
  * FP32 FMAs and one thread building every descriptor, 1.53 with this conv1 and
- * head, 1.32 with the warp-uniform issue, 1.26 with GROUPS = 2 instead of 1;
+ * head, 1.32 with the warp-uniform issue, 1.26 with GROUPS = 2 instead of 1, 1.24
+ * with the weights as one bulk copy (304 CTAs reading the same lines with plain loads
+ * waited some 6000 cycles);
  * 0.74 ms is 108 x 40 + 4 x 44 cycles per ROI and SM. */
 constexpr int IB_G = PS * PS * 16;                 /* bytes of one ci group of the buffer */
 constexpr int IB_BYTES = 4 * IB_G;
@@ -1046,6 +1053,7 @@ __global__ void __launch_bounds__(256 * INF_GROUPS, 2) net_kernel(
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float *w1 = (float *)(smem_raw + INF_W1), *bias = (float *)(smem_raw + INF_BIAS);
     __shared__ uint32_t tslot;
+    __shared__ uint64_t wbar; /* the packed weights' arrival */
     __shared__ float Wc[NC * CH], bc[NC], bl[NSUB];
     const int t = threadIdx.x % 256, lane = t & 31;
     /* warp-uniform, and known to be */
@@ -1053,10 +1061,13 @@ __global__ void __launch_bounds__(256 * INF_GROUPS, 2) net_kernel(
     InferGroup &G = ((InferGroup *)(smem_raw + INF_GRP))[grp];
     unsigned char *const buf = G.buf;
     if (threadIdx.x < 32) bamf::tc::tmem_alloc(&tslot, INF_TMEM * INF_GROUPS);
+    if (threadIdx.x == 0) {
+        bamf::tc::mbar_init(&wbar, 1);
+        bamf::tc::bulk_load(smem_raw, Wt, 3 * PKT * 2, &wbar);
+    }
     {
         const int nt = 256 * INF_GROUPS, i0 = threadIdx.x;
-        for (int i = i0; i < 3 * PKT * 2 / 16; i += nt) ((uint4 *)smem_raw)[i] = ((const uint4 *)Wt)[i];
-        for (int i = i0; i < CH * NSUB; i += nt) {
+        for (int i = i0; i < (MODE == NET_TRAIN ? 0 : CH * NSUB); i += nt) {
             const int s = i / CH, c = i - s * CH;
             bf16 *w = (bf16 *)(smem_raw + INF_WH) + (c >> 3) * (IH_N * 8) + s * 8 + (c & 7);
             float v = P[O_WL + i];
@@ -1072,9 +1083,11 @@ __global__ void __launch_bounds__(256 * INF_GROUPS, 2) net_kernel(
             const int l = i / CH;
             bias[i] = P[(l == 0 ? O_B1 : l == 1 ? O_B2 : l == 2 ? O_B3 : O_B4) + i % CH];
         }
-        for (int i = i0; i < NC * CH; i += nt) Wc[i] = P[O_WC + (i % NC) * CH + i / NC];
-        if (i0 < NSUB) bl[i0] = P[O_BL + i0];
-        if (i0 < NC) bc[i0] = P[O_BC + i0];
+        if (MODE != NET_TRAIN) {
+            for (int i = i0; i < NC * CH; i += nt) Wc[i] = P[O_WC + (i % NC) * CH + i / NC];
+            if (i0 < NSUB) bl[i0] = P[O_BL + i0];
+            if (i0 < NC) bc[i0] = P[O_BC + i0];
+        }
         const uint4 z = make_uint4(0, 0, 0, 0);
         for (int i = t; i < IB_BYTES / 16; i += 256) ((uint4 *)buf)[i] = z;
         for (int i = t; i < PS * PS; i += 256) G.xp[i] = 0.0f;
@@ -1098,7 +1111,8 @@ __global__ void __launch_bounds__(256 * INF_GROUPS, 2) net_kernel(
     const int epi = ((pe >> 4) + 1) * PS + (pe & 15) + 1;
     const uint32_t tlane = tbase + ((uint32_t)((warp & 3) * 32) << 16);
     uint32_t phase = 0;
-    const int stride = gridDim.x * INF_GROUPS, r0 = blockIdx.x * INF_GROUPS + grp;
+    /* a last round that not every group has is spread over the CTAs */
+    const int stride = gridDim.x * INF_GROUPS, r0 = blockIdx.x + gridDim.x * grp;
     float next = r0 < n ? data[(size_t)r0 * NPX + t] : 0.0f;
     /* every thread of the group waits for the group's MMAs; false (for all)
      * when the wait ran out */
@@ -1170,6 +1184,10 @@ __global__ void __launch_bounds__(256 * INF_GROUPS, 2) net_kernel(
                 if (MODE == NET_TRAIN)
                     ((uint4 *)kept.a[0])[((size_t)r * NPX + (x0 + 2 * j) * S + y) * 4 + g] = u;
             }
+        }
+        if (r == r0 && !bamf::tc::mbar_wait(&wbar, 0, 1u << 24)) {
+            G.dead = 1;
+            atomicExch(status, 1);
         }
 #pragma unroll 1
         for (int l = 0; l < 3; ++l) {
