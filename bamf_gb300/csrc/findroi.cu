@@ -1391,7 +1391,9 @@ __global__ void __launch_bounds__(256) emit_kernel(const uint8_t *__restrict__ f
  * A warp per ROI, grid-stride over the ROIs found (the count, or the range
  * [range[0], range[1]) when given, is read on the device): the box's pixels
  * in stack order, each column's run of box pixels contiguous in the frame;
- * stores coalesced. */
+ * stores coalesced.  In a frame smaller than the box the clamped corner is below 1:
+ * the box's pixels then come from the stack's values before the frame, as the
+ * linear offsets say, and are zero before the stack's first value. */
 __global__ void crop_kernel(const float *__restrict__ frames, int Ysz, int Xsz,
                             const int32_t *__restrict__ coords, const int32_t *__restrict__ corners,
                             const int64_t *__restrict__ count, const int64_t *__restrict__ range, int box,
@@ -1404,11 +1406,12 @@ __global__ void crop_kernel(const float *__restrict__ frames, int Ysz, int Xsz,
     for (int64_t b = b0 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); b < nroi;
          b += ((int64_t)gridDim.x * blockDim.x) >> 5) {
         const int sr = corners[2 * b], sc = corners[2 * b + 1], kk = coords[3 * b + 2];
-        const float *src = frames + (int64_t)(kk - 1) * plane + (int64_t)(sc - 1) * Ysz + (sr - 1);
+        const int64_t src = (int64_t)(kk - 1) * plane + (int64_t)(sc - 1) * Ysz + (sr - 1);
         float *dst = stack + b * per;
         for (int q = lane; q < per; q += 32) {
             const int col = q / box, row = q - col * box;
-            dst[q] = src[(int64_t)col * Ysz + row];
+            const int64_t at = src + (int64_t)col * Ysz + row;
+            dst[q] = at >= 0 ? frames[at] : 0.0f;
         }
     }
 }
