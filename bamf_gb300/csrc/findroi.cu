@@ -1475,12 +1475,32 @@ extern "C" void bamf_findroi_workspace_destroy(bamf_findroi_ws *ws) { delete ws;
 
 namespace {
 
+/* Frames copied from host memory at a time, `chunk_frames` at most.  A piece that
+ * takes the link as long as the device needs for it hides the device's work but
+ * for the last piece's, so a piece is no more than PIECE_BYTES, and where a CTA
+ * filters a frame (256 x 256 and the like) a multiple of the SMs, as a part of a
+ * wave takes as long as a whole one.  Smaller pieces than that would be bound by
+ * the launches of each (find and fit, us, pieces of 100 / 152 / 200 / 304 / 500 / 1000
+ * frames: 1000 frames of 256 x 256 1796 / 1534 / 1592 / 1635 / 1794 / 2169; pieces of
+ * 250 against these: 409 frames of 400 x 400 2563 / 1785, 728 of 300 x 300 2512 / 1795). */
+constexpr int64_t PIECE_BYTES = 40 << 20;
+int pinned_piece(int chunk_frames, int KX, int KY, int sms)
+{
+    const int step = std::max(1, chunk_frames);
+    const int64_t plane = (int64_t)KX * KY;
+    const int YP = (KY + FF_CW - 1) / FF_CW * FF_CW;
+    const int fit = (int)std::min<int64_t>(step, std::max<int64_t>(1, PIECE_BYTES / (plane * (int64_t)sizeof(float))));
+    if ((int64_t)KX * YP > (int64_t)FF_MAX_SLOT) return fit;
+    return fit == step ? step : std::min(step, std::max(sms, fit / sms * sms));
+}
+
 /* Passes 1-2 (the DoG) of `frames` (device) into `dog`.  With host_frames,
- * the frames are first copied from there in chunks of chunk_frames on the
- * workspace's copy stream, and each chunk's filters start on `s` as soon as
- * its copy has landed (the filters are frame-local, so a chunk is filtered
- * exactly as inside the whole stack).  The slots are in ws->b.  after_chunk, when given, is called with the number of
- * frames filtered so far after each chunk's launches. */
+ * the frames are first copied from there in pieces (pinned_piece) on the
+ * workspace's copy stream, and each piece's filters start on `s` as soon as
+ * its copy has landed (the filters are frame-local, so a piece is filtered
+ * exactly as inside the whole stack).  The slots are in ws->b.  after_chunk, when
+ * given, is called with the number of frames filtered so far after each piece's
+ * launches. */
 bamf_status run_filter(bamf_findroi_ws *ws, const float *host_frames, int chunk_frames, const float *frames,
                        int KX, int KY, int zsize, double sigma1, double sigma2, float *dog, cudaStream_t s,
                        const std::function<bamf_status(int)> *after_chunk = nullptr)
@@ -1489,7 +1509,7 @@ bamf_status run_filter(bamf_findroi_ws *ws, const float *host_frames, int chunk_
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int step = host_frames ? std::max(1, chunk_frames) : zsize;
+    const int step = host_frames ? pinned_piece(chunk_frames, KX, KY, sms) : zsize;
     const int64_t plane = (int64_t)KX * KY;
     const int YP = (KY + FF_CW - 1) / FF_CW * FF_CW;
     const size_t slot_bytes = (size_t)2 * KX * YP * sizeof(float);
@@ -1564,7 +1584,7 @@ struct FitArgs {
 /* Passes 1-5 on `frames` (device), copied first from host_frames when given
  * (run_filter; each chunk's window maxima start once it is filtered).  The
  * compaction and crop run on the whole stack at the end; with `fit`, the
- * compaction, crops and fits run after each chunk's maxima on the flag
+ * compaction, crops and fits run after every few pieces' maxima on the flag
  * chunks those complete, appended in memory order. */
 bamf_status find_roi(bamf_findroi_ws *ws, const float *host_frames, int chunk_frames, const float *frames,
                      int ysize, int xsize, int zsize, double sigma1, double sigma2, int boxsize, float minval,
@@ -1670,7 +1690,7 @@ bamf_status find_roi(bamf_findroi_ws *ws, const float *host_frames, int chunk_fr
     int64_t *total = (int64_t *)ws->total.p;
     const unsigned crop_blocks = (unsigned)((std::min<int64_t>(std::max<int64_t>(capacity, 1), (int64_t)sms * 64) + 7) / 8);
     if (fit) {
-        const int step = std::max(1, chunk_frames);
+        const int step = pinned_piece(chunk_frames, KX, KY, sms);
         if (!ws->ranges.ensure((size_t)2 * ((zsize + step - 1) / step + 2) * sizeof(int64_t))) return BAMF_ERR_CUDA;
     }
     /* compaction of flag chunks [cdone, c1), their maxima after those of the
@@ -1705,8 +1725,15 @@ bamf_status find_roi(bamf_findroi_ws *ws, const float *host_frames, int chunk_fr
         const int upto = filtered >= zsize ? zsize : filtered - reach;
         bamf_status r = maxima(done, upto);
         if (upto > done) done = upto;
-        /* the flag chunks wholly inside frames [0, upto) */
-        if (!r && fit) r = compact(upto >= zsize ? nchunks : (int64_t)upto * KX * KY / CHUNK);
+        /* the flag chunks wholly inside frames [0, upto), once they hold three pieces:
+         * the five launches of a compaction and its fits cost some 50 us, which
+         * pieces of small frames do not hide (with the fits, us, after every 250
+         * frames / half a piece / three pieces: 3000 frames of 24 x 24 878 / 501 / 492,
+         * 3000 of 128 x 128 1682 / 1442 / 1297, 1777 of 192 x 192 1948 / 1956 / 1733, 1000 of
+         * 256 x 256 1534 / 1526 / 1512, 409 of 400 x 400 1785 / 1788 / 1659) */
+        const int64_t c1 = upto >= zsize ? nchunks : (int64_t)upto * KX * KY / CHUNK;
+        if (!r && fit && (upto >= zsize || (c1 - cdone) * CHUNK * (int64_t)sizeof(float) >= 3 * PIECE_BYTES))
+            r = compact(c1);
         return r;
     };
     bamf_status st = run_filter(ws, host_frames, chunk_frames, frames, KX, KY, zsize, sigma1, sigma2, A, s,

@@ -570,7 +570,7 @@ bamf_status bamf_find_roi_host(const float *frames, int ysize, int xsize, int zs
 
 /* bamf_find_roi_device on frames that are still in host memory: copies
  * host_frames (pinned, for the copies to overlap) into dev_frames (the
- * same size, device) in chunks of chunk_frames frames on a stream of the
+ * same size, device) in chunks of at most chunk_frames frames on a stream of the
  * workspace, and starts each chunk's row and column filters on `stream`
  * as soon as its copy has landed, then the window maxima of the chunk's
  * frames (those whose windows cannot reach a frame not yet filtered); the
@@ -584,11 +584,11 @@ bamf_status bamf_find_roi_pinned(bamf_findroi_ws *ws, const float *host_frames, 
                                  int64_t *count, uint8_t *flags_out, void *stream);
 
 /* bamf_find_roi_pinned followed by gaussMLE (XYNB, CCD; gaussMLE.m:92-205
- * with the ROI stack findROI.m:157-160 crops), chunk by chunk: after each
- * chunk's window maxima, the maxima of the flag chunks those complete are
+ * with the ROI stack findROI.m:157-160 crops), while the copies go on: after every
+ * few chunks' window maxima, the maxima of the flag chunks those complete are
  * appended to the coordinates in memory order, cropped and fitted while
  * later chunks are still being copied, so the work after the last copy is
- * the last chunk's.  coords, corners, roi_stack and count are
+ * the last few chunks'.  coords, corners, roi_stack and count are
  * bamf_find_roi_pinned's (identical values); params and crlb are
  * [4][capacity]: bamf_gauss_mle_device's parameters (MATLAB Y, X, photons,
  * background) with the stride capacity, parameter k of ROI i at
