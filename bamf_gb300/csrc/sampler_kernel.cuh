@@ -1154,20 +1154,44 @@ struct ChainWarp {
                     }
                     const float base = (tBG - aBG) + (tBBG - aBBG) * (float)yl, dABG = tABG - aABG;
                     if (xo < R) {
+                        /* two columns at a time: one column's loads and
+                         * logarithms hide the other's; added in order */
 #pragma unroll 1
-                        for (int xx = x0 + xo; xx <= x1; xx += R) {
-                            float d = base + dABG * (float)xx;
-                            if (nr > 0) d += w[0] * sx[0][xx];
-                            if (nr > 1) d += w[1] * sx[1][xx];
-                            if (nr > 2) d += w[2] * sx[2][xx];
-                            if (nr > 3) d += w[3] * sx[3][xx];
-                            for (int q = 4; q < nr; ++q)
-                                d += q < na ? -SXo[q * X + xx] * SYo[q * Y + yl]
-                                            : SXn[(q - na) * X + xx] * SYn[(q - na) * Y + yl];
-                            int p = yl + Y * xx;
-                            float mt = M[p] + d;
-                            Mt[p] = mt;
-                            acc += D[p] * (__log2f(mt) - __log2f(M[p])) * LN2 - d;
+                        for (int xx = x0 + xo; xx <= x1; xx += 2 * R) {
+                            const bool two = xx + R <= x1;
+                            const int xb = two ? xx + R : xx, p0 = yl + Y * xx, p1 = yl + Y * xb;
+                            const float m0 = M[p0], m1 = M[p1], v0 = D[p0], v1 = D[p1];
+                            float d0 = base + dABG * (float)xx, d1 = base + dABG * (float)xb;
+                            if (nr > 0) {
+                                d0 += w[0] * sx[0][xx];
+                                d1 += w[0] * sx[0][xb];
+                            }
+                            if (nr > 1) {
+                                d0 += w[1] * sx[1][xx];
+                                d1 += w[1] * sx[1][xb];
+                            }
+                            if (nr > 2) {
+                                d0 += w[2] * sx[2][xx];
+                                d1 += w[2] * sx[2][xb];
+                            }
+                            if (nr > 3) {
+                                d0 += w[3] * sx[3][xx];
+                                d1 += w[3] * sx[3][xb];
+                            }
+                            for (int q = 4; q < nr; ++q) {
+                                const bool old = q < na;
+                                const float *sr = old ? SXo + q * X : SXn + (q - na) * X;
+                                const float sy = old ? SYo[q * Y + yl] : SYn[(q - na) * Y + yl];
+                                d0 = __fadd_rn(d0, __fmul_rn(old ? -sr[xx] : sr[xx], sy));
+                                d1 = __fadd_rn(d1, __fmul_rn(old ? -sr[xb] : sr[xb], sy));
+                            }
+                            const float t0 = m0 + d0, t1 = m1 + d1;
+                            Mt[p0] = t0;
+                            acc += v0 * (__log2f(t0) - __log2f(m0)) * LN2 - d0;
+                            if (two) {
+                                Mt[p1] = t1;
+                                acc += v1 * (__log2f(t1) - __log2f(m1)) * LN2 - d1;
+                            }
                         }
                     }
                 } else {
