@@ -849,39 +849,29 @@ struct ChainWarp {
     __device__ __forceinline__ void stencil_rows(int na, int nt)
     {
         const int XY = X + Y, nr = na + nt;
-        /* G rows per 32-lane pass when a row (X + Y entries) fits in 32
-         * lanes, else one row at a time over ceil(XY / 32) passes */
+        /* the rows' entries one after the other, 32 a pass: as few passes as
+         * there can be for rows that do not fill 32 lanes */
+        const int total = nr * XY;
         const float rXY = __frcp_rn((float)XY);
-        const int G = XY <= 32 ? small_div(32, rXY) : 1;
-        const int rg = XY <= 32 ? small_div(lane, rXY) : 0;
-        const int c0 = XY <= 32 ? lane - rg * XY : lane;
 #pragma unroll 1
-        for (int r0 = 0; r0 < nr; r0 += G) {
-            int r = min(r0 + rg, nr - 1);
-            bool isnew = r >= na;
-            int q = isnew ? r - na : r;
-            int k = nth_bit(isnew ? t_dirty : a_dirty, q);
+        for (int e0 = 0; e0 < total; e0 += 32) {
+            const int e = min(e0 + lane, total - 1);
+            const int r = small_div(e, rXY), c = e - r * XY;
+            const bool isnew = r >= na;
+            const int q = isnew ? r - na : r;
+            const int k = nth_bit(isnew ? t_dirty : a_dirty, q);
             /* a shuffle returns the source lane's value, so fetch both
              * states and select here (lanes of one pass may read rows of
              * different states) */
-            float Ia = __shfl_sync(BAMF_FULL, aI, k), It = __shfl_sync(BAMF_FULL, tI, k);
-            float Xa = __shfl_sync(BAMF_FULL, aX, k), Xt = __shfl_sync(BAMF_FULL, tX, k);
-            float Ya = __shfl_sync(BAMF_FULL, aY, k), Yt = __shfl_sync(BAMF_FULL, tY, k);
-            float Ik = isnew ? It : Ia, Xk = isnew ? Xt : Xa, Yk = isnew ? Yt : Ya;
-            bool on = rg < G && r0 + rg < nr;
-            float *sxr = (isnew ? SXn : SXo) + q * X, *syr = (isnew ? SYn : SYo) + q * Y;
-#pragma unroll 1
-            for (int c = c0; c < XY; c += 32) {
-                bool isx = c < X;
-                int cc = isx ? c : c - X;
-                float mu = isx ? Xk : Yk;
-                float v = 0.5f * (MT::erf_(((float)cc - mu + 1.0f) * Cst) - MT::erf_(((float)cc - mu) * Cst));
-                if (on) {
-                    if (isx) sxr[cc] = Ik * v;
-                    else syr[cc] = v;
-                }
-                if (XY <= 32) break;
-            }
+            const float Ia = __shfl_sync(BAMF_FULL, aI, k), It = __shfl_sync(BAMF_FULL, tI, k);
+            const float Xa = __shfl_sync(BAMF_FULL, aX, k), Xt = __shfl_sync(BAMF_FULL, tX, k);
+            const float Ya = __shfl_sync(BAMF_FULL, aY, k), Yt = __shfl_sync(BAMF_FULL, tY, k);
+            const bool isx = c < X;
+            const int cc = isx ? c : c - X;
+            const float mu = isx ? (isnew ? Xt : Xa) : (isnew ? Yt : Ya);
+            const float v = 0.5f * (MT::erf_(((float)cc - mu + 1.0f) * Cst) - MT::erf_(((float)cc - mu) * Cst));
+            if (e0 + lane < total)
+                ((isx ? (isnew ? SXn : SXo) + q * X : (isnew ? SYn : SYo) + q * Y))[cc] = isx ? (isnew ? It : Ia) * v : v;
         }
         __syncwarp();
     }
