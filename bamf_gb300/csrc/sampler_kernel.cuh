@@ -845,14 +845,15 @@ struct ChainWarp {
     /* Fast mode: stencil rows of the emitters a proposal changes, compact:
      * row q of SXo/SYo is the old stencil of the q-th slot of a_dirty (from
      * A), row q of SXn/SYn the new stencil of the q-th slot of t_dirty (from
-     * T). */
-    __device__ __forceinline__ void stencil_rows(int na, int nt)
+     * T).  mx, my: the columns and rows where any of them is not zero. */
+    __device__ __forceinline__ void stencil_rows(int na, int nt, uint32_t &mx, uint32_t &my)
     {
         const int XY = X + Y, nr = na + nt;
         /* the rows' entries one after the other, 32 a pass: as few passes as
          * there can be for rows that do not fill 32 lanes */
         const int total = nr * XY;
         const float rXY = __frcp_rn((float)XY);
+        uint32_t ux = 0u, uy = 0u;
 #pragma unroll 1
         for (int e0 = 0; e0 < total; e0 += 32) {
             const int e = min(e0 + lane, total - 1);
@@ -870,9 +871,14 @@ struct ChainWarp {
             const int cc = isx ? c : c - X;
             const float mu = isx ? (isnew ? Xt : Xa) : (isnew ? Yt : Ya);
             const float v = 0.5f * (MT::erf_(((float)cc - mu + 1.0f) * Cst) - MT::erf_(((float)cc - mu) * Cst));
-            if (e0 + lane < total)
-                ((isx ? (isnew ? SXn : SXo) + q * X : (isnew ? SYn : SYo) + q * Y))[cc] = isx ? (isnew ? It : Ia) * v : v;
+            const float sv = isx ? (isnew ? It : Ia) * v : v;
+            if (e0 + lane < total) ((isx ? (isnew ? SXn : SXo) + q * X : (isnew ? SYn : SYo) + q * Y))[cc] = sv;
+            const uint32_t bit = sv != 0.0f ? 1u << cc : 0u;
+            ux |= isx ? bit : 0u;
+            uy |= isx ? 0u : bit;
         }
+        mx = __reduce_or_sync(BAMF_FULL, ux);
+        my = __reduce_or_sync(BAMF_FULL, uy);
         __syncwarp();
     }
 
@@ -1096,7 +1102,8 @@ struct ChainWarp {
                 }
             } else {
                 if (na <= FAST_ROWS && nt <= FAST_ROWS) {
-                    stencil_rows(na, nt);
+                    uint32_t mx = 0u, my = 0u;
+                    stencil_rows(na, nt, mx, my);
                     const int nr = na + nt;
                     /* Support box: unless the background changes, a pixel
                      * outside the union of the changed rows' nonzero x- and
@@ -1105,15 +1112,6 @@ struct ChainWarp {
                      * sigma ~1.3 vanish in float ~7 px from the emitter. */
                     int x0 = 0, x1 = X - 1, y0 = 0, y1 = Y - 1;
                     if (tBG == aBG && tABG == aABG && tBBG == aBBG) {
-                        bool nzx = false, nzy = false;
-#pragma unroll 1
-                        for (int q = 0; q < nr; ++q) {
-                            const bool old = q < na;
-                            const int qq = old ? q : q - na;
-                            nzx |= lane < X && (old ? SXo : SXn)[qq * X + lane] != 0.0f;
-                            nzy |= lane < Y && (old ? SYo : SYn)[qq * Y + lane] != 0.0f;
-                        }
-                        const uint32_t mx = __ballot_sync(BAMF_FULL, nzx), my = __ballot_sync(BAMF_FULL, nzy);
                         if (mx == 0u || my == 0u) {
                             llr_box = 1; /* empty: Mt = M everywhere, LLR = 1 */
                             return 1.0f;
