@@ -281,6 +281,7 @@ extern "C" bamf_status bamf_rjmcmc_batch_device_noalloc(const bamf_roi_batch *ro
     B.pos_trace = out->pos_trace;
     B.pos_len = out->pos_len;
     B.pos_thin = out->pos_thin;
+    B.pos_rthin = out->pos_thin > 0 ? 1.0f / (float)out->pos_thin : 0.0f;
     if (cudaGetLastError() != cudaSuccess) return BAMF_ERR_CUDA;
 
     const bool exact = arith == BAMF_ARITH_EXACT;

@@ -597,6 +597,7 @@ extern "C" bamf_status bamf_rjmcmc_batch_device(bamf_workspace *ws, const bamf_r
     B.pos_trace = out->pos_trace;
     B.pos_len = out->pos_len;
     B.pos_thin = out->pos_thin;
+    B.pos_rthin = out->pos_thin > 0 ? 1.0f / (float)out->pos_thin : 0.0f;
     if (out->x_trace) {
         B.x_trace = out->x_trace;
         B.x_cap = out->trace_len;

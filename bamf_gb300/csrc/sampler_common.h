@@ -81,6 +81,7 @@ struct SamplerBatch {
     float *pos_trace;             /* [roi][pos_len][BAMF_POS_RECORD] thinned states */
     int32_t pos_len;
     int32_t pos_thin;
+    float pos_rthin; /* 1 / pos_thin */
     /* full chain recording (exact cRJMCMC outputs), or null */
     bamf_chain *chains;           /* device array [roi][2] of bamf_chain with device pointers */
     int32_t *queue;               /* work-queue counter (device int)       */

@@ -527,8 +527,8 @@ struct ChainWarp {
         return normpdf_f<EXACT>(x, u, s);
     }
 
-    /* a / b for 0 <= a <= 32, 1 <= b <= 64 (fast mode): (a + 1/2) / b is at least
-     * 1/128 from an integer, far more than the reciprocal's error */
+    /* a / b for 0 <= a < 2^10, 1 <= b <= 64 (fast mode): (a + 1/2) / b is at least
+     * 1/128 from an integer, far more than the reciprocal's error (2e-4) */
     static __device__ __forceinline__ int small_div(int a, float rb) { return (int)(((float)a + 0.5f) * rb); }
 
     /* ------------------------------------------------ neighbour search */
@@ -1343,7 +1343,15 @@ struct ChainWarp {
             if (lane == 0) B->nsig_trace[(int64_t)roi * B->trace_cap + entries] = (uint8_t)(an < 1 ? 0 : ns);
         }
         if (B->x_trace && entries < B->x_cap) record_x();
-        if (B->pos_trace && entries % B->pos_thin == 0 && entries / B->pos_thin < B->pos_len) record_pos();
+        if (B->pos_trace) {
+            /* every pos_thin-th entry, pos_len at most; the product with 1 / pos_thin is
+             * off by at most one below 2^22 entries and settles all others without
+             * a division */
+            const int rem = entries - (int)((float)entries * B->pos_rthin) * B->pos_thin;
+            if ((rem == 0 || rem == B->pos_thin || rem == -B->pos_thin || entries >= (1 << 22)) &&
+                entries % B->pos_thin == 0 && entries / B->pos_thin < B->pos_len)
+                record_pos();
+        }
         if (B->chains) {
             record_one(0, an, aI, aX, aY, aS, aBG, aABG, aBBG, LLR, PR, type, acc);
             record_one(1, tn, tI, tX, tY, tS, tBG, tABG, tBBG, LLR, PR, type, acc);
