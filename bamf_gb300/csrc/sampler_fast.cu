@@ -8,6 +8,8 @@
  * probabilities and independent of its state).  Also the fast launchers,
  * which pick the likelihood model's build.
  */
+#include <cmath>
+
 #include "sampler_kernel.cuh"
 #include "sampler_launch.h"
 
@@ -50,11 +52,13 @@ int blocks_per_sm_fast(int side_max, int warps_per_block, int min_ctas, int opt_
  * the first round costs `a` (it holds the brightest ROIs), later ones 0.77 a, a
  * last one that is not full 0.25 a more; less than one round costs between 0.68
  * and 1 of it.  Fitted to batches of 2,400 to 10,000 ROIs of 8, 16 and 24 px:
- * within 8%. */
-static float batch_cost(int n, int sms, int w, float a)
+ * within 8%.
+ * `whole`: the w chains are one CTA, so that less than a round leaves SMs without
+ * any instead of giving every SM fewer. */
+static float batch_cost(int n, int sms, int w, float a, bool whole)
 {
     const float x = (float)n / (float)(w * sms);
-    if (x <= 1.0f) return a * (0.68f + 0.32f * x);
+    if (x <= 1.0f) return whole ? a : a * (0.68f + 0.32f * x);
     const float frac = x - floorf(x);
     return a * (1.0f + 0.77f * (x - 1.0f) + (frac > 0.02f ? 0.25f : 0.0f));
 }
@@ -89,25 +93,31 @@ int best_fast_shape(int side_max, int opt_model, int n_rois, int sms, int *warps
                 best_per = per;
             }
         }
-    /* up to side 12, one CTA of a whole move-stream group per SM (all of
-     * the SM's warps on one instruction stream) measured faster than three
-     * CTAs of 8 chains, when it keeps as many chains resident */
-    if (side_max <= 12 && opt_model != 1) {
-        const int per = blocks_per_sm_fast(side_max, BAMF_SYNC_GROUP, 1, opt_model);
-        if (per * BAMF_SYNC_GROUP >= best_w) {
+    /* Up to side 16, one CTA of a whole move-stream group per SM (all of the SM's
+     * warps on one instruction stream) instead of three CTAs of 8 chains, when it
+     * keeps as many chains resident and fills its rounds (250 + 250 jumps, us, one /
+     * three: 16 px 2600 ROIs 3672 / 3399, 3380 3737 / 3748, 7300 5919 / 6752, 10,000
+     * 8551 / 9963, 30,000 27183 / 27373; 24 px 8140 / 7876, 11726 / 11272 at 7300 and
+     * 10,000). */
+    const int group_per = side_max <= 16 && opt_model != 1 ? blocks_per_sm_fast(side_max, BAMF_SYNC_GROUP, 1, opt_model) : 0;
+    const int group_w = group_per * BAMF_SYNC_GROUP;
+    /* Two CTAs of 8 on the larger register budget run a round in 1 / 1.42 of the
+     * time of three on the smaller (one CTA of 24: 1 / 1.25 at 8 to 12 px, 1 / 1.33 at
+     * 16), so which is faster depends on how full the last round is (16 px, 250 + 250
+     * jumps: 2432 ROIs 2812 us against 3130 with three, 5000: 5568 against 5876, 7300: 6893
+     * against 6752). */
+    float best = best_w > 0 ? batch_cost(n_rois, sms, best_w, best_mc == 2 ? 1.0f : 1.42f, false) : INFINITY;
+    if (group_w > 0 && group_w >= best_w) {
+        const float c = batch_cost(n_rois, sms, group_w, side_max <= 12 ? 1.25f : 1.33f, group_per == 1);
+        if (c < best) {
+            best = c;
             best_wpb = BAMF_SYNC_GROUP;
             best_mc = 1;
-            best_per = per;
+            best_per = group_per;
         }
     }
-    /* Two CTAs of 8 on the larger register budget run a round in 1 / 1.42 of the
-     * time of three on the smaller (8 to 12 px, one CTA of 24: 1 / 1.25), so which
-     * is faster depends on how full the last round is (16 px, 250 + 250 jumps:
-     * 2432 ROIs 3260 us against 3922, 3380: 5250 against 4636, 5000: 6422 against
-     * 7219, 7300: 8285 against 8224; uneven sides, 10,000: 11.6 ms against 12.5). */
     const int per2 = blocks_per_sm_fast(side_max, 8, 2, opt_model);
-    if (per2 * 8 >= 16 && best_w > per2 * 8 &&
-        batch_cost(n_rois, sms, per2 * 8, 1.0f) < batch_cost(n_rois, sms, best_w, best_mc == 1 ? 1.25f : 1.42f)) {
+    if (per2 * 8 >= 16 && best_w > per2 * 8 && batch_cost(n_rois, sms, per2 * 8, 1.0f, false) < best) {
         best_wpb = 8;
         best_mc = 2;
         best_per = per2;
