@@ -93,22 +93,23 @@ int best_fast_shape(int side_max, int opt_model, int n_rois, int sms, int *warps
                 best_per = per;
             }
         }
-    /* Up to side 16, one CTA of a whole move-stream group per SM (all of the SM's
+    /* Up to side 20, one CTA of a whole move-stream group per SM (all of the SM's
      * warps on one instruction stream) instead of three CTAs of 8 chains, when it
      * keeps as many chains resident and fills its rounds (250 + 250 jumps, us, one /
      * three: 16 px 2600 ROIs 3672 / 3399, 3380 3737 / 3748, 7300 5919 / 6752, 10,000
-     * 8551 / 9963, 30,000 27183 / 27373; 24 px 8140 / 7876, 11726 / 11272 at 7300 and
-     * 10,000). */
-    const int group_per = side_max <= 16 && opt_model != 1 ? blocks_per_sm_fast(side_max, BAMF_SYNC_GROUP, 1, opt_model) : 0;
+     * 8551 / 9963, 30,000 27183 / 27373; 20 px 7010 / 7723, 10660 / 11146 at 7300 and
+     * 10,000; 24 px 8140 / 7876, 11726 / 11272). */
+    const int group_per = side_max <= 20 && opt_model != 1 ? blocks_per_sm_fast(side_max, BAMF_SYNC_GROUP, 1, opt_model) : 0;
     const int group_w = group_per * BAMF_SYNC_GROUP;
     /* Two CTAs of 8 on the larger register budget run a round in 1 / 1.42 of the
      * time of three on the smaller (one CTA of 24: 1 / 1.25 at 8 to 12 px, 1 / 1.33 at
-     * 16), so which is faster depends on how full the last round is (16 px, 250 + 250
+     * 16, 1 / 1.4 at 20), so which is faster depends on how full the last round is (16 px, 250 + 250
      * jumps: 2432 ROIs 2812 us against 3130 with three, 5000: 5568 against 5876, 7300: 6893
      * against 6752). */
     float best = best_w > 0 ? batch_cost(n_rois, sms, best_w, best_mc == 2 ? 1.0f : 1.42f, false) : INFINITY;
     if (group_w > 0 && group_w >= best_w) {
-        const float c = batch_cost(n_rois, sms, group_w, side_max <= 12 ? 1.25f : 1.33f, group_per == 1);
+        const float c = batch_cost(n_rois, sms, group_w, side_max <= 12 ? 1.25f : side_max <= 16 ? 1.33f : 1.4f,
+                                   group_per == 1);
         if (c < best) {
             best = c;
             best_wpb = BAMF_SYNC_GROUP;
