@@ -78,7 +78,7 @@ struct SMath<false> {
  * proposal model Mt, per-pixel work E, sCMOS (each rounded up to 16 bytes,
  * for the vector loads of the serial sums), a pool of 2 x 32 stencil rows
  * NX/NY shared by A and T, 128 buffered uniforms.
- * Fast: D, M, Mt, the compact stencil rows SXo/SYo (old, of A) and SXn/SYn (new,
+ * Fast: D, M, Mt, the compact stencil rows SX/SY (old ones, of A, then new ones,
  * of T), the buffered uniforms and the shared draws of the next jumps; log2 M is recomputed in each likelihood pass (the
  * SFU has room; the smaller carve-out keeps 3 CTAs of 8 chains resident
  * up to 24x24 ROIs); sCMOS is read from global memory at model rebuilds
@@ -308,7 +308,7 @@ struct ChainWarp {
     int arow, trow;
     float *ubuf; /* uniforms base * 4 .. base * 4 + 127 of the stream */
     float *ahead; /* fast mode: the shared draws of MOVE_AHEAD jumps: move, then sub-branch */
-    float *SXo, *SYo, *SXn, *SYn; /* fast mode: compact stencil rows */
+    float *SX, *SY; /* fast mode: compact stencil rows */
     const float *scm; /* sCMOS: shared memory (exact) or global/null (fast) */
     /* sampled PSF (OptModel 1): [P0 y][P1 x][P2 y-sub][P3 x-sub], y fastest;
      * null for the Gaussian model */
@@ -843,8 +843,8 @@ struct ChainWarp {
     }
 
     /* Fast mode: stencil rows of the emitters a proposal changes, compact:
-     * row q of SXo/SYo is the old stencil of the q-th slot of a_dirty (from
-     * A), row q of SXn/SYn the new stencil of the q-th slot of t_dirty (from
+     * row q of SX/SY is the old stencil of the q-th slot of a_dirty (from
+     * A), row na + q the new stencil of the q-th slot of t_dirty (from
      * T).  mx, my: the columns and rows where any of them is not zero. */
     __device__ __forceinline__ void stencil_rows(int na, int nt, uint32_t &mx, uint32_t &my)
     {
@@ -872,7 +872,7 @@ struct ChainWarp {
             const float mu = isx ? (isnew ? Xt : Xa) : (isnew ? Yt : Ya);
             const float v = 0.5f * (MT::erf_(((float)cc - mu + 1.0f) * Cst) - MT::erf_(((float)cc - mu) * Cst));
             const float sv = isx ? (isnew ? It : Ia) * v : v;
-            if (e0 + lane < total) ((isx ? (isnew ? SXn : SXo) + q * X : (isnew ? SYn : SYo) + q * Y))[cc] = sv;
+            if (e0 + lane < total) (isx ? SX + r * X : SY + r * Y)[cc] = sv;
             const uint32_t bit = sv != 0.0f ? 1u << cc : 0u;
             ux |= isx ? bit : 0u;
             uy |= isx ? 0u : bit;
@@ -883,7 +883,7 @@ struct ChainWarp {
     }
 
     /* Fast mode: out = background plane + sCMOS + sum of the state's emitter
-     * stencils, one emitter at a time (its rows go through SXn/SYn row 0). */
+     * stencils, one emitter at a time (its rows go through SX/SY row 0). */
     __device__ __forceinline__ void model_stream(int n, float I, float Xv, float Yv, float BG, float ABG,
                                                  float BBG, float *out)
     {
@@ -909,15 +909,15 @@ struct ChainWarp {
                 int cc = isx ? c : c - X;
                 float mu = isx ? Xk : Yk;
                 float v = 0.5f * (MT::erf_(((float)cc - mu + 1.0f) * Cst) - MT::erf_(((float)cc - mu) * Cst));
-                if (isx) SXn[cc] = Ik * v;
-                else SYn[cc] = v;
+                if (isx) SX[cc] = Ik * v;
+                else SY[cc] = v;
             }
             __syncwarp();
             x = lane / Y;
             y = lane - (lane / Y) * Y;
 #pragma unroll 1
             for (int p = lane; p < npix; p += 32) {
-                out[p] += SXn[x] * SYn[y];
+                out[p] += SX[x] * SY[y];
                 x += px_dx;
                 y += px_dy;
                 if (y >= Y) {
@@ -1126,19 +1126,16 @@ struct ChainWarp {
                      * (h the box height); a pass covers 32 / h columns.  The
                      * model change of a pixel is bg delta + sum_q w_q(y)
                      * SX_q[x] over the changed rows q (old rows with weight
-                     * -SYo, new with +SYn); each lane holds its first four
+                     * -SY, new with +SY); each lane holds its first four
                      * weights in registers. */
                     const int h = y1 - y0 + 1;
                     const float rh = __frcp_rn((float)h);
                     const int xo = small_div(lane, rh), yl = y0 + lane - xo * h, R = small_div(32, rh);
                     float w[4];
-                    const float *sx[4];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        bool old = q < na;
-                        int qq = old ? q : q - na;
-                        w[q] = q < nr ? (old ? -SYo[qq * Y + yl] : SYn[qq * Y + yl]) : 0.0f;
-                        sx[q] = old ? SXo + qq * X : SXn + qq * X;
+                        const float sy = q < nr ? SY[q * Y + yl] : 0.0f;
+                        w[q] = q < na ? -sy : sy;
                     }
                     const float base = (tBG - aBG) + (tBBG - aBBG) * (float)yl, dABG = tABG - aABG;
                     if (xo < R) {
@@ -1151,25 +1148,25 @@ struct ChainWarp {
                             const float m0 = M[p0], m1 = M[p1], v0 = D[p0], v1 = D[p1];
                             float d0 = base + dABG * (float)xx, d1 = base + dABG * (float)xb;
                             if (nr > 0) {
-                                d0 += w[0] * sx[0][xx];
-                                d1 += w[0] * sx[0][xb];
+                                d0 += w[0] * SX[xx];
+                                d1 += w[0] * SX[xb];
                             }
                             if (nr > 1) {
-                                d0 += w[1] * sx[1][xx];
-                                d1 += w[1] * sx[1][xb];
+                                d0 += w[1] * SX[X + xx];
+                                d1 += w[1] * SX[X + xb];
                             }
                             if (nr > 2) {
-                                d0 += w[2] * sx[2][xx];
-                                d1 += w[2] * sx[2][xb];
+                                d0 += w[2] * SX[2 * X + xx];
+                                d1 += w[2] * SX[2 * X + xb];
                             }
                             if (nr > 3) {
-                                d0 += w[3] * sx[3][xx];
-                                d1 += w[3] * sx[3][xb];
+                                d0 += w[3] * SX[3 * X + xx];
+                                d1 += w[3] * SX[3 * X + xb];
                             }
                             for (int q = 4; q < nr; ++q) {
                                 const bool old = q < na;
-                                const float *sr = old ? SXo + q * X : SXn + (q - na) * X;
-                                const float sy = old ? SYo[q * Y + yl] : SYn[(q - na) * Y + yl];
+                                const float *sr = SX + q * X;
+                                const float sy = SY[q * Y + yl];
                                 d0 = __fadd_rn(d0, __fmul_rn(old ? -sr[xx] : sr[xx], sy));
                                 d1 = __fadd_rn(d1, __fmul_rn(old ? -sr[xb] : sr[xb], sy));
                             }
@@ -2286,19 +2283,17 @@ __device__ __forceinline__ bool begin_roi(ChainWarp<EXACT, NUM, TEAM> &w, const 
         w.NX = sw + 5 * npix_max;
         w.NY = w.NX + EXACT_ROWS * Bt.side_max;
         w.ubuf = w.NY + EXACT_ROWS * Bt.side_max;
-        w.SXo = w.SYo = w.SXn = w.SYn = nullptr;
+        w.SX = w.SY = nullptr;
         w.cl = (int *)(w.ubuf + UBUF);
         w.ahead = nullptr;
         w.arow = w.trow = -1;
     } else {
-        const int rs = FAST_ROWS * Bt.side_max;
+        const int rs = 2 * FAST_ROWS * Bt.side_max;
         w.E = nullptr;
         w.NX = w.NY = nullptr;
-        w.SXo = sw + 3 * npix_max;
-        w.SYo = w.SXo + rs;
-        w.SXn = w.SYo + rs;
-        w.SYn = w.SXn + rs;
-        w.ubuf = sw + ((3 * npix_max + 4 * rs + 3) & ~3);
+        w.SX = sw + 3 * npix_max;
+        w.SY = w.SX + rs;
+        w.ubuf = sw + ((3 * npix_max + 2 * rs + 3) & ~3);
         w.ahead = w.ubuf + UBUF;
         w.cl = (int *)(w.ahead + 2 * MOVE_AHEAD);
     }
