@@ -542,9 +542,10 @@ struct ChainWarp {
                 /* the reference compares (float)sqrt of the double sum; where
                  * the float sum of squares (three roundings, 1.8e-7) is more
                  * than 1e-6 from dmin^2 the answer is the same, and only the
-                 * rest, NaN included, pays for FP64 */
+                 * rest, NaN included, pays for FP64; a negative dmin has no
+                 * neighbours, whatever its square */
                 const float s = dx * dx + dy * dy, q = dmin * dmin;
-                in = q > 1e-30f && s < q * 0.999999f;
+                in = dmin > 0.0f && q > 1e-30f && s < q * 0.999999f;
                 if (!in && !(q > 1e-30f && s > q * 1.000001f))
                     in = (float)sqrt(dadd(dmul((double)dx, (double)dx), dmul((double)dy, (double)dy))) < dmin;
             } else {
