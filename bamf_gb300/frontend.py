@@ -128,7 +128,8 @@ def gaussMLE(Data, FitType: str = "Basic", CameraType: str = "CCD", Sigma=1.3, *
         d = d[:, :, None]
     sz, _, n = d.shape
     # a C-ordered array goes to the device as it lies and is reordered there
-    planes = d.flags.c_contiguous and not d.flags.f_contiguous
+    # (square windows; others are read as their Fortran-ordered values say)
+    planes = d.flags.c_contiguous and not d.flags.f_contiguous and d.shape[1] == sz
     flat = d if planes else np.ascontiguousarray(d.ravel(order="F"))
     fit_host = L.bamf_gauss_mle_fit_host_planes if planes else L.bamf_gauss_mle_fit_host
     sig = np.atleast_1d(np.asarray(Sigma, np.float64))
