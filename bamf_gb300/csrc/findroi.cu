@@ -41,6 +41,7 @@
 
 #include "bamf.h"
 #include "frontend_launch.h"
+#include "smem_limit.h"
 
 namespace {
 
@@ -1532,8 +1533,7 @@ bamf_status run_filter(bamf_findroi_ws *ws, const float *host_frames, int chunk_
     /* 256 x 256 frames (the common camera region) have their own build */
     auto ff = vec ? (KX == 256 && KY == 256 ? filter_kernel<true, 256> : filter_kernel<true, 0>)
                   : filter_kernel<false, 0>;
-    if (fused && cudaFuncSetAttribute(ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ff_smem) != cudaSuccess)
-        return cuda_fail();
+    if (fused && allow_smem(ff, ff_smem) != cudaSuccess) return cuda_fail();
     if (host_frames) {
         if (!ws->copy && cudaStreamCreateWithFlags(&ws->copy, cudaStreamNonBlocking) != cudaSuccess)
             return cuda_fail();
@@ -1660,8 +1660,7 @@ bamf_status find_roi(bamf_findroi_ws *ws, const float *host_frames, int chunk_fr
                      ? (words ? (f256 ? maxima_wide_kernel<8, 256, true> : maxima_wide_kernel<8, 0, true>)
                               : maxima_wide_kernel<8, 0, false>)
                      : (words ? maxima_wide_kernel<0, 0, true> : maxima_wide_kernel<0, 0, false>);
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(wide ? (const void *)wkern : (const void *)kern,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (smem > 48 * 1024 && allow_smem(wide ? (const void *)wkern : (const void *)kern) != cudaSuccess)
         return cuda_fail();
     auto maxima = [&](int z0, int z1) {
         if (z1 <= z0) return BAMF_OK;

@@ -15,6 +15,7 @@
 #include "bamf.h"
 #include "frontend_launch.h"
 #include "gaussmle_axis.cuh"
+#include "smem_limit.h"
 
 namespace {
 
@@ -26,7 +27,7 @@ constexpr int GROUP_FITS_PER_BLOCK = 16;  /* 128 threads */
  * jj) as ii << 8 | jj (no division in the pixel loops).  Axis rows first: they
  * are read 16 bytes at a time. */
 constexpr int AXIS_FLOATS = 2 * 4 * MAXSZ + 2 * 2 * (MAXSZ + 2);
-__host__ __device__ inline int mle_smem_floats(int sz)
+__host__ __device__ constexpr int mle_smem_floats(int sz)
 {
     return GROUP_FITS_PER_BLOCK * (AXIS_FLOATS + 2 * sz * sz) + 3 * MAXSZ + sz * sz;
 }
@@ -211,13 +212,12 @@ __global__ void __launch_bounds__(GL * GROUP_FITS_PER_BLOCK) mle_xynb_range_kern
 
 }  // namespace
 
-/* dynamic shared memory of a launch; above 48 KB (sz > 16) it is asked for */
+/* dynamic shared memory of a launch; above 48 KB (sz > 15) it is asked for */
 template <typename Kern>
 static bool gauss_mle_smem(Kern kern, int sz, size_t *bytes)
 {
     *bytes = (size_t)mle_smem_floats(sz) * sizeof(float);
-    return *bytes <= 48 * 1024 ||
-           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*bytes) == cudaSuccess;
+    return *bytes <= 48 * 1024 || allow_smem(kern, mle_smem_floats(MAXSZ) * sizeof(float)) == cudaSuccess;
 }
 
 bamf_status launch_gauss_mle_range(const float *rois, int sz, float psf_sigma, int iterations, float *params,

@@ -32,6 +32,7 @@
 
 #include "bamf.h"
 #include "gaussmle_axis.cuh"
+#include "smem_limit.h"
 
 namespace {
 
@@ -307,14 +308,18 @@ __global__ void __launch_bounds__(GL * FITS_PER_BLOCK) mle_fit_kernel(
     if (l == 0) LL[fit] = Div;
 }
 
+constexpr size_t fit_smem(int sz)
+{
+    return ((size_t)FITS_PER_BLOCK * (AXIS_FLOATS + 2 * sz * sz) + 3 * MAXSZ + (size_t)sz * sz) * sizeof(float);
+}
+
 template <int FIT, bool SCMOS>
 cudaError_t launch(const float *rois, int sz, int nfits, float sigma, const ZPar &zp, const float *coords,
                    const float *gmap, int mapsz, int iterations, float *P, float *C, float *L, cudaStream_t s)
 {
-    size_t smem = ((size_t)FITS_PER_BLOCK * (AXIS_FLOATS + 2 * sz * sz) + 3 * MAXSZ + (size_t)sz * sz) * sizeof(float);
+    const size_t smem = fit_smem(sz);
     if (smem > 48 * 1024) {
-        cudaError_t e =
-            cudaFuncSetAttribute(mle_fit_kernel<FIT, SCMOS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_smem(mle_fit_kernel<FIT, SCMOS>, fit_smem(MAXSZ));
         if (e != cudaSuccess) return e;
     }
     int blocks = (nfits + FITS_PER_BLOCK - 1) / FITS_PER_BLOCK;

@@ -28,6 +28,7 @@
 #include <cmath>
 
 #include "bamf.h"
+#include "smem_limit.h"
 
 /* a failed CUDA runtime call: clear its error so that a later call on this
  * thread does not report it again */
@@ -374,9 +375,7 @@ extern "C" bamf_status bamf_map_kmeans_device(const float *pos_trace, int pos_le
     if (n == 0) return BAMF_OK;
     if (!pos_trace || !n_entries || !map_n || !out) return BAMF_ERR_INVALID_ARG;
     const size_t smem = kmeans_smem(pos_len);
-    if (cudaFuncSetAttribute(map_kmeans_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return clear_cuda_error();
+    if (allow_smem(map_kmeans_kernel, kmeans_smem(MAX_POS_LEN)) != cudaSuccess) return clear_cuda_error();
     map_kmeans_kernel<<<n, THREADS, smem, (cudaStream_t)stream>>>(pos_trace, pos_len, pos_thin, n_entries, map_n,
                                                                   n, max_iter, out);
     return cudaGetLastError() == cudaSuccess ? BAMF_OK : BAMF_ERR_CUDA;

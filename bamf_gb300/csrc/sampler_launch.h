@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include "sampler_common.h"
+#include "smem_limit.h"
 
 namespace bamf {
 
@@ -47,12 +48,12 @@ cudaError_t launch_exact_num(const SamplerConsts &K, const SamplerBatch &B, size
                              cudaStream_t stream);
 int occupancy_exact_num(size_t smem, int threads);
 
-/* set the kernel's dynamic shared memory and launch it */
+/* launch with `smem` bytes of dynamic shared memory */
 template <typename Kern>
 inline cudaError_t launch_kernel(Kern kern, const SamplerConsts &K, const SamplerBatch &B, size_t smem, int blocks,
                                  int threads, cudaStream_t stream)
 {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern);
     if (e != cudaSuccess) return e;
     kern<<<blocks, threads, smem, stream>>>(K, B);
     return cudaGetLastError();
@@ -62,12 +63,10 @@ inline cudaError_t launch_kernel(Kern kern, const SamplerConsts &K, const Sample
 template <typename Kern>
 inline int resident_ctas(Kern kern, size_t smem, int threads)
 {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
+    if (smem > DYNAMIC_SMEM_MOST) return 0;
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) != cudaSuccess) {
+    if (allow_smem(kern) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
