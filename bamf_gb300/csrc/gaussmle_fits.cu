@@ -30,6 +30,8 @@
  */
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "bamf.h"
 #include "gaussmle_axis.cuh"
 #include "smem_limit.h"
@@ -398,6 +400,11 @@ __global__ void __launch_bounds__(256) planes_kernel(const float *__restrict__ i
     }
 }
 
+/* The planes go to the device at most so many bytes at a time (fits, in steps
+ * of planes_kernel's 32), so that a stack takes no more device memory than one
+ * that needs no reordering, but for these. */
+constexpr size_t PLANES_BYTES = (size_t)256 << 20;
+
 bamf_status fit_host(const float *rois, bool planes, int sz, int nfits, int fit_type, float psf_sigma,
                      const bamf_zfit *zfit, const float *box_corners, const float *var_gain_map, int map_size,
                      int iterations, float *params, float *crlb, float *loglik)
@@ -409,14 +416,15 @@ bamf_status fit_host(const float *rois, bool planes, int sz, int nfits, int fit_
     if (nfits == 0) return BAMF_OK;
     if (bamf_device_count() < 1) return BAMF_ERR_NO_DEVICE;
     /* one allocation for the call, its parts at multiples of 256 bytes */
-    const size_t n = (size_t)nfits, nin = n * sz * sz * 4, nout = n * np * 4;
+    const size_t n = (size_t)nfits, npx = (size_t)sz * sz, nin = n * npx * 4, nout = n * np * 4;
+    const size_t piece = std::min(n, std::max<size_t>(32, PLANES_BYTES / (npx * 4) / 32 * 32));
     size_t total = 0;
     auto part = [&](size_t bytes) {
         const size_t at = total;
         total += (bytes + 255) / 256 * 256;
         return at;
     };
-    const size_t at_r = part(nin), at_q = part(planes ? nin : 0), at_p = part(nout), at_c = part(nout),
+    const size_t at_r = part(nin), at_q = part(planes ? piece * npx * 4 : 0), at_p = part(nout), at_c = part(nout),
                  at_l = part(n * 4), at_co = part(var_gain_map ? n * 2 * 4 : 0),
                  at_m = part(var_gain_map ? (size_t)map_size * map_size * 4 : 0);
     char *mem = nullptr;
@@ -428,13 +436,20 @@ bamf_status fit_host(const float *rois, bool planes, int sz, int nfits, int fit_
           *dc = (float *)(mem + at_c), *dl = (float *)(mem + at_l);
     float *dco = var_gain_map ? (float *)(mem + at_co) : nullptr, *dm = var_gain_map ? (float *)(mem + at_m) : nullptr;
     bamf_status st = BAMF_OK;
-    if (cudaMemcpy(planes ? dq : dr, rois, nin, cudaMemcpyHostToDevice) != cudaSuccess) st = BAMF_ERR_CUDA;
+    if (!planes && cudaMemcpy(dr, rois, nin, cudaMemcpyHostToDevice) != cudaSuccess) st = BAMF_ERR_CUDA;
     if (!st && var_gain_map &&
         (cudaMemcpy(dco, box_corners, n * 2 * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
          cudaMemcpy(dm, var_gain_map, (size_t)map_size * map_size * 4, cudaMemcpyHostToDevice) != cudaSuccess))
         st = BAMF_ERR_CUDA;
-    if (!st && planes) {
-        planes_kernel<<<(nfits - 1) / 32 + 1, 256>>>(dq, sz, nfits, dr);
+    for (size_t f0 = 0; !st && planes && f0 < n; f0 += piece) {
+        const size_t m = std::min(piece, n - f0);
+        /* the planes' values of the fits f0 ..; of all fits they are one piece of memory */
+        const size_t rows = m == n ? 1 : npx, row = m == n ? npx * n : m;
+        for (size_t q = 0; !st && q < rows; ++q)
+            if (cudaMemcpy(dq + q * m, rois + f0 + q * n, row * 4, cudaMemcpyHostToDevice) != cudaSuccess)
+                st = BAMF_ERR_CUDA;
+        if (st) break;
+        planes_kernel<<<(unsigned)((m - 1) / 32 + 1), 256>>>(dq, sz, (int)m, dr + f0 * npx);
         if (cudaGetLastError() != cudaSuccess) st = BAMF_ERR_CUDA;
     }
     if (!st)
