@@ -286,6 +286,8 @@ extern "C" bamf_status bamf_rjmcmc_batch_device_noalloc(const bamf_roi_batch *ro
 
     const bool exact = arith == BAMF_ARITH_EXACT;
     const int sms = sm_count();
+    int classes = 1; /* that the batch can have; they run one after another */
+    while (class_side(classes - 1) < side_max) ++classes;
     for (int c = BAMF_N_CLASSES - 1; c >= 0; --c) {
         int lo = c == 0 ? 1 : class_side(c - 1) + 1;
         if (lo > side_max) continue;
@@ -295,7 +297,7 @@ extern "C" bamf_status bamf_rjmcmc_batch_device_noalloc(const bamf_roi_batch *ro
         Bc.side_max = std::min(class_side(c), side_max);
         int wpb = 4, mc = 2;
         int per_sm = exact ? blocks_per_sm_exact(Bc.side_max, wpb, K.opt_model)
-                           : best_fast_shape(Bc.side_max, K.opt_model, n, sms, &wpb, &mc);
+                           : best_fast_shape(Bc.side_max, K.opt_model, n, classes, sms, &wpb, &mc);
         if (per_sm < 1) return BAMF_ERR_TOO_LARGE;
         int blocks = std::min((n + wpb - 1) / wpb, per_sm * sms);
         cudaError_t e = exact ? launch_rjmcmc_exact(K, Bc, Bc.side_max, blocks, wpb, s)

@@ -1,0 +1,62 @@
+"""The rule that picks the fast sampler's CTA shape: where the size classes run one after another, the
+shape of an equal share of the batch; results do not depend on the shape."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _shape(side, n, classes=1, opt_model=0):
+    from bamf_gb300 import abi, sampler
+    f = sampler._declare().bamf_fast_shape
+    f.restype = C.c_int
+    f.argtypes = [C.c_int] * 4 + [C.POINTER(C.c_int32)] * 2
+    w, m = C.c_int32(), C.c_int32()
+    abi.check(f(side, opt_model, n, classes, C.byref(w), C.byref(m)), "bamf_fast_shape")
+    return w.value, m.value
+
+
+@pytest.mark.parametrize("classes", [2, 3, 5, 7])
+def test_classes_one_after_another_are_spread_over_the_sms(cuda_lib, classes):
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for side in (6, 8, 12, 16, 20, 24, 28, 32):
+        for n in (1, sms, 4 * sms, 8 * sms):  # no class has more than the batch
+            assert _shape(side, n, classes) == _shape(side, n)
+        for share in (8 * sms + 1, 16 * sms, 2600, 20 * sms, 24 * sms, 10_000, 30_000):
+            assert _shape(side, share * classes, classes) == _shape(side, share), (side, share)
+        w, _ = _shape(side, 16 * sms * classes, classes)
+        assert w <= 8, (side, w)  # one CTA of 24 would leave a third of the SMs without any
+
+
+def test_results_are_those_of_every_shape(cuda_lib):
+    """One image under many chain ids: the order is the ids', so a small batch's chains are the first of a
+    large one's, in another shape."""
+    import torch
+    from bamf_gb300 import rjstruct, sampler, synth
+    rj = rjstruct.uneven_rjstruct()
+    rj.N_Burnin, rj.N_Trials = 40, 35
+    p = rjstruct.mcmc_params(rj)
+    s = sampler.Sampler()
+    seen = set()
+    for side in (12, 16, 20, 24):
+        b = synth.roi_batch_uneven(1, seed=side, sides=(side,))
+        large, outs = 7300, {}
+        for n in (1, 23, 25, 152, 300, 600, 1216, 2433, 3400, large):
+            seen.add(_shape(side, n))
+            i32 = torch.full((n,), side, dtype=torch.int32, device="cuda")
+            dev = {"data": torch.from_numpy(b.data).cuda(), "offsets": torch.zeros(n, dtype=torch.int64, device="cuda"),
+                   "xsize": i32, "ysize": i32, "psf_sigma": torch.full((n,), 1.3, device="cuda"), "side_max": side}
+            o = {k: torch.zeros(n, dtype=torch.int32, device="cuda") for k in ("map_n", "final_n", "status", "llr_evals")}
+            o["counters"] = torch.zeros((n, 30), dtype=torch.int32, device="cuda")
+            o["final_state"] = torch.zeros((n, sampler.FINAL_STRIDE), device="cuda")
+            s.run_device(dev, p, rj.P_Offset, rj.P_EmPhotons, rj.P_BgEmPhotons, seed=5, outs=o,
+                         bg0=rjstruct.initial_bg(rj))
+            outs[n] = {k: v.cpu().numpy() for k, v in o.items()}
+        assert not outs[large]["status"].any() and len(np.unique(outs[large]["llr_evals"])) > 10
+        for n, o in outs.items():
+            for k, v in o.items():
+                assert v.tobytes() == outs[large][k][:n].tobytes(), (side, n, k)
+    assert {(1, 2), (2, 2), (4, 2), (8, 2), (8, 3), (24, 1)} <= seen, seen
