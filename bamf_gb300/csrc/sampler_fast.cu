@@ -120,8 +120,12 @@ int best_fast_shape(int side_max, int opt_model, int n_rois, int classes, int sm
             best_per = group_per;
         }
     }
+    /* The costs are those of CTAs of 8 and 24 chains.  More, smaller CTAs keep a few
+     * more chains resident where three of 8 do not fit, but an SM then runs as many
+     * move streams (25 px, 3000 ROIs: 6.1 ms in five CTAs of 4, 4.7 in two of 8). */
     const int per2 = blocks_per_sm_fast(side_max, 8, 2, opt_model);
-    if (per2 * 8 >= 16 && best_w > per2 * 8 && batch_cost(n, sms, per2 * 8, 1.0f, false) < best) {
+    if (per2 * 8 >= 16 && best_w > per2 * 8 &&
+        (best_wpb < 8 || batch_cost(n, sms, per2 * 8, 1.0f, false) < best)) {
         best_wpb = 8;
         best_mc = 2;
         best_per = per2;

@@ -31,6 +31,14 @@ def test_classes_one_after_another_are_spread_over_the_sms(cuda_lib, classes):
         assert w <= 8, (side, w)  # one CTA of 24 would leave a third of the SMs without any
 
 
+def test_ctas_of_eight_chains_where_two_fit(cuda_lib):
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for side in range(1, 32):  # at 32 px two CTAs of 8 do not fit
+        for n in (8 * sms + 1, 2500, 2700, 2900, 3000, 20 * sms, 22 * sms, 6000, 100_000):
+            assert _shape(side, n)[0] >= 8, (side, n, _shape(side, n))
+
+
 def test_results_are_those_of_every_shape(cuda_lib):
     """One image under many chain ids: the order is the ids', so a small batch's chains are the first of a
     large one's, in another shape."""
