@@ -1520,8 +1520,17 @@ bamf_status run_filter(bamf_findroi_ws *ws, const float *host_frames, int chunk_
      * frames whose slots would not stay in L2 one per SM, a warp per CTA, on
      * as many frames at a time as FF_SPLIT_BYTES of slots hold, and at least
      * as many as give every SM eight warps (600 frames of 320 x 320: 1.11 ms; 1.45
-     * as one launch over the stack with IEEE divisions) */
-    const bool fused = (size_t)KX * YP <= FF_MAX_SLOT && 2 * std::min(step, zsize) >= sms;
+     * as one launch over the stack with IEEE divisions).  Small frames of whole
+     * chunks, or up to 4 pixels past them, stay with a CTA per frame: its one launch
+     * and full 32-row warps outweigh the spread (findROI of 1 / 50 frames, us, fused
+     * against split: 32 x 32 39.4 / 39.4 against 43.4 / 43.4, 64 rows of 32 45.6 /
+     * 45.6 against 49.6 / 49.5, 33 x 33 37.5 / 39.3 against 39.3 / 41.4, 128 rows of 64
+     * 64.0 / 64.0 against 64.0 / 66.0; but 48 x 48, in single steps, 45.4 / 47.5
+     * against 41.5 / 43.4, 128 x 128 70.1 / 70.1 against 68.1 / 68.1) */
+    const int rest = std::max(KX % FF_CW, KY % FF_CW);
+    const bool small = std::min(KX, KY) >= FF_CW && rest <= 4 && KX <= 128 && KY <= 192 &&
+                       plane <= (rest == 0 ? 8192 : 4352);
+    const bool fused = (size_t)KX * YP <= FF_MAX_SLOT && (small || 2 * std::min(step, zsize) >= sms);
     const int ff_grid = std::min(step, sms);
     const int groups = (std::min(KX, KY) + FF_R - 1) / FF_R;
     const int per = std::min(std::min(step, 65535),
