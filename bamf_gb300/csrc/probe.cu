@@ -114,3 +114,73 @@ extern "C" bamf_status bamf_parity_math_device(int fn, const float *x, int n, fl
     cudaFree(d);
     return st;
 }
+
+/* pair i of the division check: significands, exponents and kind from a hash
+ * of i (multiply and xor-shift rounds) */
+__device__ __forceinline__ void division_pair(uint32_t i, float *a, float *b)
+{
+    uint64_t h = (uint64_t)i * 0x9E3779B97F4A7C15ull + 0xD1B54A32D192ED03ull;
+    for (int r = 0; r < 2; ++r) {
+        h ^= h >> 32;
+        h *= 0xD6E8FEB86659FD93ull;
+    }
+    h ^= h >> 32;
+    uint32_t mb = (uint32_t)h & 0x7fffffu, mq = (uint32_t)(h >> 23) & 0x7fffffu;
+    const uint32_t eb = 127u - 44u + (uint32_t)(h >> 46) % 88u; /* 2^-44 .. 2^43 */
+    const uint32_t kind = (uint32_t)(h >> 54) & 3u, low = (uint32_t)(h >> 56) & 7u;
+    if (kind == 2) mb = 0x7fffffu - low; /* next to the excluded significand */
+    *b = __uint_as_float(eb << 23 | mb);
+    const float one_b = __uint_as_float(127u << 23 | mb), q = __uint_as_float(127u << 23 | mq);
+    if (kind == 0 || kind == 2) {
+        *a = __uint_as_float((127u - 44u + (uint32_t)(h >> 40) % 88u) << 23 | mq);
+    } else if (kind == 1) {
+        /* a quotient next to the midpoint of q and the float after it */
+        const float mid = (float)((double)one_b * ((double)q + 0x1p-24));
+        const float t = __uint_as_float(__float_as_uint(mid) + low - 3u);
+        *a = t * __uint_as_float(eb << 23); /* exact: a power of two */
+    } else {
+        *a = low == 0 ? *b : __uint_as_float(__float_as_uint(one_b * q) + low - 3u) * __uint_as_float(eb << 23);
+    }
+}
+
+__global__ void parity_check_kernel(int fn, unsigned long long *bad)
+{
+    unsigned long long n = 0;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (1ull << 32); i += stride) {
+        if (fn == 3) {
+            float a, b;
+            division_pair((uint32_t)i, &a, &b);
+            const float got = bamf::pq::div_try(a, b);
+            const bool in = a >= 0x1p-40f && a < 0x1p40f && b >= 0x1p-40f && b < 0x1p40f &&
+                            (__float_as_uint(b) & 0x7fffffu) != 0x7fffffu;
+            n += in ? __float_as_uint(got) != __float_as_uint(__fdiv_rn(a, b)) : got == got;
+        } else {
+            const float x = __uint_as_float((uint32_t)i);
+            const float want = fn == 0 ? bamf_pm_erff(x) : fn == 1 ? bamf_pm_logf(x) : bamf_pm_expf(x);
+            const float got = fn == 0 ? bamf::pq::erf_q(x) : fn == 1 ? bamf::pq::log_q(x) : bamf::pq::exp_q(x);
+            n += __float_as_uint(want) != __float_as_uint(got) && !(want != want && got != got);
+        }
+    }
+    if (n) atomicAdd(bad, n);
+}
+
+extern "C" bamf_status bamf_parity_math_check(int fn, int64_t *mismatches)
+{
+    if (!mismatches || fn < 0 || fn > 3) return BAMF_ERR_INVALID_ARG;
+    if (bamf_device_count() < 1) return BAMF_ERR_NO_DEVICE;
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    unsigned long long *d = nullptr, h = 0;
+    if (cudaMalloc(&d, sizeof h) != cudaSuccess) return clear_cuda_error();
+    bamf_status st = cudaMemset(d, 0, sizeof h) == cudaSuccess ? BAMF_OK : BAMF_ERR_CUDA;
+    if (!st) {
+        parity_check_kernel<<<sms * 8, 256>>>(fn, d);
+        if (cudaMemcpy(&h, d, sizeof h, cudaMemcpyDeviceToHost) != cudaSuccess) st = BAMF_ERR_CUDA;
+    }
+    if (st) cudaGetLastError();
+    cudaFree(d);
+    *mismatches = (int64_t)h;
+    return st;
+}

@@ -705,6 +705,15 @@ bamf_status bamf_probe_peaks(double *fp32_flops, double *mufu_ops);
  * Synchronous. */
 bamf_status bamf_parity_math_device(int fn, const float *x, int n, float *out);
 
+/* The quick forms of those functions on the device against what they stand
+ * for: erf, log and exp (fn 0..2) against the header's over all 2^32 floats, the
+ * branch-free division of the likelihood terms (fn 3) against IEEE division on
+ * 2^32 pairs (any exponents around [2^-40, 2^40), quotients next to the midpoint
+ * of two floats, divisors next to the excluded significand, equal operands).
+ * *mismatches: values that differ, or that a quick division leaves open inside
+ * its range.  Synchronous, a second or less. */
+bamf_status bamf_parity_math_check(int fn, int64_t *mismatches);
+
 /* Known-answer check of the 5th-generation tensor-core path (tcgen05 MMA
  * from shared-memory descriptors into TMEM, read back with tcgen05.ld): a
  * 128 x 32 x 16 BF16 product of small integers.  *max_abs_err = the largest
