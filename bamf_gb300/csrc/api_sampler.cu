@@ -694,8 +694,9 @@ extern "C" bamf_status bamf_rjmcmc_batch_graph_launch(bamf_batch_graph *g, void 
  * the batch, with chains of `jumps` burn-in jumps, and keeps the fastest
  * per class in the workspace for later batches of that arithmetic.  In
  * fast arithmetic the chains' results do not depend on the shape (move
- * streams are keyed by slot groups), in exact arithmetic every chain is one
- * warp's, so tuning changes speed only. */
+ * streams are keyed by slot groups), in exact arithmetic a chain is one
+ * warp's whatever the shape, so tuning changes speed only.  Exact batches of at
+ * most two ROIs per SM run as teams of warps and do not take the tuned shape. */
 extern "C" bamf_status bamf_autotune(bamf_workspace *ws, const bamf_roi_batch *rois, const bamf_mcmc_params *p,
                                      const bamf_priors *priors, int arith, int jumps, int sample, void *stream)
 {

@@ -494,8 +494,12 @@ __device__ __forceinline__ Coef lane_coef(const Coef &a, const Coef &b)
  * nearly: a persistent CTA of 8 warps owns one frame at a time and one slot (two
  * images, sigma 1 then sigma 2, column-major), a lane a row (column) with both
  * sigmas' recurrences.  The grid's slots together stay within L2, so only the
- * frames are read from DRAM and only the DoG is written.  findROI of 2000 frames
- * of 256 x 256: 1.70 ms with the three-operation division, 1.68 with this. */
+ * frames are read from DRAM and only the DoG is written.  600 frames of 256 x 256
+ * take 231 us, 117k cycles per frame and SM: some 60k of slot traffic (3.6 MB at 60
+ * bytes a cycle) and 59k of issue (141M warp instructions, 51% busy), hardly
+ * overlapped; the recurrences' own latency (1,024 steps of five operations) is
+ * 22k.  (The two-operation division changed findROI of 2000 frames by 1%, 1.70 to
+ * 1.68 ms, no more than runs differ.) */
 constexpr int FW_T = 256; /* threads: rows of a row group / columns of a column group */
 /* per warp: the largest phase, two buffers of column tiles [sigma][32 columns][FF_TS] */
 constexpr int FW_FLOATS = 2 * 2 * 32 * FF_TS;
@@ -1476,11 +1480,12 @@ extern "C" void bamf_findroi_workspace_destroy(bamf_findroi_ws *ws) { delete ws;
 
 namespace {
 
-/* Frames copied from host memory at a time, `chunk_frames` at most.  A piece that
- * takes the link as long as the device needs for it hides the device's work but
- * for the last piece's, so a piece is no more than PIECE_BYTES, and where a CTA
- * filters a frame (256 x 256 and the like) a multiple of the SMs, as a part of a
- * wave takes as long as a whole one.  Smaller pieces than that would be bound by
+/* Frames copied from host memory at a time: chunk_frames, unless those are more
+ * than PIECE_BYTES.  A piece that takes the link as long as the device needs for
+ * it hides the device's work but for the last piece's; larger ones are cut to
+ * PIECE_BYTES, and where a CTA filters a frame (256 x 256 and the like) further to
+ * whole waves of the SMs, as a part of a wave takes as long as a whole one, but to
+ * no less than one wave (up to 50 MB on 152 SMs).  Smaller pieces than that would be bound by
  * the launches of each (find and fit, us, pieces of 100 / 152 / 200 / 304 / 500 / 1000
  * frames: 1000 frames of 256 x 256 1796 / 1534 / 1592 / 1635 / 1794 / 2169; pieces of
  * 250 against these: 409 frames of 400 x 400 2563 / 1785, 728 of 300 x 300 2512 / 1795). */

@@ -2443,10 +2443,10 @@ __global__ void __launch_bounds__(128, 4) rjmcmc_kernel(const __grid_constant__ 
  * The first warp runs the chain; the others take their share of every
  * proposal's pixels (the model and the likelihood-ratio terms, 40% of a
  * chain's time on one warp).  The terms are then added by the first warp in
- * pixel order, so the chain is the same.  A chain is latency-bound (about
- * 2,700 dependent warp instructions per jump, a fifth of the issue slots of
- * its scheduler).  16x16, 3000+3000 jumps, 200 ROIs: 47.0 ms with a warp per
- * chain, 38.1 ms with teams of four; one ROI: 32.4 and 28.6 ms. */
+ * pixel order, so the chain is the same.  A chain is latency-bound (3,100 warp
+ * instructions of the team per jump, issue slots 11% busy).  16x16, 3000+3000
+ * jumps, 200 ROIs: 42.1 ms with a warp per chain, 35.6 ms with teams of four; one
+ * ROI: 37.7 and 30.1 ms in the same run. */
 template <int TEAM>
 __global__ void __launch_bounds__(32 * TEAM, 2) rjmcmc_kernel_team(const __grid_constant__ SamplerConsts Kc,
                                                                 const __grid_constant__ SamplerBatch Bc)

@@ -1,9 +1,10 @@
 /*
  * sampler_launch.h - launchers of the sampler kernels, one translation unit
  * per (arithmetic, likelihood model) so the four builds compile in
- * parallel.  The fast kernel exists in two register budgets: for 2 CTAs of
- * 8 chains per SM (no spills) and for 3 (80 registers, a few spills), which
- * keeps a third CTA resident where shared memory allows (ROI sides <= 20).
+ * parallel.  The fast kernel exists in three register budgets: for 2 CTAs of
+ * 8 chains per SM (no spills), for 3 (80 registers, a few spills), which
+ * keeps a third CTA resident where shared memory allows (ROI sides up to 24),
+ * and, for the Gaussian PSF, for 1 CTA of 24 chains (80 registers).
  */
 #ifndef BAMF_SAMPLER_LAUNCH_H
 #define BAMF_SAMPLER_LAUNCH_H
@@ -15,7 +16,7 @@
 
 namespace bamf {
 
-/* fast arithmetic: min_ctas = the kernel's register budget (2 or 3 CTAs per SM) */
+/* fast arithmetic: min_ctas = the kernel's register budget (1, 2 or 3 CTAs per SM) */
 cudaError_t launch_rjmcmc_fast(const SamplerConsts &K, const SamplerBatch &B, int side_max, int blocks,
                                int warps_per_block, int min_ctas, cudaStream_t stream);
 int blocks_per_sm_fast(int side_max, int warps_per_block, int min_ctas, int opt_model);
@@ -28,9 +29,9 @@ int blocks_per_sm_exact(int side_max, int warps_per_block, int opt_model);
 
 /* the CTA shape for a fast launch of a batch of n_rois: few ROIs, one CTA per
  * SM; else the shape with the most resident chains per SM (ties: the larger
- * register budget per thread, then more chains per CTA; up to side 12, a whole
- * move-stream group per CTA when it keeps as many) or two CTAs of 8, whichever
- * takes the batch's rounds of resident chains faster.  classes: the size classes
+ * register budget per thread, then more chains per CTA), up to side 20 a whole
+ * move-stream group per CTA when it keeps as many, or two CTAs of 8, whichever
+ * takes the batch's rounds of resident chains fastest.  classes: the size classes
  * that share the batch when they run one after another (1 when they run at once).
  * Returns the CTAs per SM, 0 when none fits. */
 int best_fast_shape(int side_max, int opt_model, int n_rois, int classes, int sms, int *warps_per_block,

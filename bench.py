@@ -196,13 +196,14 @@ def plain_exact_bench(n_large: int = 4864) -> dict:
 
 def gaussmle_flops_per_fit(sz: int, iterations: int) -> int:
     """Algorithmic FP32 operations of one 'Basic' fit (an FMA counted as 2,
-    a transcendental or a reciprocal as 1): the start-up filter (sz^2
-    positions x sz^2 weighted pixels, 3 each, plus the division), every
-    Newton iteration (per pixel 25: model 3, derivatives 5, the Poisson
-    factors 5, the four num/den sums 12; per axis value 2 erf + 2 exp + 16)
-    and the Fisher information (per pixel 30) plus the 4 x 4 inversion."""
+    a transcendental or a reciprocal as 1): the start-up filter (two passes
+    of sz weighted pixels for each, plus the normalisation), every Newton
+    iteration (per pixel 25: model 3, derivatives 5, the Poisson factors 5,
+    the four num/den sums 12; per axis erf + exp + 5 at each of the sz + 1
+    edges and 10 per index) and the Fisher information (per pixel 30) plus
+    the 4 x 4 inversion."""
     px = sz * sz
-    return px * px * 3 + px + iterations * (px * 25 + 2 * sz * 20) + px * 30 + 100
+    return 4 * sz ** 3 + 2 * px + iterations * (px * 25 + 2 * ((sz + 1) * 7 + sz * 10)) + px * 30 + 100
 
 
 def frontend_bench(n_frames: int, steps: int = 5, warmup: int = 3, fp32_peak: float | None = None) -> dict:

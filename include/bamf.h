@@ -465,8 +465,9 @@ void bamf_rjmcmc_batch_graph_destroy(bamf_batch_graph *graph);
  * through the class in the batch order, so that they span its whole photon
  * range) with chains of `jumps` burn-in jumps, and keeps the fastest shape
  * in the workspace; later bamf_rjmcmc_batch_device calls on that workspace launch
- * each class with its tuned shape.  Results of a batch do not depend on
- * the shape.  Synchronises `stream`. */
+ * each class with its tuned shape (exact batches of at most two ROIs per SM
+ * run a team of warps on each chain instead).  Results of a batch do not
+ * depend on the shape.  Synchronises `stream`. */
 bamf_status bamf_autotune(bamf_workspace *ws, const bamf_roi_batch *rois, const bamf_mcmc_params *p,
                           const bamf_priors *priors, int arith, int jumps, int sample, void *stream);
 /* chains_per_cta[7]: the tuned shape per size class (sides (0,8], (8,12],
@@ -577,9 +578,9 @@ bamf_status bamf_find_roi_host(const float *frames, int ysize, int xsize, int zs
 
 /* bamf_find_roi_device on frames that are still in host memory: copies
  * host_frames (pinned, for the copies to overlap) into dev_frames (the
- * same size, device) in chunks of at most chunk_frames frames on a stream of the
- * workspace, and starts each chunk's row and column filters on `stream`
- * as soon as its copy has landed, then the window maxima of the chunk's
+ * same size, device) in chunks of chunk_frames frames (fewer where those
+ * would be more than 40 MB) on a stream of the workspace, and starts each
+ * chunk's row and column filters on `stream` as soon as its copy has landed, then the window maxima of the chunk's
  * frames (those whose windows cannot reach a frame not yet filtered); the
  * compaction and crops run on the whole stack afterwards.  Outputs
  * identical to bamf_find_roi_device on the same frames.  Enqueued on stream;
