@@ -284,8 +284,9 @@ __global__ void __launch_bounds__(256) conv1_bwd_kernel(const float *__restrict_
  * staging, took 115 us, one per layer 72, this one 64, and 58 with the weights as
  * one bulk copy under the rest of the prologue.
  *
- * The mbarrier waits are bounded; a timeout is recorded in *status, the CTA
- * writes zeros, frees its TMEM and returns. */
+ * The mbarrier waits are bounded; a timeout is recorded in *status, and the CTA
+ * starts no further copy or MMA, writes zeros, waits once more for what it has
+ * started, frees its TMEM and returns. */
 constexpr int BW_AG = S * 16;                    /* bytes of a group of act: 16 y of 8 channels */
 constexpr int BW_ACOL = 12 * BW_AG;              /* an x column of the three copies of act */
 constexpr int BW_DG = PS * 16;                   /* a group of dz */
@@ -389,6 +390,7 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const Backward 
     const uint32_t tlane = (uint32_t)((warp & 3) * 32) << 16;
     bool alive = true;
     uint32_t phase = 0;
+    int loaded = 2; /* the last layer whose weights were asked for */
 #pragma unroll 1
     for (int l = 2; l >= 0; --l) {
         bool first = true;
@@ -396,7 +398,7 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const Backward 
         for (int c = 0; c < 8; ++c) bsum[c] = 0.0f;
         bf16 *const out = l == 1 ? bw.dz[0] : bw.dz[1];
         stage();
-        if (!bamf::tc::mbar_wait(bar_wt, l & 1, 1u << 24)) { /* the layer's weights */
+        if (alive && !bamf::tc::mbar_wait(bar_wt, l & 1, 1u << 24)) { /* the layer's weights */
             atomicExch(status, 1);
             alive = false;
         }
@@ -467,7 +469,8 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const Backward 
          * first ROI and weights, and this one's sums */
         if (l > 0) {
             load(l - 1, r0);
-            if (t == 0) bamf::tc::bulk_load(smem_raw, bw.Wb + (l - 1) * PKT, PKT * 2, bar_wt);
+            if (alive) loaded = l - 1;
+            if (alive && t == 0) bamf::tc::bulk_load(smem_raw, bw.Wb + (l - 1) * PKT, PKT * 2, bar_wt);
         }
         {
             float *mine = bw.part + l * bw.pitch + (size_t)blockIdx.x * DW_PART;
@@ -501,6 +504,11 @@ __global__ void __launch_bounds__(BW_THREADS, 2) conv_bwd_kernel(const Backward 
             __syncthreads();
             if (t < CH) mine[96 * 96 + t] = alive ? (bred[0][t] + bred[1][t]) + (bred[2][t] + bred[3][t]) : 0.0f;
         }
+    }
+    if (!alive) {
+        bamf::tc::mbar_wait(bar_wt, loaded & 1, 1u << 24);
+        bamf::tc::mbar_wait(bar_in, phase ^ 1u, 1u << 24);
+        bamf::tc::mbar_wait(bar_w, phase ^ 1u, 1u << 24);
     }
     bamf::tc::fence_before_sync();
     __syncthreads();
@@ -1313,6 +1321,10 @@ __global__ void __launch_bounds__(256 * INF_GROUPS, 2) net_kernel(
             for (int k = 0; k < CH; ++k) c += Wc[k * NC + lane] * G.gmean[k];
             cnt_out[(size_t)r * NC + lane] = c;
         }
+    }
+    if (G.dead) { /* a wait ran out: once more for what the group has started */
+        bamf::tc::mbar_wait(&wbar, 0, 1u << 24);
+        bamf::tc::mbar_wait(&G.mbar, phase ^ 1u, 1u << 24);
     }
     bamf::tc::fence_before_sync();
     __syncthreads();
