@@ -286,8 +286,16 @@ extern "C" bamf_status bamf_rjmcmc_batch_device_noalloc(const bamf_roi_batch *ro
 
     const bool exact = arith == BAMF_ARITH_EXACT;
     const int sms = sm_count();
-    int classes = 1; /* that the batch can have; they run one after another */
+    /* The size classes run one after another, and only the device knows how many
+     * ROIs each has.  In fast arithmetic a class is launched in the whole batch's
+     * shape and, where that of an equal share of the batch is another, in that one
+     * too, which runs if the class has at most a quarter more than a share; the
+     * first runs otherwise; a launch that does not run takes some 3 us.  (One CTA of 24 chains
+     * per SM, right for a batch of one class, leaves most SMs without any where the
+     * batch is spread over five.) */
+    int classes = 1;
     while (class_side(classes - 1) < side_max) ++classes;
+    const int share = (n - 1) / classes + 1, near = share + share / 4;
     for (int c = BAMF_N_CLASSES - 1; c >= 0; --c) {
         int lo = c == 0 ? 1 : class_side(c - 1) + 1;
         if (lo > side_max) continue;
@@ -295,13 +303,26 @@ extern "C" bamf_status bamf_rjmcmc_batch_device_noalloc(const bamf_roi_batch *ro
         Bc.queue = (int32_t *)S + c;
         Bc.cls = c;
         Bc.side_max = std::min(class_side(c), side_max);
-        int wpb = 4, mc = 2;
+        int wpb = 4, mc = 2, share_wpb = 0, share_mc = 0, share_per = 0;
         int per_sm = exact ? blocks_per_sm_exact(Bc.side_max, wpb, K.opt_model)
-                           : best_fast_shape(Bc.side_max, K.opt_model, n, classes, sms, &wpb, &mc);
+                           : best_fast_shape(Bc.side_max, K.opt_model, n, sms, &wpb, &mc);
         if (per_sm < 1) return BAMF_ERR_TOO_LARGE;
+        if (!exact && near < n)
+            share_per = best_fast_shape(Bc.side_max, K.opt_model, share, sms, &share_wpb, &share_mc);
+        const bool two = share_per > 0 && (share_wpb != wpb || share_mc != mc);
+        if (two) {
+            Bc.count_min = near;
+            Bc.count_max = n;
+        }
         int blocks = std::min((n + wpb - 1) / wpb, per_sm * sms);
         cudaError_t e = exact ? launch_rjmcmc_exact(K, Bc, Bc.side_max, blocks, wpb, s)
                               : launch_rjmcmc_fast(K, Bc, Bc.side_max, blocks, wpb, mc, s);
+        if (two && e == cudaSuccess) {
+            Bc.count_min = 0;
+            Bc.count_max = near;
+            blocks = std::min((near + share_wpb - 1) / share_wpb, share_per * sms);
+            e = launch_rjmcmc_fast(K, Bc, Bc.side_max, blocks, share_wpb, share_mc, s);
+        }
         if (e != cudaSuccess) return clear_cuda_error();
     }
     if (want_map) {

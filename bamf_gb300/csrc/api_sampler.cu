@@ -301,7 +301,7 @@ static bamf_status launch_batch(bamf_workspace *ws, const SamplerConsts &K, Samp
          * schedulers twice; beyond, a warp per chain keeps more chains going). */
         const bool team = exact && K.opt_model == 0 && B.n_rois <= 2 * sms;
         if (exact) wpb = pick_wpb_exact(Bc.side_max, B.n_rois <= 4 * sms, K.opt_model, &per_sm);
-        else per_sm = best_fast_shape(Bc.side_max, K.opt_model, B.n_rois, 1, sms, &wpb, &mc);
+        else per_sm = best_fast_shape(Bc.side_max, K.opt_model, B.n_rois, sms, &wpb, &mc);
         if (per_sm < 1) return BAMF_ERR_TOO_LARGE;
         const int tw = ws->tuned_wpb[exact ? 0 : 1][c], tm = exact ? 0 : ws->tuned_min_ctas[c];
         if (tw > 0 && !team) {
@@ -829,16 +829,15 @@ extern "C" bamf_status bamf_autotune_shapes(const bamf_workspace *ws, int arith,
     return BAMF_OK;
 }
 
-extern "C" bamf_status bamf_fast_shape(int side_max, int opt_model, int n_rois, int classes, int32_t *chains_per_cta,
+extern "C" bamf_status bamf_fast_shape(int side_max, int opt_model, int n_rois, int32_t *chains_per_cta,
                                        int32_t *ctas_per_sm_budget)
 {
-    if (side_max < 1 || opt_model < 0 || opt_model > 1 || n_rois < 1 || classes < 1 || !chains_per_cta ||
-        !ctas_per_sm_budget)
+    if (side_max < 1 || opt_model < 0 || opt_model > 1 || n_rois < 1 || !chains_per_cta || !ctas_per_sm_budget)
         return BAMF_ERR_INVALID_ARG;
     if (side_max > BAMF_MAX_ROI_SIDE) return BAMF_ERR_TOO_LARGE;
     if (bamf_device_count() < 1) return BAMF_ERR_NO_DEVICE;
     int wpb = 0, mc = 0;
-    if (best_fast_shape(side_max, opt_model, n_rois, classes, sm_count(), &wpb, &mc) < 1) return BAMF_ERR_TOO_LARGE;
+    if (best_fast_shape(side_max, opt_model, n_rois, sm_count(), &wpb, &mc) < 1) return BAMF_ERR_TOO_LARGE;
     *chains_per_cta = wpb;
     *ctas_per_sm_budget = mc;
     return BAMF_OK;

@@ -89,6 +89,9 @@ struct SamplerBatch {
      * ROIs order[class_range[2c] .. class_range[2c+1]) of class c = cls */
     const int32_t *class_range;
     int32_t cls;
+    /* count_max > 0: the launch does nothing unless its class has more than count_min
+     * ROIs and no more than count_max (rjmcmc_kernel_sync) */
+    int32_t count_min, count_max;
 };
 
 /* Size classes by ROI side: (0,8] (8,12] (12,16] (16,20] (20,24] (24,28] (28,32]. */

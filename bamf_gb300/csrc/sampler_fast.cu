@@ -63,7 +63,7 @@ static float batch_cost(int n, int sms, int w, float a, bool whole)
     return a * (1.0f + 0.77f * (x - 1.0f) + (frac > 0.02f ? 0.25f : 0.0f));
 }
 
-int best_fast_shape(int side_max, int opt_model, int n_rois, int classes, int sms, int *warps_per_block, int *min_ctas)
+int best_fast_shape(int side_max, int opt_model, int n_rois, int sms, int *warps_per_block, int *min_ctas)
 {
     /* A batch that one CTA per SM can hold: the fewest chains per CTA that do,
      * on the register budget without spills.  Chains of a CTA wait for each
@@ -101,17 +101,14 @@ int best_fast_shape(int side_max, int opt_model, int n_rois, int classes, int sm
      * 10,000; 24 px 8140 / 7876, 11726 / 11272). */
     const int group_per = side_max <= 20 && opt_model != 1 ? blocks_per_sm_fast(side_max, BAMF_SYNC_GROUP, 1, opt_model) : 0;
     const int group_w = group_per * BAMF_SYNC_GROUP;
-    /* Where the size classes run one after another, a launch has its own class only,
-     * whose size the host does not know: the rounds are those of an equal share. */
-    const int n = (int)(((int64_t)n_rois + classes - 1) / classes);
     /* Two CTAs of 8 on the larger register budget run a round in 1 / 1.42 of the
      * time of three on the smaller (one CTA of 24: 1 / 1.25 at 8 to 12 px, 1 / 1.33 at
      * 16, 1 / 1.4 at 20), so which is faster depends on how full the last round is (16 px, 250 + 250
      * jumps: 2432 ROIs 2812 us against 3130 with three, 5000: 5568 against 5876, 7300: 6893
      * against 6752). */
-    float best = best_w > 0 ? batch_cost(n, sms, best_w, best_mc == 2 ? 1.0f : 1.42f, false) : INFINITY;
+    float best = best_w > 0 ? batch_cost(n_rois, sms, best_w, best_mc == 2 ? 1.0f : 1.42f, false) : INFINITY;
     if (group_w > 0 && group_w >= best_w) {
-        const float c = batch_cost(n, sms, group_w, side_max <= 12 ? 1.25f : side_max <= 16 ? 1.33f : 1.4f,
+        const float c = batch_cost(n_rois, sms, group_w, side_max <= 12 ? 1.25f : side_max <= 16 ? 1.33f : 1.4f,
                                    group_per == 1);
         if (c < best) {
             best = c;
@@ -125,7 +122,7 @@ int best_fast_shape(int side_max, int opt_model, int n_rois, int classes, int sm
      * move streams (25 px, 3000 ROIs: 6.1 ms in five CTAs of 4, 4.7 in two of 8). */
     const int per2 = blocks_per_sm_fast(side_max, 8, 2, opt_model);
     if (per2 * 8 >= 16 && best_w > per2 * 8 &&
-        (best_wpb < 8 || batch_cost(n, sms, per2 * 8, 1.0f, false) < best)) {
+        (best_wpb < 8 || batch_cost(n_rois, sms, per2 * 8, 1.0f, false) < best)) {
         best_wpb = 8;
         best_mc = 2;
         best_per = per2;

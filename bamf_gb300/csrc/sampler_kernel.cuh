@@ -2506,6 +2506,8 @@ __global__ void __launch_bounds__(MIN_CTAS == 1 ? 32 * BAMF_SYNC_GROUP : 256, MI
     if (Bt.class_range) {
         q_begin = Bt.class_range[2 * Bt.cls];
         q_end = Bt.class_range[2 * Bt.cls + 1];
+        const int count = q_end - q_begin;
+        if (Bt.count_max > 0 && (count <= Bt.count_min || count > Bt.count_max)) return;
     }
     for (;;) {
         __syncthreads();

@@ -31,11 +31,9 @@ int blocks_per_sm_exact(int side_max, int warps_per_block, int opt_model);
  * SM; else the shape with the most resident chains per SM (ties: the larger
  * register budget per thread, then more chains per CTA), up to side 20 a whole
  * move-stream group per CTA when it keeps as many, or two CTAs of 8, whichever
- * takes the batch's rounds of resident chains fastest.  classes: the size classes
- * that share the batch when they run one after another (1 when they run at once).
- * Returns the CTAs per SM, 0 when none fits. */
-int best_fast_shape(int side_max, int opt_model, int n_rois, int classes, int sms, int *warps_per_block,
-                    int *min_ctas);
+ * takes the batch's rounds of resident chains fastest.  Returns the CTAs per SM,
+ * 0 when none fits. */
+int best_fast_shape(int side_max, int opt_model, int n_rois, int sms, int *warps_per_block, int *min_ctas);
 
 /* per translation unit */
 cudaError_t launch_fast_gauss(const SamplerConsts &K, const SamplerBatch &B, size_t smem, int blocks, int threads,

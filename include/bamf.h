@@ -479,11 +479,8 @@ bamf_status bamf_autotune_result(const bamf_workspace *ws, int arith, int32_t *c
 bamf_status bamf_autotune_shapes(const bamf_workspace *ws, int arith, int32_t *chains_per_cta,
                                  int32_t *ctas_per_sm_budget);
 /* The shape, as bamf_autotune_shapes gives it, that a fast-arithmetic launch of
- * ROIs of up to side_max pixels takes in a batch of n_rois without tuning;
- * classes: 1 for bamf_rjmcmc_batch_device, whose size classes run at once, the
- * number of size classes up to the batch's side_max for
- * bamf_rjmcmc_batch_device_noalloc, where they run one after another. */
-bamf_status bamf_fast_shape(int side_max, int opt_model, int n_rois, int classes, int32_t *chains_per_cta,
+ * ROIs of up to side_max pixels takes in a batch of n_rois without tuning. */
+bamf_status bamf_fast_shape(int side_max, int opt_model, int n_rois, int32_t *chains_per_cta,
                             int32_t *ctas_per_sm_budget);
 
 /*

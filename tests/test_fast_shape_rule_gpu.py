@@ -1,5 +1,5 @@
-"""The rule that picks the fast sampler's CTA shape: where the size classes run one after another, the
-shape of an equal share of the batch; results do not depend on the shape."""
+"""The rule that picks the fast sampler's CTA shape, and that results do not depend on the shape, also where the
+size classes run one after another in shapes of their own."""
 import ctypes as C
 
 import numpy as np
@@ -8,27 +8,49 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def _shape(side, n, classes=1, opt_model=0):
+def _shape(side, n, opt_model=0):
     from bamf_gb300 import abi, sampler
     f = sampler._declare().bamf_fast_shape
     f.restype = C.c_int
-    f.argtypes = [C.c_int] * 4 + [C.POINTER(C.c_int32)] * 2
+    f.argtypes = [C.c_int] * 3 + [C.POINTER(C.c_int32)] * 2
     w, m = C.c_int32(), C.c_int32()
-    abi.check(f(side, opt_model, n, classes, C.byref(w), C.byref(m)), "bamf_fast_shape")
+    abi.check(f(side, opt_model, n, C.byref(w), C.byref(m)), "bamf_fast_shape")
     return w.value, m.value
 
 
-@pytest.mark.parametrize("classes", [2, 3, 5, 7])
-def test_classes_one_after_another_are_spread_over_the_sms(cuda_lib, classes):
+@pytest.mark.parametrize("n,sides", [(200, (8, 24)), (2400, (8, 12, 16, 20, 24)), (4000, (16,)), (5000, (7, 16, 32)),
+                                     (2000, (8,) * 9 + (24,))])
+def test_classes_one_after_another(cuda_lib, n, sides):
+    """Every ROI once, whether its class has an equal share of the batch, more than that or less: the results
+    of the entry point whose classes run at once."""
     import torch
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    for side in (6, 8, 12, 16, 20, 24, 28, 32):
-        for n in (1, sms, 4 * sms, 8 * sms):  # no class has more than the batch
-            assert _shape(side, n, classes) == _shape(side, n)
-        for share in (8 * sms + 1, 16 * sms, 2600, 20 * sms, 24 * sms, 10_000, 30_000):
-            assert _shape(side, share * classes, classes) == _shape(side, share), (side, share)
-        w, _ = _shape(side, 16 * sms * classes, classes)
-        assert w <= 8, (side, w)  # one CTA of 24 would leave a third of the SMs without any
+    from bamf_gb300 import abi, rjstruct, sampler, synth
+    b = synth.roi_batch_uneven(200, seed=n, sides=sides)
+    pick = np.arange(n) % 200
+    dev = {"data": torch.from_numpy(b.data).cuda(), "offsets": torch.from_numpy(b.offsets[pick]).cuda(),
+           "xsize": torch.from_numpy(b.xsize[pick]).cuda(), "ysize": torch.from_numpy(b.ysize[pick]).cuda(),
+           "psf_sigma": torch.from_numpy(b.sigma[pick]).cuda(), "side_max": int(max(sides))}
+    rj = rjstruct.uneven_rjstruct()
+    rj.N_Burnin, rj.N_Trials = 20, 15
+    p, bg0 = rjstruct.mcmc_params(rj), rjstruct.initial_bg(rj)
+    priors = (rj.P_Offset, rj.P_EmPhotons, rj.P_BgEmPhotons)
+    s = sampler.Sampler()
+    got = []
+    for call in ("workspace", "noalloc"):
+        o = {k: torch.full((n,), -7, dtype=torch.int32, device="cuda") for k in ("final_n", "status", "llr_evals")}
+        o["counters"] = torch.zeros((n, 30), dtype=torch.int32, device="cuda")
+        o["final_state"] = torch.zeros((n, sampler.FINAL_STRIDE), device="cuda")
+        if call == "workspace":
+            s.run_device(dev, p, *priors, seed=5, outs=o, bg0=bg0)
+        else:
+            f = s._L.bamf_rjmcmc_batch_device_noalloc
+            f.restype, f.argtypes = C.c_int, None
+            pr, keep, bs, rs = s._structs(dev, p, *priors, o, bg0, "reference")
+            abi.check(f(C.byref(bs), C.byref(p), C.byref(pr), C.c_uint32(5), sampler.ARITH["fast"], C.byref(rs), None), call)
+        got.append({k: v.cpu().numpy() for k, v in o.items()})
+    assert not got[0]["status"].any()
+    for k in got[0]:
+        assert got[0][k].tobytes() == got[1][k].tobytes(), k
 
 
 def test_ctas_of_eight_chains_where_two_fit(cuda_lib):
